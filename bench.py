@@ -48,7 +48,7 @@ WORKLOAD = WORKLOADS[CONFIG]
 METRIC = "s/GW iteration + tensor TFLOP/s: mixed vs FP64 GPU at Sigma err<=1e-7 Ha; CPU ref"
 # dram__bytes_read.sum + dram__bytes_write.sum summed over one iteration's launches of
 # each sliced-path GEMM kernel on C2, from one ncu capture of `bench.py --profile`.
-OZ_TRAFFIC = {"oz_gemm_kernel": 8.629e9, "oz_simt_kernel": 21.484e9}
+OZ_TRAFFIC = {}
 L2_BYTES = 129 * 1024 * 1024
 
 
@@ -214,8 +214,8 @@ def _peaks(dev):
 
 STAGE_KEYS = ("rotate_G_ms", "p0_ms", "pq_ms", "sigma_ms", "dyson_ms", "transform_ms", "solve_ms")
 PREC_LABEL = {
-    "ozaki": ("bf16 x4 fixed-point slices per operand row (Ozaki scheme) on tcgen05 kind::f16, 10 products, "
-              "exact FP32 partial sums, float-float accumulation and intermediates; FP64 W~ solve, Dyson, "
+    "ozaki": ("fp16 x3 slices per operand row (Ozaki scheme, 33 bits) on tcgen05 kind::f16, 8 products, "
+              "exact leading sums in FP32, float-float accumulation; FP64 W~ solve, Dyson, "
               "transforms, mu search, energies"),
     "fp64": "complex128 contractions on CUDA cores (the drop-in)",
     "tf32x3": ("tf32x3 (tcgen05 kind::tf32, 2 planes, 3 products, FP32 accumulate within an aux block or "
@@ -286,20 +286,8 @@ def _kernel_roofline(kern, peaks, traffic):
                 "frac": alg / peak, "executed_tflops": exe, "frac_executed": exe / peak,
                 "peak_source": "tcgen05 kind::f16 (BF16) rate measured in this run (peaks/peaks.cu), of measured",
                 "achieved_note": "algorithmic complex FLOPs (8 M N K per block GEMM) of its launches / their summed "
-                                 "CUDA-event time; executed = BF16 MMA FLOPs issued (10 slice products, real "
+                                 "CUDA-event time; executed = FP16 MMA FLOPs issued (8 slice products, real "
                                  "embedding, 128-row tiles, N and K padded to the MMA shape)",
-                "launches_per_step": k["launches"], "ms_per_step": k["ms"], "traffic": traffic.get(name),
-                "traffic_unit": "bytes per step, all launches of the kernel (ncu)"}
-    if name == "oz_simt_kernel":
-        peak = peaks["fp32_fma_tflops"]
-        alg = k["flops"] / t / 1e12
-        ins = k["mma_flops"] / t / 1e12  # FP32 instructions (48 per complex MAC) per second, in T/s
-        return {"bound": "fp32 (CUDA-core float-float)", "kernel": name, "achieved": alg, "peak": peak,
-                "unit": "TFLOP/s", "frac": alg / peak, "fp32_instr_per_s_T": ins,
-                "frac_fp32_issue": 2.0 * ins / peak,
-                "peak_source": "FP32 FMA rate measured in this run (peaks/peaks.cu, 2 flops per FMA), of measured",
-                "achieved_note": "algorithmic complex FLOPs / summed launch time; each complex MAC costs 48 FP32 "
-                                 "instructions in float-float, so frac_fp32_issue = instructions / FMA issue rate",
                 "launches_per_step": k["launches"], "ms_per_step": k["ms"], "traffic": traffic.get(name),
                 "traffic_unit": "bytes per step, all launches of the kernel (ncu)"}
     gbs = k["bytes"] / t / 1e9

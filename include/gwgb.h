@@ -45,9 +45,9 @@ extern "C" {
 #define GWGB_PREC_FP64       0  /* complex128 everywhere: the drop-in path */
 #define GWGB_PREC_TF32X3     1  /* P0/Sigma on tcgen05 kind::tf32, 3-pass split, FP32 accumulate */
 #define GWGB_PREC_BF16X3     2  /* P0/Sigma on tcgen05 kind::f16 (BF16), 3-way split, 6 products, FP32 accumulate */
-#define GWGB_PREC_OZAKI      3  /* P0/Sigma on tcgen05 kind::f16 (BF16): four fixed-point slices per operand row
-                                   (Ozaki scheme), 10 products, exact FP32 partial sums, float-float accumulation
-                                   and intermediates; Sigma error about 1e-9 of the FP64 path */
+#define GWGB_PREC_OZAKI      3  /* P0/Sigma on tcgen05 kind::f16 (FP16): three slices per operand row (Ozaki scheme),
+                                   8 products, exact leading sums in FP32, float-float accumulation; Sigma error
+                                   below 1e-9 of the FP64 path */
 
 typedef struct gwgb_handle_s *gwgb_handle;
 
@@ -69,9 +69,9 @@ typedef struct gwgb_params {
   int32_t sw_npk_max;  /* widest W-GEMM column pack (16, 32 or 64 complex columns) */
   int32_t uv_waves;    /* U/Sigma contribution slices per tau, in units of the SM count (1..16; default 8) */
   int32_t uv_simt;     /* 1: all U/Sigma tiles on the FP32 SIMT kernels (the path for AO blocks above 64) */
-  /* Sliced path (GWGB_PREC_OZAKI): block GEMMs with at most this many output
-   * columns run on the CUDA-core float-float kernel instead of tcgen05
-   * (0: the built-in 8; -1: none; at most 1024). */
+  /* Accepted for compatibility, -1 to 1024, without effect: every block GEMM of
+   * the sliced path (GWGB_PREC_OZAKI) runs on tcgen05, narrow ones several row
+   * tiles at a time. */
   int32_t oz_simt_cols;
 } gwgb_params;
 
@@ -246,15 +246,14 @@ int gwgb_synchronize(gwgb_handle h);
  * launch order.  Off by default: the events add a few microseconds per launch.
  * Switching it re-captures the iteration graph. */
 typedef struct gwgb_launch_stat {
-  int32_t stage;    /* 0 Z1 (V G2), 1 Z (G1 Z1), 2 P0 (final), 3 W (P~ V), 4 U (W G2), 5 Sigma (final) */
-  int32_t kernel;   /* 0 oz_gemm_kernel (tcgen05), 1 oz_simt_kernel (CUDA cores), 2 reduce_slices_kernel,
-                       3 oz_perm_kernel (a chunk's copy of V blocks into a concatenated operand) */
-  int32_t tasks;    /* CTA work items (kernels 0, 1) or reduced blocks (kernel 2) */
+  int32_t stage;    /* 0 Z1 (V G2), 1 Z (Z1 G1), 2 P0 (final), 3 W (V G2), 4 U (W P~), 5 Sigma (final) */
+  int32_t kernel;   /* 0 oz_gemm_kernel (tcgen05), 2 reduce_slices_kernel, 3 oz_build_kernel (operand images) */
+  int32_t tasks;    /* CTA work items (kernel 0), reduced blocks (kernel 2) or images (kernel 3) */
   int32_t ran;      /* 1 when the launch ran in the last solve / iteration */
   double ms;        /* CUDA-event time of the launch */
   double flops;     /* algorithmic: 8 M N K per complex block GEMM (0 for reductions) */
-  double mma_flops; /* kernel 0: BF16 MMA FLOPs issued (128-row tiles, N and K padded to the MMA shape,
-                       10 slice products, real embedding); kernel 1: FP32 instructions (48 per complex MAC) */
+  double mma_flops; /* kernel 0: FP16 MMA FLOPs issued (128-row tiles, N and K padded to the MMA shape,
+                       8 slice products, real embedding) */
   double bytes;     /* kernels 2, 3: bytes read + written */
 } gwgb_launch_stat;
 

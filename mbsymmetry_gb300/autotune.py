@@ -1,13 +1,8 @@
 """Empirical tuning of the contraction kernels for one workload.
 
-Sliced path (precision "ozaki"): every P0 / Sigma stage is a list of block
-GEMMs whose output width N is set by an irrep block size (AO block for the
-G products and the final Sigma GEMM, aux block for the final P0 GEMM).  A
-tcgen05 round stages 128 rows x 16 complex K whatever N is, so narrow blocks
-run faster on the CUDA-core float-float kernel.  gwgb_params.oz_simt_cols is
-the width class boundary: blocks with N <= oz_simt_cols go to the CUDA cores.
-OZAKI_CANDIDATES spans the classes (none, N <= 4, 8, 16, 32), scored on the
-whole iteration (the boundary moves work in both contractions).
+Sliced path (precision "ozaki"): the kernels choose their tiles from the block
+sizes; there is one candidate, the built-in choice, timed on the whole
+iteration.
 
 Split FP32-class paths (tf32x3 / bf16x3):
 
@@ -43,13 +38,7 @@ DEFAULT_CANDIDATES = (
     {"uvt_smem_kb": 110, "sw_npk_max": 32, "uv_waves": 8},
 )
 
-OZAKI_CANDIDATES = (
-    {"oz_simt_cols": 0},    # the built-in boundary (8)
-    {"oz_simt_cols": -1},   # every block GEMM on tcgen05
-    {"oz_simt_cols": 4},
-    {"oz_simt_cols": 16},
-    {"oz_simt_cols": 32},
-)
+OZAKI_CANDIDATES = ({"oz_simt_cols": 0},)
 
 
 def _device_key(device: int) -> str:

@@ -22,7 +22,8 @@
 #include "kernels.h"
 #include "kernels_tc.h"
 #include "kernels_sc.h"
-#include "kernels_oz.h"
+#include "dbuf.h"
+#include "oz_plan.h"
 
 namespace gwgb {
 
@@ -186,33 +187,7 @@ static Lay derive_layout(const gwgb_layout &L) {
   return l;
 }
 
-// ---------------------------------------------------------------------------
-// device buffer helper
-// ---------------------------------------------------------------------------
-// Device bytes held by the buffers of every live handle in this process.
-static std::atomic<int64_t> g_device_bytes{0};
-
-template <typename T>
-struct DBuf {
-  T *p = nullptr;
-  size_t n = 0;
-  void alloc(size_t count) {
-    free();
-    if (count) GWGB_CUDA(cudaMalloc(&p, count * sizeof(T)));
-    n = count;
-    g_device_bytes += (int64_t)(n * sizeof(T));
-  }
-  void upload(const std::vector<T> &v, cudaStream_t st) {
-    alloc(v.size());
-    if (n) GWGB_CUDA(cudaMemcpyAsync(p, v.data(), n * sizeof(T), cudaMemcpyHostToDevice, st));
-  }
-  void free() {
-    if (p) cudaFree(p);
-    g_device_bytes -= (int64_t)(n * sizeof(T));
-    p = nullptr;
-    n = 0;
-  }
-};
+std::atomic<int64_t> g_device_bytes{0};
 
 // An output block of a contraction and the contributions it sums.
 struct Owner {
@@ -254,14 +229,6 @@ struct GRef {
   int32_t stride;
 };
 
-// Host-side bounds check of one work item: [begin, begin + len) must lie in a
-// buffer of `size` elements.  Every task list is checked when it is built, so
-// no kernel launch can read or write outside its buffers whatever the layout.
-static void check_range(int64_t begin, int64_t len, int64_t size, const char *what) {
-  if (begin < 0 || len < 0 || begin + len > size)
-    throw Error(GWGB_E_INVALID, std::string("internal work list out of bounds: ") + what);
-}
-
 class Engine {
  public:
   Engine(const gwgb_params &p, const gwgb_layout &L);
@@ -274,45 +241,7 @@ class Engine {
     if (prec != prec_) drop_graphs();  // the captured graphs hold the old kernels
     prec_ = prec;
     if (prec_ == GWGB_PREC_OZAKI) {
-      if (!oz_built_) {  // the largest chunks whose buffers fit: budget 1/4, 1/8, ... of the free memory
-        oz_div_ = 4;
-        while (!build_oz_lists()) {
-          GWGB_REQUIRE(oz_div_ < 256, GWGB_E_UNSUPPORTED, "the sliced-precision buffers do not fit the device memory");
-          oz_div_ *= 2;
-        }
-      }
-      if (!ozVcat_.p) {
-        {  // the sliced path's buffers must fit the free memory: say which take it otherwise
-          const std::pair<const char *, int64_t> need[] = {
-              {"Z1", oz_z1_elems_ * 16}, {"Zcat", oz_zcat_elems_ * 16}, {"W", oz_w_elems_ * 16},
-              {"U", oz_u_elems_ * 16}, {"Vcat", oz_vcat_elems_ * 16}, {"Bcat", oz_bcat_elems_ * 16},
-              {"VcatS", oz_vcats_elems_ * 16}, {"V blocks", oz_vz_elems_ * 16}, {"partials", oz_part_elems_ * 16},
-              {"G, P~ copies", (int64_t)(Gall_.n + Pall_.n) * 16}};
-          int64_t tot = 0;
-          std::string msg;
-          for (const auto &x : need) {
-            tot += x.second;
-            msg += std::string(" ") + x.first + " " + std::to_string(x.second >> 20) + " MB";
-          }
-          size_t free_b = 0, total_b = 0;
-          GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-          GWGB_REQUIRE(tot + (256ll << 20) <= (int64_t)free_b, GWGB_E_UNSUPPORTED,
-                       "sliced-precision buffers need " + std::to_string(tot >> 20) + " MB (" + msg + " ), " +
-                           std::to_string(free_b >> 20) + " MB free");
-        }
-        ozVcat_.alloc((size_t)oz_vcat_elems_);
-        ozBcat_.alloc((size_t)oz_bcat_elems_);
-        ozVcatS_.alloc((size_t)oz_vcats_elems_);
-        ozZ1_.alloc((size_t)oz_z1_elems_);
-        ozZcat_.alloc((size_t)oz_zcat_elems_);
-        ozW_.alloc((size_t)oz_w_elems_);
-        ozU_.alloc((size_t)oz_u_elems_);
-        ozVz_.alloc((size_t)oz_vz_elems_);
-        Gff_.alloc(Gall_.n);
-        Pff_.alloc(Pall_.n);
-        ozPart_.alloc((size_t)oz_part_elems_);
-        oz_ready_ = false;
-      }
+      build_oz();
       return;
     }
     if (prec_ != GWGB_PREC_FP64 && !Wbuf_.p && wbuf_elems_) {
@@ -457,10 +386,8 @@ class Engine {
       built = true;
     }
     if (prec_ == GWGB_PREC_OZAKI && !oz_ready_) {
-      // tau-independent operands of contractions that run in one chunk: built once per upload
-      for (const OzLaunch &x : oz_static_)
-        launch_oz_perm(oz_perm_.p + x.t0, (int)x.n, static_cast<const double2 *>(oz_ptr(x.a)),
-                       static_cast<float4 *>(const_cast<void *>(oz_ptr(x.c))), st_);
+      oz_plan_[0].build_static(V_.p, st_);
+      oz_plan_[1].build_static(Vt_.p, st_);
       oz_ready_ = true;
       built = true;
     }
@@ -473,27 +400,11 @@ class Engine {
     if (built) GWGB_CUDA(cudaStreamSynchronize(st_));
   }
   bool tc_split() const { return prec_ == GWGB_PREC_TF32X3 || prec_ == GWGB_PREC_BF16X3; }
-  // Sliced (Ozaki) path: descriptors and tasks of the six GEMM stages per tau
-  // chunk, the float-float operand buffers and the copies that build the
-  // tau-independent ones from V / Vt.
-  // OZB_G, OZB_P: float-float copies of G and P~ (per iteration); OZB_V, OZB_VT: the
-  // FP64 V and pre-rotated V (sources of the operand builds); OZB_VZ: a chunk's V blocks
-  enum OzBufId { OZB_G, OZB_P, OZB_V, OZB_VT, OZB_VZ, OZB_VCAT, OZB_BCAT, OZB_VCATS, OZB_Z1, OZB_ZCAT, OZB_W, OZB_U,
-                 OZB_P0, OZB_SIG };
-  // one stage launch: tasks [t0, t0 + n); with nr > 0 the stage writes FP64 K-slice partials to
-  // ozPart_ and the ordered sums oz_red_[r0, r0 + nr) (times scale) go to buffer c afterwards
-  // simt: the CUDA-core float-float kernel; part: C is ozPart_ (K-slice partials)
-  struct OzLaunch {
-    int64_t t0, n;
-    int a, b, c;
-    bool simt = false, part = false;
-    bool perm = false;        // an operand build: oz_perm_[t0, t0 + n) from buffer a into buffer c
-    int64_t r0 = 0, nr = 0;
-    double scale = 1.0;
-    int stage = 0;            // gwgb_launch_stat.stage
-    double flops = 0, ops = 0, red_bytes = 0;
-    int red_ny = 1;           // CTAs per reduced block
-  };
+  // Sliced (Ozaki) path: one plan per contraction (0: P0, 1: Sigma) and their shared buffers.
+  OzPlan oz_plan_[2];
+  OzShared oz_buf_;
+  bool oz_built_ = false, oz_ready_ = false;
+  void build_oz();
   // per-launch profile (gwgb_set_launch_timing): records [0, n_p0) P0, then Sigma
   bool lt_on_ = false, lt_ran_p0_ = false, lt_ran_sig_ = false;
   std::vector<cudaEvent_t> lt_ev_;
@@ -508,23 +419,15 @@ class Engine {
   void lt_build() {  // one entry per GEMM launch and per reduction, in launch order
     lt_info_.clear();
     for (int l = 0; l < 2; ++l) {
-      for (const OzLaunch &x : l ? oz_sig_ : oz_p0_) {
+      for (const OzLaunch &x : oz_plan_[l].launches()) {
         gwgb_launch_stat g{};
         g.stage = x.stage;
-        g.kernel = x.perm ? 3 : x.simt ? 1 : 0;
+        g.kernel = x.kind;
         g.tasks = (int32_t)x.n;
         g.flops = x.flops;
         g.mma_flops = x.ops;
-        g.bytes = x.perm ? x.red_bytes : 0.0;
+        g.bytes = x.bytes;
         lt_info_.push_back(g);
-        if (x.nr && !x.perm) {
-          gwgb_launch_stat r{};
-          r.stage = x.stage;
-          r.kernel = 2;
-          r.tasks = (int32_t)x.nr;
-          r.bytes = x.red_bytes;
-          lt_info_.push_back(r);
-        }
       }
       if (l == 0) lt_n_p0_ = (int)lt_info_.size();
     }
@@ -561,77 +464,24 @@ class Engine {
   }
 
  private:
-  int oz_simt_n_ = 8;  // block GEMMs with at most this many output columns run on the CUDA cores
-  bool oz_built_ = false, oz_ready_ = false;
-  DBuf<OzDesc> oz_descs_;
-  DBuf<OzTask> oz_tasks_;
-  DBuf<int64_t> oz_rowtab_;
-  DBuf<RedTask> oz_red_;
-  DBuf<double2> ozPart_;
-  int64_t oz_part_elems_ = 1;
-  DBuf<float4> Gff_, Pff_, ozVz_, ozVcat_, ozBcat_, ozVcatS_, ozZ1_, ozZcat_, ozW_, ozU_;
-  int64_t oz_vz_elems_ = 1;
-  // operand builds (copies of V / Vt blocks into chunk-local Vcat, Bcat, VcatS):
-  // in the launch lists per chunk, or in oz_static_ when a contraction has one chunk
-  DBuf<OzPerm> oz_perm_;
-  std::vector<OzLaunch> oz_static_;
-  int64_t oz_vcat_elems_ = 0, oz_bcat_elems_ = 0, oz_vcats_elems_ = 0, oz_z1_elems_ = 0, oz_zcat_elems_ = 0,
-          oz_w_elems_ = 0, oz_u_elems_ = 0;
-  std::vector<OzLaunch> oz_p0_, oz_sig_;
   std::vector<P0Contrib> pc_host_;
   std::vector<SigContrib> sc_host_;
   std::vector<Owner> sig_own_host_;
-  // Builds the lists with a chunk budget of 1/oz_div_ of the free memory; false
-  // (nothing uploaded) when the buffers would take more than 85% of it.
-  bool build_oz_lists();
-  int oz_div_ = 4;
   bool tc_chunk_env_ = false;  // GWGB_TC_CHUNK_MB given: it caps the sliced path's chunks too
-  const void *oz_ptr(int id) const {
-    switch (id) {
-      case OZB_G: return Gff_.p;
-      case OZB_P: return Pff_.p;
-      case OZB_V: return V_.p;
-      case OZB_VT: return Vt_.p;
-      case OZB_VZ: return ozVz_.p;
-      case OZB_VCAT: return ozVcat_.p;
-      case OZB_BCAT: return ozBcat_.p;
-      case OZB_VCATS: return ozVcatS_.p;
-      case OZB_Z1: return ozZ1_.p;
-      case OZB_ZCAT: return ozZcat_.p;
-      case OZB_W: return ozW_.p;
-      case OZB_U: return ozU_.p;
-      case OZB_P0: return Pall_.p;
-      default: return Sig_.p;
-    }
-  }
-  // rec: first profile record of this list (P0: 0, Sigma: lt_n_p0_)
-  void oz_run(const std::vector<OzLaunch> &ls, int rec) {
+  // Run a contraction's plan (0: P0 into Pall_, 1: Sigma into Sig_).
+  void oz_run(int which, double scale) {
     if (lt_on_ && lt_ev_.size() < 2 * lt_info_.size()) {
       const size_t n0 = lt_ev_.size();
       lt_ev_.resize(2 * lt_info_.size());
       for (size_t i = n0; i < lt_ev_.size(); ++i) GWGB_CUDA(cudaEventCreate(&lt_ev_[i]));
     }
-    for (const OzLaunch &x : ls) {
-      void *c = x.part ? static_cast<void *>(ozPart_.p) : const_cast<void *>(oz_ptr(x.c));
-      const void *a = oz_ptr(x.a), *b = oz_ptr(x.b);
-      const float4 *af = static_cast<const float4 *>(a), *bf = static_cast<const float4 *>(b);
+    int rec = which ? lt_n_p0_ : 0;
+    for (const OzLaunch &x : oz_plan_[which].launches()) {
       if (lt_on_) rec_ev(lt_ev_[2 * rec]);
-      if (x.perm)
-        launch_oz_perm(oz_perm_.p + x.t0, (int)x.n, static_cast<const double2 *>(a), static_cast<float4 *>(c), st_);
-      else if (x.simt)
-        launch_oz_simt(oz_descs_.p, oz_tasks_.p + x.t0, (int)x.n, af, bf, c, oz_rowtab_.p, st_);
-      else
-        launch_oz_gemm(oz_descs_.p, oz_tasks_.p + x.t0, (int)x.n, af, bf, c, oz_rowtab_.p, nsm_, bad_.p + 2, st_);
+      oz_plan_[which].run_one(x, oz_buf_, which ? Vt_.p : V_.p, Gall_.p, which ? Pall_.p : Gall_.p,
+                              which ? Sig_.p : Pall_.p, nts_, scale, nsm_, bad_.p + 2, st_);
       if (lt_on_) rec_ev(lt_ev_[2 * rec + 1]);
       ++rec;
-      if (x.nr) {
-        if (lt_on_) rec_ev(lt_ev_[2 * rec]);
-        launch_reduce_slices(oz_red_.p + x.r0, (int)x.nr, ozPart_.p,
-                             static_cast<double2 *>(const_cast<void *>(oz_ptr(x.c))), nts_, x.scale, 0, st_,
-                             x.red_ny);
-        if (lt_on_) rec_ev(lt_ev_[2 * rec + 1]);
-        ++rec;
-      }
     }
   }
   struct P0Group { int64_t pout; int32_t pstride, qb, c0, c1; };
@@ -721,7 +571,6 @@ Engine::Engine(const gwgb_params &p, const gwgb_layout &L) {
   GWGB_REQUIRE(p.uv_waves >= 0 && p.uv_waves <= 16, GWGB_E_INVALID, "uv_waves must be in [0, 16]");
   GWGB_REQUIRE(p.uv_simt == 0 || p.uv_simt == 1, GWGB_E_INVALID, "uv_simt must be 0 or 1");
   GWGB_REQUIRE(p.oz_simt_cols >= -1 && p.oz_simt_cols <= 1024, GWGB_E_INVALID, "oz_simt_cols must be in [-1, 1024]");
-  oz_simt_n_ = p.oz_simt_cols == 0 ? 8 : std::max(0, p.oz_simt_cols);
   tune_uvt_kb_ = p.uvt_smem_kb;
   tune_simt_ = p.uv_simt;
   if (p.sw_npk_max) tune_npk_ = p.sw_npk_max;
@@ -800,9 +649,7 @@ Engine::~Engine() {
                            &Tnt_, &Ttn_, &TntBF_, &TtnFB_};
   sw_tiles_.free(); bc_tasks_.free(); sig_wref_.free(); Wbuf_.free(); Bcat_.free(); uv_red_.free();
   pz_tasks_.free(); vc_tasks_.free(); pk_tiles_.free(); pr_tiles_.free(); Zbuf_.free(); Vcat_.free(); Ppart_.free();
-  oz_descs_.free(); oz_tasks_.free(); oz_perm_.free(); oz_rowtab_.free();
-  for (DBuf<float4> *b : {&Gff_, &Pff_, &ozVz_, &ozVcat_, &ozBcat_, &ozVcatS_, &ozZ1_, &ozZcat_, &ozW_, &ozU_}) b->free();
-  oz_red_.free(); ozPart_.free();
+  oz_plan_[0].free(); oz_plan_[1].free(); oz_buf_.free();
   for (auto *b : bufs) b->free();
   tct_f_.free(); tct_l_.free(); mu_dev_.free(); ws_.free(); bad_.free(); leak_.free();
   qoff_irr_.free(); qsz_irr_.free();
@@ -1573,731 +1420,93 @@ void Engine::build_work_lists() {
 }
 
 // ---------------------------------------------------------------------------
-// sliced (Ozaki) path: work lists of the six GEMM stages
+// sliced (Ozaki) path: the two contractions as chains of block GEMMs (oz_plan.h)
 // ---------------------------------------------------------------------------
-namespace {
-
-// Inclusive extent of the offsets of rows [0, M) of a row map.
-void oz_rows_extent(const OzRows &m, int M, int64_t &lo, int64_t &hi) {
-  const int64_t qmax = (M - 1) / m.d, rmax = std::min<int64_t>(m.d, M) - 1;
-  lo = m.base + std::min<int64_t>(0, qmax * m.s1) + std::min<int64_t>(0, rmax * m.s0);
-  hi = m.base + std::max<int64_t>(0, qmax * m.s1) + std::max<int64_t>(0, rmax * m.s0);
-}
-
-void oz_widen(int64_t &lo, int64_t &hi, int64_t step, int64_t count) {
-  const int64_t e = (count - 1) * step;
-  lo += std::min<int64_t>(0, e);
-  hi += std::max<int64_t>(0, e);
-}
-
-// Every element that the tasks of descriptor d (nrep repetitions) read or
-// write lies inside its buffers of na, nb, nc elements.
-void oz_check(const OzDesc &d, int nrep, int64_t na, int64_t nb, int64_t nc, const char *what) {
-  GWGB_REQUIRE(d.M >= 1 && d.N >= 1 && d.K >= 1 && nrep >= 1 && d.a.d >= 0 && d.b.d >= 0 && d.c.d >= 0 &&
-                   d.cnd >= 1 && (d.a.d != 0 || d.aks == 1),
-               GWGB_E_INVALID, std::string("internal work list out of bounds: empty sliced GEMM in ") + what);
-  int64_t lo, hi;
-  if (d.a.d != 0) {  // table-mapped rows are checked entry by entry where the table is built
-    oz_rows_extent(d.a, d.M, lo, hi);
-    oz_widen(lo, hi, d.aks, d.K);
-    oz_widen(lo, hi, d.ra, nrep);
-    check_range(lo, hi - lo + 1, na, what);
-  }
-  GWGB_REQUIRE(d.b.d != 0, GWGB_E_INVALID, std::string("internal work list: B rows must not be table-mapped in ") + what);
-  oz_rows_extent(d.b, d.N, lo, hi);
-  oz_widen(lo, hi, d.bks, d.K);
-  oz_widen(lo, hi, d.rb, nrep);
-  check_range(lo, hi - lo + 1, nb, what);
-  if (d.c.d == 0) return;
-  oz_rows_extent(d.c, d.M, lo, hi);
-  const int64_t qmax = (d.N - 1) / d.cnd, rmax = std::min<int64_t>(d.cnd, d.N) - 1;
-  lo += std::min<int64_t>(0, qmax * d.cn1) + std::min<int64_t>(0, rmax * d.cn0);
-  hi += std::max<int64_t>(0, qmax * d.cn1) + std::max<int64_t>(0, rmax * d.cn0);
-  oz_widen(lo, hi, d.rc, nrep);
-  check_range(lo, hi - lo + 1, nc, what);
-}
-
-}  // namespace
-
-bool Engine::build_oz_lists() {
-  // Layouts (float-float, complex elements).  The contractions run in chunks of
-  // output blocks (P0: output blocks (q_irr, iq); Sigma: AO blocks (k_irr, i1)
-  // with their spins), each chunk over all tau (a block whose own buffers exceed
-  // the budget: over tau ranges), so the final GEMMs (P0, Sigma) get full
-  // 128-row tiles of (tau, row); a chunk's tau-dependent buffers are
-  // sequences of tau slabs with one stride (z1t, zct, wct, uct elements per
-  // tau), so one repetition offset serves every row of a packed GEMM.
-  //   Z1[tau][pack][m][row]      row = (c, P, t) of the contributions sharing G2's block
-  //   Zcat[tau][group][P][K]     K = (c, s, m, p) of the P0 output block (q_irr, iq)
-  //   Vcat[group][Q][K]          = V_c[Q][p][m] at the same K (per chunk, or all chunks once per upload)
-  //   W[tau][group][Q][col]      col = (c, j, n) of the chunk's contributions in the P~ block group
-  //   U[tau][owner][j][K]        K = (c, Q, m) of the Sigma owner (k_irr, i1, s)
-  //   VcatS[owner][i][K]         = Vt_c[Q][i][m] at the same K (per chunk, or all chunks once per upload)
-  // Per-tau stages (Z1, Z, U) pack the chunk's contributions that share their
-  // G-block operand (same block and spin) into one GEMM with a row table.
+void Engine::build_oz() {
+  if (oz_built_) return;
   const Lay &l = l_;
-  const int ns = ns_, nts = nts_, half = nts / 2;
-  const std::vector<P0Contrib> &pc = pc_host_;
-  const std::vector<SigContrib> &sc = sc_host_;
-  std::vector<OzDesc> ds;
-  std::vector<OzTask> ts;
-  std::vector<int64_t> rt;  // row table
-  constexpr int REPG = 8;   // tau per task in the per-tau stages (Z, U)
-  // narrow[id]: descriptor id runs on the CUDA-core kernel.  The choice uses a
-  // width that does not depend on the chunking (width < 0: d.N), so chunked and
-  // unchunked runs use the same arithmetic for every output element.
-  std::vector<char> narrow_d;
-  auto add = [&](const OzDesc &d, int nrep, int repg, int width = -1) {
-    const int id = (int)ds.size();
-    ds.push_back(d);
-    narrow_d.push_back((width < 0 ? d.N : width) <= oz_simt_n_);
-    const int mtn = (d.M + OZ_M - 1) / OZ_M, ntn = (d.N + OZ_NC - 1) / OZ_NC;
-    GWGB_REQUIRE(mtn < 65536 && ntn < 65536, GWGB_E_UNSUPPORTED, "sliced GEMM too large");
-    for (int r0 = 0; r0 < nrep; r0 += repg)
-      for (int mt = 0; mt < mtn; ++mt)
-        for (int nt = 0; nt < ntn; ++nt) ts.push_back({id, r0, std::min(repg, nrep - r0), (mt << 16) | nt});
-  };
-  // tasks of one stage (appended since t0): the tensor-core tasks, then the
-  // narrow ones (at most oz_simt_n_ output columns) for the CUDA-core kernel,
-  // each heaviest first; one launch per kind.  The last launch carries `last`.
-  auto narrow = [&](const OzTask &t) { return narrow_d[t.desc] != 0; };
-  int cur_stage = 0;  // gwgb_launch_stat.stage of the launches being built
-  auto stage = [&](std::vector<OzLaunch> &v, size_t t0, int a, int b, int c, bool part = false,
-                   const OzLaunch *last = nullptr) {
-    auto cost = [&](const OzTask &t) { return (int64_t)t.nrep * ds[t.desc].K; };
-    std::stable_sort(ts.begin() + t0, ts.end(), [&](const OzTask &x, const OzTask &y) {
-      const bool nx = narrow(x), ny = narrow(y);
-      return nx != ny ? ny : cost(x) > cost(y);
-    });
-    const size_t t1 = std::find_if(ts.begin() + t0, ts.end(), narrow) - ts.begin();
-    const size_t n0 = v.size();
-    for (int k = 0; k < 2; ++k) {
-      const size_t lo = k ? t1 : t0, hi = k ? ts.size() : t1;
-      if (hi == lo) continue;
-      OzLaunch l{(int64_t)lo, (int64_t)(hi - lo), a, b, c};
-      l.simt = k == 1;
-      l.part = part;
-      l.stage = cur_stage;
-      for (size_t t = lo; t < hi; ++t) {  // algorithmic FLOPs; tcgen05 MMA FLOPs or FP32 instructions
-        const OzTask &tk = ts[t];
-        const OzDesc &d = ds[tk.desc];
-        const int Mt = std::min(OZ_M, d.M - (tk.mtnt >> 16) * OZ_M), Nt = std::min(OZ_NC, d.N - (tk.mtnt & 0xffff) * OZ_NC);
-        const double cmac = (double)Mt * Nt * d.K * tk.nrep;
-        l.flops += 8.0 * cmac;
-        if (l.simt) {
-          l.ops += 48.0 * cmac;
-        } else {
-          const int ksteps = (d.K / OZ_KR) * 2 + ((d.K % OZ_KR) + 7) / 8;  // MMA K steps of 8 complex
-          l.ops += 10.0 * 2.0 * OZ_M * (16.0 * ((Nt + 7) / 8)) * 16.0 * ksteps * tk.nrep;
-        }
+  const int ns = ns_, nts = nts_;
+  std::vector<OzContrib> cs;
+  std::vector<OzOwner> own;
+  // memory free for the images of V that do not change between iterations (V itself may not be allocated yet)
+  size_t free_b = 0, total_b = 0;
+  GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  const int64_t avail = (int64_t)free_b - (V_.p ? 0 : 16 * l.flat_V);
+  const int64_t persist = std::max<int64_t>(0, avail / 4);
+  // intermediates of one chunk: large chunks mean fewer, fuller launches (hex 8 k: 1 GB 66 ms, 8 GB 56 ms)
+  const int64_t budget = tc_chunk_env_ ? tc_chunk_bytes_ : std::min<int64_t>(OZ_CHUNK_BYTES, std::max<int64_t>(64ll << 20, avail / 8));
+  // P0[Q][P] = sum V[Q][p][m] G1(beta - tau)[t][p] conj(V[P][t][n]) G2(tau)[m][n]
+  for (const P0Group &g : p0_groups_) {
+    const int c0 = (int)cs.size();
+    for (int c = g.c0; c < g.c1; ++c)
+      for (int s = 0; s < ns; ++s) {
+        const P0Contrib &x = pc_host_[c];
+        const int qb = g.qb, b1 = x.b1, b2 = x.b2;
+        OzContrib o{};
+        o.nL = b2; o.nx = qb; o.ny = b1; o.nz = b1; o.N = qb; o.K1 = b2;
+        o.vid = c;
+        o.v = x.v;
+        o.sx = b1 * b2; o.sy = b2; o.sk = 1; o.conj1 = 1;
+        o.sn = b1 * b2; o.sL = 1; o.sz = b2;
+        o.ga = x.gb + (int64_t)s * x.sb; o.gt = (int64_t)ns * x.sb; o.gL = b2; o.gk = 1;
+        o.b2 = x.ga + ((int64_t)(nts - 1) * ns + s) * x.sa; o.b2t = -(int64_t)ns * x.sa; o.b2z = 1; o.b2y = b1;
+        cs.push_back(o);
       }
-      v.push_back(l);
-    }
-    if (last && v.size() > n0) {
-      v.back().r0 = last->r0;
-      v.back().nr = last->nr;
-      v.back().scale = last->scale;
-      v.back().red_bytes = last->red_bytes;
-      v.back().red_ny = last->red_ny;
-    }
-  };
-  // Final GEMMs (P0, Sigma) in K slices: each slice writes an FP64 partial block
-  // [slice][rows][cols] to ozPart_; the slices are summed in order afterwards
-  // (reduce_slices_kernel), so the result does not depend on the launch order.
-  // The slice count depends on the block alone (about two waves of CTAs for
-  // that block, at least 32 rounds of K per slice), so results do not depend on
-  // how blocks are grouped into chunks.
-  std::vector<RedTask> red;
-  // mfull: rows of the block over all tau (the slice count must not depend on the tau chunking)
-  struct Fin { OzDesc d; int64_t out; int32_t ostride, nt, elems, mfull; };
-  auto final_stage = [&](std::vector<OzLaunch> &v, const std::vector<Fin> &fins, int a, int b, int c, double scale,
-                         int64_t na, int64_t nb, int64_t nout, const char *what) {
-    const size_t t0 = ts.size(), r0 = red.size();
-    int64_t part = 0;
-    for (const Fin &f : fins) {
-      const int64_t tiles = (int64_t)((f.mfull + OZ_M - 1) / OZ_M) * ((f.d.N + OZ_NC - 1) / OZ_NC);
-      const int64_t want = (2 * (int64_t)std::max(1, nsm_) + tiles - 1) / tiles;
-      const int nk16 = (f.d.K + OZ_KR - 1) / OZ_KR;
-      const int nsl = (int)std::max<int64_t>(1, std::min<int64_t>(want, nk16 / 32));
-      const int per = (nk16 + nsl - 1) / nsl * OZ_KR;
-      const int64_t mn = (int64_t)f.d.M * f.d.N;
-      int used = 0;
-      for (int k0 = 0; k0 < f.d.K; k0 += per, ++used) {
-        OzDesc d = f.d;
-        d.a.base += k0;
-        d.b.base += k0;
-        d.K = std::min(per, f.d.K - k0);
-        d.c = {part + used * mn, f.elems, 1, f.d.c.d};
-        d.alpha = 1.0;
-        d.flags |= OZ_OUT_F64;
-        oz_check(d, 1, na, nb, (int64_t)1 << 62, what);
-        add(d, 1, 1);
-      }
-      red.push_back({part, f.out, f.ostride, f.elems, 0, f.nt, used, 0});
-      check_range(f.out, (int64_t)(f.nt - 1) * f.ostride + f.elems, nout, what);
-      part += used * mn;
-    }
-    oz_part_elems_ = std::max(oz_part_elems_, part);
-    OzLaunch red_info{0, 0, a, b, c};
-    red_info.r0 = (int64_t)r0;
-    red_info.nr = (int64_t)(red.size() - r0);
-    red_info.scale = scale;
-    int64_t maxn = 1;
-    for (size_t r = r0; r < red.size(); ++r) {  // partials read, output written
-      red_info.red_bytes += 16.0 * red[r].nt * red[r].elems * (red[r].nslice + 1);
-      maxn = std::max<int64_t>(maxn, (int64_t)red[r].nt * red[r].elems);
-    }
-    // enough CTAs for about four waves of 256-thread blocks, none with under 1024 elements
-    const int64_t nblk = std::max<int64_t>(1, (int64_t)(red.size() - r0));
-    const int64_t want = (4 * 8 * (int64_t)std::max(1, nsm_) + nblk - 1) / nblk;
-    red_info.red_ny = (int)std::max<int64_t>(1, std::min<int64_t>({want, (maxn + 1023) / 1024, 4096}));
-    stage(v, t0, a, b, c, true, &red_info);
-  };
-  // Row-table checks: every entry (plus the row's K extent and reps) inside the buffer.
-  auto check_tab = [&](int64_t base, int M, int64_t klen, int64_t rep, int nrep, int64_t size, const char *what) {
-    for (int r = 0; r < M; ++r) {
-      int64_t lo = rt[base + r], hi = lo + klen - 1;
-      oz_widen(lo, hi, rep, nrep);
-      check_range(lo, hi - lo + 1, size, what);
-    }
-  };
-  oz_p0_.clear();
-  oz_sig_.clear();
-  oz_part_elems_ = 1;
-  const int64_t gsz = (int64_t)Gall_.n, psz = (int64_t)Pall_.n, ssz = (int64_t)nts * ns * l.flat_ao;
-  const double pref = -1.0 / l.nk * (ns == 1 ? 2.0 : 1.0);  // cugw_qkpt_block.cu:210, cugw_solver_block.cpp:303
-
-  // ---- P0 -------------------------------------------------------------------
-  // Operand builds (copies of V / Vt blocks): one launch per chunk and buffer, or
-  // a launch in oz_static_ (once per upload) when the contraction has one chunk.
-  std::vector<OzPerm> perms;
-  oz_static_.clear();
-  auto perm_launch = [&](std::vector<OzLaunch> &v, size_t p0, int src, int dst, bool once) {
-    if (perms.size() == p0) return;
-    OzLaunch l{(int64_t)p0, (int64_t)(perms.size() - p0), src, src, dst};
-    l.perm = true;
-    l.stage = cur_stage;
-    for (size_t t = p0; t < perms.size(); ++t) l.red_bytes += 32.0 * perms[t].X * perms[t].Y * perms[t].Z;
-    (once ? oz_static_ : v).push_back(l);
-  };
-  struct PG { int64_t voff; int zld; };  // Vcat offset (chunk-local) and row length of a P0 group
-  std::vector<PG> pg;
-  std::vector<int> zcol(pc.size() * ns), cgrp(pc.size());
-  for (size_t gi = 0; gi < p0_groups_.size(); ++gi) {
-    const P0Group &g = p0_groups_[gi];
-    int zld = 0;
-    for (int c = g.c0; c < g.c1; ++c) {
-      cgrp[c] = (int)gi;
-      for (int sp = 0; sp < ns; ++sp) {
-        zcol[c * ns + sp] = zld;
-        zld += pc[c].b1 * pc[c].b2;
-      }
-    }
-    pg.push_back({0, zld});
+    own.push_back({g.pout, g.pstride, g.qb, g.qb, g.qb, 1, c0, (int32_t)cs.size()});
   }
-  // chunks of output blocks: Z1, Zcat, Vcat and V blocks of a chunk (all nts/2 tau) within
-  // the budget: 1/oz_div_ of the memory free now (after V), at most GWGB_TC_CHUNK_MB
-  // when that is given, at least 64 MB.  Every buffer is sized to its largest chunk and
-  // the P0 and Sigma buffers coexist; the caller halves the budget until they fit.
-  int64_t budget;  // complex float-float elements
-  {
-    size_t free_b = 0, total_b = 0;
-    GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const int64_t by_free = std::max<int64_t>(64ll << 20, (int64_t)(free_b / oz_div_));
-    budget = std::max<int64_t>(1, (tc_chunk_env_ ? std::min<int64_t>(tc_chunk_bytes_, by_free) : by_free) / 16);
+  oz_plan_[0].build(3, cs, own, nts / 2, 0, budget, persist, nsm_, l.flat_V, (int64_t)Gall_.n, (int64_t)Gall_.n,
+                    (int64_t)Pall_.n, st_);
+  // Sigma[i][j] = sum Vt[Q][i][m] G2(tau)[m][n] P~(tau)[Q][P] conj(Vt[P][j][n])
+  cs.clear();
+  own.clear();
+  for (const Owner &ow : sig_own_host_) {
+    const int c0 = (int)cs.size();
+    for (int c = ow.c0; c < ow.c1; ++c) {
+      const SigContrib &x = sc_host_[c];
+      const int qb = x.qb, b1 = sig_b1_[c], b2 = x.b2;
+      OzContrib o{};
+      o.nL = b2; o.nx = b1; o.ny = qb; o.nz = qb; o.N = b1; o.K1 = b2;
+      o.vid = c;
+      o.v = x.v;
+      o.sx = b2; o.sy = b1 * b2; o.sk = 1;
+      o.sn = b2; o.sL = 1; o.sz = b1 * b2; o.conj3 = 1;
+      o.ga = x.gb + (int64_t)ow.s * x.sb; o.gt = (int64_t)ns * x.sb; o.gL = 1; o.gk = b2;
+      o.b2 = x.pq; o.b2t = x.pstride; o.b2z = 1; o.b2y = qb; o.b2conj = (int8_t)x.pconj;
+      cs.push_back(o);
+    }
+    own.push_back({ow.out, ow.ostride, ow.n, ow.n, 1, ow.n, c0, (int32_t)cs.size()});
   }
-  // The concatenated operands of every chunk are kept (built once per upload) when
-  // together they take at most a quarter of the free memory; otherwise each chunk
-  // builds its own in the launch list.
-  bool persist;
-  {
+  oz_plan_[1].build(3, cs, own, nts, 3, budget, std::max<int64_t>(0, persist - oz_plan_[0].bytes_V()), nsm_,
+                    (int64_t)Vt_.n, (int64_t)Gall_.n, (int64_t)Pall_.n, (int64_t)nts * ns * l.flat_ao, st_);
+  {  // the buffers must fit the free memory: say which take it otherwise
+    const OzPlan &p = oz_plan_[0], &s = oz_plan_[1];
+    const int64_t a1 = std::max(p.bytes_A1(), s.bytes_A1()), b2 = std::max(p.bytes_B2(), s.bytes_B2()),
+                  x1 = std::max(p.bytes_X1(), s.bytes_X1()), x2 = std::max(p.bytes_X2(), s.bytes_X2()),
+                  part = std::max(p.part_elems(), s.part_elems());
+    const std::pair<const char *, int64_t> need[] = {{"V images", p.bytes_V() + s.bytes_V()}, {"G images", a1},
+                                                     {"stage-2 operands", b2}, {"X1", x1}, {"X2", x2},
+                                                     {"partials", 16 * part}};
     int64_t tot = 0;
-    for (size_t gi = 0; gi < p0_groups_.size(); ++gi) tot += 2 * (int64_t)p0_groups_[gi].qb * pg[gi].zld;
-    for (const SigContrib &x : sc) tot += 2 * (int64_t)x.qb * x.b2 * 64;  // Bcat + VcatS, AO blocks <= 64
-    size_t free_b = 0, total_b = 0;
+    std::string msg;
+    for (const auto &x : need) {
+      tot += x.second;
+      msg += std::string(" ") + x.first + " " + std::to_string(x.second >> 20) + " MB";
+    }
     GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    persist = tot * 16 <= (int64_t)(free_b / 4);
+    GWGB_REQUIRE(tot + (256ll << 20) + (V_.p ? 0 : 16 * l.flat_V) <= (int64_t)free_b, GWGB_E_UNSUPPORTED,
+                 "sliced-precision buffers need " + std::to_string(tot >> 20) + " MB (" + msg + " ), " +
+                     std::to_string(free_b >> 20) + " MB free");
+    oz_plan_[0].alloc_images();
+    oz_plan_[1].alloc_images();
+    oz_buf_.A1.alloc((size_t)a1);
+    oz_buf_.B2.alloc((size_t)b2);
+    oz_buf_.X1.alloc((size_t)x1);
+    oz_buf_.X2.alloc((size_t)x2);
+    oz_buf_.part.alloc((size_t)part);
   }
-  int64_t vcat_base = 0, vz_base = 0, bcat_base = 0, vcats_base = 0;  // persistent: each chunk's offset
-  // persistent: where a block's operand copy already is (tau chunks of one block share it)
-  std::vector<int64_t> vcat_at(p0_groups_.size(), -1), vz_at(pc.size(), -1);
-  std::map<std::pair<int, int>, int64_t> bcat_at, vcats_at;
-  // A group whose own need is above the budget gets chunks of its own over tau ranges.
-  struct Chunk { int first, second, t0, t1; };  // output blocks [first, second), tau [t0, t1)
-  std::vector<Chunk> pchunks;
-  {
-    auto need = [&](size_t g, int nt) {  // Z1 and Zcat per tau, Vcat and V blocks once
-      return (2 * (int64_t)nt + 2) * p0_groups_[g].qb * pg[g].zld;
-    };
-    for (size_t g0 = 0; g0 < p0_groups_.size();) {
-      if (need(g0, half) > budget) {
-        const int64_t per = 2 * (int64_t)p0_groups_[g0].qb * pg[g0].zld;
-        const int nt = (int)std::max<int64_t>(1, std::min<int64_t>(half, (budget - per) / per));
-        for (int t0 = 0; t0 < half; t0 += nt) pchunks.push_back({(int)g0, (int)g0 + 1, t0, std::min(half, t0 + nt)});
-        ++g0;
-        continue;
-      }
-      size_t g1 = g0;
-      int64_t tot = 0;
-      while (g1 < p0_groups_.size() && need(g1, half) <= budget && (g1 == g0 || tot + need(g1, half) <= budget))
-        tot += need(g1++, half);
-      pchunks.push_back({(int)g0, (int)g1, 0, half});
-      g0 = g1;
-    }
-  }
-  oz_z1_elems_ = oz_zcat_elems_ = oz_vcat_elems_ = oz_vz_elems_ = 1;
-  struct PackRow { int c; int64_t pos; };
-  for (const auto &ch : pchunks) {
-    const int t0 = ch.t0, ntc = ch.t1 - ch.t0;  // the chunk's tau range
-    {  // Vcat of the chunk's groups: Vcat[Q][zcol + m b1 + p] = V_c[Q][p][m]
-      const size_t p0 = perms.size();
-      int64_t voff = persist ? vcat_base : 0;
-      for (int gi = ch.first; gi < ch.second; ++gi) {
-        const P0Group &g = p0_groups_[gi];
-        if (persist && vcat_at[gi] >= 0) {
-          pg[gi].voff = vcat_at[gi];
-          continue;
-        }
-        pg[gi].voff = voff;
-        vcat_at[gi] = voff;
-        for (int c = g.c0; c < g.c1; ++c)
-          for (int sp = 0; sp < ns; ++sp)
-            perms.push_back({pc[c].v, voff + zcol[c * ns + sp], pg[gi].zld, 1, pc[c].b1, g.qb, pc[c].b1, pc[c].b2, 0});
-        voff += (int64_t)g.qb * pg[gi].zld;
-      }
-      oz_vcat_elems_ = std::max(oz_vcat_elems_, voff);
-      for (size_t t = p0; t < perms.size(); ++t) {
-        const OzPerm &x = perms[t];
-        check_range(x.src, (int64_t)x.X * x.Y * x.Z, l.flat_V, "sliced Vcat source");
-        check_range(x.dst, (x.X - 1) * x.dx + (x.Y - 1) * x.dy + (x.Z - 1) * x.dz + 1, voff, "sliced Vcat");
-      }
-      if (persist) vcat_base = voff;
-      cur_stage = 2;
-      perm_launch(oz_p0_, p0, OZB_V, OZB_VCAT, persist || pchunks.size() == 1);
-    }
-    std::vector<int64_t> vz(pc.size(), -1);  // the chunk's V blocks in float-float (the Z1 stage's A rows)
-    int64_t vz_elems = persist ? vz_base : 0;
-    {
-      const size_t p0 = perms.size();
-      int64_t &off = vz_elems;
-      for (int gi = ch.first; gi < ch.second; ++gi)
-        for (int c = p0_groups_[gi].c0; c < p0_groups_[gi].c1; ++c) {
-          const int qb = p0_groups_[gi].qb, b1 = pc[c].b1, b2 = pc[c].b2;
-          if (persist && vz_at[c] >= 0) {
-            vz[c] = vz_at[c];
-            continue;
-          }
-          vz[c] = vz_at[c] = off;
-          perms.push_back({pc[c].v, off, (int64_t)b1 * b2, b2, 1, qb, b1, b2, 0});
-          check_range(pc[c].v, (int64_t)qb * b1 * b2, l.flat_V, "sliced V block source");
-          off += (int64_t)qb * b1 * b2;
-        }
-      oz_vz_elems_ = std::max(oz_vz_elems_, off);
-      if (persist) vz_base = off;
-      cur_stage = 0;
-      perm_launch(oz_p0_, p0, OZB_V, OZB_VZ, persist || pchunks.size() == 1);
-    }
-    // chunk-local per-tau layouts
-    std::vector<int64_t> zc(p0_groups_.size(), 0);
-    int64_t zct = 0;
-    for (int gi = ch.first; gi < ch.second; ++gi) {
-      zc[gi] = zct;
-      zct += (int64_t)p0_groups_[gi].qb * pg[gi].zld;
-    }
-    std::map<std::pair<int64_t, int>, std::vector<PackRow>> z1p, zp;
-    for (int gi = ch.first; gi < ch.second; ++gi)
-      for (int c = p0_groups_[gi].c0; c < p0_groups_[gi].c1; ++c)
-        for (int sp = 0; sp < ns; ++sp) {
-          auto &v = z1p[{pc[c].gb, sp}];
-          const int64_t pos =
-              v.empty() ? 0 : v.back().pos + (int64_t)p0_groups_[cgrp[v.back().c]].qb * pc[v.back().c].b1;
-          v.push_back({c, pos});
-          zp[{pc[c].ga, sp}].push_back({c, 0});
-        }
-    std::map<int, int64_t> z1pack, z1mp, z1pos;  // keyed by c * ns + s
-    int64_t z1t = 0;
-    for (auto &kv : z1p) {
-      const auto &v = kv.second;
-      const int64_t mp = v.back().pos + (int64_t)p0_groups_[cgrp[v.back().c]].qb * pc[v.back().c].b1;
-      for (const PackRow &x : v) {
-        const int k = x.c * ns + kv.first.second;
-        z1pack[k] = z1t;
-        z1mp[k] = mp;
-        z1pos[k] = x.pos;
-      }
-      z1t += mp * pc[v[0].c].b2;
-    }
-    const int64_t z1_elems = z1t * ntc, zcat_elems = zct * ntc;
-    oz_z1_elems_ = std::max(oz_z1_elems_, z1_elems);
-    oz_zcat_elems_ = std::max(oz_zcat_elems_, zcat_elems);
-    size_t s0 = ts.size();
-    for (auto &kv : z1p) {  // Z1[tau][m][(c,P,t)] = sum_n conj(V_c[P][t][n]) G2(tau)[m][n]
-      const int sp = kv.first.second;
-      const auto &v = kv.second;
-      const P0Contrib &c0 = pc[v[0].c];
-      const int b2 = c0.b2, k0 = v[0].c * ns + sp;
-      const int64_t tab = (int64_t)rt.size();
-      for (const PackRow &x : v) {
-        const P0Contrib &cb = pc[x.c];
-        const int qb = p0_groups_[cgrp[x.c]].qb;
-        for (int P = 0; P < qb; ++P)
-          for (int t = 0; t < cb.b1; ++t) rt.push_back(vz[x.c] + ((int64_t)P * cb.b1 + t) * b2);
-      }
-      OzDesc d{};
-      d.M = (int)(rt.size() - tab);
-      d.a = {tab, 0, 0, 0};
-      d.b = {c0.gb + ((int64_t)t0 * ns + sp) * c0.sb, (int64_t)ns * c0.sb, b2, b2};  // G2(tau) rows (tau, m)
-      d.c = {z1pack[k0], 1, 0, 1};
-      d.cn1 = z1t;
-      d.cn0 = (int32_t)z1mp[k0];
-      d.cnd = b2;
-      d.aks = d.bks = 1;
-      d.N = ntc * b2;
-      d.K = b2;
-      d.flags = OZ_CONJ_A;
-      check_tab(tab, d.M, b2, 0, 1, vz_elems, "P0 stage Z1 (V rows)");
-      oz_check(d, 1, vz_elems, gsz, z1_elems, "P0 stage Z1");
-      add(d, 1, 1, half * b2);  // routed by the width over all tau (every tau chunk the same way)
-    }
-    cur_stage = 0;
-    stage(oz_p0_, s0, OZB_VZ, OZB_G, OZB_Z1);
-    s0 = ts.size();
-    for (auto &kv : zp) {  // Zcat[tau][P][K = (c,s,m,p)] = sum_t G1(beta-tau)[t][p] Z1[tau][m][(c,P,t)]
-      const int sp = kv.first.second;
-      const auto &v = kv.second;
-      const P0Contrib &c0 = pc[v[0].c];
-      const int b1 = c0.b1;
-      const int64_t taba = (int64_t)rt.size();
-      for (const PackRow &x : v) {
-        const P0Contrib &cb = pc[x.c];
-        const int qb = p0_groups_[cgrp[x.c]].qb, k = x.c * ns + sp;
-        for (int P = 0; P < qb; ++P)
-          for (int m = 0; m < cb.b2; ++m) rt.push_back(z1pack[k] + m * z1mp[k] + z1pos[k] + (int64_t)P * b1);
-      }
-      const int64_t tabc = (int64_t)rt.size();
-      for (const PackRow &x : v) {
-        const P0Contrib &cb = pc[x.c];
-        const int gi = cgrp[x.c], qb = p0_groups_[gi].qb, k = x.c * ns + sp;
-        for (int P = 0; P < qb; ++P)
-          for (int m = 0; m < cb.b2; ++m) rt.push_back(zc[gi] + (int64_t)P * pg[gi].zld + zcol[k] + (int64_t)m * b1);
-      }
-      OzDesc d{};
-      d.M = (int)(tabc - taba);
-      d.a = {taba, 0, 0, 0};
-      d.ra = z1t;
-      d.b = {c0.ga + ((int64_t)(nts - 1 - t0) * ns + sp) * c0.sa, 1, 0, 1};  // G1(beta - tau)
-      d.bks = b1;
-      d.rb = -(int64_t)ns * c0.sa;
-      d.c = {tabc, 0, 0, 0};
-      d.rc = zct;
-      d.cn1 = 1;
-      d.cnd = 1;
-      d.aks = 1;
-      d.N = b1;
-      d.K = b1;
-      check_tab(taba, d.M, b1, z1t, ntc, z1_elems, "P0 stage Z (Z1 rows)");
-      check_tab(tabc, d.M, b1, zct, ntc, zcat_elems, "P0 stage Z (Zcat rows)");
-      oz_check(d, ntc, z1_elems, gsz, zcat_elems, "P0 stage Z");
-      add(d, ntc, REPG);
-    }
-    cur_stage = 1;
-    stage(oz_p0_, s0, OZB_Z1, OZB_G, OZB_ZCAT);
-    std::vector<Fin> fins;
-    for (int gi = ch.first; gi < ch.second; ++gi) {  // P0[Q][P] = sum_K Zcat[(tau,P)][K] Vcat[Q][K]
-      const P0Group &g = p0_groups_[gi];
-      if (g.c1 == g.c0) continue;
-      OzDesc d{};
-      d.a = {zc[gi], zct, pg[gi].zld, g.qb};
-      d.b = {pg[gi].voff, pg[gi].zld, 0, 1};
-      d.c = {0, 0, 1, g.qb};  // partial [slice][(tau, P)][Q]: rows (tau, P), column Q at Q * qb
-      d.cn1 = g.qb;
-      d.cnd = 1;
-      d.aks = d.bks = 1;
-      d.M = ntc * g.qb;
-      d.N = g.qb;
-      d.K = pg[gi].zld;
-      oz_check(d, 1, zcat_elems, oz_vcat_elems_, (int64_t)1 << 62, "P0 stage P0");
-      fins.push_back({d, g.pout + (int64_t)t0 * g.pstride, g.pstride, ntc, g.qb * g.qb, half * g.qb});
-    }
-    cur_stage = 2;
-    final_stage(oz_p0_, fins, OZB_ZCAT, OZB_VCAT, OZB_P0, pref, zcat_elems, oz_vcat_elems_, psz, "P0 stage P0");
-  }
-
-  // ---- Sigma ----------------------------------------------------------------
-  // Bcat per P~ block group, columns in contribution order (so the columns of a
-  // chunk of AO-block owners are contiguous in every group); chunk-local copies
-  struct SG { int qb, ncol; };
-  std::vector<SG> sg;
-  std::vector<int> cgroup(sc.size(), -1), ccol(sc.size(), 0);
-  std::vector<std::vector<int>> gcs;  // contributions of each group (increasing)
-  for (const auto &grp : sig_groups_) {
-    const std::vector<int> &cs = grp.second;
-    const int qb = sc[cs[0]].qb;
-    int ncol = 0;
-    for (int c : cs) {
-      cgroup[c] = (int)sg.size();
-      ccol[c] = ncol;
-      ncol += sig_b1_[c] * sc[c].b2;
-    }
-    sg.push_back({qb, ncol});
-    gcs.push_back(cs);
-  }
-  // AO-block owners (k_irr, i1): the owners of their spins share (c0, c1)
-  std::vector<int> ucol(sc.size(), 0);
-  std::map<std::pair<int, int>, int> uldk;  // (c0, c1) -> row length of U and VcatS
-  std::vector<std::pair<int, int>> aoo;     // distinct (c0, c1) in owner order
-  std::map<std::pair<int, int>, int> aoidx; // (c0, c1) -> index in aoo
-  std::map<std::pair<int, int>, int> aon;   // (c0, c1) -> block size (rows of VcatS)
-  for (size_t oi = 0; oi < sig_own_host_.size(); ++oi) {
-    const Owner &o = sig_own_host_[oi];
-    const auto key = std::make_pair(o.c0, o.c1);
-    if (uldk.count(key)) continue;
-    int uld = 0;
-    for (int c = o.c0; c < o.c1; ++c) {
-      ucol[c] = uld;
-      uld += sc[c].qb * sc[c].b2;
-    }
-    uldk[key] = uld;
-    aon[key] = o.n;
-    aoidx[key] = (int)aoo.size();
-    aoo.push_back(key);
-  }
-  // chunks of AO-block owners: W and U of a chunk (all nts tau) and its Bcat and
-  // VcatS within the budget
-  // An owner whose own need is above the budget gets chunks of its own over tau ranges.
-  auto ao_w = [&](const std::pair<int, int> &key) {
-    int64_t w = 0;
-    for (int c = key.first; c < key.second; ++c) w += (int64_t)sc[c].qb * sig_b1_[c] * sc[c].b2;
-    return w;
-  };
-  auto ao_need = [&](const std::pair<int, int> &key, int nt) {  // W and U per tau, Bcat and VcatS once
-    const int64_t w = ao_w(key);
-    return (1 + ns) * w * nt + w + (int64_t)aon[key] * uldk[key];
-  };
-  std::vector<Chunk> schunks;  // ranges of aoo, tau ranges
-  for (size_t a0 = 0; a0 < aoo.size();) {
-    if (ao_need(aoo[a0], nts) > budget) {
-      const int64_t per = (1 + ns) * ao_w(aoo[a0]), fixed = ao_need(aoo[a0], 0);
-      const int nt = (int)std::max<int64_t>(1, std::min<int64_t>(nts, (budget - fixed) / per));
-      for (int t0 = 0; t0 < nts; t0 += nt) schunks.push_back({(int)a0, (int)a0 + 1, t0, std::min(nts, t0 + nt)});
-      ++a0;
-      continue;
-    }
-    size_t a1 = a0;
-    int64_t tot = 0;
-    while (a1 < aoo.size() && ao_need(aoo[a1], nts) <= budget && (a1 == a0 || tot + ao_need(aoo[a1], nts) <= budget))
-      tot += ao_need(aoo[a1++], nts);
-    schunks.push_back({(int)a0, (int)a1, 0, nts});
-    a0 = a1;
-  }
-  oz_w_elems_ = oz_u_elems_ = oz_bcat_elems_ = oz_vcats_elems_ = 1;
-  for (const auto &ch : schunks) {
-    const int t0 = ch.t0, ntc = ch.t1 - ch.t0;                           // the chunk's tau range
-    const int cA = aoo[ch.first].first, cB = aoo[ch.second - 1].second;  // contributions [cA, cB)
-    // W: per group, the chunk's columns (contiguous: contributions in [cA, cB)); the
-    // chunk's Bcat holds those columns, group after group: Bcat[col][P] = conj(Vt_c[P][j][n])
-    struct WG { int g, col0, ncol; int64_t wc, boff; };
-    std::vector<WG> wg;
-    std::vector<int> wgi(sg.size(), -1);
-    int64_t wct = 0, boff = persist ? bcat_base : 0;
-    const size_t pb0 = perms.size();
-    for (size_t gi = 0; gi < sg.size(); ++gi) {
-      int col0 = -1, ncol = 0;
-      for (int c : gcs[gi])
-        if (c >= cA && c < cB) {
-          if (col0 < 0) col0 = ccol[c];
-          ncol += sig_b1_[c] * sc[c].b2;
-        }
-      if (ncol == 0) continue;
-      const int qb = sg[gi].qb;
-      int64_t at = boff;
-      auto hit = bcat_at.find({(int)gi, cA});
-      if (persist && hit != bcat_at.end()) {
-        at = hit->second;
-      } else {
-        for (int c : gcs[gi])
-          if (c >= cA && c < cB)
-            perms.push_back({sc[c].v, boff + (int64_t)(ccol[c] - col0) * qb, 1, (int64_t)sc[c].b2 * qb, qb, qb,
-                             sig_b1_[c], sc[c].b2, 1});
-        bcat_at[{(int)gi, cA}] = boff;
-        boff += (int64_t)qb * ncol;
-      }
-      wgi[gi] = (int)wg.size();
-      wg.push_back({(int)gi, col0, ncol, wct, at});
-      wct += (int64_t)qb * ncol;
-    }
-    oz_bcat_elems_ = std::max(oz_bcat_elems_, boff);
-    for (size_t t = pb0; t < perms.size(); ++t) {
-      const OzPerm &x = perms[t];
-      check_range(x.src, (int64_t)x.X * x.Y * x.Z, (int64_t)Vt_.n, "sliced Bcat source");
-      check_range(x.dst, (x.X - 1) * x.dx + (x.Y - 1) * x.dy + (x.Z - 1) * x.dz + 1, boff, "sliced Bcat");
-    }
-    if (persist) bcat_base = boff;
-    cur_stage = 3;
-    perm_launch(oz_sig_, pb0, OZB_VT, OZB_BCAT, persist || schunks.size() == 1);
-    // VcatS of the chunk's owner blocks: VcatS[i][ucol + Q b2 + n] = Vt_c[Q][i][n]
-    const size_t ps0 = perms.size();
-    std::map<std::pair<int, int>, std::pair<int64_t, int>> vs;  // (c0, c1) -> (VcatS offset, uld)
-    int64_t vsoff = persist ? vcats_base : 0;
-    for (int ai = ch.first; ai < ch.second; ++ai) {
-      const auto key = aoo[ai];
-      const int uld = uldk[key];
-      auto hit = vcats_at.find(key);
-      if (persist && hit != vcats_at.end()) {
-        vs[key] = {hit->second, uld};
-        continue;
-      }
-      vs[key] = {vsoff, uld};
-      vcats_at[key] = vsoff;
-      for (int c = key.first; c < key.second; ++c)
-        perms.push_back({sc[c].v, vsoff + ucol[c], sc[c].b2, uld, 1, sc[c].qb, sig_b1_[c], sc[c].b2, 0});
-      vsoff += (int64_t)aon[key] * uld;
-    }
-    oz_vcats_elems_ = std::max(oz_vcats_elems_, vsoff);
-    for (size_t t = ps0; t < perms.size(); ++t) {
-      const OzPerm &x = perms[t];
-      check_range(x.src, (int64_t)x.X * x.Y * x.Z, (int64_t)Vt_.n, "sliced VcatS source");
-      check_range(x.dst, (x.X - 1) * x.dx + (x.Y - 1) * x.dy + (x.Z - 1) * x.dz + 1, vsoff, "sliced VcatS");
-    }
-    if (persist) vcats_base = vsoff;
-    cur_stage = 5;
-    perm_launch(oz_sig_, ps0, OZB_VT, OZB_VCATS, persist || schunks.size() == 1);
-    // U: the chunk's owners (all spins)
-    std::vector<int64_t> uoff(sig_own_host_.size(), -1);
-    int64_t uct = 0;
-    for (size_t oi = 0; oi < sig_own_host_.size(); ++oi) {
-      const Owner &o = sig_own_host_[oi];
-      const int ai = aoidx[std::make_pair(o.c0, o.c1)];
-      if (ai < ch.first || ai >= ch.second) continue;
-      uoff[oi] = uct;
-      uct += (int64_t)o.n * vs[std::make_pair(o.c0, o.c1)].second;
-    }
-    const int64_t w_elems = std::max<int64_t>(1, wct * ntc), u_elems = std::max<int64_t>(1, uct * ntc);
-    oz_w_elems_ = std::max(oz_w_elems_, w_elems);
-    oz_u_elems_ = std::max(oz_u_elems_, u_elems);
-    size_t s0 = ts.size();
-    for (const WG &w : wg) {  // W[tau][Q][(c,j,n)] = sum_P op(P~(tau))[Q][P] conj(Vt_c[P][j][n])
-      const SigContrib &c0 = sc[gcs[w.g][0]];
-      const int qb = c0.qb;
-      OzDesc d{};
-      d.a = {c0.pq + (int64_t)t0 * c0.pstride, c0.pstride, qb, qb};  // P~ rows (tau, Q) of the tau range
-      d.b = {w.boff, qb, 0, 1};  // the chunk's Bcat columns of this group
-      d.c = {w.wc, wct, w.ncol, qb};
-      d.cn1 = 1;
-      d.cnd = 1;
-      d.aks = d.bks = 1;
-      d.M = ntc * qb;
-      d.N = w.ncol;
-      d.K = qb;
-      d.flags = c0.pconj ? OZ_CONJ_A : 0;
-      oz_check(d, 1, psz, oz_bcat_elems_, w_elems, "Sigma stage W");
-      add(d, 1, 1, sg[w.g].ncol);  // routed by the group's full width (every chunk the same way)
-    }
-    cur_stage = 3;
-    stage(oz_sig_, s0, OZB_P, OZB_BCAT, OZB_W);
-    s0 = ts.size();
-    // U packs: (G2 block, spin) -> [(owner, contribution)]
-    std::map<std::pair<int64_t, int>, std::vector<std::pair<int, int>>> up;
-    for (size_t oi = 0; oi < sig_own_host_.size(); ++oi) {
-      if (uoff[oi] < 0) continue;
-      const Owner &o = sig_own_host_[oi];
-      for (int c = o.c0; c < o.c1; ++c) up[{sc[c].gb, o.s}].push_back({(int)oi, c});
-    }
-    for (auto &kv : up) {  // U[tau][j][(c,Q,m)] = sum_n W[tau][Q][(c,j,n)] G2(tau)[m][n]
-      const int sp = kv.first.second;
-      const auto &v = kv.second;
-      const SigContrib &c0 = sc[v[0].second];
-      const int b2 = c0.b2;
-      const int64_t taba = (int64_t)rt.size();
-      for (const auto &x : v) {
-        const int c = x.second, b1 = sig_b1_[c];
-        const WG &w = wg[wgi[cgroup[c]]];
-        for (int Q = 0; Q < sc[c].qb; ++Q)
-          for (int j = 0; j < b1; ++j)
-            rt.push_back(w.wc + (int64_t)Q * w.ncol + (ccol[c] - w.col0) + (int64_t)j * b2);
-      }
-      const int64_t tabc = (int64_t)rt.size();
-      for (const auto &x : v) {
-        const int c = x.second, b1 = sig_b1_[c];
-        const Owner &o = sig_own_host_[x.first];
-        const int uld = vs[std::make_pair(o.c0, o.c1)].second;
-        for (int Q = 0; Q < sc[c].qb; ++Q)
-          for (int j = 0; j < b1; ++j) rt.push_back(uoff[x.first] + ucol[c] + (int64_t)Q * b2 + (int64_t)j * uld);
-      }
-      OzDesc d{};
-      d.M = (int)(tabc - taba);
-      d.a = {taba, 0, 0, 0};
-      d.ra = wct;
-      d.b = {c0.gb + ((int64_t)t0 * ns + sp) * c0.sb, b2, 0, 1};  // G2(tau), tau from t0
-      d.rb = (int64_t)ns * c0.sb;
-      d.c = {tabc, 0, 0, 0};
-      d.rc = uct;
-      d.cn1 = 1;
-      d.cnd = 1;
-      d.aks = d.bks = 1;
-      d.N = b2;
-      d.K = b2;
-      check_tab(taba, d.M, b2, wct, ntc, w_elems, "Sigma stage U (W rows)");
-      check_tab(tabc, d.M, b2, uct, ntc, u_elems, "Sigma stage U (U rows)");
-      oz_check(d, ntc, w_elems, gsz, u_elems, "Sigma stage U");
-      add(d, ntc, REPG);
-    }
-    cur_stage = 4;
-    stage(oz_sig_, s0, OZB_W, OZB_G, OZB_U);
-    std::vector<Fin> fins;
-    for (size_t oi = 0; oi < sig_own_host_.size(); ++oi) {  // Sigma[i][j] = sum_K U[(tau,j)][K] VcatS[i][K]
-      if (uoff[oi] < 0) continue;
-      const Owner &o = sig_own_host_[oi];
-      const auto &v = vs[std::make_pair(o.c0, o.c1)];
-      if (v.second == 0) continue;
-      OzDesc d{};
-      d.a = {uoff[oi], uct, v.second, o.n};
-      d.b = {v.first, v.second, 0, 1};
-      d.c = {0, 0, 1, o.n};  // partial [slice][(tau, j)][i]: rows (tau, j), column i at i * b1
-      d.cn1 = o.n;
-      d.cnd = 1;
-      d.aks = d.bks = 1;
-      d.M = ntc * o.n;
-      d.N = o.n;
-      d.K = v.second;
-      oz_check(d, 1, u_elems, oz_vcats_elems_, (int64_t)1 << 62, "Sigma stage Sigma");
-      fins.push_back({d, o.out + (int64_t)t0 * o.ostride, o.ostride, ntc, o.n * o.n, nts * o.n});
-    }
-    cur_stage = 5;
-    final_stage(oz_sig_, fins, OZB_U, OZB_VCATS, OZB_SIG, -1.0 / l.nk, u_elems, oz_vcats_elems_, ssz,
-                "Sigma stage Sigma");
-  }
-  GWGB_REQUIRE(ts.size() < (size_t)INT32_MAX, GWGB_E_UNSUPPORTED, "too many sliced GEMM tasks");
-  {  // buffers and lists within 85% of the free memory, or a smaller budget
-    const int64_t bufs = 16 * (oz_z1_elems_ + oz_zcat_elems_ + oz_w_elems_ + oz_u_elems_ + oz_vcat_elems_ +
-                               oz_bcat_elems_ + oz_vcats_elems_ + oz_vz_elems_ + oz_part_elems_ +
-                               (int64_t)(Gall_.n + Pall_.n)) +
-                         (int64_t)(ds.size() * sizeof(OzDesc) + ts.size() * sizeof(OzTask) + rt.size() * 8);
-    size_t free_b = 0, total_b = 0;
-    GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    if (bufs > (int64_t)(0.85 * (double)free_b) && oz_div_ < 256) return false;
-  }
-  {
-    const int64_t lists = (int64_t)(ds.size() * sizeof(OzDesc) + ts.size() * sizeof(OzTask) + rt.size() * 8 +
-                                    perms.size() * sizeof(OzPerm) + red.size() * sizeof(RedTask));
-    size_t free_b = 0, total_b = 0;
-    GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    GWGB_REQUIRE(lists + (256ll << 20) <= (int64_t)free_b, GWGB_E_UNSUPPORTED,
-                 "sliced-precision work lists need " + std::to_string(lists >> 20) + " MB (row tables " +
-                     std::to_string((rt.size() * 8) >> 20) + " MB, tasks " +
-                     std::to_string((ts.size() * sizeof(OzTask)) >> 20) + " MB), " + std::to_string(free_b >> 20) +
-                     " MB free");
-  }
-  oz_descs_.upload(ds, st_);
-  oz_tasks_.upload(ts, st_);
-  oz_rowtab_.upload(rt.empty() ? std::vector<int64_t>(1, 0) : rt, st_);
-  for (const RedTask &r : red) check_range(r.part, (int64_t)r.nslice * r.nt * r.elems, oz_part_elems_, "sliced partials");
-  oz_red_.upload(red.empty() ? std::vector<RedTask>(1, RedTask{}) : red, st_);
-  oz_perm_.upload(perms.empty() ? std::vector<OzPerm>(1, OzPerm{}) : perms, st_);
-  GWGB_CUDA(cudaStreamSynchronize(st_));
+  oz_ready_ = false;
   lt_build();
   oz_built_ = true;
-  return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -2398,9 +1607,8 @@ void Engine::k_p0(int mirror) {
   const double pref = -1.0 / l_.nk * (ns_ == 1 ? 2.0 : 1.0);  // cugw_qkpt_block.cu:210, cugw_solver_block.cpp:303
   if (prec_ == GWGB_PREC_OZAKI) {  // sliced contractions: Z1 -> Z -> P0 per tau chunk
     GWGB_REQUIRE(oz_ready_, GWGB_E_STATE, "sliced-precision operands not prepared");
-    launch_to_ffc(Gall_.p, Gff_.p, (int64_t)Gall_.n, st_);
     GWGB_CUDA(cudaMemsetAsync(Pall_.p, 0, Pall_.n * sizeof(double2), st_));  // blocks without contributions
-    oz_run(oz_p0_, 0);
+    oz_run(0, pref);
     lt_ran_p0_ = lt_on_;
     if (mirror) launch_mirror(Pall_.p, qoff_irr_.p, qsz_irr_.p, l_.ink, nts_, st_);
   } else if (prec_ != GWGB_PREC_FP64) {  // tcgen05 split contractions
@@ -2431,10 +1639,8 @@ void Engine::k_pq(bool mirror_first) {
 void Engine::k_sigma() {
   if (prec_ == GWGB_PREC_OZAKI) {  // sliced contractions: W -> U -> Sigma per tau chunk
     GWGB_REQUIRE(oz_ready_, GWGB_E_STATE, "sliced-precision operands not prepared");
-    launch_to_ffc(Gall_.p, Gff_.p, (int64_t)Gall_.n, st_);
-    launch_to_ffc(Pall_.p, Pff_.p, (int64_t)Pall_.n, st_);
     GWGB_CUDA(cudaMemsetAsync(Sig_.p, 0, Sig_.n * sizeof(double2), st_));  // blocks without contributions
-    oz_run(oz_sig_, lt_n_p0_);
+    oz_run(1, -1.0 / l_.nk);
     lt_ran_sig_ = lt_on_;
   } else if (prec_ != GWGB_PREC_FP64) {  // tcgen05 split contractions
     GWGB_REQUIRE(Wbuf_.p || !wbuf_elems_, GWGB_E_STATE, "mixed-precision work buffer missing");
@@ -2524,10 +1730,8 @@ void Engine::finish_stats(bool with_dyson, bool with_gw, bool with_pq, bool with
     const int64_t sg = tc ? sgt
                           : (sig_tiles_.n ? 1 : 0) + (sig_red_.n ? 1 : 0);
     if (prec_ == GWGB_PREC_OZAKI) {
-      int64_t a = 1, b = 2;  // G (and P~) to float-float
-      for (const OzLaunch &x : oz_p0_) a += x.n ? 1 : 0;
-      for (const OzLaunch &x : oz_sig_) b += x.n ? 1 : 0;
-      launches += (rotG_.n ? 1 : 0) + a + 1 + 3 + b;
+      const int64_t a = (int64_t)oz_plan_[0].launches().size(), b = (int64_t)oz_plan_[1].launches().size();
+      launches += (rotG_.n ? 1 : 0) + a + 1 + 3 + b;  // 1: the tau mirror of P0
     } else
     launches += (rotG_.n ? 1 : 0) + p0 + 3 + sg;
   }
@@ -2952,7 +2156,7 @@ static int on_handle(gwgb_handle h, F &&f) {
 extern "C" {
 
 const char *gwgb_version(void) {
-  return "gwgb 0.5 (sm_103a; FP64, sliced BF16 (Ozaki), TF32x3 and BF16x3 contraction paths)";
+  return "gwgb 0.5 (sm_103a; FP64, sliced FP16 (Ozaki), TF32x3 and BF16x3 contraction paths)";
 }
 
 const char *gwgb_last_error(void) { return gwgb::g_last_error.c_str(); }

@@ -1,40 +1,28 @@
-// Error-free sliced complex GEMMs on tcgen05 for the P0 and Sigma stages.
+// Sliced complex GEMMs on tcgen05 for the P0 and Sigma stages.
 //
 // Why: a TF32/BF16 split with FP32 accumulation carries about 24 bits, and the
 // GW contractions sum many terms of both signs, so their error stays near
 // 1e-6 relative -- far from 1e-7 Ha absolute on Sigma.  Here each operand row
-// is cut, per round of OZ_KR complex K, into four BF16 slices of a fixed-point
-// representation (the Ozaki scheme: Ozaki, Ogita, Oishi, Rump, Numer. Algor.
-// 59 (2012) 95-118; Ootomo, Ozaki, Yokota, IJHPCA 2024):
-//   x = 2^(E-7) (s0 + s1 2^-8 + s2 2^-16 + s3 2^-24) + O(2^(E-32)),
-//   E: the row's exponent (|x| < 2^E), s_i integers with |s_i| <= 129,
-// stored as BF16 values s_i 2^(-8 i) (exact: 8 significant bits).  The
-// product of two such rows is a sum of slice products whose class c = i + j
-// carries weight 2^(-8 c); the classes 0 to 3 are computed (10 MMAs per K
-// step) into three TMEM accumulators:
-//   D0 = class 0 (s0 t0: integers <= 2^14 per term, a round's sum < 2^20),
-//   D1 = class 1 (integer multiples of 2^-8 below 2^13 per term),
-//   D2 = classes 2 and 3 (below 2^-2 per term),
-// so D0 and D1 are exact in FP32 and D2's rounding lies near 2^-40 of the
-// row-by-column scale.  Dropped terms (classes 4 to 6) and the slice
-// remainder are below 2^-30 of that scale.  After every round the three
-// accumulators are combined, scaled by 2^(Ea + Eb - 14) (exact) and added to
-// a float-float accumulator (two FP32 numbers, about 48 bits) in registers.
-// No FP64 arithmetic runs in the GEMM except the final conversion of
-// FP64-valued outputs.  Complex products use the real embedding
-//   A = [Ar Ai] (K interleaved), B rows (n, 0) = [Br -Bi], (n, 1) = [Bi Br],
-// so C[r][(n,0)] = Re, C[r][(n,1)] = Im of sum_k A[r][k] B[n][k].
-//
-// Kernel structure: persistent, two CTAs per SM (80 KB shared memory and 256
-// TMEM columns each), 128 threads; tasks in list order with a grid stride.
-// Per round every thread stages one A row (max, exponent, slices: K-major
-// no-swizzle core-matrix layout), four threads stage one complex B row (two
-// real rows), one thread issues the 20 MMAs and commits to an mbarrier, all
-// threads wait (bounded) and drain their TMEM lane.  The other CTA on the SM
-// overlaps its staging and drain with these MMAs.
-#include "common.h"
+// is held, per round of at most 32 complex K, as three FP16 slices of its value
+// relative to the row's exponent E (|x| < 2^E) (the Ozaki scheme: Ozaki, Ogita,
+// Oishi, Rump, Numer. Algor. 59 (2012) 95-118; Mukunoki, Ozaki, Ogita, Imamura,
+// ISC 2020 for FP16 tensor cores):
+//   x 2^(15-E) = s0 + s1 + s2,  s0 a multiple of 2^6 (|s0| <= 2^15),
+//   s1 a multiple of 2^(5-b) (|s1| <= 2^5), s2 the rest rounded to FP16,
+// b = 9 bits for rounds of 3 or 4 octets of K, 10 for 2, 11 for 1.  The
+// remainder is below 2^(E-32) and 2^(E-33) rms (s2 floats).  The products
+// (i, j) with i + j <= 3 (8 MMAs per K step) go to four TMEM accumulators:
+//   (0, 0): multiples of 2^12, at most 2^30 each: a round of 64 real terms stays
+//           within 24 bits, so FP32 accumulation is exact;
+//   (0, 1) and (1, 0), one each: 9 + b bits per term and the round's 6, 5 or 4: exact;
+//   the rest: weight 2^-19 and less; its FP32 rounding lies near 2^-41.
+// Dropped: s2 t2, below 2^-37 of the row-by-column scale.  Complex products use
+// the real embedding A = [Ar Ai] (K interleaved), B rows (n, 0) = [Br -Bi],
+// (n, 1) = [Bi Br], so D[r][(n,0)] = Re, D[r][(n,1)] = Im of sum_k A[r][k] B[n][k].
 #include "kernels_oz.h"
-#include <cuda_bf16.h>
+
+#include <algorithm>
+#include <cuda_fp16.h>
 
 #include "tc_common.cuh"
 
@@ -42,13 +30,7 @@ namespace gwgb {
 
 namespace {
 
-constexpr int OZ_NR = 2 * OZ_NC;            // real columns (rows of the real-embedded B)
-constexpr int OZ_KP = 2 * OZ_KR;            // real K per round (BF16 elements per operand row)
-constexpr int OZ_SBO = (OZ_KP / 8) * 128;   // bytes between 8-row groups of core matrices
-constexpr int OZ_PA = OZ_M * OZ_KP * 2;     // bytes of one A slice plane
-constexpr int OZ_PB = OZ_NR * OZ_KP * 2;    // bytes of one B slice plane
-constexpr int OZ_EMIN = -100, OZ_EMAX = 100;
-static_assert(OZ_KP % 16 == 0, "a round is a whole number of BF16 MMA K steps");
+constexpr int OZ_EMIN = -100, OZ_EMAX = 128;
 
 // E with |x| < 2^E for every |x| <= m (m >= 0), clamped to [OZ_EMIN, OZ_EMAX].
 __device__ __forceinline__ int oz_exponent(float m) {
@@ -57,547 +39,668 @@ __device__ __forceinline__ int oz_exponent(float m) {
   return e > OZ_EMAX ? OZ_EMAX : e;
 }
 
-// 2^e as a float for e in [-126, 127]; 0 below (the term underflows).
-__device__ __forceinline__ float oz_pow2(int e) {
-  if (e < -126) return 0.f;
-  return __uint_as_float((uint32_t)(e > 127 ? 254 : e + 127) << 23);
-}
+// 2^e for e in [-126, 127].
+__device__ __forceinline__ float oz_pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
 
-// Four fixed-point slices of x = hi + lo in units of 2^(E-7) (f = 2^(7-E)),
-// returned with their weights: s0, s1 2^-8, s2 2^-16, s3 2^-24.
-__device__ __forceinline__ void oz_slice(float hi, float lo, float f, float (&s)[4]) {
-  const float h = hi * f, l = lo * f;  // exact scalings
-  const float s0 = rintf(h);
-  const float r = h - s0;              // exact, |r| <= 1/2
-  const float rh = r + l;              // two-sum of r and l
-  const float bb = rh - r;
-  const float rl = (r - (rh - bb)) + (l - bb);
-  const float t1 = rh * 256.f;
-  const float s1 = rintf(t1);
-  const float t2 = ((t1 - s1) + rl * 256.f) * 256.f;
-  const float s2 = rintf(t2);
-  const float s3 = rintf((t2 - s2) * 256.f);
-  s[0] = s0;
-  s[1] = s1 * 0x1p-8f;
-  s[2] = s2 * 0x1p-16f;
-  s[3] = s3 * 0x1p-24f;
-}
-
-__device__ __forceinline__ uint32_t bf2(float lo_elem, float hi_elem) {
-  return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(lo_elem)) |
-         ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi_elem)) << 16);
-}
-
+// s = fl(a + b), e = a + b - s.
 __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
   s = a + b;
   const float bb = s - a;
   e = (a - (s - bb)) + (b - bb);
 }
 
-// (h, l) += (vh, vl), float-float addition.
-__device__ __forceinline__ void ff_add(float &h, float &l, float vh, float vl) {
-  float s, e;
-  two_sum(h, vh, s, e);
-  e += l + vl;
-  h = s + e;
-  l = e - (h - s);
+// The three slices of h + l (v = fl(h + l), f = 2^(15-E)); adding and subtracting 1.5 2^(23+g) rounds
+// to multiples of 2^g, and h f - s0 is exact.
+__device__ __forceinline__ void oz_slice(float h, float l, float v, float f, float m1, float (&s)[3]) {
+  constexpr float M0 = 1.5f * 536870912.f;  // 1.5 2^29
+  s[0] = fmaf(v, f, M0) - M0;
+  const float t = fmaf(l, f, fmaf(h, f, -s[0]));
+  s[1] = (t + m1) - m1;
+  s[2] = t - s[1];
 }
 
-// Byte offset of the 16-byte row segment (8 BF16 elements from real column k8,
-// a multiple of 8) of row r in a K-major no-swizzle tile.
-__device__ __forceinline__ uint32_t seg_off(int r, int k8) {
-  return (uint32_t)((r >> 3) * OZ_SBO + (k8 >> 3) * 128 + (r & 7) * 16);
+// The rounding constant of s1 for an image of nks octets of K.
+__device__ __forceinline__ float oz_m1(int nks) {
+  return nks == 1 ? 1.5f * 131072.f : nks == 2 ? 1.5f * 262144.f : 1.5f * 524288.f;  // 1.5 2^(28-b)
 }
 
-// Offset of local row r of a row map (d == 0: from the row table).
-__device__ __forceinline__ int64_t row_off(const OzRows &m, int r, const int64_t *__restrict__ rowtab) {
-  if (m.d == 0) return __ldg(rowtab + m.base + r);
-  if (m.d == 1) return m.base + (int64_t)r * m.s1;
-  return m.base + (int64_t)(r / m.d) * m.s1 + (int64_t)(r % m.d) * m.s0;
+__device__ __forceinline__ uint32_t h2(float a, float b) {
+  const __half2 v = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t *>(&v);
 }
 
-// 32 lanes x 8 consecutive 32-bit columns from registers into TMEM (this warp's lane quarter).
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr),
-               "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
-               "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
-               "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+// One 32-byte sector (an octet of one row and plane), its 16-byte halves
+// swapped in rows 4-7 of every 8 (the 32-byte swizzle).
+__device__ __forceinline__ void st_octet(char *p, const uint32_t (&w)[8], bool swap) {
+  uint32_t v[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = swap ? w[j ^ 4] : w[j];
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
 }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-constexpr int OZ_THREADS = 512;         // warps 0-7 drain (TMEM lanes), 8-15 stage; lane 0 of warp 8 issues MMAs
-constexpr int OZ_ACC = 3 * OZ_NR;       // TMEM columns of one accumulator set D0 | D1 | D2
-constexpr int OZ_TMEM_WS = 512;         // two accumulator sets, then the float-float sums (hi | lo)
-constexpr int OZ_SUM = 2 * OZ_ACC;      // TMEM column of the running sums of multi-round GEMMs
-constexpr int OZ_BUF = 4 * OZ_PA + 4 * OZ_PB;
-constexpr int OZ_SMEM_WS = 120 * 1024;  // two tile buffers (96 KB); more than half an SM: one CTA per SM
-static_assert(2 * OZ_BUF + 1024 <= OZ_SMEM_WS, "two tile buffers must fit the requested shared memory");
-static_assert(2 * OZ_ACC + 2 * OZ_NR <= OZ_TMEM_WS, "two accumulator sets and the sums must fit the TMEM allocation");
-
-// Combined, scaled value of one accumulator column: (D0 + D1 + D2) * sc as a
-// float-float pair (D0, D1 exact; D2 small).
-__device__ __forceinline__ void oz_combine(float x0, float x1, float x2, float sc, float &h, float &l) {
-  float vh, vl;
-  two_sum(x0, x1, vh, vl);
-  vl += x2;
-  h = vh + vl;
-  l = (vl - (h - vh)) * sc;
-  h *= sc;
+// K-major operand in the 32-byte swizzle: rows of 32 bytes, 8-row groups 256 bytes apart.
+__device__ __forceinline__ uint64_t sw32_desc(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
+  d |= (uint64_t)1 << 16;            // leading dimension: unused, K is one atom wide
+  d |= (uint64_t)(256 >> 4) << 32;   // stride between 8-row groups
+  d |= (uint64_t)1 << 46;            // descriptor version of the sm_100 family
+  d |= (uint64_t)6 << 61;            // SWIZZLE_32B
+  return d;
+}
+// D = F32, A = B = F16, both K-major.
+__device__ __forceinline__ uint32_t idesc_f16(int N) {
+  return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(OZ_M >> 4) << 24);
 }
 
-__device__ __forceinline__ void oz_store(void *Cg, int64_t o, bool f64, double alpha, float rh, float ih, float rl,
-                                         float il) {
-  if (f64)
-    reinterpret_cast<double2 *>(Cg)[o] =
-        make_double2(alpha * ((double)rh + (double)rl), alpha * ((double)ih + (double)il));
-  else
-    reinterpret_cast<float4 *>(Cg)[o] = make_float4(rh, ih, rl, il);
+// 32 lanes x 8 consecutive 32-bit columns; the caller waits (tmem_wait_ld) before use.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void bulk_load(uint32_t dst, const char *src, uint32_t bytes, uint64_t *mbar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(tc::smem_u32(mbar))
+               : "memory");
+}
+__device__ __forceinline__ void expect_tx(uint64_t *mbar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(mbar)), "r"(bytes)
+               : "memory");
 }
 
-// Persistent warp-specialised sliced GEMM.  Every role walks the same work
-// sequence (tasks of this CTA with a grid stride, repetitions, rounds of
-// OZ_KR complex K), counting rounds i.  Rings: 2 shared tile buffers
-// (full / empty), 2 TMEM accumulator sets (done / afree), 4 exponent slots
-// (eready / efree).  Every wait is bounded; a wait that runs out sets the error
-// word and an abort flag that ends every role's loop, and TMEM is released only
-// after the MMAs issued so far have completed (bounded wait on `last`).
-__global__ void __launch_bounds__(OZ_THREADS, 1)
-    oz_gemm_kernel(const OzDesc *__restrict__ descs, const OzTask *__restrict__ tasks, int ntasks,
-                   const float4 *__restrict__ Ag, const float4 *__restrict__ Bg, void *__restrict__ Cg,
-                   const int64_t *__restrict__ rowtab, int *__restrict__ err) {
+// The sequence of rounds of one task: `outer` row tiles of R rounds (stages 1
+// and 2, the column operand held over the row tiles), or R rounds (stage 3).
+template <int NS, int STAGE> struct Job {
+  static constexpr int OCT = OzCfg<NS>::OCT;
+  int outer, R, noct, kos;
+  int G;                 // row tiles per accumulator set
+  const char *a, *b;
+  int64_t atile;
+  const OzRnd *rt;
+  __device__ __forceinline__ void init(const OzArgs &g, const OzTask &t) {
+    rt = nullptr;
+    if constexpr (STAGE == 0) {
+      const OzS1 d = static_cast<const OzS1 *>(g.desc)[t.d];
+      const OzCol1 c = static_cast<const OzCol1 *>(g.aux1)[t.i];
+      kos = d.kos;
+      R = (kos + OCT - 1) / OCT;
+      outer = t.n;
+      noct = c.ngrp * c.gs;
+      atile = (int64_t)NS * kos * 4096 + 512 * R;
+      a = g.A + d.a + t.m0 * atile;
+      b = g.B + c.b;
+    } else if constexpr (STAGE == 1) {
+      const OzS2 d = static_cast<const OzS2 *>(g.desc)[t.d];
+      const int tau = t.i & 0xffff, zt = t.i >> 16;
+      kos = d.kos;
+      R = (kos + OCT - 1) / OCT;
+      outer = t.n;
+      noct = min(OCT, d.zos - zt * OCT);
+      atile = d.t2bytes;
+      a = g.A + d.a + ((int64_t)tau * d.nt2 + t.m0) * atile;
+      b = g.B + d.b + tau * d.bt + zt * d.bz;
+    } else {
+      const OzS3 d = static_cast<const OzS3 *>(g.desc)[t.d];
+      const int f = t.i & 0xffff, ct = t.i >> 16;
+      kos = 0;
+      R = d.nkr;
+      outer = t.n;
+      noct = min(OCT, (d.N + 7) / 8 - ct * OCT);
+      atile = d.fbytes;
+      a = g.A + d.a + f * d.fbytes;
+      b = g.B + d.b + ct * d.bz;
+      rt = static_cast<const OzRnd *>(g.aux1) + d.rt;
+    }
+    G = STAGE == 0 ? 1 : OCT / noct;
+  }
+  __device__ __forceinline__ int nks(int r) const { return STAGE == 2 ? rt[r].nks : min(OCT, kos - r * OCT); }
+  __device__ __forceinline__ const char *aptr(int m, int r) const {
+    return a + m * atile + (STAGE == 2 ? (int64_t)rt[r].a16 * 16 : r * oz_abytes(NS, OCT));
+  }
+  __device__ __forceinline__ const char *bptr(int r) const {
+    return b + noct * (STAGE == 2 ? (int64_t)rt[r].b16 * 16 : r * oz_bbytes1(NS, OCT));
+  }
+};
+
+constexpr int OZ_RING = 16;             // largest operand ring (K steps)
+constexpr int OZ_SC = 32;               // scale rings: deeper than the operand rings plus the accumulator sets
+constexpr int OZ_SMEM = 200 * 1024;
+constexpr int OZ_THREADS = 320;         // warps 0-7 drain, warp 8 copies, warp 9 issues the MMAs
+
+// One lane of a converged warp.  The copy and MMA loops are warp-uniform and
+// elect a lane only around the instruction itself: their descriptors then stay in
+// uniform registers.  In a one-lane branch every MMA took 161 cycles to issue,
+// whatever its N; this way the N = 64 MMA takes 48, its operand reads.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred P;\nelect.sync _|P, 0xffffffff;\nselp.b32 %0, 1, 0, P;\n}\n" : "=r"(p));
+  return p != 0;
+}
+
+// Ring position.
+struct Ring {
+  int slot = 0, phase = 0, n;
+  __device__ __forceinline__ explicit Ring(int n_) : n(n_) {}
+  __device__ __forceinline__ void next() {
+    if (++slot == n) {
+      slot = 0;
+      phase ^= 1;
+    }
+  }
+};
+
+// Persistent warp-specialised GEMM over operand images.  Bound: the drain's
+// CUDA-core work (about 40 FP32 instructions per complex output of stages 1
+// and 2) and the L2 / HBM traffic of the images; the operands need no CUDA-core
+// work at all, a K step (8 complex) is 8 MMAs, and two TMEM accumulator sets let
+// one round multiply while the other drains.  Operands stream through rings of
+// K steps (12 KB of A, at most 6 KB of B); stages 1 and 2 hold the column
+// operand of a task over its row tiles.  A column tile of one octet (two) fills
+// a quarter (half) of an accumulator set, so stages 2 and 3 put G = OCT / noct
+// row tiles into one.
+//
+// Every wait is bounded: a wait that runs out sets the error word and an abort
+// flag; the copy and MMA roles then leave, the drain warps walk on through
+// their work without waiting (their named barriers stay matched).  Copies and
+// MMAs in flight are waited for (bounded) before TMEM is released.
+template <int NS, int STAGE>
+__global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) {
+  constexpr int OCT = OzCfg<NS>::OCT, NACC = OzCfg<NS>::NACC, HO = OCT / 2;
+  constexpr int NR = 16 * OCT, SETC = NACC * NR;
+  constexpr uint32_t SA = NS * 4096, SB = NS * 512 * OCT;  // ring slots
+  static_assert(2 * SETC <= 512, "two accumulator sets must fit TMEM");
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint32_t tslot;
-  __shared__ __align__(8) uint64_t full[2], empty[2], done[2], afree[2], eready[4], efree[4], last;
-  __shared__ int ea_s[4][OZ_M], eb_s[4][OZ_NC];
-  __shared__ float amax[2][2][OZ_M];  // per tile buffer: partial row maxima of the two A halves
-  __shared__ __align__(8) uint64_t mx[2];
-  __shared__ int abort_flag, issued;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  if (warp == 0) tc::tmem_alloc(&tslot, OZ_TMEM_WS);
+  __shared__ __align__(8) uint64_t full[OZ_RING], emptyA[OZ_RING], emptyB[OZ_RING], done[2], tfree[2], last;
+  __shared__ __align__(16) float sA[OZ_SC][OZ_M], sB[OZ_SC][8 * OCT];
+  __shared__ float gmax[2][OCT][OZ_M];
+  __shared__ int abort_flag;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  if (warp == 0) tc::tmem_alloc(&tslot, 512);
   if (tid == 0) {
-    for (int j = 0; j < 2; ++j) {
-      tc::mbar_init(&full[j], 256);
-      tc::mbar_init(&empty[j], 1);
-      tc::mbar_init(&done[j], 1);
-      tc::mbar_init(&afree[j], 256);
+    for (int j = 0; j < OZ_RING; ++j) {
+      tc::mbar_init(&full[j], 1);
+      tc::mbar_init(&emptyA[j], 1);
+      tc::mbar_init(&emptyB[j], 1);
     }
-    for (int j = 0; j < 4; ++j) {
-      tc::mbar_init(&eready[j], 256);
-      tc::mbar_init(&efree[j], 256);
+    for (int j = 0; j < 2; ++j) {
+      tc::mbar_init(&done[j], 1);
+      tc::mbar_init(&tfree[j], 8);
     }
     tc::mbar_init(&last, 1);
-    tc::mbar_init(&mx[0], 256);
-    tc::mbar_init(&mx[1], 256);
     abort_flag = 0;
-    issued = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tm = tslot;
-  // bounded wait; false when it ran out (error word and abort flag set) or another role aborted.
-  // Each poll may suspend the thread for up to 20 us (hint) until the phase completes, so
-  // waiting roles do not take issue slots from the working ones; 2^16 polls bound the wait.
+  const uint32_t tm = __shfl_sync(0xffffffffu, tslot, 0);
+  // Bounded wait of a converged warp; false (in every lane) when it ran out (error word and abort
+  // flag set) or another role aborted.  Each poll may suspend for up to 20 us (hint).
   auto bwait = [&](uint64_t *b, uint32_t par) -> bool {
-    for (int rep = 0; rep < 256; ++rep) {
-      for (int it = 0; it < 256; ++it) {
+    bool hit = false;
+    for (int rep = 0; rep < 256 && !hit; ++rep) {
+      for (int it = 0; it < 256 && !hit; ++it) {
         uint32_t ok;
         asm volatile(
             "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.b32 %0, 1, 0, p;\n}\n"
             : "=r"(ok)
             : "r"(tc::smem_u32(b)), "r"(par), "r"(20000u)
             : "memory");
-        if (ok) return true;
+        hit = ok != 0;
       }
-      if (*(volatile int *)&abort_flag) return false;
+      if (!hit && *(volatile int *)&abort_flag) break;
+      if (!hit && rep == 255) {
+        atomicExch(g.err, 1);
+        *(volatile int *)&abort_flag = 1;
+      }
     }
-    atomicExch(err, 1);
-    *(volatile int *)&abort_flag = 1;
-    return false;
+    return __all_sync(0xffffffffu, hit);
   };
-  auto aborted = [&]() { return *(volatile int *)&abort_flag != 0; };
-  // Every stop decision is taken by the whole warp (the tcgen05 loads, the
-  // shuffles and the warp barrier of the staging loop need all 32 lanes): a
-  // warp stops when any lane saw the abort flag or a wait that ran out.  Each
-  // lane's wait is bounded, so the votes end, and a timed-out wait can never
-  // leave part of a warp waiting for lanes that left the loop.
-  auto warp_aborted = [&]() { return __any_sync(0xffffffffu, aborted()); };
-  auto warp_ok = [&](bool ok) { return __all_sync(0xffffffffu, ok); };
+  const uint32_t smA = tc::smem_u32(smem), smB = smA + (uint32_t)g.nA * SA;
 
-  if (warp >= 8) {
-    // ------------------------------ producers (and the MMA issuer) ------------------------------
-    // A: two threads per row (h = K half); B: eight threads per complex row (two complex K each).
-    const int pt = tid - 256;
-    const int ar = pt & 127, ah = pt >> 7;
-    const int bn = pt >> 3, bq = pt & 7;
-    int i = 0, nissued = 0;
-    bool stop = false;
-    for (int ti = blockIdx.x; ti < ntasks && !stop; ti += gridDim.x) {
-      const OzTask tk = tasks[ti];
-      const OzDesc dg = descs[tk.desc];
-      const int mt = tk.mtnt >> 16, nt = tk.mtnt & 0xffff;
-      const int Mt = min(OZ_M, dg.M - mt * OZ_M), Nt = min(OZ_NC, dg.N - nt * OZ_NC);
-      const int ngrp = (Nt + 7) >> 3;
-      const bool rv = ar < Mt, bv = bn < Nt, bw = bn < 8 * ngrp;
-      const int64_t arow0 = rv ? row_off(dg.a, mt * OZ_M + ar, rowtab) : 0;
-      const int64_t brow0 = bv ? row_off(dg.b, nt * OZ_NC + bn, rowtab) : 0;
-      const bool ca = dg.flags & OZ_CONJ_A, cb = dg.flags & OZ_CONJ_B;
-      for (int rr = 0; rr < tk.nrep && !stop; ++rr) {
-        const int rep = tk.rep0 + rr;
-        const float4 *arow = Ag + arow0 + (int64_t)rep * dg.ra;
-        const float4 *brow = Bg + brow0 + (int64_t)rep * dg.rb;
-        for (int k0 = 0; k0 < dg.K; k0 += OZ_KR, ++i) {
-          if (warp_aborted()) { stop = true; break; }
-          const int b = i & 1, e = i & 3;
-          if (i >= 2 && !warp_ok(bwait(&empty[b], ((i >> 1) - 1) & 1))) { stop = true; break; }
-          if (i >= 4 && !warp_ok(bwait(&efree[e], ((i >> 2) - 1) & 1))) { stop = true; break; }
-          const int kn = min(OZ_KR, dg.K - k0);
-          const int nks = (kn + 7) >> 3;  // MMA K steps this round (8 complex each)
-          const int kw = 4 * nks;         // complex K per thread of an A row (4 or 8)
-          unsigned char *As = smem + b * OZ_BUF, *Bs = As + 4 * OZ_PA;
-          {  // A: this thread's half [kw h, kw h + kw) of row ar; exponent from both halves
-            float4 v[8];
-            float m = 0.f;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const int kk = kw * ah + k;
-              v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-              if (rv && k < kw && kk < kn) v[k] = __ldg(arow + (int64_t)(k0 + kk) * dg.aks);
-              m = fmaxf(m, fmaxf(fabsf(v[k].x), fabsf(v[k].y)));
-            }
-            amax[b][ah][ar] = m;
-            tc::mbar_arrive(&mx[b]);  // both halves' maxima posted (bounded wait, no named barrier)
-            if (!warp_ok(bwait(&mx[b], (i >> 1) & 1))) { stop = true; break; }
-            const int ea = oz_exponent(fmaxf(amax[b][0][ar], amax[b][1][ar]));
-            const float f = oz_pow2(7 - ea);
-#pragma unroll
-            for (int g = 0; g < 2; ++g) {  // segments of 4 complex (8 reals per plane)
-              if (4 * g < kw) {
-                uint32_t w[4][4];
-                if (rv) {
-#pragma unroll
-                  for (int j = 0; j < 4; ++j) {
-                    float4 x = v[g * 4 + j];
-                    if (ca) { x.y = -x.y; x.w = -x.w; }
-                    float sr[4], si[4];
-                    oz_slice(x.x, x.z, f, sr);
-                    oz_slice(x.y, x.w, f, si);
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) w[p][j] = bf2(sr[p], si[p]);
-                  }
-                } else {
-#pragma unroll
-                  for (int p = 0; p < 4; ++p) w[p][0] = w[p][1] = w[p][2] = w[p][3] = 0u;
+  if (warp == 8) {
+    // ------------------------------ copies ------------------------------
+    Ring ra(g.nA), rb(g.nB);
+    int ia = 0, ib = 0, ra_rounds = 0, rb_rounds = 0;  // K steps and rounds copied
+    bool ok = true;
+    for (int ti = blockIdx.x; ti < g.ntasks && ok; ti += gridDim.x) {
+      Job<NS, STAGE> job;
+      job.init(g, g.tasks[ti]);
+      const uint32_t bb = (uint32_t)(job.noct * NS * 512), sb = (uint32_t)(32 * job.noct);
+      for (int m0 = 0; m0 < job.outer && ok; m0 += job.G) {
+        const int Gm = min(job.G, job.outer - m0);
+        for (int r = 0; r < job.R && ok; ++r) {
+          const int nks = job.nks(r);
+          for (int gi = 0; gi < Gm && ok; ++gi) {
+            const bool nb = gi == 0 && (STAGE == 2 || m0 == 0);
+            const char *ap = job.aptr(m0 + gi, r), *bp = job.bptr(r);
+            for (int ks = 0; ks < nks; ++ks) {
+              if (ia >= g.nA && !bwait(&emptyA[ra.slot], ra.phase ^ 1)) { ok = false; break; }
+              if (nb && ib >= g.nB && !bwait(&emptyB[rb.slot], rb.phase ^ 1)) { ok = false; break; }
+              uint64_t *f = &full[ra.slot];
+              if (elect_one()) {
+                expect_tx(f, SA + (ks == 0 ? 512u : 0u) + (nb ? bb + (ks == 0 ? sb : 0u) : 0u));
+                bulk_load(smA + ra.slot * SA, ap + ks * SA, SA, f);
+                if (ks == 0) bulk_load(tc::smem_u32(sA[ra_rounds & (OZ_SC - 1)]), ap + nks * SA, 512, f);
+                if (nb) {
+                  bulk_load(smB + rb.slot * SB, bp + ks * bb, bb, f);
+                  if (ks == 0) bulk_load(tc::smem_u32(sB[rb_rounds & (OZ_SC - 1)]), bp + nks * bb, sb, f);
                 }
-                const uint32_t o = seg_off(ar, 8 * (kw * ah / 4 + g));
-#pragma unroll
-                for (int p = 0; p < 4; ++p)
-                  *reinterpret_cast<uint4 *>(As + p * OZ_PA + o) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
               }
+              __syncwarp();
+              if (nb) {
+                rb.next();
+                ++ib;
+              }
+              ra.next();
+              ++ia;
             }
-            if (ah == 0) ea_s[e][ar] = ea;
+            ++ra_rounds;
+            if (nb) ++rb_rounds;
           }
-          {  // B: rows (n,0) = [Br -Bi], (n,1) = [Bi Br]; complex K [2 bq, 2 bq + 2) of row bn
-            float4 v[2];
-            float mb = 0.f;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              const int k = 2 * bq + j;
-              v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-              if (bv && k < kn) v[j] = __ldg(brow + (int64_t)(k0 + k) * dg.bks);
-              if (cb) { v[j].y = -v[j].y; v[j].w = -v[j].w; }
-              mb = fmaxf(mb, fmaxf(fabsf(v[j].x), fabsf(v[j].y)));
-            }
-            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 1));
-            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 2));
-            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 4));
-            const int eb = oz_exponent(mb);
-            if (bq == 0) eb_s[e][bn] = eb;
-            if (bw && 2 * bq < 8 * nks) {
-              uint32_t w0[4][2], w1[4][2];
-              if (bv) {
-                const float f = oz_pow2(7 - eb);
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                  float sr[4], si[4];
-                  oz_slice(v[j].x, v[j].z, f, sr);
-                  oz_slice(v[j].y, v[j].w, f, si);
-#pragma unroll
-                  for (int p = 0; p < 4; ++p) {
-                    w0[p][j] = bf2(sr[p], -si[p]);
-                    w1[p][j] = bf2(si[p], sr[p]);
-                  }
-                }
-              } else {
-#pragma unroll
-                for (int p = 0; p < 4; ++p) w0[p][0] = w0[p][1] = w1[p][0] = w1[p][1] = 0u;
-              }
-              // 8-byte halves of the 16-byte core-matrix row segments of complex K [4 (bq/2), +4)
-              const uint32_t o0 = seg_off(2 * bn, 8 * (bq >> 1)) + 8 * (bq & 1);
-              const uint32_t o1 = seg_off(2 * bn + 1, 8 * (bq >> 1)) + 8 * (bq & 1);
-#pragma unroll
-              for (int p = 0; p < 4; ++p) {
-                *reinterpret_cast<uint2 *>(Bs + p * OZ_PB + o0) = make_uint2(w0[p][0], w0[p][1]);
-                *reinterpret_cast<uint2 *>(Bs + p * OZ_PB + o1) = make_uint2(w1[p][0], w1[p][1]);
-              }
-            }
-          }
-          tc::fence_async_smem();
-          tc::mbar_arrive(&eready[e]);
-          tc::mbar_arrive(&full[b]);
-          if (pt == 0) {  // MMA issue for this round once all producers have staged it
-            const int a = i & 1;
-            bool ok = bwait(&full[b], (i >> 1) & 1);
-            if (ok && i >= 2) ok = bwait(&afree[a], ((i >> 1) - 1) & 1);
-            if (ok) {
+        }
+      }
+    }
+    // every copy issued has landed before the CTA may end
+    Ring rw(g.nA);
+    const int first = max(0, ia - g.nA);
+    for (int q = 0; q < ia; ++q) {
+      if (q >= first) tc::mbar_wait(&full[rw.slot], rw.phase, 4000000);
+      rw.next();
+    }
+  } else if (warp == 9) {
+    // ------------------------------ MMAs ------------------------------
+    Ring ra(g.nA), rb(g.nB);
+    int n = 0;  // accumulator sets filled
+    bool ok = true;
+    for (int ti = blockIdx.x; ti < g.ntasks && ok; ti += gridDim.x) {
+      Job<NS, STAGE> job;
+      job.init(g, g.tasks[ti]);
+      const int noct = __shfl_sync(0xffffffffu, job.noct, 0);
+      const uint32_t id = idesc_f16(16 * noct);
+      const uint32_t bstep = 512u * noct;
+      const Ring r0 = rb;
+      for (int m0 = 0; m0 < job.outer && ok; m0 += job.G) {
+        const int Gm = min(job.G, job.outer - m0);
+        const bool lastm = STAGE == 2 || m0 + job.G >= job.outer;
+        if (STAGE != 2) rb = r0;
+        for (int r = 0; r < job.R && ok; ++r, ++n) {
+          const int set = n & 1, nks = __shfl_sync(0xffffffffu, job.nks(r), 0);
+          if (n >= 2 && !bwait(&tfree[set], ((n >> 1) - 1) & 1)) { ok = false; break; }
+          const Ring rr = rb;
+          for (int gi = 0; gi < Gm && ok; ++gi) {
+            rb = rr;
+            const uint32_t d0 = tm + (uint32_t)(set * SETC + gi * 16 * noct);
+            for (int ks = 0; ks < nks; ++ks) {
+              if (!bwait(&full[ra.slot], ra.phase)) { ok = false; break; }
               tc::fence_after_sync();
-              const uint32_t id = tc::idesc_bf16(OZ_M, 16 * ngrp);
-              const uint32_t a0 = tc::smem_u32(As), b0 = a0 + 4 * OZ_PA;
-              const uint32_t d0 = tm + (uint32_t)(a * OZ_ACC), d1 = d0 + OZ_NR, d2 = d0 + 2 * OZ_NR;
-              for (int ks = 0; ks < nks; ++ks) {
-                auto da = [&](int p) { return tc::make_desc(a0 + p * OZ_PA + ks * 256, 128, OZ_SBO); };
-                auto db = [&](int p) { return tc::make_desc(b0 + p * OZ_PB + ks * 256, 128, OZ_SBO); };
-                const uint32_t acc = ks > 0 ? 1u : 0u;
-                tc::mma_bf16(d0, da(0), db(0), id, acc);
-                tc::mma_bf16(d1, da(0), db(1), id, acc);
-                tc::mma_bf16(d1, da(1), db(0), id, 1u);
-                tc::mma_bf16(d2, da(0), db(2), id, acc);
-                tc::mma_bf16(d2, da(1), db(1), id, 1u);
-                tc::mma_bf16(d2, da(2), db(0), id, 1u);
-                tc::mma_bf16(d2, da(0), db(3), id, 1u);
-                tc::mma_bf16(d2, da(1), db(2), id, 1u);
-                tc::mma_bf16(d2, da(2), db(1), id, 1u);
-                tc::mma_bf16(d2, da(3), db(0), id, 1u);
+              const uint32_t a0 = smA + ra.slot * SA, b0 = smB + rb.slot * SB;
+              const uint32_t more = ks > 0 ? 1u : 0u;
+              if (elect_one()) {
+#pragma unroll
+                for (int c = 0; c <= OzCfg<NS>::CMAX; ++c)
+#pragma unroll
+                  for (int p = 0; p < NS; ++p) {
+                    const int q = c - p;
+                    if (q < 0 || q >= NS) continue;
+                    // (0,0) | (0,1) | (1,0) | the rest
+                    const int acc = c == 0 ? 0 : c == 1 ? 1 + p : 3;
+                    const bool fresh = c < 2 || (c == 2 && p == 0);
+                    tc::mma_bf16(d0 + acc * NR, sw32_desc(a0 + p * 4096u), sw32_desc(b0 + q * bstep), id,
+                                 fresh ? more : 1u);  // kind::f16, types from the descriptor
+                  }
+                tc::commit(&emptyA[ra.slot]);
+                if (lastm && gi == Gm - 1) tc::commit(&emptyB[rb.slot]);
               }
-              tc::commit(&empty[b]);
-              tc::commit(&done[a]);
-              ++nissued;
+              __syncwarp();
+              ra.next();
+              rb.next();
             }
           }
+          if (!ok) break;
+          if (elect_one()) tc::commit(&done[set]);
           __syncwarp();
         }
       }
     }
-    if (pt == 0) {
-      if (nissued > 0) tc::commit(&last);  // arrives when every MMA issued above has completed
-      issued = nissued;
-    }
+    if (elect_one()) tc::commit(&last);  // arrives when every MMA issued above has completed
+    __syncwarp();
   } else {
     // ------------------------------ drain ------------------------------
-    // warp w: TMEM lanes (rows) 32 (w & 3) .. + 31, complex columns [16 (w >> 2), + 16)
-    const int r = 32 * (warp & 3) + (tid & 31), ch = warp >> 2;
-    const uint32_t tlane = tm + ((uint32_t)(32 * (warp & 3)) << 16);
-    const uint32_t sum_h = tlane + OZ_SUM, sum_l = sum_h + OZ_NR;
-    int i = 0;
-    bool stop = false;
-    for (int ti = blockIdx.x; ti < ntasks && !stop; ti += gridDim.x) {
-      const OzTask tk = tasks[ti];
-      const OzDesc dg = descs[tk.desc];
-      const int mt = tk.mtnt >> 16, nt = tk.mtnt & 0xffff;
-      const int Mt = min(OZ_M, dg.M - mt * OZ_M), Nt = min(OZ_NC, dg.N - nt * OZ_NC);
-      const int ngrp = (Nt + 7) >> 3;
-      const bool rv = r < Mt, f64 = dg.flags & OZ_OUT_F64;
-      const int64_t crow0 = rv ? row_off(dg.c, mt * OZ_M + r, rowtab) : 0;
-      const int ng0 = nt * OZ_NC + 16 * ch;
-      const int nq0 = ng0 / dg.cnd, nr0 = ng0 - nq0 * dg.cnd;  // column ng0 = nq0 * cnd + nr0
-      for (int rr = 0; rr < tk.nrep && !stop; ++rr) {
-        const int64_t co = crow0 + (int64_t)(tk.rep0 + rr) * dg.rc;
-        for (int k0 = 0; k0 < dg.K; k0 += OZ_KR, ++i) {
-          if (warp_aborted()) { stop = true; break; }
-          const int a = i & 1, e = i & 3;
-          if (!warp_ok(bwait(&done[a], (i >> 1) & 1) && bwait(&eready[e], (i >> 2) & 1))) { stop = true; break; }
+    // warp w: TMEM lanes (rows) 32 (w & 3) .. + 31, octets HO (w >> 2) .. + HO - 1 of the set.
+    // The rows' destinations are read while the set still multiplies.
+    const int lq = warp & 3, half = warp >> 2, row = 32 * lq + lane;
+    const uint32_t tbase = tm + ((uint32_t)(32 * lq) << 16) + 16u * HO * half;
+    int n = 0, i0 = 0, j0 = 0, tile = 0;  // sets, row tiles and column images consumed
+    bool dead = false;
+    for (int ti = blockIdx.x; ti < g.ntasks; ti += gridDim.x) {
+      const OzTask tk = g.tasks[ti];
+      Job<NS, STAGE> job;
+      job.init(g, tk);
+      int gi[HO], oct[HO];  // row tile in the set, octet in the tile
+#pragma unroll
+      for (int q = 0; q < HO; ++q) {
+        gi[q] = (half * HO + q) / job.noct;
+        oct[q] = half * HO + q - gi[q] * job.noct;
+      }
+      // stage 1: the row and its destination
+      int rg = 0, M = 0, nL = 1, tau = 0, Lr = 0, dtau = 0, dL = 0, gs = 1, goff = 0, nLg = 1, glog = 0, nt2 = 1;
+      int64_t t2bytes = 0;
+      char *xbase = g.X;
+      // stage 2
+      const OzRow *rows = nullptr;
+      OzRow rw[HO];
+      int zos = 1;
+      if constexpr (STAGE == 0) {
+        const OzS1 d = static_cast<const OzS1 *>(g.desc)[tk.d];
+        const OzCol1 col = static_cast<const OzCol1 *>(g.aux1)[tk.i];
+        const OzDst1 d1 = static_cast<const OzDst1 *>(g.aux2)[col.dst];
+        M = d.M;
+        nL = d.nL;
+        gs = col.gs;
+        nLg = d1.nLg;
+        glog = d1.glog;
+        goff = d1.gbase + col.x0 * nLg;
+        nt2 = d1.nt2;
+        t2bytes = d1.t2bytes;
+        xbase += d1.base + col.yoff;
+        rg = tk.m0 * OZ_M + row;
+        tau = rg / nL;
+        Lr = rg - tau * nL;
+        dtau = OZ_M / nL;
+        dL = OZ_M - dtau * nL;
+      } else if constexpr (STAGE == 1) {
+        const OzS2 d = static_cast<const OzS2 *>(g.desc)[tk.d];
+        gs = job.noct;
+        glog = d.glog;
+        zos = d.zos;
+        tau = tk.i & 0xffff;
+        xbase += (tk.i >> 16) * oz_abytes(NS, OCT);
+        rows = static_cast<const OzRow *>(g.aux1) + d.rows + tk.m0 * OZ_M + row;
+#pragma unroll
+        for (int q = 0; q < HO; ++q) {
+          rw[q] = {-1, 0, 0};
+          if (gi[q] < min(job.G, job.outer)) rw[q] = rows[gi[q] * OZ_M];
+        }
+      }
+      for (int m0 = 0; m0 < job.outer; m0 += job.G, ++tile) {
+        const int Gm = min(job.G, job.outer - m0);
+        OzDst2 d2[HO];
+        OzRow rw1[HO];
+        if constexpr (STAGE == 1) {
+#pragma unroll
+          for (int q = 0; q < HO; ++q) {
+            if (rw[q].dst >= 0) d2[q] = static_cast<const OzDst2 *>(g.aux2)[rw[q].dst];
+            rw1[q] = {-1, 0, 0};
+            if (m0 + job.G + gi[q] < job.outer) rw1[q] = rows[(m0 + job.G + gi[q]) * OZ_M];
+          }
+        }
+        float H[HO][16], L[HO][16];  // value H + L of this thread's octets
+#pragma unroll
+        for (int q = 0; q < HO; ++q)
+#pragma unroll
+          for (int e = 0; e < 16; ++e) H[q][e] = L[q][e] = 0.f;
+        for (int r = 0; r < job.R; ++r, ++n, i0 += Gm) {
+          const int set = n & 1;
+          if (!dead) dead = !bwait(&done[set], (n >> 1) & 1);
+          if (dead) continue;
           tc::fence_after_sync();
-          const bool first = k0 == 0, lastr = k0 + OZ_KR >= dg.K;
-          const int ea = ea_s[e][r];
-          const uint32_t base = tlane + (uint32_t)(a * OZ_ACC);
-          int nq = nq0, nrr = nr0;  // output column cursor
+          const float *sbp = sB[(j0 + r) & (OZ_SC - 1)];
+          const uint32_t base = tbase + (uint32_t)(set * SETC);
 #pragma unroll
-          for (int gl = 0; gl < 4; ++gl) {  // this warp's groups of 8 real columns (4 complex)
-            const int g = 4 * ch + gl;
-            if (g < 2 * ngrp) {
-              float x0[8], x1[8], x2[8], sh[8], sl[8];
-              tc::tmem_ld8(base + (uint32_t)(8 * g), x0);
-              tc::tmem_ld8(base + (uint32_t)(OZ_NR + 8 * g), x1);
-              tc::tmem_ld8(base + (uint32_t)(2 * OZ_NR + 8 * g), x2);
-              if (!first) {
-                tc::tmem_ld8(sum_h + (uint32_t)(8 * g), sh);
-                tc::tmem_ld8(sum_l + (uint32_t)(8 * g), sl);
-              }
+          for (int q = 0; q < HO; ++q) {
+            if (gi[q] >= Gm) continue;
+            const float sa = sA[(i0 + gi[q]) & (OZ_SC - 1)][row];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const float sc = oz_pow2(ea + eb_s[e][4 * g + (j >> 1)] - 14);
-                float vh, vl;
-                oz_combine(x0[j], x1[j], x2[j], sc, vh, vl);
-                if (first) {
-                  sh[j] = vh;
-                  sl[j] = vl;
+            for (int hf = 0; hf < 2; ++hf) {
+              uint32_t x0[8], x1[8], x2[8], x3[8];
+              tmem_ld8(base + 16 * q + 8 * hf, x0);
+              tmem_ld8(base + NR + 16 * q + 8 * hf, x1);
+              tmem_ld8(base + 2 * NR + 16 * q + 8 * hf, x2);
+              tmem_ld8(base + 3 * NR + 16 * q + 8 * hf, x3);
+              const float4 sb4 = *reinterpret_cast<const float4 *>(sbp + 8 * oct[q] + 4 * hf);
+              const float sb[4] = {sb4.x, sb4.y, sb4.z, sb4.w};
+              tmem_wait_ld();
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                const float sc = sa * sb[e >> 1];
+                const float lo = (__uint_as_float(x1[e]) + __uint_as_float(x2[e])) + __uint_as_float(x3[e]);
+                if (r == 0) {
+                  H[q][8 * hf + e] = __uint_as_float(x0[e]) * sc;
+                  L[q][8 * hf + e] = lo * sc;
                 } else {
-                  ff_add(sh[j], sl[j], vh, vl);
+                  float s, er;
+                  two_sum(H[q][8 * hf + e], __uint_as_float(x0[e]) * sc, s, er);
+                  H[q][8 * hf + e] = s;
+                  L[q][8 * hf + e] += fmaf(lo, sc, er);
                 }
-              }
-              if (lastr) {
-#pragma unroll
-                for (int j = 0; j < 8; j += 2) {
-                  const int n = 4 * g + (j >> 1);
-                  if (rv && n < Nt) {
-                    oz_store(Cg, co + nq * dg.cn1 + nrr * dg.cn0, f64, dg.alpha, sh[j], sh[j + 1], sl[j], sl[j + 1]);
-                    if (++nrr == dg.cnd) {
-                      nrr = 0;
-                      ++nq;
-                    }
-                  }
-                }
-              } else {
-                tmem_st8(sum_h + (uint32_t)(8 * g), sh);
-                tmem_st8(sum_l + (uint32_t)(8 * g), sl);
               }
             }
           }
-          if (!lastr) tmem_wait_st();
           tc::fence_before_sync();
-          tc::mbar_arrive(&afree[a]);
-          tc::mbar_arrive(&efree[e]);
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&tfree[set]);
+        }
+        if constexpr (STAGE == 2) {  // FP64 partial of this K slice
+          j0 += job.R;
+          const OzS3 d = static_cast<const OzS3 *>(g.desc)[tk.d];
+#pragma unroll
+          for (int q = 0; q < HO; ++q) {
+            const int fr = ((tk.i & 0xffff) + m0 + gi[q]) * OZ_M + row, n0 = ((tk.i >> 16) * OCT + oct[q]) * 8;
+            if (gi[q] < Gm && fr < d.M && !dead) {
+              const int t = fr / d.nx, x = fr - t * d.nx;
+              double2 *o = g.part + d.part + (int64_t)t * d.elems + (int64_t)x * d.sx;
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                if (n0 + e < d.N)
+                  o[(int64_t)(n0 + e) * d.sn] = make_double2((double)H[q][2 * e] + (double)L[q][2 * e],
+                                                             (double)H[q][2 * e + 1] + (double)L[q][2 * e + 1]);
+            }
+          }
+        } else {
+          float V[HO][16], mx[HO];
+          bool valid[HO];
+#pragma unroll
+          for (int q = 0; q < HO; ++q) {
+            valid[q] = gi[q] < Gm && (STAGE == 0 ? rg < M : rw[q].dst >= 0);
+            float mo[8];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              V[q][e] = H[q][e] + L[q][e];
+              if (e & 1) mo[e >> 1] = fmaxf(fabsf(V[q][e - 1]), fabsf(V[q][e]));
+            }
+            mx[q] = fmaxf(fmaxf(fmaxf(mo[0], mo[1]), fmaxf(mo[2], mo[3])),
+                          fmaxf(fmaxf(mo[4], mo[5]), fmaxf(mo[6], mo[7])));
+            if (!valid[q]) mx[q] = 0.f;
+          }
+          if (gs > 1) {  // octets that share an exponent
+            float mo = mx[0];
+#pragma unroll
+            for (int q = 1; q < HO; ++q) mo = fmaxf(mo, mx[q]);
+            if (gs > HO) {  // some are in the other warp of this lane quarter
+              gmax[tile & 1][half][row] = mo;
+              asm volatile("bar.sync %0, 64;" ::"r"(1 + lq) : "memory");
+              mo = fmaxf(mo, gmax[tile & 1][half ^ 1][row]);
+            }
+#pragma unroll
+            for (int q = 0; q < HO; ++q) mx[q] = mo;
+          }
+          if constexpr (STAGE == 1)  // rows L of one K round share the exponent of their (tau, x)
+            for (int dlt = 1; dlt < (1 << glog); dlt <<= 1)
+#pragma unroll
+              for (int q = 0; q < HO; ++q) mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], dlt));
+#pragma unroll
+          for (int q = 0; q < HO; ++q) {
+            if (!valid[q] || dead) continue;
+            // the row's blob, its row and K step there
+            char *blob = xbase;
+            int nksb = gs, rr, ks;
+            if constexpr (STAGE == 0) {
+              const int grp = oct[q] / gs;
+              const int slot = ((goff + grp * nLg + (Lr >> glog)) << glog) + (Lr & ((1 << glog) - 1));
+              blob += ((int64_t)tau * nt2 + (slot >> 7)) * t2bytes;
+              rr = slot & 127;
+              ks = oct[q] - grp * gs;
+            } else {
+              const int fr = tau * d2[q].nx + rw[q].x, Lg = rw[q].L >> glog;
+              if (glog) nksb = min(1 << glog, d2[q].nL - (Lg << glog)) * zos;
+              ks = (rw[q].L & ((1 << glog) - 1)) * zos + oct[q];
+              blob += d2[q].base + (fr >> 7) * d2[q].fbytes + d2[q].kbase + (int64_t)Lg * d2[q].lgbytes;
+              rr = fr & 127;
+            }
+            const int e2 = oz_exponent(mx[q]);
+            const float f = oz_pow2(15 - e2), m1 = oz_m1(nksb);
+            uint32_t w[NS][8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              float sr[NS], si[NS];
+              oz_slice(H[q][2 * e], L[q][2 * e], V[q][2 * e], f, m1, sr);
+              oz_slice(H[q][2 * e + 1], L[q][2 * e + 1], V[q][2 * e + 1], f, m1, si);
+#pragma unroll
+              for (int p = 0; p < NS; ++p) w[p][e] = h2(sr[p], si[p]);
+            }
+            char *o = blob + ks * SA + rr * 32;
+            const bool sw = (rr >> 2) & 1;
+#pragma unroll
+            for (int p = 0; p < NS; ++p) st_octet(o + p * 4096, w[p], sw);
+            if (ks == 0) reinterpret_cast<float *>(blob + (int64_t)nksb * SA)[rr] = oz_pow2(e2 - 15);
+          }
+        }
+        if constexpr (STAGE == 0) {  // the next row tile
+          rg += OZ_M;
+          tau += dtau;
+          Lr += dL;
+          if (Lr >= nL) {
+            Lr -= nL;
+            ++tau;
+          }
+        } else if constexpr (STAGE == 1) {
+#pragma unroll
+          for (int q = 0; q < HO; ++q) rw[q] = rw1[q];
         }
       }
+      if (STAGE != 2) j0 += job.R;
     }
   }
   __syncthreads();
-  if (tid == 0 && issued > 0) tc::mbar_wait(&last, 0u, 4000000);  // every issued MMA has completed
+  if (tid == 0) tc::mbar_wait(&last, 0u, 4000000);  // every issued MMA has completed
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  if (warp == 0) tc::tmem_dealloc(tm, OZ_TMEM_WS);
+  if (warp == 0) tc::tmem_dealloc(tm, 512);
 }
 
-// (h, l) += (a + al)(b + bl) without renormalising (the a_l b_l term, below
-// 2^-48 of the product, is dropped): the product's rounding error comes from an
-// FMA (exact), the sum's from a two-sum; both go to the low word.
-__device__ __forceinline__ void ff_mac(float &h, float &l, float a, float al, float b, float bl) {
-  const float p = a * b;
-  float e = fmaf(a, b, -p);
-  e = fmaf(a, bl, e);
-  e = fmaf(al, b, e);
-  const float s = h + p;
-  const float bb = s - h;
-  l += ((h - (s - bb)) + (p - bb)) + e;
-  h = s;
-}
-
-// Narrow block GEMMs (few output columns) on the CUDA cores in float-float:
-// the same descriptors and tasks as oz_gemm_kernel (one CTA per task, one
-// thread per row of the 128-row tile, four output columns at a time), for
-// shapes where a tensor-core round would stage 128 x 16 slices for a handful
-// of columns.  Every operand keeps its float-float value (no slicing), so the
-// result carries about 46 bits.  B is read with addresses uniform across the
-// warp (broadcast loads).
-__global__ void __launch_bounds__(OZ_M) oz_simt_kernel(const OzDesc *__restrict__ descs,
-                                                       const OzTask *__restrict__ tasks, const float4 *__restrict__ Ag,
-                                                       const float4 *__restrict__ Bg, void *__restrict__ Cg,
-                                                       const int64_t *__restrict__ rowtab) {
-  const OzTask tk = tasks[blockIdx.x];
-  const OzDesc dg = descs[tk.desc];
-  const int mt = tk.mtnt >> 16, nt = tk.mtnt & 0xffff;
-  const int Mt = min(OZ_M, dg.M - mt * OZ_M), Nt = min(OZ_NC, dg.N - nt * OZ_NC);
-  const int r = threadIdx.x;
-  if (r >= Mt) return;
-  const int64_t arow0 = row_off(dg.a, mt * OZ_M + r, rowtab), crow0 = row_off(dg.c, mt * OZ_M + r, rowtab);
-  const float sa = (dg.flags & OZ_CONJ_A) ? -1.f : 1.f, sb = (dg.flags & OZ_CONJ_B) ? -1.f : 1.f;
-  const bool f64 = dg.flags & OZ_OUT_F64;
-  for (int rr = 0; rr < tk.nrep; ++rr) {
-    const int rep = tk.rep0 + rr;
-    const float4 *arow = Ag + arow0 + (int64_t)rep * dg.ra;
-    const int64_t co = crow0 + (int64_t)rep * dg.rc;
-    for (int n0 = 0; n0 < Nt; n0 += 4) {
-      const int nc = min(4, Nt - n0);
-      const float4 *bp[4];
+// Operand images from FP64 data: one CTA per image, OCT lanes per row (one
+// octet each), the row's exponent by a shuffle over them.
+template <int NS>
+__global__ void __launch_bounds__(128) oz_build_kernel(const OzBuild *__restrict__ tasks,
+                                                       const double2 *__restrict__ src, char *__restrict__ dst) {
+  constexpr int OCT = OzCfg<NS>::OCT;
+  const OzBuild t = tasks[blockIdx.x];
+  const int q = threadIdx.x % OCT;
+  const int nks = t.nks;
+  char *blob = dst + t.dst;
+  const int64_t pstride = t.isb ? 64 * t.rows : 4096;  // one K step of one plane
+  for (int lr = threadIdx.x / OCT; lr < t.rows; lr += 128 / OCT) {
+    const int r = t.r0 + lr, r1 = r / t.rd, r0 = r - r1 * t.rd;
+    const bool rv = r0 < t.rv && r1 < t.rn && q < nks;
+    const double2 *s = src + t.src + r1 * t.rs1 + (int64_t)r0 * t.rs0;
+    double2 v[8];
+    float m = 0.f;
 #pragma unroll
-      for (int c = 0; c < 4; ++c)  // columns past the tile re-read column n0 (results unused)
-        bp[c] = Bg + row_off(dg.b, nt * OZ_NC + n0 + (c < nc ? c : 0), rowtab) + (int64_t)rep * dg.rb;
-      float acc[4][4];  // per column: re (h, l), im (h, l)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[c][0] = acc[c][1] = acc[c][2] = acc[c][3] = 0.f;
-      for (int k = 0; k < dg.K; ++k) {
-        const float4 a = __ldg(arow + (int64_t)k * dg.aks);
-        const float ai = sa * a.y, ail = sa * a.w;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float4 b = __ldg(bp[c] + (int64_t)k * dg.bks);
-          const float bi = sb * b.y, bil = sb * b.w;
-          ff_mac(acc[c][0], acc[c][1], a.x, a.z, b.x, b.z);    // re += ar br
-          ff_mac(acc[c][0], acc[c][1], -ai, -ail, bi, bil);    //     - ai bi
-          ff_mac(acc[c][2], acc[c][3], a.x, a.z, bi, bil);     // im += ar bi
-          ff_mac(acc[c][2], acc[c][3], ai, ail, b.x, b.z);     //     + ai br
-        }
+    for (int e = 0; e < 8; ++e) {
+      const int k = 8 * q + e, k1 = k / t.kd, k0 = k - k1 * t.kd;
+      v[e] = make_double2(0.0, 0.0);
+      if (rv && k0 < t.kv && k1 < t.kn) {
+        v[e] = s[k1 * t.ks1 + (int64_t)k0 * t.ks0];
+        if (t.conj) v[e].y = -v[e].y;
       }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        if (c < nc) {
-          const int n = nt * OZ_NC + n0 + c;
-          const int nq = n / dg.cnd, nr = n - nq * dg.cnd;
-          const float rh = acc[c][0] + acc[c][1], ih = acc[c][2] + acc[c][3];
-          const float rl = acc[c][1] - (rh - acc[c][0]), il = acc[c][3] - (ih - acc[c][2]);
-          oz_store(Cg, co + nq * dg.cn1 + (int64_t)nr * dg.cn0, f64, dg.alpha, rh, ih, rl, il);
-        }
-      }
+      m = fmaxf(m, fmaxf(fabsf((float)v[e].x), fabsf((float)v[e].y)));
     }
-  }
-}
-
-__global__ void to_ffc_kernel(const double2 *__restrict__ x, float4 *__restrict__ y, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double2 v = x[i];
-    const float hr = __double2float_rn(v.x), hi = __double2float_rn(v.y);
-    y[i] = make_float4(hr, hi, __double2float_rn(v.x - (double)hr), __double2float_rn(v.y - (double)hi));
-  }
-}
-
-__global__ void oz_perm_kernel(const OzPerm *__restrict__ tasks, const double2 *__restrict__ src,
-                               float4 *__restrict__ dst) {
-  const OzPerm t = tasks[blockIdx.x];
-  const int yz = t.Y * t.Z, n = t.X * yz;
-  for (int e = threadIdx.x; e < n; e += blockDim.x) {
-    const int x = e / yz, y = (e / t.Z) % t.Y, z = e % t.Z;
-    double2 v = src[t.src + e];
-    if (t.conj) v.y = -v.y;
-    const float hr = __double2float_rn(v.x), hi = __double2float_rn(v.y);
-    dst[t.dst + x * t.dx + y * t.dy + z * t.dz] =
-        make_float4(hr, hi, __double2float_rn(v.x - (double)hr), __double2float_rn(v.y - (double)hi));
+#pragma unroll
+    for (int d = 1; d < OCT; d <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+    const int e2 = oz_exponent(m);
+    const float f = oz_pow2(15 - e2), m1 = oz_m1(nks);
+    if (q < nks) {
+      uint32_t w[NS][8];
+      float sr[8][NS], si[8][NS];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float hr = (float)v[e].x, hi = (float)v[e].y;
+        oz_slice(hr, (float)(v[e].x - (double)hr), hr, f, m1, sr[e]);
+        oz_slice(hi, (float)(v[e].y - (double)hi), hi, f, m1, si[e]);
+      }
+      if (!t.isb) {
+#pragma unroll
+        for (int p = 0; p < NS; ++p) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) w[p][e] = h2(sr[e][p], si[e][p]);
+          st_octet(blob + (q * NS + p) * pstride + lr * 32, w[p], (lr >> 2) & 1);
+        }
+      } else {  // rows (n, 0) = [Br -Bi], (n, 1) = [Bi Br]
+#pragma unroll
+        for (int p = 0; p < NS; ++p) {
+          char *o = blob + (q * NS + p) * pstride + lr * 64;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) w[p][e] = h2(sr[e][p], -si[e][p]);
+          st_octet(o, w[p], (lr >> 1) & 1);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) w[p][e] = h2(si[e][p], sr[e][p]);
+          st_octet(o + 32, w[p], (lr >> 1) & 1);
+        }
+      }
+      if (q == 0) reinterpret_cast<float *>(blob + NS * nks * pstride)[lr] = oz_pow2(e2 - 15);
+    }
   }
 }
 
 }  // namespace
 
 void set_oz_kernel_attributes() {
-  GWGB_CUDA(cudaFuncSetAttribute(oz_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM_WS));
+  GWGB_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<3, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
+  GWGB_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
+  GWGB_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
 }
 
-void launch_oz_gemm(const OzDesc *descs, const OzTask *tasks, int ntasks, const float4 *A, const float4 *B, void *C,
-                    const int64_t *rowtab, int nsm, int *err, cudaStream_t st) {
-  if (ntasks == 0) return;
-  const int grid = std::min(ntasks, std::max(1, nsm));
-  oz_gemm_kernel<<<grid, OZ_THREADS, OZ_SMEM_WS, st>>>(descs, tasks, ntasks, A, B, C, rowtab, err);
+// Stages 1 and 2 hold the column operand of a task (all K steps) and prefetch
+// the next task's; stage 3 streams both operands.
+void oz_rings(int ns, int stage, int max_kos, OzArgs *a) {
+  const int slotA = ns * 4096, slotB = ns * 512 * OzCfg<3>::OCT;
+  if (stage == 2) {
+    a->nA = a->nB = std::min(OZ_RING, OZ_SMEM / (slotA + slotB));
+  } else {
+    a->nB = std::min(OZ_RING, 2 * max_kos);
+    a->nA = std::min(OZ_RING, (OZ_SMEM - a->nB * slotB) / slotA);
+  }
+  GWGB_REQUIRE(a->nA >= 2 && a->nB >= (stage == 2 ? 2 : max_kos), GWGB_E_UNSUPPORTED, "sliced GEMM rings too small");
+}
+
+void launch_oz_gemm(int ns, int stage, const OzArgs &a, int nsm, cudaStream_t st) {
+  if (a.ntasks == 0) return;
+  (void)ns;
+  const int grid = std::min(a.ntasks, std::max(1, nsm));
+  if (stage == 0)
+    oz_gemm_kernel<3, 0><<<grid, OZ_THREADS, OZ_SMEM, st>>>(a);
+  else if (stage == 1)
+    oz_gemm_kernel<3, 1><<<grid, OZ_THREADS, OZ_SMEM, st>>>(a);
+  else
+    oz_gemm_kernel<3, 2><<<grid, OZ_THREADS, OZ_SMEM, st>>>(a);
   GWGB_CUDA(cudaGetLastError());
 }
 
-void launch_oz_simt(const OzDesc *descs, const OzTask *tasks, int ntasks, const float4 *A, const float4 *B, void *C,
-                    const int64_t *rowtab, cudaStream_t st) {
-  if (ntasks == 0) return;
-  oz_simt_kernel<<<ntasks, OZ_M, 0, st>>>(descs, tasks, A, B, C, rowtab);
-  GWGB_CUDA(cudaGetLastError());
-}
-
-void launch_to_ffc(const double2 *x, float4 *y, int64_t n, cudaStream_t st) {
-  if (n == 0) return;
-  const int64_t blocks = std::min<int64_t>((n + 255) / 256, 8 * 1024);
-  to_ffc_kernel<<<(int)blocks, 256, 0, st>>>(x, y, n);
-  GWGB_CUDA(cudaGetLastError());
-}
-
-void launch_oz_perm(const OzPerm *tasks, int ntasks, const double2 *src, float4 *dst, cudaStream_t st) {
-  if (ntasks == 0) return;
-  oz_perm_kernel<<<ntasks, 256, 0, st>>>(tasks, src, dst);
-  GWGB_CUDA(cudaGetLastError());
+void launch_oz_build(int ns, const OzBuild *tasks, int64_t ntasks, const double2 *src, char *dst, cudaStream_t st) {
+  (void)ns;
+  if (ntasks > 0) {
+    oz_build_kernel<3><<<(unsigned)ntasks, 128, 0, st>>>(tasks, src, dst);
+    GWGB_CUDA(cudaGetLastError());
+  }
 }
 
 }  // namespace gwgb

@@ -1,87 +1,123 @@
-// Error-free sliced contractions on tcgen05 ("BF16 x4 fixed-point slices"):
-// work descriptors and launchers.
+// Sliced contractions on tcgen05 (FP16 fixed-point slices, the Ozaki scheme):
+// operand images, work descriptors and launchers.
 //
-// Every contraction stage of the GW iteration (P0: Z1, Z, P0; Sigma: W, U,
-// Sigma) is a batch of complex GEMMs C = A B^T over the irrep blocks.  Here
-// they all run through one grouped persistent kernel (oz_gemm_kernel) whose
-// tasks are (descriptor, repetition, row tile, column tile).  Operands are
-// "float-float" complex numbers: float4 {re_hi, im_hi, re_lo, im_lo}, value
-// (re_hi + re_lo) + i (im_hi + im_lo), about 48 significant bits.
+// A contraction (P0 or Sigma) is a chain of three block GEMMs per V block:
+//   stage 1   X1[(tau, L)][(x, y)] = sum_k  G[(tau, L)][k]   V1[(x, y)][k]
+//   stage 2   X2[tau][(x, L)][z]   = sum_y  X1[tau][(x, L)][y]  B2[tau][z][y]
+//   stage 3   C[(tau, x)][n]       = sum_(c, L, z) X2[(tau, x)][(c, L, z)]  V3[n][(c, L, z)]
+// with, for P0:     L = m, x = P, y = t, z = p, n = Q, k = n',  B2 = G(k1, beta - tau)
+//      for Sigma:   L = n, x = i, y = Q, z = P, n = j, k = m,   B2 = P~(tau).
+//
+// Every operand lives in memory as the image the tensor core reads: the row's
+// value as NS FP16 slices (planes), K interleaved (re, im) in 32-byte steps of
+// 8 complex ("octets"), 128 rows (A) or 16 rows per 8 complex columns (B, the
+// real embedding) per step, in the 32-byte swizzle of the shared-memory matrix
+// descriptors.  One image ("blob") covers at most OCT octets of K (one round:
+// one exponent per row) and carries one FP32 scale per row behind the planes:
+//   A blob: [step][plane][128 rows][32 B], float scale[128]
+//   B blob: [step][plane][16 noct rows][32 B], float scale[8 noct]
+// so the GEMM moves blobs with bulk copies and does no work on its operands.
 #pragma once
 
 #include "common.h"
 
 namespace gwgb {
 
-// Row map of an operand or of the output: local row r (of the whole descriptor,
-// not of a tile) -> base + (r / d) * s1 + (r % d) * s0 (complex elements), or,
-// with d == 0, -> rowtab[base + r] (a table of row offsets).
-struct OzRows {
-  int64_t base;
-  int64_t s1;
-  int32_t s0;
-  int32_t d;
-};
-
-constexpr int OZ_CONJ_A = 1;  // A read conjugated
-constexpr int OZ_CONJ_B = 2;  // B read conjugated
-constexpr int OZ_OUT_F64 = 4; // C written as complex FP64, alpha * value (else float-float)
-
-// C[r][n] = sum_k A[r][k] B[n][k] for r < M, n < N, k < K (complex).
-//   A[r][k] at A + a(r) + k * aks + rep * ra, B[n][k] at B + b(n) + k * bks + rep * rb,
-//   C[r][n] at C + c(r) + (n / cnd) * cn1 + (n % cnd) * cn0 + rep * rc.
-// Every output element is written by exactly one task (no accumulation across
-// tasks), so the result is independent of the launch order.
-struct OzDesc {
-  OzRows a, b, c;
-  int64_t cn1;
-  int64_t ra, rb, rc;
-  double alpha;      // OZ_OUT_F64 only
-  int32_t cn0, cnd;
-  int32_t aks, bks;
-  int32_t M, N, K;
-  int32_t flags;
-};
-
-// One CTA work item: rows [128 mt, 128 mt + 128) and complex columns
-// [32 nt, 32 nt + 32) of descriptor `desc` at repetitions [rep0, rep0 + nrep)
-// (independent GEMMs done one after the other); mtnt = mt << 16 | nt.
-struct OzTask {
-  int32_t desc, rep0, nrep, mtnt;
-};
-
-// Element copy of a [X][Y][Z] block into float-float form at
-//   dst + x * dx + y * dy + z * dz (optionally conjugated): builds the
-// tau-independent operands (concatenated V blocks, their transposes) once per
-// V / rotation upload.
-struct OzPerm {
-  int64_t src, dst;
-  int64_t dx, dy, dz;
-  int32_t X, Y, Z;
-  int32_t conj;
-};
-
-// Tile geometry (shared with the host's work-list checks).
 constexpr int OZ_M = 128;   // rows per tile (TMEM lanes)
-constexpr int OZ_NC = 32;   // complex columns per tile
-constexpr int OZ_KR = 16;   // complex K per round (one slicing exponent per row and round)
+// X1 + X2 of one chunk, when that is at most an eighth of the free memory.
+constexpr int64_t OZ_CHUNK_BYTES = 8ll << 30;
+
+// Geometry of one slicing: NS planes; OCT octets (of 8 complex) per round and per column tile.
+template <int NS> struct OzCfg;
+template <> struct OzCfg<3> {  // 33-bit operands: the split-precision path
+  static constexpr int OCT = 4, NACC = 4, CMAX = 3;
+};
+
+__host__ __device__ constexpr int64_t oz_abytes(int ns, int nks) { return (int64_t)ns * nks * 4096 + 512; }
+// B blob bytes per octet of columns
+__host__ __device__ constexpr int64_t oz_bbytes1(int ns, int nks) { return (int64_t)ns * nks * 512 + 32; }
+
+// Stage 1: the images of one G block (all tau), row tile mt, round r at
+// a + mt * (bytes of all rounds) + r * oz_abytes(full round).
+struct OzS1 {
+  int64_t a;
+  int32_t M, nL;   // rows = n_tau * nL, row = tau * nL + L
+  int32_t kos;     // octets of K
+  int32_t pad;
+};
+// Stage-1 column tile: ngrp consecutive x of one contribution, gs octets of y each.
+struct OzCol1 {
+  int64_t b;       // its B blobs, rounds consecutive
+  int32_t dst;     // OzDst1
+  int32_t yoff;    // byte offset of the stage-2 round these columns are in
+  int16_t x0;
+  int8_t ngrp, gs;
+  int32_t pad;
+};
+// Where the stage-1 output of a contribution goes: stage-2 row slots
+//   group gi = gbase + x * nLg + (L >> glog), slot = (gi << glog) + (L & (2^glog - 1)),
+// tile slot / 128 of base + (tau * nt2 + tile) * t2bytes.
+struct OzDst1 {
+  int64_t base, t2bytes;
+  int32_t nt2, gbase, nLg, glog;
+};
+// Stage 2: one pack (contributions that share the B2 operand and glog).
+struct OzS2 {
+  int64_t a, t2bytes;      // X1 images of the pack
+  int64_t b, bt, bz;       // B2 images: b + tau * bt + (column tile) * bz
+  int32_t nt2, kos, zos, glog;
+  int32_t rows;            // first entry of the row map
+  int32_t pad;
+};
+struct OzRow { int32_t dst; int16_t x, L; };  // stage-2 row slot; dst < 0: empty
+// Where the stage-2 output of a contribution goes: final row tau * nx + x in
+// row tile f at base + f * fbytes; the round of L group Lg at kbase + Lg * lgbytes.
+struct OzDst2 {
+  int64_t base, fbytes;
+  int32_t kbase, lgbytes, nx, nL;
+};
+// Stage 3: one unit (a K slice of an output block).
+struct OzS3 {
+  int64_t a, fbytes;       // X2 images: a + f * fbytes + round offset
+  int64_t b, bz;           // V3 images: b + (column tile) * bz + round offset * octets
+  int64_t part;            // FP64 partial: part + tau * elems + n * sn + x * sx
+  int32_t rt, nkr;         // rounds [rt, rt + nkr) of the round table
+  int32_t M, N, nx, elems, sn, sx;
+};
+struct OzRnd { int32_t a16, b16, nks, pad; };  // byte offsets / 16 in the row tile and per octet of the column tile
+
+// One CTA work item.  Stage 1: OzS1 d, column tile i, row tiles [m0, m0 + n);
+// stage 2: pack d, i = tau | ztile << 16, row tiles [m0, m0 + n);
+// stage 3: unit d, i = first row tile | column tile << 16, n row tiles (at most OCT / octets of the column tile).
+struct OzTask { int32_t d, i, m0, n; };
+
+// One operand image built from FP64 data: row r (r0 + local) at (r / rd) * rs1 + (r % rd) * rs0,
+// valid when r % rd < rv and r / rd < rn; K index k at (k / kd) * ks1 + (k % kd) * ks0, valid likewise.
+struct OzBuild {
+  int64_t src, dst;
+  int64_t rs1, ks1;
+  int32_t rs0, ks0, rd, kd, rv, kv, rn, kn, r0;
+  int16_t rows, nks;       // rows of the image (complex), K octets
+  int8_t isb, conj;
+  int16_t pad;
+};
+
+struct OzArgs {
+  const void *desc;
+  const OzTask *tasks;
+  int ntasks;
+  const void *aux1, *aux2;   // stage 1: OzCol1, OzDst1; stage 2: OzRow, OzDst2; stage 3: OzRnd
+  const char *A, *B;
+  char *X;                   // stages 1, 2: output images
+  double2 *part;             // stage 3
+  int nA, nB;                // operand rings (K steps)
+  int *err;
+};
 
 void set_oz_kernel_attributes();
-
-// All tasks of one stage in one persistent launch (two CTAs per SM, tasks
-// taken in list order with a stride of the grid size).  err: set to 1 when a
-// bounded tensor-core completion wait ran out.
-void launch_oz_gemm(const OzDesc *descs, const OzTask *tasks, int ntasks, const float4 *A, const float4 *B, void *C,
-                    const int64_t *rowtab, int nsm, int *err, cudaStream_t st);
-
-// The same tasks on the CUDA cores in float-float arithmetic (one CTA per task):
-// for block GEMMs with few output columns.
-void launch_oz_simt(const OzDesc *descs, const OzTask *tasks, int ntasks, const float4 *A, const float4 *B, void *C,
-                    const int64_t *rowtab, cudaStream_t st);
-
-// y[i] = float-float(x[i]) for n complex elements.
-void launch_to_ffc(const double2 *x, float4 *y, int64_t n, cudaStream_t st);
-
-void launch_oz_perm(const OzPerm *tasks, int ntasks, const double2 *src, float4 *dst, cudaStream_t st);
+// Ring sizes of a launch; max_kos: most octets of K of its tasks (stages 1 and 2).
+void oz_rings(int ns, int stage, int max_kos, OzArgs *a);
+void launch_oz_gemm(int ns, int stage, const OzArgs &a, int nsm, cudaStream_t st);
+void launch_oz_build(int ns, const OzBuild *tasks, int64_t ntasks, const double2 *src, char *dst, cudaStream_t st);
 
 }  // namespace gwgb

@@ -1,0 +1,95 @@
+// Work lists and buffers of one sliced contraction (P0 or Sigma).
+#pragma once
+
+#include <vector>
+
+#include "dbuf.h"
+#include "kernels_oz.h"
+
+namespace gwgb {
+
+// One V block (and spin) of a contraction, in the names of kernels_oz.h.
+// Offsets and strides in complex elements of the source buffers.
+struct OzContrib {
+  int32_t nL, nx, ny, nz, N, K1;
+  int32_t vid;                 // V block id: contributions with the same id share their V images
+  int64_t v;                   // V block in the V source
+  int32_t sx, sy, sk;          // stage 1: V1[(x, y)][k]
+  int32_t sn, sL, sz;          // stage 3: V3[n][(L, z)]
+  int8_t conj1, conj3;
+  int64_t ga, gt;              // stage 1 operand G[(tau, L)][k]: ga + tau * gt + L * gL + k * gk
+  int32_t gL, gk;
+  int64_t b2, b2t;             // stage 2 operand B2[tau][z][y]: b2 + tau * b2t + z * b2z + y * b2y
+  int32_t b2z, b2y;
+  int8_t b2conj;
+};
+
+// One output block and its contributions [c0, c1) in K order.
+struct OzOwner {
+  int64_t out;                 // block at tau = 0
+  int32_t ostride, N, nx;
+  int32_t sn, sx;              // element (n, x) at n * sn + x * sx
+  int32_t c0, c1;
+};
+
+// One launch; kind as in gwgb_launch_stat.kernel.
+struct OzLaunch {
+  int kind = 0, stage = 0;     // 0 oz_gemm_kernel, 2 reduce_slices_kernel, 3 oz_build_kernel
+  int64_t t0 = 0, n = 0;       // tasks
+  int64_t d0 = 0;              // descriptors / auxiliary lists of the launch
+  int src = 0, dst = 0;        // builds: source (0 V, 1 G, 2 B2 source) and image buffer
+  OzArgs args{};               // rings (pointers are filled in when it runs)
+  int ny = 1;                  // reductions: CTAs per task
+  double flops = 0, ops = 0, bytes = 0;
+};
+
+// Buffers that the plans of one handle share (they run one after the other).
+struct OzShared {
+  DBuf<char> A1, B2, X1, X2;
+  DBuf<double2> part;
+  void free() {
+    A1.free(); B2.free(); X1.free(); X2.free(); part.free();
+  }
+};
+
+class OzPlan {
+ public:
+  enum { IMG_V, IMG_A1, IMG_B2 };
+  // stage0: gwgb_launch_stat.stage of stage 1; budget: bytes of X1 + X2 per chunk; persist_bytes: the
+  // V images are kept (built once per upload) when they take at most this, else built per chunk.
+  void build(int ns, const std::vector<OzContrib> &cs, const std::vector<OzOwner> &own, int ntau, int stage0,
+             int64_t budget, int64_t persist_bytes, int nsm, int64_t nV, int64_t nG, int64_t nB2, int64_t nout,
+             cudaStream_t st);
+  int64_t bytes_V() const { return vimg_; }
+  int64_t bytes_A1() const { return a1_; }
+  int64_t bytes_B2() const { return b2_; }
+  int64_t bytes_X1() const { return x1_; }
+  int64_t bytes_X2() const { return x2_; }
+  int64_t part_elems() const { return part_; }
+  void alloc_images() { V_.alloc((size_t)vimg_); }
+  // the operand images that do not change between iterations (after a V / rotation upload)
+  void build_static(const double2 *V, cudaStream_t st);
+  void run_one(const OzLaunch &l, OzShared &sh, const double2 *V, const double2 *G, const double2 *B2, double2 *out,
+               int nts, double scale, int nsm, int *err, cudaStream_t st) const;
+  const std::vector<OzLaunch> &launches() const { return launches_; }
+  void free();
+
+ private:
+  int ns_ = 3;
+  int64_t vimg_ = 0, a1_ = 0, b2_ = 0, x1_ = 0, x2_ = 0, part_ = 0;
+  std::vector<OzLaunch> launches_, static_;
+  DBuf<char> V_;
+  DBuf<OzBuild> builds_;
+  DBuf<OzTask> tasks_;
+  DBuf<OzS1> s1_;
+  DBuf<OzCol1> col1_;
+  DBuf<OzDst1> dst1_;
+  DBuf<OzS2> s2_;
+  DBuf<OzRow> rows_;
+  DBuf<OzDst2> dst2_;
+  DBuf<OzS3> s3_;
+  DBuf<OzRnd> rnd_;
+  DBuf<RedTask> red_;
+};
+
+}  // namespace gwgb

@@ -33,9 +33,9 @@ class GWSolver:
     def __init__(self, layout: BlockLayout, ns: int, transforms: IRTransforms,
                  precision: str = "fp64", device: int = 0, tune: dict = None):
         """tune: optional gwgb_params settings chosen by autotune.autotune()
-        (its "best" entry): oz_simt_cols, the width-class boundary of the
-        sliced path, or the tile settings of the FP32-class tcgen05 Sigma
-        path (uvt_smem_kb, sw_npk_max, uv_waves)."""
+        (its "best" entry): the tile settings of the FP32-class tcgen05 Sigma
+        path (uvt_smem_kb, sw_npk_max, uv_waves); oz_simt_cols is accepted
+        without effect."""
         self.lib = _abi.load()
         self.layout = layout
         self.ns = ns
