@@ -240,7 +240,7 @@ class Engine {
                  GWGB_E_INVALID, "unknown precision");
     if (prec != prec_) drop_graphs();  // the captured graphs hold the old kernels
     prec_ = prec;
-    if (prec_ == GWGB_PREC_OZAKI) {
+    if (prec_ == GWGB_PREC_OZAKI || prec_ == GWGB_PREC_FP64) {
       build_oz();
       return;
     }
@@ -385,10 +385,11 @@ class Engine {
       vcat_ready_ = false;
       built = true;
     }
-    if (prec_ == GWGB_PREC_OZAKI && !oz_ready_) {
-      oz_plan_[0].build_static(V_.p, st_);
-      oz_plan_[1].build_static(Vt_.p, st_);
-      oz_ready_ = true;
+    build_oz();
+    if (OzSet *o = oz_set(); o && !o->ready) {
+      o->plan[0].build_static(V_.p, st_);
+      o->plan[1].build_static(Vt_.p, st_);
+      o->ready = true;
       built = true;
     }
     if (tc_split() && !vcat_ready_) {
@@ -400,16 +401,27 @@ class Engine {
     if (built) GWGB_CUDA(cudaStreamSynchronize(st_));
   }
   bool tc_split() const { return prec_ == GWGB_PREC_TF32X3 || prec_ == GWGB_PREC_BF16X3; }
-  // Sliced (Ozaki) path: one plan per contraction (0: P0, 1: Sigma) and their shared buffers.
-  OzPlan oz_plan_[2];
+  // Sliced contractions: one plan per contraction (0: P0, 1: Sigma), in three
+  // slices (GWGB_PREC_OZAKI) and in six (GWGB_PREC_FP64), and their shared buffers.
+  // The FP64 FMA kernels are left for what the six slices do not serve: memory too
+  // small for the images (off), and contractions too small to fill the GPU.
+  struct OzSet {
+    OzPlan plan[2];
+    bool built = false, ready = false, off = false;
+  };
+  OzSet oz_[2];
   OzShared oz_buf_;
-  bool oz_built_ = false, oz_ready_ = false;
   void build_oz();
+  OzSet *oz_set() {  // the set that runs the contractions, if one does
+    OzSet *o = prec_ == GWGB_PREC_OZAKI ? &oz_[0] : prec_ == GWGB_PREC_FP64 ? &oz_[1] : nullptr;
+    return o && o->built && !o->off ? o : nullptr;
+  }
   // per-launch profile (gwgb_set_launch_timing): records [0, n_p0) P0, then Sigma
   bool lt_on_ = false, lt_ran_p0_ = false, lt_ran_sig_ = false;
   std::vector<cudaEvent_t> lt_ev_;
   std::vector<gwgb_launch_stat> lt_info_;
   int lt_n_p0_ = 0;
+  OzSet *lt_set_ = nullptr;  // the set whose launches the profile lists
   void rec_ev(cudaEvent_t e) {
     if (capturing_)
       GWGB_CUDA(cudaEventRecordWithFlags(e, st_, cudaEventRecordExternal));
@@ -417,9 +429,12 @@ class Engine {
       GWGB_CUDA(cudaEventRecord(e, st_));
   }
   void lt_build() {  // one entry per GEMM launch and per reduction, in launch order
+    lt_set_ = oz_set();
     lt_info_.clear();
+    lt_free();
+    lt_ran_p0_ = lt_ran_sig_ = false;
     for (int l = 0; l < 2; ++l) {
-      for (const OzLaunch &x : oz_plan_[l].launches()) {
+      for (const OzLaunch &x : oz_set()->plan[l].launches()) {
         gwgb_launch_stat g{};
         g.stage = x.stage;
         g.kernel = x.kind;
@@ -470,16 +485,17 @@ class Engine {
   bool tc_chunk_env_ = false;  // GWGB_TC_CHUNK_MB given: it caps the sliced path's chunks too
   // Run a contraction's plan (0: P0 into Pall_, 1: Sigma into Sig_).
   void oz_run(int which, double scale) {
+    OzSet &o = *oz_set();
     if (lt_on_ && lt_ev_.size() < 2 * lt_info_.size()) {
       const size_t n0 = lt_ev_.size();
       lt_ev_.resize(2 * lt_info_.size());
       for (size_t i = n0; i < lt_ev_.size(); ++i) GWGB_CUDA(cudaEventCreate(&lt_ev_[i]));
     }
     int rec = which ? lt_n_p0_ : 0;
-    for (const OzLaunch &x : oz_plan_[which].launches()) {
+    for (const OzLaunch &x : o.plan[which].launches()) {
       if (lt_on_) rec_ev(lt_ev_[2 * rec]);
-      oz_plan_[which].run_one(x, oz_buf_, which ? Vt_.p : V_.p, Gall_.p, which ? Pall_.p : Gall_.p,
-                              which ? Sig_.p : Pall_.p, nts_, scale, nsm_, bad_.p + 2, st_);
+      o.plan[which].run_one(x, oz_buf_, which ? Vt_.p : V_.p, Gall_.p, which ? Pall_.p : Gall_.p,
+                            which ? Sig_.p : Pall_.p, nts_, scale, nsm_, bad_.p + 2, st_);
       if (lt_on_) rec_ev(lt_ev_[2 * rec + 1]);
       ++rec;
     }
@@ -649,7 +665,8 @@ Engine::~Engine() {
                            &Tnt_, &Ttn_, &TntBF_, &TtnFB_};
   sw_tiles_.free(); bc_tasks_.free(); sig_wref_.free(); Wbuf_.free(); Bcat_.free(); uv_red_.free();
   pz_tasks_.free(); vc_tasks_.free(); pk_tiles_.free(); pr_tiles_.free(); Zbuf_.free(); Vcat_.free(); Ppart_.free();
-  oz_plan_[0].free(); oz_plan_[1].free(); oz_buf_.free();
+  for (OzSet &o : oz_) o.plan[0].free(), o.plan[1].free();
+  oz_buf_.free();
   for (auto *b : bufs) b->free();
   tct_f_.free(); tct_l_.free(); mu_dev_.free(); ws_.free(); bad_.free(); leak_.free();
   qoff_irr_.free(); qsz_irr_.free();
@@ -1423,7 +1440,14 @@ void Engine::build_work_lists() {
 // sliced (Ozaki) path: the two contractions as chains of block GEMMs (oz_plan.h)
 // ---------------------------------------------------------------------------
 void Engine::build_oz() {
-  if (oz_built_) return;
+  if (prec_ != GWGB_PREC_OZAKI && prec_ != GWGB_PREC_FP64) return;
+  const bool f64 = prec_ == GWGB_PREC_FP64;
+  OzSet &set = oz_[f64 ? 1 : 0];
+  if (set.built) {
+    if (lt_set_ != &set && !set.off) lt_build();
+    return;
+  }
+  const int NS = f64 ? 6 : 3;
   const Lay &l = l_;
   const int ns = ns_, nts = nts_;
   std::vector<OzContrib> cs;
@@ -1454,7 +1478,7 @@ void Engine::build_oz() {
       }
     own.push_back({g.pout, g.pstride, g.qb, g.qb, g.qb, 1, c0, (int32_t)cs.size()});
   }
-  oz_plan_[0].build(3, cs, own, nts / 2, 0, budget, persist, nsm_, l.flat_V, (int64_t)Gall_.n, (int64_t)Gall_.n,
+  set.plan[0].build(NS, cs, own, nts / 2, 0, budget, persist, nsm_, l.flat_V, (int64_t)Gall_.n, (int64_t)Gall_.n,
                     (int64_t)Pall_.n, st_);
   // Sigma[i][j] = sum Vt[Q][i][m] G2(tau)[m][n] P~(tau)[Q][P] conj(Vt[P][j][n])
   cs.clear();
@@ -1476,13 +1500,17 @@ void Engine::build_oz() {
     }
     own.push_back({ow.out, ow.ostride, ow.n, ow.n, 1, ow.n, c0, (int32_t)cs.size()});
   }
-  oz_plan_[1].build(3, cs, own, nts, 3, budget, std::max<int64_t>(0, persist - oz_plan_[0].bytes_V()), nsm_,
+  set.plan[1].build(NS, cs, own, nts, 3, budget, std::max<int64_t>(0, persist - set.plan[0].bytes_V()), nsm_,
                     (int64_t)Vt_.n, (int64_t)Gall_.n, (int64_t)Pall_.n, (int64_t)nts * ns * l.flat_ao, st_);
-  {  // the buffers must fit the free memory: say which take it otherwise
-    const OzPlan &p = oz_plan_[0], &s = oz_plan_[1];
-    const int64_t a1 = std::max(p.bytes_A1(), s.bytes_A1()), b2 = std::max(p.bytes_B2(), s.bytes_B2()),
-                  x1 = std::max(p.bytes_X1(), s.bytes_X1()), x2 = std::max(p.bytes_X2(), s.bytes_X2()),
-                  part = std::max(p.part_elems(), s.part_elems());
+  {  // the buffers (shared with the other set, if it is built) must fit the free memory
+    const OzPlan &p = set.plan[0], &s = set.plan[1];
+    auto grow = [](int64_t a, int64_t b, size_t have) {
+      const int64_t m = std::max(a, b);
+      return m > (int64_t)have ? m : 0;
+    };
+    const int64_t a1 = grow(p.bytes_A1(), s.bytes_A1(), oz_buf_.A1.n), b2 = grow(p.bytes_B2(), s.bytes_B2(), oz_buf_.B2.n),
+                  x1 = grow(p.bytes_X1(), s.bytes_X1(), oz_buf_.X1.n), x2 = grow(p.bytes_X2(), s.bytes_X2(), oz_buf_.X2.n),
+                  part = grow(p.part_elems(), s.part_elems(), oz_buf_.part.n);
     const std::pair<const char *, int64_t> need[] = {{"V images", p.bytes_V() + s.bytes_V()}, {"G images", a1},
                                                      {"stage-2 operands", b2}, {"X1", x1}, {"X2", x2},
                                                      {"partials", 16 * part}};
@@ -1493,20 +1521,39 @@ void Engine::build_oz() {
       msg += std::string(" ") + x.first + " " + std::to_string(x.second >> 20) + " MB";
     }
     GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    GWGB_REQUIRE(tot + (256ll << 20) + (V_.p ? 0 : 16 * l.flat_V) <= (int64_t)free_b, GWGB_E_UNSUPPORTED,
+    // Six slices against the FMA kernels: the MMAs (padded to octets of columns and 128 rows) run at 160 to
+    // 400 TFLOP/s including their drains, the launches around them take about 0.1 ms; the FMA kernels run at
+    // 1.2 TFLOP/s.  s+p (AO blocks 1-4): 1.03 ms against 1.04; s+p+d (1-8): 21 against 94; hexagonal 4 k
+    // (AO 7-30): 28 against 222; blocks of a single orbital stay on the FMA kernels.
+    double ops = 0;
+    for (const OzPlan *q : {&p, &s})
+      for (const OzLaunch &x : q->launches()) ops += x.ops;
+    // (GWGB_FP64_SLICES=1 / 0 in the environment forces one or the other)
+    const char *force = std::getenv("GWGB_FP64_SLICES");
+    const bool slow = f64 && force ? force[0] == '0' : f64 && ops / 1.8e14 + 1e-4 > (p0_flops_ + sig_flops_) / 1.2e12;
+    const bool fits = !slow && tot + (256ll << 20) + (V_.p ? 0 : 16 * l.flat_V) <= (int64_t)free_b;
+    set.built = true;
+    if (f64 && !fits) {  // the FMA kernels, which need no images
+      set.off = true;
+      set.plan[0].free();
+      set.plan[1].free();
+      return;
+    }
+    set.built = fits;
+    GWGB_REQUIRE(fits, GWGB_E_UNSUPPORTED,
                  "sliced-precision buffers need " + std::to_string(tot >> 20) + " MB (" + msg + " ), " +
                      std::to_string(free_b >> 20) + " MB free");
-    oz_plan_[0].alloc_images();
-    oz_plan_[1].alloc_images();
-    oz_buf_.A1.alloc((size_t)a1);
-    oz_buf_.B2.alloc((size_t)b2);
-    oz_buf_.X1.alloc((size_t)x1);
-    oz_buf_.X2.alloc((size_t)x2);
-    oz_buf_.part.alloc((size_t)part);
+    if (a1 || b2 || x1 || x2 || part) drop_graphs();  // they hold the old buffers' addresses
+    set.plan[0].alloc_images();
+    set.plan[1].alloc_images();
+    if (a1) oz_buf_.A1.alloc((size_t)a1);
+    if (b2) oz_buf_.B2.alloc((size_t)b2);
+    if (x1) oz_buf_.X1.alloc((size_t)x1);
+    if (x2) oz_buf_.X2.alloc((size_t)x2);
+    if (part) oz_buf_.part.alloc((size_t)part);
   }
-  oz_ready_ = false;
+  set.ready = false;
   lt_build();
-  oz_built_ = true;
 }
 
 // ---------------------------------------------------------------------------
@@ -1527,7 +1574,8 @@ void Engine::upload_V(const double *V, int64_t n) {
   h2d(V_.p, V, (size_t)n * sizeof(double2), st_);
   GWGB_CUDA(cudaStreamSynchronize(st_));
   have_V_ = true;
-  vt_ready_ = vcat_ready_ = oz_ready_ = false;  // rebuilt before the next solve
+  vt_ready_ = vcat_ready_ = oz_[0].ready = oz_[1].ready = false;  // rebuilt before the next solve
+  build_oz();  // the lists, with the other set-up of a handle that will contract
 }
 
 void Engine::set_reps(const double *orep, int64_t no, const double *auxrep, int64_t na) {
@@ -1536,7 +1584,7 @@ void Engine::set_reps(const double *orep, int64_t no, const double *auxrep, int6
   h2d(auxrep_.p, auxrep, (size_t)na * sizeof(double2), st_);
   GWGB_CUDA(cudaStreamSynchronize(st_));
   have_reps_ = true;
-  vt_ready_ = vcat_ready_ = oz_ready_ = false;  // rebuilt before the next solve
+  vt_ready_ = vcat_ready_ = oz_[0].ready = oz_[1].ready = false;  // rebuilt before the next solve
 }
 
 void Engine::set_transforms(const double *Tnt, const double *Ttn, const double *TntBF, const double *TtnFB,
@@ -1605,8 +1653,8 @@ void Engine::k_rotate_G() {
 
 void Engine::k_p0(int mirror) {
   const double pref = -1.0 / l_.nk * (ns_ == 1 ? 2.0 : 1.0);  // cugw_qkpt_block.cu:210, cugw_solver_block.cpp:303
-  if (prec_ == GWGB_PREC_OZAKI) {  // sliced contractions: Z1 -> Z -> P0 per tau chunk
-    GWGB_REQUIRE(oz_ready_, GWGB_E_STATE, "sliced-precision operands not prepared");
+  if (OzSet *o = oz_set()) {
+    GWGB_REQUIRE(o->ready, GWGB_E_STATE, "sliced operands not prepared");
     GWGB_CUDA(cudaMemsetAsync(Pall_.p, 0, Pall_.n * sizeof(double2), st_));  // blocks without contributions
     oz_run(0, pref);
     lt_ran_p0_ = lt_on_;
@@ -1637,8 +1685,8 @@ void Engine::k_pq(bool mirror_first) {
 
 
 void Engine::k_sigma() {
-  if (prec_ == GWGB_PREC_OZAKI) {  // sliced contractions: W -> U -> Sigma per tau chunk
-    GWGB_REQUIRE(oz_ready_, GWGB_E_STATE, "sliced-precision operands not prepared");
+  if (OzSet *o = oz_set()) {
+    GWGB_REQUIRE(o->ready, GWGB_E_STATE, "sliced operands not prepared");
     GWGB_CUDA(cudaMemsetAsync(Sig_.p, 0, Sig_.n * sizeof(double2), st_));  // blocks without contributions
     oz_run(1, -1.0 / l_.nk);
     lt_ran_sig_ = lt_on_;
@@ -1729,8 +1777,8 @@ void Engine::finish_stats(bool with_dyson, bool with_gw, bool with_pq, bool with
                           : (p0_tiles_.n ? 1 : 0) + (p0_red_.n ? 1 : 0);
     const int64_t sg = tc ? sgt
                           : (sig_tiles_.n ? 1 : 0) + (sig_red_.n ? 1 : 0);
-    if (prec_ == GWGB_PREC_OZAKI) {
-      const int64_t a = (int64_t)oz_plan_[0].launches().size(), b = (int64_t)oz_plan_[1].launches().size();
+    if (OzSet *o = oz_set()) {
+      const int64_t a = (int64_t)o->plan[0].launches().size(), b = (int64_t)o->plan[1].launches().size();
       launches += (rotG_.n ? 1 : 0) + a + 1 + 3 + b;  // 1: the tau mirror of P0
     } else
     launches += (rotG_.n ? 1 : 0) + p0 + 3 + sg;
@@ -2089,6 +2137,7 @@ void Engine::sc_loop(int niter, double alpha, const gwgb_mu_search &ms, int fina
   if (nmain < niter) {  // the last iteration with the FP64 contractions
     GWGB_CUDA(cudaStreamSynchronize(st_));
     set_precision(GWGB_PREC_FP64);
+    prepare_operands();
     capture(&sc_exec_, [&] { k_sc_iteration(alpha, ms); });
     sc_alpha_ = alpha;
     sc_ms_ = ms;

@@ -16,7 +16,18 @@
 //           within 24 bits, so FP32 accumulation is exact;
 //   (0, 1) and (1, 0), one each: 9 + b bits per term and the round's 6, 5 or 4: exact;
 //   the rest: weight 2^-19 and less; its FP32 rounding lies near 2^-41.
-// Dropped: s2 t2, below 2^-37 of the row-by-column scale.  Complex products use
+// Dropped: s2 t2, below 2^-37 of the row-by-column scale.
+//
+// The FP64 contractions are the same chains with six slices: x 2^(8-E) = sum_p
+// d_p 2^(-9p), |d_p| <= 2^8, d_0 .. d_4 integers and d_5 the rest rounded to FP16,
+// so a row is held to 2^(E-57) of its scale (FP64 itself holds an element to
+// 2^-53).  The products of class i + j <= 6 (26 MMAs per K step) go to one
+// accumulator per class; classes 0 to 3 are exact in FP32 (at most 4 products of
+// 2^16 over 64 real terms), classes 4 to 6 have weight 2^-36 and less, class 7 is
+// dropped (2^-61).  The drain sums the classes without error into three FP32
+// numbers.  Measured against 64-bit references the error is below the FP64
+// FMA kernels'.  Their rate is the FP64 pipe's (2 FMA per cycle and SM); one
+// complex output of K = 32 takes 64 cycles there and about 3 here.  Complex products use
 // the real embedding A = [Ar Ai] (K interleaved), B rows (n, 0) = [Br -Bi],
 // (n, 1) = [Bi Br], so D[r][(n,0)] = Re, D[r][(n,1)] = Im of sum_k A[r][k] B[n][k].
 #include "kernels_oz.h"
@@ -31,6 +42,8 @@ namespace gwgb {
 namespace {
 
 constexpr int OZ_EMIN = -100, OZ_EMAX = 128;
+// NS = 6: exponents of the images; a row without a nonzero value has -OZ_ELIM
+constexpr int OZ_ELIM = 4000, OZ_ENONE = -1000000;
 
 // E with |x| < 2^E for every |x| <= m (m >= 0), clamped to [OZ_EMIN, OZ_EMAX].
 __device__ __forceinline__ int oz_exponent(float m) {
@@ -58,6 +71,62 @@ __device__ __forceinline__ void oz_slice(float h, float l, float v, float f, flo
   s[1] = (t + m1) - m1;
   s[2] = t - s[1];
 }
+
+// Unevaluated sum of three FP32 numbers, h the rounded value.
+struct Tri {
+  float h, m, l;
+};
+
+// The value of the class sums D0 .. D6 (weights 2^(-9c)); D0 to D3 are exact integers.
+__device__ __forceinline__ Tri tri_of(const float (&d)[7]) {
+  constexpr float W1 = 0x1p-9f, W2 = 0x1p-18f, W3 = 0x1p-27f, W4 = 0x1p-36f;
+  float h, e1, s, e2, e3;
+  two_sum(d[0], d[1] * W1, h, e1);
+  two_sum(d[2] * W2, d[3] * W3, s, e2);
+  two_sum(e1, s, e1, e3);
+  float l = fmaf(fmaf(fmaf(d[6], W1, d[5]), W1, d[4]), W4, e2 + e3);
+  // h is zero only when the value is (all of it can lie in the low classes)
+  two_sum(h, e1, h, e1);
+  two_sum(e1, l, e1, e2);
+  Tri t;
+  two_sum(h, e1, t.h, t.m);
+  t.l = e2;
+  return t;
+}
+
+// a += b, and a normalised (h the rounded value).
+__device__ __forceinline__ void tri_add(Tri &a, const Tri &b) {
+  float h, e1, m, e2, e3;
+  two_sum(a.h, b.h, h, e1);
+  two_sum(a.m, b.m, m, e2);
+  two_sum(m, e1, m, e3);
+  const float l = (a.l + b.l) + (e2 + e3);
+  two_sum(h, m, h, m);
+  two_sum(m, l, m, a.l);
+  two_sum(h, m, a.h, a.m);
+}
+
+// The six digits of h + m + l (f = 2^(8-E)).
+__device__ __forceinline__ void tri_digits(const Tri &x, float f, float (&s)[6]) {
+  constexpr float MG = 1.5f * 8388608.f;  // 1.5 2^23: rounds to integers
+  s[0] = fmaf(x.h, f, MG) - MG;
+  float t, te;
+  two_sum(fmaf(x.h, f, -s[0]), x.m * f, t, te);  // the first is exact
+  te = fmaf(x.l, f, te);
+  s[1] = fmaf(t, 512.f, MG) - MG;
+  t = fmaf(t, 512.f, -s[1]);
+  s[2] = fmaf(t, 512.f, MG) - MG;
+  t = fmaf(t, 512.f, -s[2]);
+  two_sum(t, te * 262144.f, t, te);
+  s[3] = fmaf(t, 512.f, MG) - MG;
+  t = fmaf(t, 512.f, -s[3]);
+  s[4] = fmaf(t, 512.f, MG) - MG;
+  t = fmaf(t, 512.f, -s[4]);
+  s[5] = fmaf(te, 134217728.f, t * 512.f);  // te 2^27
+}
+
+// 2^e for any e, 0 below the FP32 range.
+__device__ __forceinline__ float oz_pow2c(int e) { return e < -126 ? 0.f : oz_pow2(min(e, 127)); }
 
 // The rounding constant of s1 for an image of nks octets of K.
 __device__ __forceinline__ float oz_m1(int nks) {
@@ -99,6 +168,11 @@ __device__ __forceinline__ uint32_t idesc_f16(int N) {
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
@@ -170,7 +244,11 @@ template <int NS, int STAGE> struct Job {
 constexpr int OZ_RING = 16;             // largest operand ring (K steps)
 constexpr int OZ_SC = 32;               // scale rings: deeper than the operand rings plus the accumulator sets
 constexpr int OZ_SMEM = 200 * 1024;
-constexpr int OZ_THREADS = 320;         // warps 0-7 drain, warp 8 copies, warp 9 issues the MMAs
+// Drain warps (then one warp copies and one issues the MMAs): three slices take two octets per
+// thread in 8 warps (hex 8 k: 61 ms against 69 with one octet in 16 warps), six slices one octet
+// in 16 warps (s+p+d: 24 ms against 33: unrolled over two octets the code misses the instruction cache).
+template <int NS> constexpr int oz_drain = 4 * OzCfg<NS>::OCT / OzCfg<NS>::HO;
+template <int NS> constexpr int oz_threads = 32 * (oz_drain<NS> + 2);
 
 // One lane of a converged warp.  The copy and MMA loops are warp-uniform and
 // elect a lane only around the instruction itself: their descriptors then stay in
@@ -208,15 +286,17 @@ struct Ring {
 // flag; the copy and MMA roles then leave, the drain warps walk on through
 // their work without waiting (their named barriers stay matched).  Copies and
 // MMAs in flight are waited for (bounded) before TMEM is released.
-template <int NS, int STAGE>
-__global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) {
-  constexpr int OCT = OzCfg<NS>::OCT, NACC = OzCfg<NS>::NACC, HO = OCT / 2;
+// MULTI (stages 1 and 2): tasks with more than one round of K.
+template <int NS, int STAGE, bool MULTI>
+__global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs g) {
+  constexpr int OCT = OzCfg<NS>::OCT, NACC = OzCfg<NS>::NACC, HO = OzCfg<NS>::HO, DW = oz_drain<NS>;
   constexpr int NR = 16 * OCT, SETC = NACC * NR;
   constexpr uint32_t SA = NS * 4096, SB = NS * 512 * OCT;  // ring slots
-  static_assert(2 * SETC <= 512, "two accumulator sets must fit TMEM");
+  constexpr int SETS = OzCfg<NS>::SETS;
+  static_assert(SETS * SETC <= 512, "the accumulator sets must fit TMEM");
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint32_t tslot;
-  __shared__ __align__(8) uint64_t full[OZ_RING], emptyA[OZ_RING], emptyB[OZ_RING], done[2], tfree[2], last;
+  __shared__ __align__(8) uint64_t full[OZ_RING], emptyA[OZ_RING], emptyB[OZ_RING], done[SETS], tfree[SETS], last;
   __shared__ __align__(16) float sA[OZ_SC][OZ_M], sB[OZ_SC][8 * OCT];
   __shared__ float gmax[2][OCT][OZ_M];
   __shared__ int abort_flag;
@@ -229,9 +309,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) 
       tc::mbar_init(&emptyA[j], 1);
       tc::mbar_init(&emptyB[j], 1);
     }
-    for (int j = 0; j < 2; ++j) {
+    for (int j = 0; j < SETS; ++j) {
       tc::mbar_init(&done[j], 1);
-      tc::mbar_init(&tfree[j], 8);
+      tc::mbar_init(&tfree[j], DW);
     }
     tc::mbar_init(&last, 1);
     abort_flag = 0;
@@ -265,7 +345,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) 
   };
   const uint32_t smA = tc::smem_u32(smem), smB = smA + (uint32_t)g.nA * SA;
 
-  if (warp == 8) {
+  if (warp == DW) {
     // ------------------------------ copies ------------------------------
     Ring ra(g.nA), rb(g.nB);
     int ia = 0, ib = 0, ra_rounds = 0, rb_rounds = 0;  // K steps and rounds copied
@@ -315,7 +395,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) 
       if (q >= first) tc::mbar_wait(&full[rw.slot], rw.phase, 4000000);
       rw.next();
     }
-  } else if (warp == 9) {
+  } else if (warp == DW + 1) {
     // ------------------------------ MMAs ------------------------------
     Ring ra(g.nA), rb(g.nB);
     int n = 0;  // accumulator sets filled
@@ -332,8 +412,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) 
         const bool lastm = STAGE == 2 || m0 + job.G >= job.outer;
         if (STAGE != 2) rb = r0;
         for (int r = 0; r < job.R && ok; ++r, ++n) {
-          const int set = n & 1, nks = __shfl_sync(0xffffffffu, job.nks(r), 0);
-          if (n >= 2 && !bwait(&tfree[set], ((n >> 1) - 1) & 1)) { ok = false; break; }
+          const int set = n % SETS, nks = __shfl_sync(0xffffffffu, job.nks(r), 0);
+          if (n >= SETS && !bwait(&tfree[set], (n / SETS - 1) & 1)) { ok = false; break; }
           const Ring rr = rb;
           for (int gi = 0; gi < Gm && ok; ++gi) {
             rb = rr;
@@ -350,9 +430,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) 
                   for (int p = 0; p < NS; ++p) {
                     const int q = c - p;
                     if (q < 0 || q >= NS) continue;
-                    // (0,0) | (0,1) | (1,0) | the rest
-                    const int acc = c == 0 ? 0 : c == 1 ? 1 + p : 3;
-                    const bool fresh = c < 2 || (c == 2 && p == 0);
+                    // NS = 3: (0,0) | (0,1) | (1,0) | the rest; NS = 6: one per class
+                    const int acc = NS == 6 ? c : c == 0 ? 0 : c == 1 ? 1 + p : 3;
+                    const bool fresh = NS == 6 ? p == max(0, c - NS + 1) : c < 2 || (c == 2 && p == 0);
                     tc::mma_bf16(d0 + acc * NR, sw32_desc(a0 + p * 4096u), sw32_desc(b0 + q * bstep), id,
                                  fresh ? more : 1u);  // kind::f16, types from the descriptor
                   }
@@ -376,19 +456,20 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) 
     // ------------------------------ drain ------------------------------
     // warp w: TMEM lanes (rows) 32 (w & 3) .. + 31, octets HO (w >> 2) .. + HO - 1 of the set.
     // The rows' destinations are read while the set still multiplies.
-    const int lq = warp & 3, half = warp >> 2, row = 32 * lq + lane;
-    const uint32_t tbase = tm + ((uint32_t)(32 * lq) << 16) + 16u * HO * half;
+    const int lq = warp & 3, os0 = HO * (warp >> 2), row = 32 * lq + lane;
+    const uint32_t tbase = tm + ((uint32_t)(32 * lq) << 16) + 16u * os0;
     int n = 0, i0 = 0, j0 = 0, tile = 0;  // sets, row tiles and column images consumed
     bool dead = false;
     for (int ti = blockIdx.x; ti < g.ntasks; ti += gridDim.x) {
       const OzTask tk = g.tasks[ti];
       Job<NS, STAGE> job;
       job.init(g, tk);
-      int gi[HO], oct[HO];  // row tile in the set, octet in the tile
+      // row tile in the set, octet in the tile, valid columns of the octet
+      int gi[HO], oct[HO], nv[HO];
 #pragma unroll
       for (int q = 0; q < HO; ++q) {
-        gi[q] = (half * HO + q) / job.noct;
-        oct[q] = half * HO + q - gi[q] * job.noct;
+        gi[q] = (os0 + q) / job.noct;
+        oct[q] = os0 + q - gi[q] * job.noct;
       }
       // stage 1: the row and its destination
       int rg = 0, M = 0, nL = 1, tau = 0, Lr = 0, dtau = 0, dL = 0, gs = 1, goff = 0, nLg = 1, glog = 0, nt2 = 1;
@@ -416,6 +497,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) 
         Lr = rg - tau * nL;
         dtau = OZ_M / nL;
         dL = OZ_M - dtau * nL;
+#pragma unroll
+        for (int q = 0; q < HO; ++q) nv[q] = col.ny - 8 * (oct[q] % gs);
       } else if constexpr (STAGE == 1) {
         const OzS2 d = static_cast<const OzS2 *>(g.desc)[tk.d];
         gs = job.noct;
@@ -426,9 +509,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) 
         rows = static_cast<const OzRow *>(g.aux1) + d.rows + tk.m0 * OZ_M + row;
 #pragma unroll
         for (int q = 0; q < HO; ++q) {
+          nv[q] = d.nz - 8 * ((tk.i >> 16) * OCT + oct[q]);
           rw[q] = {-1, 0, 0};
           if (gi[q] < min(job.G, job.outer)) rw[q] = rows[gi[q] * OZ_M];
         }
+      } else {
+#pragma unroll
+        for (int q = 0; q < HO; ++q)
+          nv[q] = static_cast<const OzS3 *>(g.desc)[tk.d].N - 8 * ((tk.i >> 16) * OCT + oct[q]);
       }
       for (int m0 = 0; m0 < job.outer; m0 += job.G, ++tile) {
         const int Gm = min(job.G, job.outer - m0);
@@ -442,44 +530,93 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) 
             if (m0 + job.G + gi[q] < job.outer) rw1[q] = rows[(m0 + job.G + gi[q]) * OZ_M];
           }
         }
-        float H[HO][16], L[HO][16];  // value H + L of this thread's octets
+        // this thread's octets: value H + L (NS = 3), (H + M + L) 2^ex (NS = 6)
+        float H[HO][16], L[HO][16], M3[NS == 6 ? HO : 1][16];
+        int ex[HO];
 #pragma unroll
-        for (int q = 0; q < HO; ++q)
+        for (int q = 0; q < HO; ++q) {
+          ex[q] = 0;
 #pragma unroll
-          for (int e = 0; e < 16; ++e) H[q][e] = L[q][e] = 0.f;
+          for (int e = 0; e < 16; ++e) H[q][e] = L[q][e] = M3[NS == 6 ? q : 0][e] = 0.f;
+        }
         for (int r = 0; r < job.R; ++r, ++n, i0 += Gm) {
-          const int set = n & 1;
-          if (!dead) dead = !bwait(&done[set], (n >> 1) & 1);
+          const int set = n % SETS;
+          if (!dead) dead = !bwait(&done[set], (n / SETS) & 1);
           if (dead) continue;
           tc::fence_after_sync();
-          const float *sbp = sB[(j0 + r) & (OZ_SC - 1)];
-          const uint32_t base = tbase + (uint32_t)(set * SETC);
+          const bool first = STAGE == 2 || MULTI ? r == 0 : true;
 #pragma unroll
           for (int q = 0; q < HO; ++q) {
             if (gi[q] >= Gm) continue;
+            const float *sbp = sB[(j0 + r) & (OZ_SC - 1)] + 8 * oct[q];
+            const uint32_t base = tbase + (uint32_t)(set * SETC) + 16u * q;
             const float sa = sA[(i0 + gi[q]) & (OZ_SC - 1)][row];
+            if constexpr (NS == 3) {
 #pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-              uint32_t x0[8], x1[8], x2[8], x3[8];
-              tmem_ld8(base + 16 * q + 8 * hf, x0);
-              tmem_ld8(base + NR + 16 * q + 8 * hf, x1);
-              tmem_ld8(base + 2 * NR + 16 * q + 8 * hf, x2);
-              tmem_ld8(base + 3 * NR + 16 * q + 8 * hf, x3);
-              const float4 sb4 = *reinterpret_cast<const float4 *>(sbp + 8 * oct[q] + 4 * hf);
-              const float sb[4] = {sb4.x, sb4.y, sb4.z, sb4.w};
-              tmem_wait_ld();
+              for (int hf = 0; hf < 2; ++hf) {
+                if (4 * hf >= nv[q]) continue;
+                uint32_t x0[8], x1[8], x2[8], x3[8];
+                tmem_ld8(base + 8 * hf, x0);
+                tmem_ld8(base + NR + 8 * hf, x1);
+                tmem_ld8(base + 2 * NR + 8 * hf, x2);
+                tmem_ld8(base + 3 * NR + 8 * hf, x3);
+                const float4 sb4 = *reinterpret_cast<const float4 *>(sbp + 4 * hf);
+                const float sb[4] = {sb4.x, sb4.y, sb4.z, sb4.w};
+                tmem_wait_ld();
 #pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const float sc = sa * sb[e >> 1];
-                const float lo = (__uint_as_float(x1[e]) + __uint_as_float(x2[e])) + __uint_as_float(x3[e]);
-                if (r == 0) {
-                  H[q][8 * hf + e] = __uint_as_float(x0[e]) * sc;
-                  L[q][8 * hf + e] = lo * sc;
-                } else {
-                  float s, er;
-                  two_sum(H[q][8 * hf + e], __uint_as_float(x0[e]) * sc, s, er);
-                  H[q][8 * hf + e] = s;
-                  L[q][8 * hf + e] += fmaf(lo, sc, er);
+                for (int e = 0; e < 8; ++e) {
+                  const float sc = sa * sb[e >> 1];
+                  const float lo = (__uint_as_float(x1[e]) + __uint_as_float(x2[e])) + __uint_as_float(x3[e]);
+                  if (first) {
+                    H[q][8 * hf + e] = __uint_as_float(x0[e]) * sc;
+                    L[q][8 * hf + e] = lo * sc;
+                  } else {
+                    float s, er;
+                    two_sum(H[q][8 * hf + e], __uint_as_float(x0[e]) * sc, s, er);
+                    H[q][8 * hf + e] = s;
+                    L[q][8 * hf + e] += fmaf(lo, sc, er);
+                  }
+                }
+              }
+            } else {
+              // exponent of the row and of this octet's columns, relative column factors
+              const int4 b0 = *reinterpret_cast<const int4 *>(sbp), b1 = *reinterpret_cast<const int4 *>(sbp + 4);
+              const int eb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+              const int em = max(max(max(eb[0], eb[1]), max(eb[2], eb[3])), max(max(eb[4], eb[5]), max(eb[6], eb[7])));
+              const int er = __float_as_int(sa) + em;
+              float fo = 1.f, fn = 1.f;  // factors of the sum so far and of this round
+              if (first) {
+                ex[q] = er;
+              } else if (er > ex[q]) {
+                fo = oz_pow2c(ex[q] - er);
+                ex[q] = er;
+              } else {
+                fn = oz_pow2c(er - ex[q]);
+              }
+#pragma unroll
+              for (int hf = 0; hf < 4; ++hf) {
+                if (2 * hf >= nv[q]) continue;
+                uint32_t x[7][4];
+#pragma unroll
+                for (int c = 0; c < 7; ++c) tmem_ld4(base + c * NR + 4 * hf, x[c]);
+                tmem_wait_ld();
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const int i = 4 * hf + e;
+                  float d[7];
+#pragma unroll
+                  for (int c = 0; c < 7; ++c) d[c] = __uint_as_float(x[c][e]);
+                  Tri t = tri_of(d);
+                  const float sc = oz_pow2c(eb[i >> 1] - em) * fn;
+                  t = {t.h * sc, t.m * sc, t.l * sc};
+                  if (!first) {
+                    Tri o{H[q][i] * fo, M3[q][i] * fo, L[q][i] * fo};
+                    tri_add(o, t);
+                    t = o;
+                  }
+                  H[q][i] = t.h;
+                  M3[q][i] = t.m;
+                  L[q][i] = t.l;
                 }
               }
             }
@@ -493,49 +630,77 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) 
           const OzS3 d = static_cast<const OzS3 *>(g.desc)[tk.d];
 #pragma unroll
           for (int q = 0; q < HO; ++q) {
-            const int fr = ((tk.i & 0xffff) + m0 + gi[q]) * OZ_M + row, n0 = ((tk.i >> 16) * OCT + oct[q]) * 8;
-            if (gi[q] < Gm && fr < d.M && !dead) {
-              const int t = fr / d.nx, x = fr - t * d.nx;
-              double2 *o = g.part + d.part + (int64_t)t * d.elems + (int64_t)x * d.sx;
+            const int fr = ((tk.i & 0xffff) + m0 + gi[q]) * OZ_M + row, n0 = d.N - nv[q];
+            if (gi[q] >= Gm || fr >= d.M || dead) continue;
+            const int t = fr / d.nx, x = fr - t * d.nx;
+            double2 *o = g.part + d.part + (int64_t)t * d.elems + (int64_t)x * d.sx;
 #pragma unroll
-              for (int e = 0; e < 8; ++e)
-                if (n0 + e < d.N)
-                  o[(int64_t)(n0 + e) * d.sn] = make_double2((double)H[q][2 * e] + (double)L[q][2 * e],
-                                                             (double)H[q][2 * e + 1] + (double)L[q][2 * e + 1]);
-            }
+            for (int e = 0; e < 8; ++e)
+              if (e < nv[q]) {
+                double re, im;
+                if constexpr (NS == 6) {
+                  re = scalbn((double)H[q][2 * e] + ((double)M3[q][2 * e] + (double)L[q][2 * e]), ex[q]);
+                  im = scalbn((double)H[q][2 * e + 1] + ((double)M3[q][2 * e + 1] + (double)L[q][2 * e + 1]), ex[q]);
+                } else {
+                  re = (double)H[q][2 * e] + (double)L[q][2 * e];
+                  im = (double)H[q][2 * e + 1] + (double)L[q][2 * e + 1];
+                }
+                o[(int64_t)(n0 + e) * d.sn] = make_double2(re, im);
+              }
           }
         } else {
-          float V[HO][16], mx[HO];
+          // largest component of each octet, as a value (NS = 3) or an exponent (NS = 6)
           bool valid[HO];
+          float mx[HO];
+          int ee[HO];
 #pragma unroll
           for (int q = 0; q < HO; ++q) {
             valid[q] = gi[q] < Gm && (STAGE == 0 ? rg < M : rw[q].dst >= 0);
             float mo[8];
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              V[q][e] = H[q][e] + L[q][e];
-              if (e & 1) mo[e >> 1] = fmaxf(fabsf(V[q][e - 1]), fabsf(V[q][e]));
-            }
+            for (int e = 0; e < 8; ++e)
+              mo[e] = NS == 3 ? fmaxf(fabsf(H[q][2 * e] + L[q][2 * e]), fabsf(H[q][2 * e + 1] + L[q][2 * e + 1]))
+                              : fmaxf(fabsf(H[q][2 * e]), fabsf(H[q][2 * e + 1]));
             mx[q] = fmaxf(fmaxf(fmaxf(mo[0], mo[1]), fmaxf(mo[2], mo[3])),
                           fmaxf(fmaxf(mo[4], mo[5]), fmaxf(mo[6], mo[7])));
-            if (!valid[q]) mx[q] = 0.f;
-          }
-          if (gs > 1) {  // octets that share an exponent
-            float mo = mx[0];
-#pragma unroll
-            for (int q = 1; q < HO; ++q) mo = fmaxf(mo, mx[q]);
-            if (gs > HO) {  // some are in the other warp of this lane quarter
-              gmax[tile & 1][half][row] = mo;
-              asm volatile("bar.sync %0, 64;" ::"r"(1 + lq) : "memory");
-              mo = fmaxf(mo, gmax[tile & 1][half ^ 1][row]);
+            ee[q] = mx[q] > 0.f || mx[q] != mx[q] ? oz_exponent(mx[q]) + ex[q] : OZ_ENONE;
+            if (!valid[q]) {
+              mx[q] = 0.f;
+              ee[q] = OZ_ENONE;
             }
-#pragma unroll
-            for (int q = 0; q < HO; ++q) mx[q] = mo;
           }
-          if constexpr (STAGE == 1)  // rows L of one K round share the exponent of their (tau, x)
-            for (int dlt = 1; dlt < (1 << glog); dlt <<= 1)
+          if (gs > HO) {  // octets that share the exponent are in other warps of this lane quarter
 #pragma unroll
-              for (int q = 0; q < HO; ++q) mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], dlt));
+            for (int q = 0; q < HO; ++q) gmax[tile & 1][os0 + q][row] = NS == 6 ? __int_as_float(ee[q]) : mx[q];
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + lq), "n"(32 * OCT / HO) : "memory");
+#pragma unroll
+            for (int q = 0; q < HO; ++q) {
+              const int g0 = os0 + q - oct[q] % gs;
+              for (int k = 0; k < gs; ++k) {
+                const float o = gmax[tile & 1][min(g0 + k, OCT - 1)][row];
+                if constexpr (NS == 6) {
+                  ee[q] = max(ee[q], __float_as_int(o));
+                } else {
+                  mx[q] = fmaxf(mx[q], o);
+                }
+              }
+            }
+          } else if (HO == 2 && gs == 2) {
+            mx[0] = mx[HO - 1] = fmaxf(mx[0], mx[HO - 1]);
+            ee[0] = ee[HO - 1] = max(ee[0], ee[HO - 1]);
+          }
+          if constexpr (STAGE == 1) {  // rows L of one K round share the exponent of their (tau, x)
+            for (int dlt = 1; dlt < (1 << glog); dlt <<= 1) {
+#pragma unroll
+              for (int q = 0; q < HO; ++q) {
+                if constexpr (NS == 6) {
+                  ee[q] = max(ee[q], __shfl_xor_sync(0xffffffffu, ee[q], dlt));
+                } else {
+                  mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], dlt));
+                }
+              }
+            }
+          }
 #pragma unroll
           for (int q = 0; q < HO; ++q) {
             if (!valid[q] || dead) continue;
@@ -555,22 +720,39 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_kernel(const OzArgs g) 
               blob += d2[q].base + (fr >> 7) * d2[q].fbytes + d2[q].kbase + (int64_t)Lg * d2[q].lgbytes;
               rr = fr & 127;
             }
-            const int e2 = oz_exponent(mx[q]);
-            const float f = oz_pow2(15 - e2), m1 = oz_m1(nksb);
             uint32_t w[NS][8];
+            float scale;
+            const int e2 = NS == 3 ? oz_exponent(mx[q]) : max(ee[q], -OZ_ELIM);
+            if constexpr (NS == 3) {
+              scale = oz_pow2(e2 - 15);
+            } else {
+              scale = __int_as_float(e2 - 8);
+            }
+            // NS = 6: 2^(8 - e2 + ex); e2 - ex is at least the exponent of an FP32 value
+            const float f = NS == 3 ? oz_pow2(15 - e2) : oz_pow2c(8 - e2 + ex[q]), m1 = oz_m1(nksb);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
+              if (e == 4 && nv[q] <= 4) {  // the second half is padding
+#pragma unroll
+                for (int p = 0; p < NS; ++p) w[p][4] = w[p][5] = w[p][6] = w[p][7] = 0u;
+                break;
+              }
               float sr[NS], si[NS];
-              oz_slice(H[q][2 * e], L[q][2 * e], V[q][2 * e], f, m1, sr);
-              oz_slice(H[q][2 * e + 1], L[q][2 * e + 1], V[q][2 * e + 1], f, m1, si);
+              if constexpr (NS == 3) {
+                oz_slice(H[q][2 * e], L[q][2 * e], H[q][2 * e] + L[q][2 * e], f, m1, sr);
+                oz_slice(H[q][2 * e + 1], L[q][2 * e + 1], H[q][2 * e + 1] + L[q][2 * e + 1], f, m1, si);
+              } else {
+                tri_digits({H[q][2 * e], M3[q][2 * e], L[q][2 * e]}, f, sr);
+                tri_digits({H[q][2 * e + 1], M3[q][2 * e + 1], L[q][2 * e + 1]}, f, si);
+              }
 #pragma unroll
               for (int p = 0; p < NS; ++p) w[p][e] = h2(sr[p], si[p]);
             }
-            char *o = blob + ks * SA + rr * 32;
+            char *o = blob + ks * (int)SA + rr * 32;
             const bool sw = (rr >> 2) & 1;
 #pragma unroll
             for (int p = 0; p < NS; ++p) st_octet(o + p * 4096, w[p], sw);
-            if (ks == 0) reinterpret_cast<float *>(blob + (int64_t)nksb * SA)[rr] = oz_pow2(e2 - 15);
+            if (ks == 0) reinterpret_cast<float *>(blob + (int64_t)nksb * SA)[rr] = scale;
           }
         }
         if constexpr (STAGE == 0) {  // the next row tile
@@ -613,7 +795,7 @@ __global__ void __launch_bounds__(128) oz_build_kernel(const OzBuild *__restrict
     const bool rv = r0 < t.rv && r1 < t.rn && q < nks;
     const double2 *s = src + t.src + r1 * t.rs1 + (int64_t)r0 * t.rs0;
     double2 v[8];
-    float m = 0.f;
+    double m = 0.0;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int k = 8 * q + e, k1 = k / t.kd, k0 = k - k1 * t.kd;
@@ -622,20 +804,49 @@ __global__ void __launch_bounds__(128) oz_build_kernel(const OzBuild *__restrict
         v[e] = s[k1 * t.ks1 + (int64_t)k0 * t.ks0];
         if (t.conj) v[e].y = -v[e].y;
       }
-      m = fmaxf(m, fmaxf(fabsf((float)v[e].x), fabsf((float)v[e].y)));
+      m = fmax(m, fmax(fabs(v[e].x), fabs(v[e].y)));
     }
 #pragma unroll
-    for (int d = 1; d < OCT; d <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-    const int e2 = oz_exponent(m);
-    const float f = oz_pow2(15 - e2), m1 = oz_m1(nks);
+    for (int d = 1; d < OCT; d <<= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, d));
+    int e2 = 0;
+    float f = 0.f, m1 = 0.f, scale;
+    double fd = 1.0;
+    if constexpr (NS == 3) {
+      e2 = oz_exponent((float)m);
+      f = oz_pow2(15 - e2);
+      m1 = oz_m1(nks);
+      scale = oz_pow2(e2 - 15);
+    } else {
+      // FP64's own exponent range; subnormal numbers count as the smallest normal exponent
+      const int be = (int)((__double_as_longlong(m) >> 52) & 0x7ff);
+      e2 = m > 0.0 ? max(be, 1) - 1022 : -OZ_ELIM;
+      scale = __int_as_float(e2 - 8);
+      // 2^-E
+      fd = !(m > 0.0) ? 0.0
+           : e2 < 1023 ? __longlong_as_double((long long)(1023 - e2) << 52)
+                       : 0x1p-1022 * (e2 == 1023 ? 0.5 : 0.25);
+    }
     if (q < nks) {
       uint32_t w[NS][8];
       float sr[8][NS], si[8][NS];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        const float hr = (float)v[e].x, hi = (float)v[e].y;
-        oz_slice(hr, (float)(v[e].x - (double)hr), hr, f, m1, sr[e]);
-        oz_slice(hi, (float)(v[e].y - (double)hi), hi, f, m1, si[e]);
+        if constexpr (NS == 3) {
+          const float hr = (float)v[e].x, hi = (float)v[e].y;
+          oz_slice(hr, (float)(v[e].x - (double)hr), hr, f, m1, sr[e]);
+          oz_slice(hi, (float)(v[e].y - (double)hi), hi, f, m1, si[e]);
+        } else {
+          const double xr = v[e].x * fd, xi = v[e].y * fd;  // exact, below 1
+          Tri a, b;
+          a.h = (float)xr;
+          a.m = (float)(xr - (double)a.h);
+          a.l = (float)((xr - (double)a.h) - (double)a.m);
+          b.h = (float)xi;
+          b.m = (float)(xi - (double)b.h);
+          b.l = (float)((xi - (double)b.h) - (double)b.m);
+          tri_digits(a, 256.f, sr[e]);
+          tri_digits(b, 256.f, si[e]);
+        }
       }
       if (!t.isb) {
 #pragma unroll
@@ -656,51 +867,63 @@ __global__ void __launch_bounds__(128) oz_build_kernel(const OzBuild *__restrict
           st_octet(o + 32, w[p], (lr >> 1) & 1);
         }
       }
-      if (q == 0) reinterpret_cast<float *>(blob + NS * nks * pstride)[lr] = oz_pow2(e2 - 15);
+      if (q == 0) reinterpret_cast<float *>(blob + NS * nks * pstride)[lr] = scale;
     }
   }
 }
 
 }  // namespace
 
+template <int NS>
+static void set_attributes() {
+  for (auto k : {oz_gemm_kernel<NS, 0, false>, oz_gemm_kernel<NS, 0, true>, oz_gemm_kernel<NS, 1, false>,
+                 oz_gemm_kernel<NS, 1, true>, oz_gemm_kernel<NS, 2, false>})
+    GWGB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
+}
+
 void set_oz_kernel_attributes() {
-  GWGB_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<3, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
-  GWGB_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
-  GWGB_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
+  set_attributes<3>();
+  set_attributes<6>();
 }
 
 // Stages 1 and 2 hold the column operand of a task (all K steps) and prefetch
-// the next task's; stage 3 streams both operands.
+// the next task's as far as three K steps of A leave room; stage 3 streams both.
 void oz_rings(int ns, int stage, int max_kos, OzArgs *a) {
-  const int slotA = ns * 4096, slotB = ns * 512 * OzCfg<3>::OCT;
+  const int slotA = ns * 4096, slotB = ns * 512 * OZ_OCT;
   if (stage == 2) {
     a->nA = a->nB = std::min(OZ_RING, OZ_SMEM / (slotA + slotB));
   } else {
-    a->nB = std::min(OZ_RING, 2 * max_kos);
+    a->nB = std::min({OZ_RING, 2 * max_kos, std::max(max_kos, (OZ_SMEM - 3 * slotA) / slotB)});
     a->nA = std::min(OZ_RING, (OZ_SMEM - a->nB * slotB) / slotA);
   }
   GWGB_REQUIRE(a->nA >= 2 && a->nB >= (stage == 2 ? 2 : max_kos), GWGB_E_UNSUPPORTED, "sliced GEMM rings too small");
 }
 
-void launch_oz_gemm(int ns, int stage, const OzArgs &a, int nsm, cudaStream_t st) {
+template <int NS>
+static void launch(int stage, bool multi, const OzArgs &a, int grid, cudaStream_t st) {
+  auto k = stage == 0 ? (multi ? oz_gemm_kernel<NS, 0, true> : oz_gemm_kernel<NS, 0, false>)
+           : stage == 1 ? (multi ? oz_gemm_kernel<NS, 1, true> : oz_gemm_kernel<NS, 1, false>)
+                        : oz_gemm_kernel<NS, 2, false>;
+  k<<<grid, oz_threads<NS>, OZ_SMEM, st>>>(a);
+}
+
+void launch_oz_gemm(int ns, int stage, bool multi, const OzArgs &a, int nsm, cudaStream_t st) {
   if (a.ntasks == 0) return;
-  (void)ns;
   const int grid = std::min(a.ntasks, std::max(1, nsm));
-  if (stage == 0)
-    oz_gemm_kernel<3, 0><<<grid, OZ_THREADS, OZ_SMEM, st>>>(a);
-  else if (stage == 1)
-    oz_gemm_kernel<3, 1><<<grid, OZ_THREADS, OZ_SMEM, st>>>(a);
+  if (ns == 3)
+    launch<3>(stage, multi, a, grid, st);
   else
-    oz_gemm_kernel<3, 2><<<grid, OZ_THREADS, OZ_SMEM, st>>>(a);
+    launch<6>(stage, multi, a, grid, st);
   GWGB_CUDA(cudaGetLastError());
 }
 
 void launch_oz_build(int ns, const OzBuild *tasks, int64_t ntasks, const double2 *src, char *dst, cudaStream_t st) {
-  (void)ns;
-  if (ntasks > 0) {
+  if (ntasks == 0) return;
+  if (ns == 3)
     oz_build_kernel<3><<<(unsigned)ntasks, 128, 0, st>>>(tasks, src, dst);
-    GWGB_CUDA(cudaGetLastError());
-  }
+  else
+    oz_build_kernel<6><<<(unsigned)ntasks, 128, 0, st>>>(tasks, src, dst);
+  GWGB_CUDA(cudaGetLastError());
 }
 
 }  // namespace gwgb

@@ -13,9 +13,10 @@
 // 8 complex ("octets"), 128 rows (A) or 16 rows per 8 complex columns (B, the
 // real embedding) per step, in the 32-byte swizzle of the shared-memory matrix
 // descriptors.  One image ("blob") covers at most OCT octets of K (one round:
-// one exponent per row) and carries one FP32 scale per row behind the planes:
-//   A blob: [step][plane][128 rows][32 B], float scale[128]
-//   B blob: [step][plane][16 noct rows][32 B], float scale[8 noct]
+// one exponent per row) and carries one scale per row behind the planes (NS = 3:
+// an FP32 factor, NS = 6: an int32 exponent, so that the range is that of FP64):
+//   A blob: [step][plane][128 rows][32 B], scale[128]
+//   B blob: [step][plane][16 noct rows][32 B], scale[8 noct]
 // so the GEMM moves blobs with bulk copies and does no work on its operands.
 #pragma once
 
@@ -27,11 +28,16 @@ constexpr int OZ_M = 128;   // rows per tile (TMEM lanes)
 // X1 + X2 of one chunk, when that is at most an eighth of the free memory.
 constexpr int64_t OZ_CHUNK_BYTES = 8ll << 30;
 
-// Geometry of one slicing: NS planes; OCT octets (of 8 complex) per round and per column tile.
+// Geometry of one slicing: NS planes; OCT octets (of 8 complex) per round and per column tile; NACC
+// accumulators of slice products up to class CMAX, SETS sets of them in TMEM; HO octets per drain thread.
 template <int NS> struct OzCfg;
 template <> struct OzCfg<3> {  // 33-bit operands: the split-precision path
-  static constexpr int OCT = 4, NACC = 4, CMAX = 3;
+  static constexpr int OCT = 4, NACC = 4, CMAX = 3, SETS = 2, HO = 2;
 };
+template <> struct OzCfg<6> {  // 57-bit operands: the FP64 contractions
+  static constexpr int OCT = 4, NACC = 7, CMAX = 6, SETS = 1, HO = 1;
+};
+constexpr int OZ_OCT = 4;
 
 __host__ __device__ constexpr int64_t oz_abytes(int ns, int nks) { return (int64_t)ns * nks * 4096 + 512; }
 // B blob bytes per octet of columns
@@ -52,7 +58,7 @@ struct OzCol1 {
   int32_t yoff;    // byte offset of the stage-2 round these columns are in
   int16_t x0;
   int8_t ngrp, gs;
-  int32_t pad;
+  int32_t ny;      // valid y of this round
 };
 // Where the stage-1 output of a contribution goes: stage-2 row slots
 //   group gi = gbase + x * nLg + (L >> glog), slot = (gi << glog) + (L & (2^glog - 1)),
@@ -67,7 +73,7 @@ struct OzS2 {
   int64_t b, bt, bz;       // B2 images: b + tau * bt + (column tile) * bz
   int32_t nt2, kos, zos, glog;
   int32_t rows;            // first entry of the row map
-  int32_t pad;
+  int32_t nz;              // valid z
 };
 struct OzRow { int32_t dst; int16_t x, L; };  // stage-2 row slot; dst < 0: empty
 // Where the stage-2 output of a contribution goes: final row tau * nx + x in
@@ -117,7 +123,8 @@ struct OzArgs {
 void set_oz_kernel_attributes();
 // Ring sizes of a launch; max_kos: most octets of K of its tasks (stages 1 and 2).
 void oz_rings(int ns, int stage, int max_kos, OzArgs *a);
-void launch_oz_gemm(int ns, int stage, const OzArgs &a, int nsm, cudaStream_t st);
+// multi (stages 1 and 2): the tasks have more than one round of K.
+void launch_oz_gemm(int ns, int stage, bool multi, const OzArgs &a, int nsm, cudaStream_t st);
 void launch_oz_build(int ns, const OzBuild *tasks, int64_t ntasks, const double2 *src, char *dst, cudaStream_t st);
 
 }  // namespace gwgb

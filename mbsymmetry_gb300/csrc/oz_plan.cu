@@ -10,6 +10,7 @@
 #include "oz_plan.h"
 
 #include <algorithm>
+#include <cstring>
 #include <map>
 #include <tuple>
 
@@ -43,8 +44,9 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
                    int64_t budget, int64_t persist_bytes, int nsm, int64_t nV, int64_t nG, int64_t nB2, int64_t nout,
                    cudaStream_t st) {
   ns_ = ns;
-  const int OCT = OzCfg<3>::OCT, NS = ns;
+  const int OCT = OZ_OCT, NS = ns;
   const int FK = 8 * OCT;  // complex K of a full round
+  const double nprod = ns == 3 ? 8 : 26;  // slice products per K step
   const int64_t fullA = oz_abytes(NS, OCT);
   launches_.clear();
   static_.clear();
@@ -330,7 +332,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
         l2.flops += 8.0 * rowsx * x.ny * x.nz;
         l3.flops += 8.0 * rowsx * x.nz * x.N;
       }
-      for (const OzRnd &q : rr) l3.ops += 16.0 * OZ_M * 16.0 * nos * 16.0 * q.nks * nf;
+      for (const OzRnd &q : rr) l3.ops += nprod * 2.0 * OZ_M * 16.0 * nos * 16.0 * q.nks * nf;
       // partials
       if (un.idx == 0)
         red.push_back({part, ow.out, ow.ostride, ow.N * ow.nx, 0, ntau, un.nunits, 0});
@@ -356,7 +358,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
       const int64_t t2b = (int64_t)NS * kos * 4096 + 512 * R;
       const B2 &b2 = b2_of[std::make_pair(x0.b2, (int)x0.b2conj)];
       const int id = (int)s2.size();
-      s2.push_back({x1, t2b, b2.b, b2.bt, b2.bz, nt2, kos, zos, gl, (int32_t)rows.size(), 0});
+      s2.push_back({x1, t2b, b2.b, b2.bt, b2.bz, nt2, kos, zos, gl, (int32_t)rows.size(), x0.nz});
       const size_t r0 = rows.size();
       rows.resize(r0 + (size_t)nt2 * OZ_M, OzRow{-1, 0, 0});
       for (int ui : p.cs) {
@@ -379,7 +381,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
       for (int t = 0; t < ntau; ++t)
         for (int zt = 0; zt < nzt; ++zt)
           for (int m = 0; m < nt2; m += per2) t2.push_back({id, t | zt << 16, m, std::min(per2, nt2 - m)});
-      l2.ops += 16.0 * OZ_M * 16.0 * zos * 16.0 * kos * nt2 * ntau;
+      l2.ops += nprod * 2.0 * OZ_M * 16.0 * zos * 16.0 * kos * nt2 * ntau;
     }
     x1_ = std::max(x1_, x1);
     // stage 1: column tiles of every use
@@ -395,7 +397,8 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
           const int gs = std::min(OCT, yos - yr * OCT), ng = OCT / gs;
           for (int xa = 0; xa < x.nx; xa += ng) {
             const int n = std::min(ng, x.nx - xa), noct = n * gs;
-            v.cols.push_back({voff, 0, (int32_t)(yr * fullA), (int16_t)xa, (int8_t)n, (int8_t)gs, 0});
+            v.cols.push_back({voff, 0, (int32_t)(yr * fullA), (int16_t)xa, (int8_t)n, (int8_t)gs,
+                              std::min(8 * gs, x.ny - yr * FK)});
             for (int r = 0; r < R; ++r) {
               const int nks = std::min(OCT, kos - r * OCT);
               builds.push_back({x.v + (int64_t)xa * x.sx + (int64_t)yr * FK * x.sy + (int64_t)r * FK * x.sk, voff, x.sx,
@@ -413,7 +416,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
         cl.dst = us.d1;
         t1.push_back({d, (int32_t)col1.size(), 0, nmt});
         col1.push_back(cl);
-        l1.ops += 16.0 * OZ_M * 16.0 * cl.ngrp * cl.gs * 16.0 * kos * nmt;
+        l1.ops += nprod * 2.0 * OZ_M * 16.0 * cl.ngrp * cl.gs * 16.0 * kos * nmt;
       }
       m_kos1 = std::max(m_kos1, kos);
     }
@@ -434,13 +437,25 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
       l.kind = 0;
       l.t0 = (int64_t)tasks.size();
       l.n = (int64_t)t.size();
+      if (t.empty()) return;
       tasks.insert(tasks.end(), t.begin(), t.end());
       oz_rings(NS, stage, kos, &l.args);
       l.d0 = stage;
       launches_.push_back(l);
     };
-    add_gemm(l1, t1, 0, m_kos1);
-    add_gemm(l2, t2, 1, m_kos2);
+    // tasks of one round of K, then those of more; the launch statistics go with the larger list
+    auto split = [&](OzLaunch l, std::vector<OzTask> &t, int stage, int kos, auto &&kos_of) {
+      auto mid = std::stable_partition(t.begin(), t.end(), [&](const OzTask &k) { return kos_of(k) <= OCT; });
+      const std::vector<OzTask> one(t.begin(), mid), more(mid, t.end());
+      OzLaunch lm = l;
+      lm.multi = true;
+      OzLaunch &rest = one.size() >= more.size() ? lm : l;
+      rest.flops = rest.ops = 0;
+      add_gemm(l, one, stage, std::min(kos, OCT));
+      add_gemm(lm, more, stage, kos);
+    };
+    split(l1, t1, 0, m_kos1, [&](const OzTask &k) { return s1[k.d].kos; });
+    split(l2, t2, 1, m_kos2, [&](const OzTask &k) { return s2[k.d].kos; });
     add_gemm(l3, t3, 2, 1);
     for (size_t s = s3_0; s < s3.size(); ++s) {
       check_range(s3[s].a, (int64_t)cdiv(s3[s].M, OZ_M) * s3[s].fbytes, x2, "sliced X2 unit");
@@ -460,17 +475,27 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
   GWGB_REQUIRE(tasks.size() < (size_t)INT32_MAX && rows.size() < (size_t)INT32_MAX && rnd.size() < (size_t)INT32_MAX &&
                    col1.size() < (size_t)INT32_MAX,
                GWGB_E_UNSUPPORTED, "too many sliced GEMM tasks");
-  builds_.upload(builds, st);
-  tasks_.upload(tasks, st);
-  s1_.upload(s1, st);
-  col1_.upload(col1, st);
-  dst1_.upload(dst1, st);
-  s2_.upload(s2, st);
-  rows_.upload(rows, st);
-  dst2_.upload(dst2, st);
-  s3_.upload(s3, st);
-  rnd_.upload(rnd, st);
-  red_.upload(red, st);
+  // one allocation for all lists: each separate one cost about as much as building it
+  size_t total = 0;
+  auto place = [&](const auto &v, auto &l) {
+    total = (total + 255) / 256 * 256;
+    l.n = v.size();
+    l.p = reinterpret_cast<decltype(l.p)>(total);  // its offset, until the buffer exists
+    total += v.size() * sizeof(v[0]);
+  };
+  auto each = [&](auto &&f) {
+    f(builds, builds_); f(tasks, tasks_); f(s1, s1_); f(col1, col1_); f(dst1, dst1_); f(s2, s2_); f(rows, rows_);
+    f(dst2, dst2_); f(s3, s3_); f(rnd, rnd_); f(red, red_);
+  };
+  each(place);
+  std::vector<char> host(total);
+  lists_.alloc(total);
+  each([&](const auto &v, auto &l) {
+    const size_t off = reinterpret_cast<size_t>(l.p);
+    if (!v.empty()) std::memcpy(host.data() + off, v.data(), v.size() * sizeof(v[0]));
+    l.p = reinterpret_cast<decltype(l.p)>(lists_.p + off);
+  });
+  if (total) GWGB_CUDA(cudaMemcpyAsync(lists_.p, host.data(), total, cudaMemcpyHostToDevice, st));
   GWGB_CUDA(cudaStreamSynchronize(st));
 }
 
@@ -516,12 +541,12 @@ void OzPlan::run_one(const OzLaunch &l, OzShared &sh, const double2 *V, const do
     a.B = V_.p;
     a.X = nullptr;
   }
-  launch_oz_gemm(ns_, (int)l.d0, a, nsm, st);
+  launch_oz_gemm(ns_, (int)l.d0, l.multi, a, nsm, st);
 }
 
 void OzPlan::free() {
-  V_.free(); builds_.free(); tasks_.free(); s1_.free(); col1_.free(); dst1_.free(); s2_.free(); rows_.free();
-  dst2_.free(); s3_.free(); rnd_.free(); red_.free();
+  V_.free();
+  lists_.free();
   launches_.clear();
   static_.clear();
 }

@@ -39,6 +39,7 @@ struct OzLaunch {
   int64_t d0 = 0;              // descriptors / auxiliary lists of the launch
   int src = 0, dst = 0;        // builds: source (0 V, 1 G, 2 B2 source) and image buffer
   OzArgs args{};               // rings (pointers are filled in when it runs)
+  bool multi = false;          // stages 1, 2: tasks of more than one round of K
   int ny = 1;                  // reductions: CTAs per task
   double flops = 0, ops = 0, bytes = 0;
 };
@@ -79,17 +80,23 @@ class OzPlan {
   int64_t vimg_ = 0, a1_ = 0, b2_ = 0, x1_ = 0, x2_ = 0, part_ = 0;
   std::vector<OzLaunch> launches_, static_;
   DBuf<char> V_;
-  DBuf<OzBuild> builds_;
-  DBuf<OzTask> tasks_;
-  DBuf<OzS1> s1_;
-  DBuf<OzCol1> col1_;
-  DBuf<OzDst1> dst1_;
-  DBuf<OzS2> s2_;
-  DBuf<OzRow> rows_;
-  DBuf<OzDst2> dst2_;
-  DBuf<OzS3> s3_;
-  DBuf<OzRnd> rnd_;
-  DBuf<RedTask> red_;
+  // the work lists, one allocation
+  template <typename T> struct List {
+    T *p = nullptr;
+    size_t n = 0;
+  };
+  DBuf<char> lists_;
+  List<OzBuild> builds_;
+  List<OzTask> tasks_;
+  List<OzS1> s1_;
+  List<OzCol1> col1_;
+  List<OzDst1> dst1_;
+  List<OzS2> s2_;
+  List<OzRow> rows_;
+  List<OzDst2> dst2_;
+  List<OzS3> s3_;
+  List<OzRnd> rnd_;
+  List<RedTask> red_;
 };
 
 }  // namespace gwgb
