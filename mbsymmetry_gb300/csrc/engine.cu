@@ -12,6 +12,7 @@
 #include <cstddef>
 #include <cstdlib>
 #include <cstring>
+#include <future>
 #include <map>
 #include <mutex>
 #include <numeric>
@@ -386,7 +387,7 @@ class Engine {
       built = true;
     }
     build_oz();
-    if (OzSet *o = oz_set(); o && !o->ready) {
+    if (OzSet *o = oz_set(); o && alloc_oz(*o) && !o->ready) {
       o->plan[0].build_static(V_.p, st_);
       o->plan[1].build_static(Vt_.p, st_);
       o->ready = true;
@@ -405,13 +406,26 @@ class Engine {
   // slices (GWGB_PREC_OZAKI) and in six (GWGB_PREC_FP64), and their shared buffers.
   // The FP64 FMA kernels are left for what the six slices do not serve: memory too
   // small for the images (off), and contractions too small to fill the GPU.
+  // tau <-> omega transforms in six slices; a transform without its plan (memory, no slabs) runs in FP64 FMAs
+  enum { XF_P0, XF_P, XF_SIGMA, XF_G, XF_E, XF_N };
+  OzTransform xf_[XF_N];
+  DBuf<char> xf_img_;
+  void build_xf(int which, const std::vector<TSlab> &slabs, int nout, int nin, int row0, int64_t nX, int64_t nY);
+  void transform(int which, const DBuf<TSlab> &slabs, int max_cols, const double2 *T, int nout, int nin, int row0,
+                 const double2 *X, double2 *Y) {
+    if (xf_[which].ready)
+      xf_[which].run(X, Y, xf_img_.p, nsm_, bad_.p + 2, st_);
+    else
+      launch_transform(slabs.p, (int)slabs.n, max_cols, T, nout, nin, row0, X, Y, st_);
+  }
   struct OzSet {
     OzPlan plan[2];
-    bool built = false, ready = false, off = false;
+    bool built = false, alloc = false, ready = false, off = false;
   };
   OzSet oz_[2];
   OzShared oz_buf_;
   void build_oz();
+  bool alloc_oz(OzSet &set);
   OzSet *oz_set() {  // the set that runs the contractions, if one does
     OzSet *o = prec_ == GWGB_PREC_OZAKI ? &oz_[0] : prec_ == GWGB_PREC_FP64 ? &oz_[1] : nullptr;
     return o && o->built && !o->off ? o : nullptr;
@@ -667,6 +681,8 @@ Engine::~Engine() {
   pz_tasks_.free(); vc_tasks_.free(); pk_tiles_.free(); pr_tiles_.free(); Zbuf_.free(); Vcat_.free(); Ppart_.free();
   for (OzSet &o : oz_) o.plan[0].free(), o.plan[1].free();
   oz_buf_.free();
+  for (OzTransform &x : xf_) x.free();
+  xf_img_.free();
   for (auto *b : bufs) b->free();
   tct_f_.free(); tct_l_.free(); mu_dev_.free(); ws_.free(); bad_.free(); leak_.free();
   qoff_irr_.free(); qsz_irr_.free();
@@ -1373,6 +1389,10 @@ void Engine::build_work_lists() {
   slab_p_bwd_.upload(pb, st_);
   slab_s_fwd_.upload(sf, st_);
   slab_g_bwd_.upload(gb, st_);
+  build_xf(XF_P0, pf, nw_b_, ncheb_, 1, (int64_t)nts_ * fq, (int64_t)nw_b_ * fq);
+  build_xf(XF_P, pb, nts_, nw_b_, 0, (int64_t)nw_b_ * fq, (int64_t)nts_ * fq);
+  build_xf(XF_SIGMA, sf, nw_, ncheb_, 1, (int64_t)nts_ * ns_ * fa, (int64_t)nw_ * ns_ * fa);
+  build_xf(XF_G, gb, nts_, nw_, 0, (int64_t)nw_ * ns_ * fa, (int64_t)nts_ * ns_ * fa);
   {  // traces over the stored k (weight = mesh k mapped to each) and the M G slabs
     std::vector<double> wk(ink, 0.0);
     for (int k = 0; k < nk; ++k) wk[l.irre_index[k]] += 1.0;
@@ -1387,6 +1407,7 @@ void Engine::build_work_lists() {
       }
     tr_tasks_.upload(tt, st_);
     slab_e_.upload(se, st_);
+    build_xf(XF_E, se, ncheb_, ncheb_, 1, (int64_t)nts_ * ns_ * fa, (int64_t)ncheb_ * ns_ * fa);
   }
   {
     const int64_t gsz = (int64_t)nts_ * ns_ * fa, wsz = (int64_t)nw_ * ns_ * fa, pwsz = (int64_t)nw_b_ * fq;
@@ -1439,6 +1460,55 @@ void Engine::build_work_lists() {
 // ---------------------------------------------------------------------------
 // sliced (Ozaki) path: the two contractions as chains of block GEMMs (oz_plan.h)
 // ---------------------------------------------------------------------------
+// The images and work buffers of the active set, on its first use (a handle that only solves
+// Dyson or W~ never needs them).  False: no memory (FP64 falls back to the FMA kernels).
+bool Engine::alloc_oz(OzSet &set) {
+  if (set.alloc) return true;
+  const OzPlan &p = set.plan[0], &s = set.plan[1];
+  drop_graphs();  // they may hold the addresses of smaller buffers
+  auto grow = [](auto &buf, int64_t a, int64_t b) {
+    const int64_t m = std::max(a, b);
+    if (m > (int64_t)buf.n) buf.alloc((size_t)m);
+  };
+  try {
+    set.plan[0].alloc_images();
+    set.plan[1].alloc_images();
+    grow(oz_buf_.A1, p.bytes_A1(), s.bytes_A1());
+    grow(oz_buf_.B2, p.bytes_B2(), s.bytes_B2());
+    grow(oz_buf_.X1, p.bytes_X1(), s.bytes_X1());
+    grow(oz_buf_.X2, p.bytes_X2(), s.bytes_X2());
+    grow(oz_buf_.part, p.part_elems(), s.part_elems());
+  } catch (const Error &e) {
+    if (&set != &oz_[1] || e.code != GWGB_E_NOMEM) throw;
+    cudaGetLastError();
+    set.off = true;
+    set.plan[0].free();
+    set.plan[1].free();
+    oz_buf_.free();
+    oz_[0].alloc = oz_[0].ready = false;  // its buffers, too, are allocated again on its next use
+    return false;
+  }
+  set.alloc = true;
+  return true;
+}
+
+void Engine::build_xf(int which, const std::vector<TSlab> &slabs, int nout, int nin, int row0, int64_t nX, int64_t nY) {
+  // below 40 MFLOP the FP64 kernel's single launch is the shorter one (s+p: 15 to 30 us against 22 and up);
+  // 12000 columns at 120 points: 1.28 ms there, 0.20 here
+  double flops = 0;
+  for (const TSlab &x : slabs) flops += 8.0 * x.ncols * nout * nin;
+  if (flops < 4e7) return;
+  xf_[which].build(slabs, nout, nin, row0, nX, nY, nsm_, st_);
+  if (!xf_[which].built() || xf_[which].bytes_A() <= (int64_t)xf_img_.n) return;
+  size_t free_b = 0, total_b = 0;
+  GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  if (xf_[which].bytes_A() > (int64_t)(free_b / 16)) {
+    xf_[which].free();
+    return;
+  }
+  xf_img_.alloc((size_t)xf_[which].bytes_A());
+}
+
 void Engine::build_oz() {
   if (prec_ != GWGB_PREC_OZAKI && prec_ != GWGB_PREC_FP64) return;
   const bool f64 = prec_ == GWGB_PREC_FP64;
@@ -1478,8 +1548,11 @@ void Engine::build_oz() {
       }
     own.push_back({g.pout, g.pstride, g.qb, g.qb, g.qb, 1, c0, (int32_t)cs.size()});
   }
-  set.plan[0].build(NS, cs, own, nts / 2, 0, budget, persist, nsm_, l.flat_V, (int64_t)Gall_.n, (int64_t)Gall_.n,
-                    (int64_t)Pall_.n, st_);
+  // the lists of the two contractions are built side by side
+  auto p0_built = std::async(std::launch::async, [&set, cs, own, NS, nts, budget, persist, this] {
+    set.plan[0].build(NS, cs, own, nts / 2, 0, budget, persist / 2, nsm_, l_.flat_V, (int64_t)Gall_.n, (int64_t)Gall_.n,
+                      (int64_t)Pall_.n);
+  });
   // Sigma[i][j] = sum Vt[Q][i][m] G2(tau)[m][n] P~(tau)[Q][P] conj(Vt[P][j][n])
   cs.clear();
   own.clear();
@@ -1500,8 +1573,9 @@ void Engine::build_oz() {
     }
     own.push_back({ow.out, ow.ostride, ow.n, ow.n, 1, ow.n, c0, (int32_t)cs.size()});
   }
-  set.plan[1].build(NS, cs, own, nts, 3, budget, std::max<int64_t>(0, persist - set.plan[0].bytes_V()), nsm_,
-                    (int64_t)Vt_.n, (int64_t)Gall_.n, (int64_t)Pall_.n, (int64_t)nts * ns * l.flat_ao, st_);
+  set.plan[1].build(NS, cs, own, nts, 3, budget, persist / 2, nsm_, (int64_t)Vt_.n, (int64_t)Gall_.n, (int64_t)Pall_.n,
+                    (int64_t)nts * ns * l.flat_ao);
+  p0_built.get();
   {  // the buffers (shared with the other set, if it is built) must fit the free memory
     const OzPlan &p = set.plan[0], &s = set.plan[1];
     auto grow = [](int64_t a, int64_t b, size_t have) {
@@ -1543,14 +1617,8 @@ void Engine::build_oz() {
     GWGB_REQUIRE(fits, GWGB_E_UNSUPPORTED,
                  "sliced-precision buffers need " + std::to_string(tot >> 20) + " MB (" + msg + " ), " +
                      std::to_string(free_b >> 20) + " MB free");
-    if (a1 || b2 || x1 || x2 || part) drop_graphs();  // they hold the old buffers' addresses
-    set.plan[0].alloc_images();
-    set.plan[1].alloc_images();
-    if (a1) oz_buf_.A1.alloc((size_t)a1);
-    if (b2) oz_buf_.B2.alloc((size_t)b2);
-    if (x1) oz_buf_.X1.alloc((size_t)x1);
-    if (x2) oz_buf_.X2.alloc((size_t)x2);
-    if (part) oz_buf_.part.alloc((size_t)part);
+    set.plan[0].upload(st_);
+    set.plan[1].upload(st_);
   }
   set.ready = false;
   lt_build();
@@ -1608,6 +1676,10 @@ void Engine::set_transforms(const double *Tnt, const double *Ttn, const double *
     h2d(tct_f_.p, tf, ncheb_ * sizeof(double), st_);
     h2d(tct_l_.p, tl, ncheb_ * sizeof(double), st_);
   }
+  const double2 *T[XF_E] = {TntBF_.p, TtnFB_.p, Tnt_.p, Ttn_.p};
+  const double *Th[XF_E] = {TntBF, TtnFB, Tnt, Ttn};
+  for (int i = 0; i < XF_E; ++i)
+    if (xf_[i].built()) xf_[i].set_matrix(Th[i], T[i], st_);
   GWGB_CUDA(cudaStreamSynchronize(st_));
   have_T_ = true;
 }
@@ -1675,11 +1747,11 @@ void Engine::k_p0(int mirror) {
 void Engine::k_pq(bool mirror_first) {
   if (mirror_first) launch_mirror(Pall_.p, qoff_irr_.p, qsz_irr_.p, l_.ink, nts_, st_);
   record(8);
-  launch_transform(slab_p_fwd_.p, (int)slab_p_fwd_.n, max_cols_p_, TntBF_.p, nw_b_, ncheb_, 1, Pall_.p, Pw_.p, st_);
+  transform(XF_P0, slab_p_fwd_, max_cols_p_, TntBF_.p, nw_b_, ncheb_, 1, Pall_.p, Pw_.p);
   record(9);
   launch_inverse(inv_w_.p, (int)inv_w_.n, l_.max_aux, Pw_.p, nullptr, nullptr, nullptr, beta_, 0.0, 0, bad_.p, st_);
   record(10);
-  launch_transform(slab_p_bwd_.p, (int)slab_p_bwd_.n, max_cols_p_, TtnFB_.p, nts_, nw_b_, 0, Pw_.p, Pall_.p, st_);
+  transform(XF_P, slab_p_bwd_, max_cols_p_, TtnFB_.p, nts_, nw_b_, 0, Pw_.p, Pall_.p);
   record(11);
 }
 
@@ -1707,9 +1779,9 @@ void Engine::k_sigma() {
 }
 
 void Engine::k_dyson() {
-  launch_transform(slab_s_fwd_.p, (int)slab_s_fwd_.n, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p, st_);
+  transform(XF_SIGMA, slab_s_fwd_, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p);
   launch_inverse(inv_d_.p, (int)inv_d_.n, l_.max_ao, Ww_.p, S_.p, F_.p, ws_.p, beta_, 0.0, 1, bad_.p + 1, st_);
-  launch_transform(slab_g_bwd_.p, (int)slab_g_bwd_.n, max_cols_g_, Ttn_.p, nts_, nw_, 0, Ww_.p, Gall_.p, st_);
+  transform(XF_G, slab_g_bwd_, max_cols_g_, Ttn_.p, nts_, nw_, 0, Ww_.p, Gall_.p);
   if (has_tct_) {
     GWGB_CUDA(cudaMemsetAsync(leak_.p, 0, 2 * sizeof(unsigned long long), st_));
     launch_leakage(slab_g_bwd_.p, (int)slab_g_bwd_.n, Gall_.p, tct_f_.p, tct_l_.p, ncheb_, leak_.p, st_);
@@ -1872,11 +1944,11 @@ void Engine::dyson(double mu) {
   GWGB_REQUIRE(have_F_, GWGB_E_STATE, "F and S have not been set");
   // mu enters the inverse kernel by value here (no graph)
   record(5);
-  launch_transform(slab_s_fwd_.p, (int)slab_s_fwd_.n, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p, st_);
+  transform(XF_SIGMA, slab_s_fwd_, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p);
   record(12);
   launch_inverse(inv_d_.p, (int)inv_d_.n, l_.max_ao, Ww_.p, S_.p, F_.p, ws_.p, beta_, mu, 1, bad_.p + 1, st_);
   record(13);
-  launch_transform(slab_g_bwd_.p, (int)slab_g_bwd_.n, max_cols_g_, Ttn_.p, nts_, nw_, 0, Ww_.p, Gall_.p, st_);
+  transform(XF_G, slab_g_bwd_, max_cols_g_, Ttn_.p, nts_, nw_, 0, Ww_.p, Gall_.p);
   record(14);
   if (has_tct_) {
     GWGB_CUDA(cudaMemsetAsync(leak_.p, 0, 2 * sizeof(unsigned long long), st_));
@@ -1911,11 +1983,11 @@ void Engine::iteration(double mu) {
     record(4);
     k_sigma();
     record(5);
-    launch_transform(slab_s_fwd_.p, (int)slab_s_fwd_.n, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p, st_);
+    transform(XF_SIGMA, slab_s_fwd_, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p);
     record(12);
     launch_inverse(inv_d_.p, (int)inv_d_.n, l_.max_ao, Ww_.p, S_.p, F_.p, ws_.p, beta_, mu, 1, bad_.p + 1, st_);
     record(13);
-    launch_transform(slab_g_bwd_.p, (int)slab_g_bwd_.n, max_cols_g_, Ttn_.p, nts_, nw_, 0, Ww_.p, Gall_.p, st_);
+    transform(XF_G, slab_g_bwd_, max_cols_g_, Ttn_.p, nts_, nw_, 0, Ww_.p, Gall_.p);
     record(14);
     if (has_tct_) {
       GWGB_CUDA(cudaMemsetAsync(leak_.p, 0, 2 * sizeof(unsigned long long), st_));
@@ -1959,6 +2031,7 @@ void Engine::set_energy_matrix(const double *M, int n) {
   for (size_t i = 0; i < m.size(); ++i) m[i] = make_double2(M[i], 0.0);
   if (!Me_.p) Me_.alloc(m.size());
   h2d(Me_.p, m.data(), m.size() * sizeof(double2), st_);
+  if (xf_[XF_E].built()) xf_[XF_E].set_matrix(&m[0].x, Me_.p, st_);
   GWGB_CUDA(cudaStreamSynchronize(st_));
   if (!have_M_) drop_graphs();
   have_M_ = true;
@@ -2001,7 +2074,7 @@ void Engine::k_mu_search(const gwgb_mu_search &ms) {
 void Engine::k_dyson_dev() {
   launch_inverse(inv_d_.p, (int)inv_d_.n, l_.max_ao, Ww_.p, S_.p, F_.p, ws_.p, beta_, 0.0, 1, bad_.p + 1, st_,
                  mu_dev_.p);
-  launch_transform(slab_g_bwd_.p, (int)slab_g_bwd_.n, max_cols_g_, Ttn_.p, nts_, nw_, 0, Ww_.p, Gall_.p, st_);
+  transform(XF_G, slab_g_bwd_, max_cols_g_, Ttn_.p, nts_, nw_, 0, Ww_.p, Gall_.p);
   if (has_tct_) {
     GWGB_CUDA(cudaMemsetAsync(leak_.p, 0, 2 * sizeof(unsigned long long), st_));
     launch_leakage(slab_g_bwd_.p, (int)slab_g_bwd_.n, Gall_.p, tct_f_.p, tct_l_.p, ncheb_, leak_.p, st_);
@@ -2010,7 +2083,7 @@ void Engine::k_dyson_dev() {
 
 void Engine::k_energy_record(bool with_energy) {
   if (with_energy)
-    launch_transform(slab_e_.p, (int)slab_e_.n, max_cols_g_, Me_.p, ncheb_, ncheb_, 1, Gall_.p, Hm_.p, st_);
+    transform(XF_E, slab_e_, max_cols_g_, Me_.p, ncheb_, ncheb_, 1, Gall_.p, Hm_.p);
   EnergyArgs a{};
   a.tasks = tr_tasks_.p;
   a.ntasks = (int)tr_tasks_.n;
@@ -2041,7 +2114,7 @@ void Engine::k_sc_iteration(double alpha, const gwgb_mu_search &ms) {
   k_pq(false);
   k_sigma();
   launch_mix(Sig_.p, Sold_.p, (int64_t)Sig_.n, alpha, st_);
-  launch_transform(slab_s_fwd_.p, (int)slab_s_fwd_.n, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p, st_);
+  transform(XF_SIGMA, slab_s_fwd_, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p);
   k_mu_search(ms);
   k_dyson_dev();
   k_energy_record(have_M_);
@@ -2080,7 +2153,7 @@ void Engine::find_mu(const gwgb_mu_search &ms, double *mu_out, double *n_out) {
   check_mu_search(ms);
   init_mu_state(ms);
   record(5);
-  launch_transform(slab_s_fwd_.p, (int)slab_s_fwd_.n, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p, st_);
+  transform(XF_SIGMA, slab_s_fwd_, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p);
   k_mu_search(ms);
   k_dyson_dev();
   k_energy_record(false);

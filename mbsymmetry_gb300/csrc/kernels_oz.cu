@@ -224,7 +224,7 @@ template <int NS, int STAGE> struct Job {
       kos = 0;
       R = d.nkr;
       outer = t.n;
-      noct = min(OCT, (d.N + 7) / 8 - ct * OCT);
+      noct = min(d.oct, (d.N + 7) / 8 - ct * d.oct);
       atile = d.fbytes;
       a = g.A + d.a + f * d.fbytes;
       b = g.B + d.b + ct * d.bz;
@@ -515,8 +515,10 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
         }
       } else {
 #pragma unroll
-        for (int q = 0; q < HO; ++q)
-          nv[q] = static_cast<const OzS3 *>(g.desc)[tk.d].N - 8 * ((tk.i >> 16) * OCT + oct[q]);
+        for (int q = 0; q < HO; ++q) {
+          const OzS3 &d = static_cast<const OzS3 *>(g.desc)[tk.d];
+          nv[q] = d.N - 8 * ((tk.i >> 16) * d.oct + oct[q]);
+        }
       }
       for (int m0 = 0; m0 < job.outer; m0 += job.G, ++tile) {
         const int Gm = min(job.G, job.outer - m0);
@@ -779,11 +781,51 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
   if (warp == 0) tc::tmem_dealloc(tm, 512);
 }
 
+// The six digits of x relative to 2^E, |x| < 2^E, from its bits: x 2^(60-E) as a 64-bit integer
+// (rounded towards zero: below 2^(E-60)), digits of 9 bits from the top, the last one with 7 bits of
+// fraction.  Infinities and NaN give NaN.
+__device__ __forceinline__ void double_digits(double x, int e2, float (&s)[6]) {
+  const long long b = __double_as_longlong(x);
+  const int be = (int)((b >> 52) & 0x7ff);
+  long long m = b & 0xfffffffffffffll;
+  if (be) m |= 1ll << 52;
+  const int sh = e2 + 1022 - max(be, 1);  // x = m 2^(max(be, 1) - 1075): F = m 2^(7 - sh)
+  long long F = sh <= 7 ? m << (7 - sh) : sh < 64 ? m >> (sh - 7) : 0ll;
+  if (b < 0) F = -F;
+  auto digit = [](int d) { return __int_as_float(0x4b400000 + d) - 12582912.f; };  // |d| < 2^22, exact
+#pragma unroll
+  for (int p = 0; p < 5; ++p) {
+    const int k = 52 - 9 * p;
+    const int d = (int)((F + (1ll << (k - 1))) >> k);
+    F -= (long long)d << k;
+    s[p] = digit(d);
+  }
+  s[5] = digit((int)F) * 0x1p-7f;
+  if (be == 0x7ff) s[0] = __int_as_float(0x7fffffff);
+}
+
+// Element k of row source s of an image (zero outside).
+__device__ __forceinline__ double2 load(const double2 *__restrict__ s, const OzBuild &t, bool rv, int k,
+                                        const double *__restrict__ scale) {
+  double2 v = make_double2(0.0, 0.0);
+  const int k1 = k / t.kd, k0 = k - k1 * t.kd;
+  if (rv && k0 < t.kv && k1 < t.kn) {
+    v = s[k1 * t.ks1 + (int64_t)k0 * t.ks0];
+    if (t.conj) v.y = -v.y;
+    if (t.kx >= 0) {
+      const double f = scale[t.kx + k];
+      v = make_double2(v.x * f, v.y * f);
+    }
+  }
+  return v;
+}
+
 // Operand images from FP64 data: one CTA per image, OCT lanes per row (one
 // octet each), the row's exponent by a shuffle over them.
 template <int NS>
 __global__ void __launch_bounds__(128) oz_build_kernel(const OzBuild *__restrict__ tasks,
-                                                       const double2 *__restrict__ src, char *__restrict__ dst) {
+                                                       const double2 *__restrict__ src, char *__restrict__ dst,
+                                                       const double *__restrict__ scale_k) {
   constexpr int OCT = OzCfg<NS>::OCT;
   const OzBuild t = tasks[blockIdx.x];
   const int q = threadIdx.x % OCT;
@@ -795,36 +837,36 @@ __global__ void __launch_bounds__(128) oz_build_kernel(const OzBuild *__restrict
     const bool rv = r0 < t.rv && r1 < t.rn && q < nks;
     const double2 *s = src + t.src + r1 * t.rs1 + (int64_t)r0 * t.rs0;
     double2 v[8];
-    double m = 0.0;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int k = 8 * q + e, k1 = k / t.kd, k0 = k - k1 * t.kd;
-      v[e] = make_double2(0.0, 0.0);
-      if (rv && k0 < t.kv && k1 < t.kn) {
-        v[e] = s[k1 * t.ks1 + (int64_t)k0 * t.ks0];
-        if (t.conj) v[e].y = -v[e].y;
-      }
-      m = fmax(m, fmax(fabs(v[e].x), fabs(v[e].y)));
-    }
-#pragma unroll
-    for (int d = 1; d < OCT; d <<= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, d));
-    int e2 = 0;
+    int e2;        // the row's exponent
     float f = 0.f, m1 = 0.f, scale;
-    double fd = 1.0;
     if constexpr (NS == 3) {
-      e2 = oz_exponent((float)m);
+      float m = 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        v[e] = load(s, t, rv, 8 * q + e, scale_k);
+        m = fmaxf(m, fmaxf(fabsf((float)v[e].x), fabsf((float)v[e].y)));
+      }
+#pragma unroll
+      for (int d = 1; d < OCT; d <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+      e2 = oz_exponent(m);
       f = oz_pow2(15 - e2);
       m1 = oz_m1(nks);
       scale = oz_pow2(e2 - 15);
     } else {
-      // FP64's own exponent range; subnormal numbers count as the smallest normal exponent
-      const int be = (int)((__double_as_longlong(m) >> 52) & 0x7ff);
-      e2 = m > 0.0 ? max(be, 1) - 1022 : -OZ_ELIM;
-      scale = __int_as_float(e2 - 8);
-      // 2^-E
-      fd = !(m > 0.0) ? 0.0
-           : e2 < 1023 ? __longlong_as_double((long long)(1023 - e2) << 52)
-                       : 0x1p-1022 * (e2 == 1023 ? 0.5 : 0.25);
+      // FP64's own exponent range, by integer operations (the FP64 pipe is 64 times slower)
+      int be = 0;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        v[e] = load(s, t, rv, 8 * q + e, scale_k);
+        const int hx = __double2hiint(v[e].x) & 0x7fffffff, hy = __double2hiint(v[e].y) & 0x7fffffff;
+        // subnormal numbers have the smallest normal number's exponent; zero has none
+        be = max(be, max(hx >> 20, hy >> 20));
+        if ((hx | hy | __double2loint(v[e].x) | __double2loint(v[e].y)) != 0) be = max(be, 1);
+      }
+#pragma unroll
+      for (int d = 1; d < OCT; d <<= 1) be = max(be, __shfl_xor_sync(0xffffffffu, be, d));
+      e2 = be - 1022;
+      scale = __int_as_float((be ? e2 : -OZ_ELIM) - 8);
     }
     if (q < nks) {
       uint32_t w[NS][8];
@@ -836,16 +878,8 @@ __global__ void __launch_bounds__(128) oz_build_kernel(const OzBuild *__restrict
           oz_slice(hr, (float)(v[e].x - (double)hr), hr, f, m1, sr[e]);
           oz_slice(hi, (float)(v[e].y - (double)hi), hi, f, m1, si[e]);
         } else {
-          const double xr = v[e].x * fd, xi = v[e].y * fd;  // exact, below 1
-          Tri a, b;
-          a.h = (float)xr;
-          a.m = (float)(xr - (double)a.h);
-          a.l = (float)((xr - (double)a.h) - (double)a.m);
-          b.h = (float)xi;
-          b.m = (float)(xi - (double)b.h);
-          b.l = (float)((xi - (double)b.h) - (double)b.m);
-          tri_digits(a, 256.f, sr[e]);
-          tri_digits(b, 256.f, si[e]);
+          double_digits(v[e].x, e2, sr[e]);
+          double_digits(v[e].y, e2, si[e]);
         }
       }
       if (!t.isb) {
@@ -917,12 +951,13 @@ void launch_oz_gemm(int ns, int stage, bool multi, const OzArgs &a, int nsm, cud
   GWGB_CUDA(cudaGetLastError());
 }
 
-void launch_oz_build(int ns, const OzBuild *tasks, int64_t ntasks, const double2 *src, char *dst, cudaStream_t st) {
+void launch_oz_build(int ns, const OzBuild *tasks, int64_t ntasks, const double2 *src, char *dst, cudaStream_t st,
+                     const double *scale) {
   if (ntasks == 0) return;
   if (ns == 3)
-    oz_build_kernel<3><<<(unsigned)ntasks, 128, 0, st>>>(tasks, src, dst);
+    oz_build_kernel<3><<<(unsigned)ntasks, 128, 0, st>>>(tasks, src, dst, scale);
   else
-    oz_build_kernel<6><<<(unsigned)ntasks, 128, 0, st>>>(tasks, src, dst);
+    oz_build_kernel<6><<<(unsigned)ntasks, 128, 0, st>>>(tasks, src, dst, scale);
   GWGB_CUDA(cudaGetLastError());
 }
 

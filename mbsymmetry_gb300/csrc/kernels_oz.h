@@ -89,6 +89,7 @@ struct OzS3 {
   int64_t part;            // FP64 partial: part + tau * elems + n * sn + x * sx
   int32_t rt, nkr;         // rounds [rt, rt + nkr) of the round table
   int32_t M, N, nx, elems, sn, sx;
+  int32_t oct, pad;        // octets per column tile
 };
 struct OzRnd { int32_t a16, b16, nks, pad; };  // byte offsets / 16 in the row tile and per octet of the column tile
 
@@ -98,7 +99,8 @@ struct OzRnd { int32_t a16, b16, nks, pad; };  // byte offsets / 16 in the row t
 struct OzTask { int32_t d, i, m0, n; };
 
 // One operand image built from FP64 data: row r (r0 + local) at (r / rd) * rs1 + (r % rd) * rs0,
-// valid when r % rd < rv and r / rd < rn; K index k at (k / kd) * ks1 + (k % kd) * ks0, valid likewise.
+// valid when r % rd < rv and r / rd < rn; K index k at (k / kd) * ks1 + (k % kd) * ks0, valid likewise;
+// kx >= 0: element k is multiplied by scale[kx + k] (powers of two).
 struct OzBuild {
   int64_t src, dst;
   int64_t rs1, ks1;
@@ -106,6 +108,7 @@ struct OzBuild {
   int16_t rows, nks;       // rows of the image (complex), K octets
   int8_t isb, conj;
   int16_t pad;
+  int32_t kx, pad2;
 };
 
 struct OzArgs {
@@ -125,6 +128,7 @@ void set_oz_kernel_attributes();
 void oz_rings(int ns, int stage, int max_kos, OzArgs *a);
 // multi (stages 1 and 2): the tasks have more than one round of K.
 void launch_oz_gemm(int ns, int stage, bool multi, const OzArgs &a, int nsm, cudaStream_t st);
-void launch_oz_build(int ns, const OzBuild *tasks, int64_t ntasks, const double2 *src, char *dst, cudaStream_t st);
+void launch_oz_build(int ns, const OzBuild *tasks, int64_t ntasks, const double2 *src, char *dst, cudaStream_t st,
+                     const double *scale = nullptr);
 
 }  // namespace gwgb

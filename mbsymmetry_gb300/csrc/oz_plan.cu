@@ -10,6 +10,7 @@
 #include "oz_plan.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <map>
 #include <tuple>
@@ -41,8 +42,7 @@ int choose_glog(int zos, int nL, int oct) {
 }  // namespace
 
 void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<OzOwner> &own, int ntau, int stage0,
-                   int64_t budget, int64_t persist_bytes, int nsm, int64_t nV, int64_t nG, int64_t nB2, int64_t nout,
-                   cudaStream_t st) {
+                   int64_t budget, int64_t persist_bytes, int nsm, int64_t nV, int64_t nG, int64_t nB2, int64_t nout) {
   ns_ = ns;
   const int OCT = OZ_OCT, NS = ns;
   const int FK = 8 * OCT;  // complex K of a full round
@@ -97,7 +97,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
       for (int r = 0; r < R; ++r) {
         const int nks = std::min(OCT, kos - r * OCT);
         builds.push_back({c.ga + (int64_t)r * FK * c.gk, a1_, c.gt, 0, c.gL, c.gk, c.nL, 1 << 20, c.nL,
-                          c.K1 - r * FK, ntau, 1, mt * OZ_M, OZ_M, (int16_t)nks, 0, 0, 0});
+                          c.K1 - r * FK, ntau, 1, mt * OZ_M, OZ_M, (int16_t)nks, 0, 0, 0, -1, 0});
         a1_ += oz_abytes(NS, nks);
       }
   }
@@ -115,7 +115,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
           const int nks = std::min(OCT, kos - r * OCT);
           builds.push_back({c.b2 + t * c.b2t + (int64_t)z0 * 8 * c.b2z + (int64_t)r * FK * c.b2y, b2_, 0, 0, c.b2z,
                             c.b2y, 1 << 20, 1 << 20, c.nz - 8 * z0, c.ny - r * FK, 1, 1, 0, (int16_t)(8 * noct),
-                            (int16_t)nks, 1, c.b2conj, 0});
+                            (int16_t)nks, 1, c.b2conj, 0, -1, 0});
           b2_ += noct * oz_bbytes1(NS, nks);
         }
       }
@@ -304,14 +304,14 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
             builds.push_back({x.v + (int64_t)ct * FK * x.sn + (int64_t)w.Lg * g * x.sL + (int64_t)w.zt * FK * x.sz,
                               voff + ct * bz + w.b16 * 16 * noct, 0, x.sL, x.sn, x.sz, 1 << 20, 8 * zr,
                               x.N - ct * FK, std::min(8 * zr, x.nz - w.zt * FK), 1, w.nks / zr, 0,
-                              (int16_t)(8 * noct), (int16_t)w.nks, 1, x.conj3, 0});
+                              (int16_t)(8 * noct), (int16_t)w.nks, 1, x.conj3, 0, -1, 0});
           }
         }
         voff += (int64_t)nos * vb;
       }
       const int id = (int)s3.size();
       s3.push_back({x2, fb, hit->second.first, bz, part, (int32_t)rnd.size(), (int32_t)rr.size(), ntau * ow.nx, ow.N,
-                    ow.nx, ow.N * ow.nx, ow.sn, ow.sx});
+                    ow.nx, ow.N * ow.nx, ow.sn, ow.sx, OCT, 0});
       rnd.insert(rnd.end(), rr.begin(), rr.end());
       for (int ct = 0; ct < nct; ++ct)
         for (int f = 0, G = OCT / std::min(OCT, nos - ct * OCT); f < nf; f += G)
@@ -403,7 +403,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
               const int nks = std::min(OCT, kos - r * OCT);
               builds.push_back({x.v + (int64_t)xa * x.sx + (int64_t)yr * FK * x.sy + (int64_t)r * FK * x.sk, voff, x.sx,
                                 0, x.sy, x.sk, 8 * gs, 1 << 20, std::min(8 * gs, x.ny - yr * FK), x.K1 - r * FK, n, 1,
-                                0, (int16_t)(8 * noct), (int16_t)nks, 1, x.conj1, 0});
+                                0, (int16_t)(8 * noct), (int16_t)nks, 1, x.conj1, 0, -1, 0});
               voff += noct * oz_bbytes1(NS, nks);
             }
           }
@@ -488,15 +488,19 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
     f(dst2, dst2_); f(s3, s3_); f(rnd, rnd_); f(red, red_);
   };
   each(place);
-  std::vector<char> host(total);
-  lists_.alloc(total);
+  host_.resize(total);
   each([&](const auto &v, auto &l) {
-    const size_t off = reinterpret_cast<size_t>(l.p);
-    if (!v.empty()) std::memcpy(host.data() + off, v.data(), v.size() * sizeof(v[0]));
-    l.p = reinterpret_cast<decltype(l.p)>(lists_.p + off);
+    if (!v.empty()) std::memcpy(host_.data() + reinterpret_cast<size_t>(l.p), v.data(), v.size() * sizeof(v[0]));
   });
-  if (total) GWGB_CUDA(cudaMemcpyAsync(lists_.p, host.data(), total, cudaMemcpyHostToDevice, st));
+}
+
+void OzPlan::upload(cudaStream_t st) {
+  lists_.alloc(host_.size());
+  auto at = [&](auto &l) { l.p = reinterpret_cast<decltype(l.p)>(lists_.p + reinterpret_cast<size_t>(l.p)); };
+  at(builds_); at(tasks_); at(s1_); at(col1_); at(dst1_); at(s2_); at(rows_); at(dst2_); at(s3_); at(rnd_); at(red_);
+  if (!host_.empty()) GWGB_CUDA(cudaMemcpyAsync(lists_.p, host_.data(), host_.size(), cudaMemcpyHostToDevice, st));
   GWGB_CUDA(cudaStreamSynchronize(st));
+  host_ = std::vector<char>();
 }
 
 void OzPlan::build_static(const double2 *V, cudaStream_t st) {
@@ -544,9 +548,112 @@ void OzPlan::run_one(const OzLaunch &l, OzShared &sh, const double2 *V, const do
   launch_oz_gemm(ns_, (int)l.d0, l.multi, a, nsm, st);
 }
 
+void OzTransform::build(const std::vector<TSlab> &slabs, int nout, int nin, int row0, int64_t nX, int64_t nY, int nsm,
+                        cudaStream_t st) {
+  const int NS = 6, OCT = OZ_OCT, FK = 8 * OCT;
+  const int kos = cdiv(nin, 8), R = cdiv(kos, OCT), nos = cdiv(nout, 8);
+  nout_ = nout;
+  nin_ = nin;
+  const int64_t fb = (int64_t)NS * kos * 4096 + 512 * R, vb = (int64_t)NS * kos * 512 + 32 * R;
+  std::vector<OzBuild> builds;
+  std::vector<OzTask> tasks;
+  std::vector<OzS3> s3;
+  std::vector<OzRnd> rnd;
+  int64_t tiles = 0;
+  for (const TSlab &x : slabs) tiles += cdiv(x.ncols, OZ_M);
+  // the widest column tile (octets) that gives every SM a task: wide tiles read X's images less often
+  int oct = OCT;
+  while (oct > 1 && tiles * cdiv(nos, oct) < nsm) oct >>= 1;
+  for (int r = 0; r < R; ++r)
+    rnd.push_back({(int32_t)(r * oz_abytes(NS, OCT) / 16), (int32_t)(r * oz_bbytes1(NS, OCT) / 16),
+                   std::min(OCT, kos - r * OCT), 0});
+  a_ = 0;
+  for (size_t i = 0; i < slabs.size(); ++i) {
+    const TSlab &x = slabs[i];
+    check_range(x.x, (int64_t)(row0 + nin - 1) * x.ldx + x.ncols, nX, "transform input");
+    check_range(x.y, (int64_t)(nout - 1) * x.ldy + x.ncols, nY, "transform output");
+    s3.push_back({a_, fb, 0, oct * vb, x.y, 0, R, x.ncols, nout, 1 << 30, 0, x.ldy, 1, oct, 0});
+    for (int f = 0; f * OZ_M < x.ncols; ++f) {
+      for (int r = 0; r < R; ++r) {
+        const int nks = std::min(OCT, kos - r * OCT);
+        builds.push_back({x.x + (int64_t)(row0 + r * FK) * x.ldx, a_, 0, 0, 1, x.ldx, 1 << 30, 1 << 20, x.ncols,
+                          nin - r * FK, 1, 1, f * OZ_M, OZ_M, (int16_t)nks, 0, 0, 0, r * FK, 0});
+        a_ += oz_abytes(NS, nks);
+      }
+      GWGB_REQUIRE(f < 65536, GWGB_E_UNSUPPORTED, "transform slab too large");
+      for (int ct = 0; ct * oct < nos; ++ct) tasks.push_back({(int32_t)i, f | ct << 16, 0, 1});
+    }
+  }
+  nbuild_ = (int64_t)builds.size();
+  int64_t tb = 0;
+  for (int ct = 0; ct * oct < nos; ++ct) {
+    const int noct = std::min(oct, nos - ct * oct);
+    for (int r = 0; r < R; ++r) {
+      const int nks = std::min(OCT, kos - r * OCT);
+      builds.push_back({(int64_t)ct * oct * 8 * nin + r * FK, tb, 0, 0, nin, 1, 1 << 20, 1 << 20, nout - ct * oct * 8,
+                        nin - r * FK, 1, 1, 0, (int16_t)(8 * noct), (int16_t)nks, 1, 0, 0, nin + r * FK, 0});
+      tb += noct * oz_bbytes1(NS, nks);
+    }
+  }
+  nT_ = (int64_t)builds.size() - nbuild_;
+  gemm_ = OzLaunch{};
+  gemm_.n = (int64_t)tasks.size();
+  if (tasks.empty()) return;
+  oz_rings(NS, 2, 1, &gemm_.args);
+  builds_.upload(builds, st);
+  tasks_.upload(tasks, st);
+  s3_.upload(s3, st);
+  rnd_.upload(rnd, st);
+  T_.alloc((size_t)tb);
+  GWGB_CUDA(cudaStreamSynchronize(st));
+}
+
+void OzTransform::set_matrix(const double *T_host, const double2 *T, cudaStream_t st) {
+  std::vector<double> scale(2 * (size_t)nin_, 1.0);
+  for (int i = 0; i < nin_; ++i) {
+    double m = 0.0;
+    for (int r = 0; r < nout_; ++r) {
+      const double *t = T_host + 2 * ((size_t)r * nin_ + i);
+      m = std::max(m, std::max(std::fabs(t[0]), std::fabs(t[1])));
+    }
+    if (!(m > 0x1p-500 && m < 0x1p500)) continue;
+    int e;
+    std::frexp(m, &e);
+    scale[i] = std::ldexp(1.0, e);
+    scale[nin_ + i] = std::ldexp(1.0, -e);
+  }
+  scale_.upload(scale, st);
+  launch_oz_build(6, builds_.p + nbuild_, nT_, T, T_.p, st, scale_.p);
+  GWGB_CUDA(cudaStreamSynchronize(st));
+  ready = true;
+}
+
+void OzTransform::run(const double2 *X, double2 *Y, char *A, int nsm, int *err, cudaStream_t st) const {
+  launch_oz_build(6, builds_.p, nbuild_, X, A, st, scale_.p);
+  OzArgs a = gemm_.args;
+  a.desc = s3_.p;
+  a.tasks = tasks_.p;
+  a.ntasks = (int)gemm_.n;
+  a.aux1 = rnd_.p;
+  a.aux2 = nullptr;
+  a.A = A;
+  a.B = T_.p;
+  a.X = nullptr;
+  a.part = Y;
+  a.err = err;
+  launch_oz_gemm(6, 2, false, a, nsm, st);
+}
+
+void OzTransform::free() {
+  builds_.free(); tasks_.free(); s3_.free(); rnd_.free(); T_.free(); scale_.free();
+  gemm_.n = 0;
+  ready = false;
+}
+
 void OzPlan::free() {
   V_.free();
   lists_.free();
+  host_ = std::vector<char>();
   launches_.clear();
   static_.clear();
 }

@@ -53,14 +53,44 @@ struct OzShared {
   }
 };
 
+// A tau <-> omega transform Y[slab][r][c] = sum_i T[r][i] X[slab][row0 + i][c] as a stage-3
+// GEMM in six slices: rows c, K = i, columns r.  The tau grids are dense at their ends, where the
+// weights in T are small and X is large: X[i] is scaled by the power of two of the largest
+// |T[r][i]| and T by its inverse, so that the slices of a row are relative to its largest term.
+class OzTransform {
+ public:
+  void build(const std::vector<TSlab> &slabs, int nout, int nin, int row0, int64_t nX, int64_t nY, int nsm,
+             cudaStream_t st);
+  int64_t bytes_A() const { return a_; }
+  bool built() const { return gemm_.n > 0; }
+  bool ready = false;           // the matrix has been set
+  // T: host and device copies, [nout][nin]
+  void set_matrix(const double *T_host, const double2 *T, cudaStream_t st);
+  // A: bytes_A() bytes of scratch
+  void run(const double2 *X, double2 *Y, char *A, int nsm, int *err, cudaStream_t st) const;
+  void free();
+
+ private:
+  int64_t a_ = 0, nbuild_ = 0, nT_ = 0;
+  int nout_ = 0, nin_ = 0;
+  OzLaunch gemm_;
+  DBuf<OzBuild> builds_;        // images of X, then those of T
+  DBuf<OzTask> tasks_;
+  DBuf<OzS3> s3_;
+  DBuf<OzRnd> rnd_;
+  DBuf<char> T_;
+  DBuf<double> scale_;          // [nin] of X, [nin] of T
+};
+
 class OzPlan {
  public:
   enum { IMG_V, IMG_A1, IMG_B2 };
   // stage0: gwgb_launch_stat.stage of stage 1; budget: bytes of X1 + X2 per chunk; persist_bytes: the
   // V images are kept (built once per upload) when they take at most this, else built per chunk.
+  // Host side only (no CUDA calls); upload() then moves the lists to the device.
   void build(int ns, const std::vector<OzContrib> &cs, const std::vector<OzOwner> &own, int ntau, int stage0,
-             int64_t budget, int64_t persist_bytes, int nsm, int64_t nV, int64_t nG, int64_t nB2, int64_t nout,
-             cudaStream_t st);
+             int64_t budget, int64_t persist_bytes, int nsm, int64_t nV, int64_t nG, int64_t nB2, int64_t nout);
+  void upload(cudaStream_t st);
   int64_t bytes_V() const { return vimg_; }
   int64_t bytes_A1() const { return a1_; }
   int64_t bytes_B2() const { return b2_; }
@@ -85,6 +115,7 @@ class OzPlan {
     T *p = nullptr;
     size_t n = 0;
   };
+  std::vector<char> host_;      // the lists until they are uploaded
   DBuf<char> lists_;
   List<OzBuild> builds_;
   List<OzTask> tasks_;
