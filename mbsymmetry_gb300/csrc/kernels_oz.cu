@@ -232,16 +232,20 @@ template <int NS, int STAGE> struct Job {
     }
     G = STAGE == 0 ? 1 : OCT / noct;
   }
-  __device__ __forceinline__ int nks(int r) const { return STAGE == 2 ? rt[r].nks : min(OCT, kos - r * OCT); }
-  __device__ __forceinline__ const char *aptr(int m, int r) const {
-    return a + m * atile + (STAGE == 2 ? (int64_t)rt[r].a16 * 16 : r * oz_abytes(NS, OCT));
+  // Round r (stage 3: from the round table, read one round ahead).
+  __device__ __forceinline__ OzRnd round(int r) const {
+    if constexpr (STAGE == 2) return rt[min(r, R - 1)];
+    return {0, 0, min(OCT, kos - r * OCT), 0};
   }
-  __device__ __forceinline__ const char *bptr(int r) const {
-    return b + noct * (STAGE == 2 ? (int64_t)rt[r].b16 * 16 : r * oz_bbytes1(NS, OCT));
+  __device__ __forceinline__ const char *aptr(int m, int r, const OzRnd &q) const {
+    return a + m * atile + (STAGE == 2 ? (int64_t)q.a16 * 16 : r * oz_abytes(NS, OCT));
+  }
+  __device__ __forceinline__ const char *bptr(int r, const OzRnd &q) const {
+    return b + noct * (STAGE == 2 ? (int64_t)q.b16 * 16 : r * oz_bbytes1(NS, OCT));
   }
 };
 
-constexpr int OZ_RING = 16;             // largest operand ring (K steps)
+constexpr int OZ_RING = 16;             // largest operand ring
 constexpr int OZ_SC = 32;               // scale rings: deeper than the operand rings plus the accumulator sets
 constexpr int OZ_SMEM = 200 * 1024;
 // Drain warps (then one warp copies and one issues the MMAs): three slices take two octets per
@@ -277,10 +281,13 @@ struct Ring {
 // and 2) and the L2 / HBM traffic of the images; the operands need no CUDA-core
 // work at all, a K step (8 complex) is 8 MMAs, and two TMEM accumulator sets let
 // one round multiply while the other drains.  Operands stream through rings of
-// K steps (12 KB of A, at most 6 KB of B); stages 1 and 2 hold the column
-// operand of a task over its row tiles.  A column tile of one octet (two) fills
-// a quarter (half) of an accumulator set, so stages 2 and 3 put G = OCT / noct
-// row tiles into one.
+// segments of SEG K steps; stages 1 and 2 hold the column operand of a task over
+// its row tiles.  The copy and MMA warps' own loops count: with one K step per
+// segment and a table entry read per step they alone took 7.0 of the 10.4 ms of the
+// hexagonal 8 k Sigma stage (three slices).  With segments of 4 it takes 7.0 (of 2: 7.7); stages
+// 1 and 2 keep 2, which leaves room for the next task's columns (s+p+d: 1.33 ms against 1.52).
+// A column tile of one octet (two) fills a quarter (half) of an accumulator set, so
+// stages 2 and 3 put G = OCT / noct row tiles into one.
 //
 // Every wait is bounded: a wait that runs out sets the error word and an abort
 // flag; the copy and MMA roles then leave, the drain warps walk on through
@@ -291,12 +298,13 @@ template <int NS, int STAGE, bool MULTI>
 __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs g) {
   constexpr int OCT = OzCfg<NS>::OCT, NACC = OzCfg<NS>::NACC, HO = OzCfg<NS>::HO, DW = oz_drain<NS>;
   constexpr int NR = 16 * OCT, SETC = NACC * NR;
-  constexpr uint32_t SA = NS * 4096, SB = NS * 512 * OCT;  // ring slots
+  constexpr int SEG = STAGE == 2 ? OzCfg<NS>::SEG3 : OzCfg<NS>::SEG;
+  constexpr uint32_t SA = NS * 4096, SB = NS * 512 * OCT;  // one K step
   constexpr int SETS = OzCfg<NS>::SETS;
   static_assert(SETS * SETC <= 512, "the accumulator sets must fit TMEM");
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint32_t tslot;
-  __shared__ __align__(8) uint64_t full[OZ_RING], emptyA[OZ_RING], emptyB[OZ_RING], done[SETS], tfree[SETS], last;
+  __shared__ __align__(8) uint64_t full[OZ_RING], emptyA[OZ_RING], emptyB[OZ_RING], fullB[2], done[SETS], tfree[SETS], last;
   __shared__ __align__(16) float sA[OZ_SC][OZ_M], sB[OZ_SC][8 * OCT];
   __shared__ float gmax[2][OCT][OZ_M];
   __shared__ int abort_flag;
@@ -309,6 +317,8 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
       tc::mbar_init(&emptyA[j], 1);
       tc::mbar_init(&emptyB[j], 1);
     }
+    tc::mbar_init(&fullB[0], 1);
+    tc::mbar_init(&fullB[1], 1);
     for (int j = 0; j < SETS; ++j) {
       tc::mbar_init(&done[j], 1);
       tc::mbar_init(&tfree[j], DW);
@@ -323,18 +333,20 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
   const uint32_t tm = __shfl_sync(0xffffffffu, tslot, 0);
   // Bounded wait of a converged warp; false (in every lane) when it ran out (error word and abort
   // flag set) or another role aborted.  Each poll may suspend for up to 20 us (hint).
+  auto poll = [&](uint64_t *b, uint32_t par) -> bool {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.b32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(tc::smem_u32(b)), "r"(par), "r"(20000u)
+        : "memory");
+    return ok != 0;
+  };
   auto bwait = [&](uint64_t *b, uint32_t par) -> bool {
+    if (__all_sync(0xffffffffu, poll(b, par))) return true;
     bool hit = false;
     for (int rep = 0; rep < 256 && !hit; ++rep) {
-      for (int it = 0; it < 256 && !hit; ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.b32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok)
-            : "r"(tc::smem_u32(b)), "r"(par), "r"(20000u)
-            : "memory");
-        hit = ok != 0;
-      }
+      for (int it = 0; it < 256 && !hit; ++it) hit = poll(b, par);
       if (!hit && *(volatile int *)&abort_flag) break;
       if (!hit && rep == 255) {
         atomicExch(g.err, 1);
@@ -343,47 +355,68 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
     }
     return __all_sync(0xffffffffu, hit);
   };
-  const uint32_t smA = tc::smem_u32(smem), smB = smA + (uint32_t)g.nA * SA;
+  // rings: nA segments of A, then nB segments of B (stage 3) or tasksB tasks' B of nB K steps
+  const uint32_t smA = tc::smem_u32(smem), smB = smA + (uint32_t)g.nA * SEG * SA;
 
   if (warp == DW) {
     // ------------------------------ copies ------------------------------
-    Ring ra(g.nA), rb(g.nB);
-    int ia = 0, ib = 0, ra_rounds = 0, rb_rounds = 0;  // K steps and rounds copied
+    Ring ra(g.nA), rb(STAGE == 2 ? g.nB : g.tasksB);
+    int ia = 0, ib = 0, na = 0, nb = 0;  // segments (of A, of B or tasks), rounds copied
     bool ok = true;
     for (int ti = blockIdx.x; ti < g.ntasks && ok; ti += gridDim.x) {
       Job<NS, STAGE> job;
       job.init(g, g.tasks[ti]);
       const uint32_t bb = (uint32_t)(job.noct * NS * 512), sb = (uint32_t)(32 * job.noct);
+      if constexpr (STAGE != 2) {  // the task's column operand, all rounds
+        if (ib >= g.tasksB && !bwait(&emptyB[rb.slot], rb.phase ^ 1)) { ok = false; break; }
+        if (elect_one()) {
+          uint64_t *f = &fullB[rb.slot];
+          expect_tx(f, job.kos * bb + job.R * sb);
+          for (int r = 0; r < job.R; ++r) {
+            const int nks = min(OCT, job.kos - r * OCT);
+            const char *bp = job.bptr(r, OzRnd{});
+            bulk_load(smB + rb.slot * (g.nB * SB) + r * OCT * bb, bp, nks * bb, f);
+            bulk_load(tc::smem_u32(sB[(nb + r) & (OZ_SC - 1)]), bp + nks * bb, sb, f);
+          }
+        }
+        __syncwarp();
+        nb += job.R;
+        rb.next();
+        ++ib;
+      }
       for (int m0 = 0; m0 < job.outer && ok; m0 += job.G) {
         const int Gm = min(job.G, job.outer - m0);
+        OzRnd nx = job.round(0);
         for (int r = 0; r < job.R && ok; ++r) {
-          const int nks = job.nks(r);
+          const OzRnd q = nx;
+          nx = job.round(r + 1);
           for (int gi = 0; gi < Gm && ok; ++gi) {
-            const bool nb = gi == 0 && (STAGE == 2 || m0 == 0);
-            const char *ap = job.aptr(m0 + gi, r), *bp = job.bptr(r);
-            for (int ks = 0; ks < nks; ++ks) {
+            const bool withb = STAGE == 2 && gi == 0;
+            const char *ap = job.aptr(m0 + gi, r, q), *bp = job.bptr(r, q);
+            for (int ks = 0; ks < q.nks; ks += SEG) {
+              const int n = min(SEG, q.nks - ks);
               if (ia >= g.nA && !bwait(&emptyA[ra.slot], ra.phase ^ 1)) { ok = false; break; }
-              if (nb && ib >= g.nB && !bwait(&emptyB[rb.slot], rb.phase ^ 1)) { ok = false; break; }
-              uint64_t *f = &full[ra.slot];
+              if (withb && ib >= g.nB && !bwait(&emptyB[rb.slot], rb.phase ^ 1)) { ok = false; break; }
               if (elect_one()) {
-                expect_tx(f, SA + (ks == 0 ? 512u : 0u) + (nb ? bb + (ks == 0 ? sb : 0u) : 0u));
-                bulk_load(smA + ra.slot * SA, ap + ks * SA, SA, f);
-                if (ks == 0) bulk_load(tc::smem_u32(sA[ra_rounds & (OZ_SC - 1)]), ap + nks * SA, 512, f);
-                if (nb) {
-                  bulk_load(smB + rb.slot * SB, bp + ks * bb, bb, f);
-                  if (ks == 0) bulk_load(tc::smem_u32(sB[rb_rounds & (OZ_SC - 1)]), bp + nks * bb, sb, f);
+                uint64_t *f = &full[ra.slot];
+                expect_tx(f, n * SA + (ks == 0 ? 512u : 0u) + (withb ? n * bb + (ks == 0 ? sb : 0u) : 0u));
+                bulk_load(smA + ra.slot * (SEG * SA), ap + ks * SA, n * SA, f);
+                if (withb) bulk_load(smB + rb.slot * (SEG * SB), bp + ks * bb, n * bb, f);
+                if (ks == 0) {
+                  bulk_load(tc::smem_u32(sA[na & (OZ_SC - 1)]), ap + q.nks * SA, 512, f);
+                  if (withb) bulk_load(tc::smem_u32(sB[nb & (OZ_SC - 1)]), bp + q.nks * bb, sb, f);
                 }
               }
               __syncwarp();
-              if (nb) {
+              if (withb) {
                 rb.next();
                 ++ib;
               }
               ra.next();
               ++ia;
             }
-            ++ra_rounds;
-            if (nb) ++rb_rounds;
+            ++na;
+            if (withb) ++nb;
           }
         }
       }
@@ -395,9 +428,16 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
       if (q >= first) tc::mbar_wait(&full[rw.slot], rw.phase, 4000000);
       rw.next();
     }
+    if constexpr (STAGE != 2) {
+      Ring rv(g.tasksB);
+      for (int q = 0; q < ib; ++q) {
+        if (q >= ib - g.tasksB) tc::mbar_wait(&fullB[rv.slot], rv.phase, 4000000);
+        rv.next();
+      }
+    }
   } else if (warp == DW + 1) {
     // ------------------------------ MMAs ------------------------------
-    Ring ra(g.nA), rb(g.nB);
+    Ring ra(g.nA), rb(STAGE == 2 ? g.nB : g.tasksB);
     int n = 0;  // accumulator sets filled
     bool ok = true;
     for (int ti = blockIdx.x; ti < g.ntasks && ok; ti += gridDim.x) {
@@ -405,49 +445,62 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
       job.init(g, g.tasks[ti]);
       const int noct = __shfl_sync(0xffffffffu, job.noct, 0);
       const uint32_t id = idesc_f16(16 * noct);
-      const uint32_t bstep = 512u * noct;
-      const Ring r0 = rb;
+      const uint32_t bstep = 512u * noct;  // one plane of one K step
+      if (STAGE != 2 && !bwait(&fullB[rb.slot], rb.phase)) { ok = false; break; }
+      const uint32_t bt = smB + rb.slot * (g.nB * SB);
       for (int m0 = 0; m0 < job.outer && ok; m0 += job.G) {
         const int Gm = min(job.G, job.outer - m0);
-        const bool lastm = STAGE == 2 || m0 + job.G >= job.outer;
-        if (STAGE != 2) rb = r0;
+        OzRnd nx = job.round(0);
         for (int r = 0; r < job.R && ok; ++r, ++n) {
-          const int set = n % SETS, nks = __shfl_sync(0xffffffffu, job.nks(r), 0);
+          const int set = n % SETS, nks = __shfl_sync(0xffffffffu, nx.nks, 0);
+          nx = job.round(r + 1);
           if (n >= SETS && !bwait(&tfree[set], (n / SETS - 1) & 1)) { ok = false; break; }
           const Ring rr = rb;
           for (int gi = 0; gi < Gm && ok; ++gi) {
-            rb = rr;
+            if (STAGE == 2) rb = rr;
             const uint32_t d0 = tm + (uint32_t)(set * SETC + gi * 16 * noct);
-            for (int ks = 0; ks < nks; ++ks) {
+            for (int ks = 0; ks < nks; ks += SEG) {
               if (!bwait(&full[ra.slot], ra.phase)) { ok = false; break; }
               tc::fence_after_sync();
-              const uint32_t a0 = smA + ra.slot * SA, b0 = smB + rb.slot * SB;
-              const uint32_t more = ks > 0 ? 1u : 0u;
+              const uint32_t a0 = smA + ra.slot * (SEG * SA);
+              const uint32_t b0 = STAGE == 2 ? smB + rb.slot * (SEG * SB) : bt + (r * OCT + ks) * NS * bstep;
               if (elect_one()) {
 #pragma unroll
-                for (int c = 0; c <= OzCfg<NS>::CMAX; ++c)
+                for (int k = 0; k < SEG; ++k) {
+                  if (ks + k >= nks) break;
+                  const uint32_t more = ks + k > 0 ? 1u : 0u;
 #pragma unroll
-                  for (int p = 0; p < NS; ++p) {
-                    const int q = c - p;
-                    if (q < 0 || q >= NS) continue;
-                    // NS = 3: (0,0) | (0,1) | (1,0) | the rest; NS = 6: one per class
-                    const int acc = NS == 6 ? c : c == 0 ? 0 : c == 1 ? 1 + p : 3;
-                    const bool fresh = NS == 6 ? p == max(0, c - NS + 1) : c < 2 || (c == 2 && p == 0);
-                    tc::mma_bf16(d0 + acc * NR, sw32_desc(a0 + p * 4096u), sw32_desc(b0 + q * bstep), id,
-                                 fresh ? more : 1u);  // kind::f16, types from the descriptor
-                  }
+                  for (int c = 0; c <= OzCfg<NS>::CMAX; ++c)
+#pragma unroll
+                    for (int p = 0; p < NS; ++p) {
+                      const int q = c - p;
+                      if (q < 0 || q >= NS) continue;
+                      // NS = 3: (0,0) | (0,1) | (1,0) | the rest; NS = 6: one per class
+                      const int acc = NS == 6 ? c : c == 0 ? 0 : c == 1 ? 1 + p : 3;
+                      const bool fresh = NS == 6 ? p == max(0, c - NS + 1) : c < 2 || (c == 2 && p == 0);
+                      tc::mma_bf16(d0 + acc * NR, sw32_desc(a0 + k * SA + p * 4096u),
+                                   sw32_desc(b0 + (k * NS + q) * bstep), id,
+                                   fresh ? more : 1u);  // kind::f16, types from the descriptor
+                    }
+                }
                 tc::commit(&emptyA[ra.slot]);
-                if (lastm && gi == Gm - 1) tc::commit(&emptyB[rb.slot]);
+                if (STAGE == 2 && gi == Gm - 1) tc::commit(&emptyB[rb.slot]);
               }
               __syncwarp();
               ra.next();
-              rb.next();
+              if (STAGE == 2) rb.next();
             }
           }
           if (!ok) break;
           if (elect_one()) tc::commit(&done[set]);
           __syncwarp();
         }
+      }
+      if (STAGE != 2) {
+        if (!ok) break;
+        if (elect_one()) tc::commit(&emptyB[rb.slot]);
+        __syncwarp();
+        rb.next();
       }
     }
     if (elect_one()) tc::commit(&last);  // arrives when every MMA issued above has completed
@@ -460,8 +513,11 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
     const uint32_t tbase = tm + ((uint32_t)(32 * lq) << 16) + 16u * os0;
     int n = 0, i0 = 0, j0 = 0, tile = 0;  // sets, row tiles and column images consumed
     bool dead = false;
+    OzTask tk1{};
+    if (blockIdx.x < (unsigned)g.ntasks) tk1 = g.tasks[blockIdx.x];
     for (int ti = blockIdx.x; ti < g.ntasks; ti += gridDim.x) {
-      const OzTask tk = g.tasks[ti];
+      const OzTask tk = tk1;
+      if (ti + (int)gridDim.x < g.ntasks) tk1 = g.tasks[ti + gridDim.x];
       Job<NS, STAGE> job;
       job.init(g, tk);
       // row tile in the set, octet in the tile, valid columns of the octet
@@ -920,17 +976,20 @@ void set_oz_kernel_attributes() {
   set_attributes<6>();
 }
 
-// Stages 1 and 2 hold the column operand of a task (all K steps) and prefetch
-// the next task's as far as three K steps of A leave room; stage 3 streams both.
+// Stages 1 and 2 hold the column operand of a task (max_kos K steps) and, where that leaves room
+// for three segments of A, that of the next; stage 3 streams both operands.
 void oz_rings(int ns, int stage, int max_kos, OzArgs *a) {
-  const int slotA = ns * 4096, slotB = ns * 512 * OZ_OCT;
+  const int seg = ns == 3 ? (stage == 2 ? OzCfg<3>::SEG3 : OzCfg<3>::SEG)
+                          : (stage == 2 ? OzCfg<6>::SEG3 : OzCfg<6>::SEG);
+  const int slotA = seg * ns * 4096, stepB = ns * 512 * OZ_OCT;
   if (stage == 2) {
-    a->nA = a->nB = std::min(OZ_RING, OZ_SMEM / (slotA + slotB));
+    a->nA = a->nB = std::min(OZ_RING, OZ_SMEM / (slotA + seg * stepB));
   } else {
-    a->nB = std::min({OZ_RING, 2 * max_kos, std::max(max_kos, (OZ_SMEM - 3 * slotA) / slotB)});
-    a->nA = std::min(OZ_RING, (OZ_SMEM - a->nB * slotB) / slotA);
+    a->nB = max_kos;
+    a->tasksB = (OZ_SMEM - 2 * a->nB * stepB) / slotA >= 3 ? 2 : 1;
+    a->nA = std::min(OZ_RING, (OZ_SMEM - a->tasksB * a->nB * stepB) / slotA);
   }
-  GWGB_REQUIRE(a->nA >= 2 && a->nB >= (stage == 2 ? 2 : max_kos), GWGB_E_UNSUPPORTED, "sliced GEMM rings too small");
+  GWGB_REQUIRE(a->nA >= 2, GWGB_E_UNSUPPORTED, "sliced GEMM rings too small");
 }
 
 template <int NS>
