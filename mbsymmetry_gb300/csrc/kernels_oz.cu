@@ -55,36 +55,61 @@ __device__ __forceinline__ int oz_exponent(float m) {
 // 2^e for e in [-126, 127].
 __device__ __forceinline__ float oz_pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
 
+// Two FP32 numbers per instruction (the drains are bound by their issue slots).
+struct F2 {
+  float x, y;
+};
+__device__ __forceinline__ F2 both(float a) { return {a, a}; }
+#define OZ_F2_OP(op, ...)                                                                                   \
+  F2 r;                                                                                                     \
+  asm("{\n.reg .b64 a, b, c;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\n" op "mov.b64 {%0, %1}, c;\n}\n" \
+      : "=f"(r.x), "=f"(r.y)                                                                                \
+      : __VA_ARGS__);                                                                                       \
+  return r
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  OZ_F2_OP("add.rn.f32x2 c, a, b;\n", "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  OZ_F2_OP("mul.rn.f32x2 c, a, b;\n", "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 d) {
+  OZ_F2_OP(".reg .b64 d;\nmov.b64 d, {%6, %7};\nfma.rn.f32x2 c, a, b, d;\n", "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y),
+           "f"(d.x), "f"(d.y));
+}
+#undef OZ_F2_OP
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, both(-1.f), a); }
+
 // s = fl(a + b), e = a + b - s.
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
-  s = a + b;
-  const float bb = s - a;
-  e = (a - (s - bb)) + (b - bb);
+__device__ __forceinline__ void two_sum(F2 a, F2 b, F2 &s, F2 &e) {
+  s = add2(a, b);
+  const F2 bb = sub2(s, a);
+  e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
 }
 
 // The three slices of h + l (v = fl(h + l), f = 2^(15-E)); adding and subtracting 1.5 2^(23+g) rounds
 // to multiples of 2^g, and h f - s0 is exact.
-__device__ __forceinline__ void oz_slice(float h, float l, float v, float f, float m1, float (&s)[3]) {
+__device__ __forceinline__ void oz_slice(F2 h, F2 l, F2 v, F2 f, F2 m1, F2 (&s)[3]) {
   constexpr float M0 = 1.5f * 536870912.f;  // 1.5 2^29
-  s[0] = fmaf(v, f, M0) - M0;
-  const float t = fmaf(l, f, fmaf(h, f, -s[0]));
-  s[1] = (t + m1) - m1;
-  s[2] = t - s[1];
+  const F2 r = fma2(v, f, both(M0));
+  s[0] = add2(r, both(-M0));
+  const F2 t = fma2(l, f, fma2(h, f, sub2(both(M0), r)));
+  s[1] = sub2(add2(t, m1), m1);
+  s[2] = sub2(t, s[1]);
 }
 
-// Unevaluated sum of three FP32 numbers, h the rounded value.
+// Unevaluated sums of three FP32 numbers, h the rounded value.
 struct Tri {
-  float h, m, l;
+  F2 h, m, l;
 };
 
 // The value of the class sums D0 .. D6 (weights 2^(-9c)); D0 to D3 are exact integers.
-__device__ __forceinline__ Tri tri_of(const float (&d)[7]) {
-  constexpr float W1 = 0x1p-9f, W2 = 0x1p-18f, W3 = 0x1p-27f, W4 = 0x1p-36f;
-  float h, e1, s, e2, e3;
-  two_sum(d[0], d[1] * W1, h, e1);
-  two_sum(d[2] * W2, d[3] * W3, s, e2);
+__device__ __forceinline__ Tri tri_of(const F2 (&d)[7]) {
+  const F2 W1 = both(0x1p-9f), W2 = both(0x1p-18f), W3 = both(0x1p-27f), W4 = both(0x1p-36f);
+  F2 h, e1, s, e2, e3;
+  two_sum(d[0], mul2(d[1], W1), h, e1);
+  two_sum(mul2(d[2], W2), mul2(d[3], W3), s, e2);
   two_sum(e1, s, e1, e3);
-  float l = fmaf(fmaf(fmaf(d[6], W1, d[5]), W1, d[4]), W4, e2 + e3);
+  const F2 l = fma2(fma2(fma2(d[6], W1, d[5]), W1, d[4]), W4, add2(e2, e3));
   // h is zero only when the value is (all of it can lie in the low classes)
   two_sum(h, e1, h, e1);
   two_sum(e1, l, e1, e2);
@@ -96,33 +121,34 @@ __device__ __forceinline__ Tri tri_of(const float (&d)[7]) {
 
 // a += b, and a normalised (h the rounded value).
 __device__ __forceinline__ void tri_add(Tri &a, const Tri &b) {
-  float h, e1, m, e2, e3;
+  F2 h, e1, m, e2, e3;
   two_sum(a.h, b.h, h, e1);
   two_sum(a.m, b.m, m, e2);
   two_sum(m, e1, m, e3);
-  const float l = (a.l + b.l) + (e2 + e3);
+  const F2 l = add2(add2(a.l, b.l), add2(e2, e3));
   two_sum(h, m, h, m);
   two_sum(m, l, m, a.l);
   two_sum(h, m, a.h, a.m);
 }
 
 // The six digits of h + m + l (f = 2^(8-E)).
-__device__ __forceinline__ void tri_digits(const Tri &x, float f, float (&s)[6]) {
-  constexpr float MG = 1.5f * 8388608.f;  // 1.5 2^23: rounds to integers
-  s[0] = fmaf(x.h, f, MG) - MG;
-  float t, te;
-  two_sum(fmaf(x.h, f, -s[0]), x.m * f, t, te);  // the first is exact
-  te = fmaf(x.l, f, te);
-  s[1] = fmaf(t, 512.f, MG) - MG;
-  t = fmaf(t, 512.f, -s[1]);
-  s[2] = fmaf(t, 512.f, MG) - MG;
-  t = fmaf(t, 512.f, -s[2]);
-  two_sum(t, te * 262144.f, t, te);
-  s[3] = fmaf(t, 512.f, MG) - MG;
-  t = fmaf(t, 512.f, -s[3]);
-  s[4] = fmaf(t, 512.f, MG) - MG;
-  t = fmaf(t, 512.f, -s[4]);
-  s[5] = fmaf(te, 134217728.f, t * 512.f);  // te 2^27
+__device__ __forceinline__ void tri_digits(const Tri &x, F2 f, F2 (&s)[6]) {
+  const F2 MG = both(1.5f * 8388608.f), NM = both(-1.5f * 8388608.f);  // 1.5 2^23: rounds to integers
+  const F2 B = both(512.f);
+  s[0] = add2(fma2(x.h, f, MG), NM);
+  F2 t, te;
+  two_sum(sub2(mul2(x.h, f), s[0]), mul2(x.m, f), t, te);  // products and difference are exact
+  te = fma2(x.l, f, te);
+  s[1] = add2(fma2(t, B, MG), NM);
+  t = sub2(mul2(t, B), s[1]);
+  s[2] = add2(fma2(t, B, MG), NM);
+  t = sub2(mul2(t, B), s[2]);
+  two_sum(t, mul2(te, both(262144.f)), t, te);
+  s[3] = add2(fma2(t, B, MG), NM);
+  t = sub2(mul2(t, B), s[3]);
+  s[4] = add2(fma2(t, B, MG), NM);
+  t = sub2(mul2(t, B), s[4]);
+  s[5] = fma2(te, both(134217728.f), mul2(t, B));  // te 2^27
 }
 
 // 2^e for any e, 0 below the FP32 range.
@@ -133,8 +159,8 @@ __device__ __forceinline__ float oz_m1(int nks) {
   return nks == 1 ? 1.5f * 131072.f : nks == 2 ? 1.5f * 262144.f : 1.5f * 524288.f;  // 1.5 2^(28-b)
 }
 
-__device__ __forceinline__ uint32_t h2(float a, float b) {
-  const __half2 v = __floats2half2_rn(a, b);
+__device__ __forceinline__ uint32_t h2(F2 a) {
+  const __half2 v = __floats2half2_rn(a.x, a.y);
   return *reinterpret_cast<const uint32_t *>(&v);
 }
 
@@ -589,13 +615,13 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
           }
         }
         // this thread's octets: value H + L (NS = 3), (H + M + L) 2^ex (NS = 6)
-        float H[HO][16], L[HO][16], M3[NS == 6 ? HO : 1][16];
+        F2 H[HO][8], L[HO][8], M3[NS == 6 ? HO : 1][8];
         int ex[HO];
 #pragma unroll
         for (int q = 0; q < HO; ++q) {
           ex[q] = 0;
 #pragma unroll
-          for (int e = 0; e < 16; ++e) H[q][e] = L[q][e] = M3[NS == 6 ? q : 0][e] = 0.f;
+          for (int e = 0; e < 8; ++e) H[q][e] = L[q][e] = M3[NS == 6 ? q : 0][e] = both(0.f);
         }
         for (int r = 0; r < job.R; ++r, ++n, i0 += Gm) {
           const int set = n % SETS;
@@ -622,17 +648,21 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
                 const float sb[4] = {sb4.x, sb4.y, sb4.z, sb4.w};
                 tmem_wait_ld();
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  const float sc = sa * sb[e >> 1];
-                  const float lo = (__uint_as_float(x1[e]) + __uint_as_float(x2[e])) + __uint_as_float(x3[e]);
+                for (int e = 0; e < 4; ++e) {
+                  auto at = [&](const uint32_t(&x)[8]) {
+                    return F2{__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1])};
+                  };
+                  const int c = 4 * hf + e;
+                  const F2 sc = both(sa * sb[e]);
+                  const F2 lo = add2(add2(at(x1), at(x2)), at(x3));
                   if (first) {
-                    H[q][8 * hf + e] = __uint_as_float(x0[e]) * sc;
-                    L[q][8 * hf + e] = lo * sc;
+                    H[q][c] = mul2(at(x0), sc);
+                    L[q][c] = mul2(lo, sc);
                   } else {
-                    float s, er;
-                    two_sum(H[q][8 * hf + e], __uint_as_float(x0[e]) * sc, s, er);
-                    H[q][8 * hf + e] = s;
-                    L[q][8 * hf + e] += fmaf(lo, sc, er);
+                    F2 s, er;
+                    two_sum(H[q][c], mul2(at(x0), sc), s, er);
+                    H[q][c] = s;
+                    L[q][c] = add2(L[q][c], fma2(lo, sc, er));
                   }
                 }
               }
@@ -659,16 +689,17 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
                 for (int c = 0; c < 7; ++c) tmem_ld4(base + c * NR + 4 * hf, x[c]);
                 tmem_wait_ld();
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const int i = 4 * hf + e;
-                  float d[7];
+                for (int e = 0; e < 2; ++e) {
+                  const int i = 2 * hf + e;
+                  F2 d[7];
 #pragma unroll
-                  for (int c = 0; c < 7; ++c) d[c] = __uint_as_float(x[c][e]);
+                  for (int c = 0; c < 7; ++c) d[c] = {__uint_as_float(x[c][2 * e]), __uint_as_float(x[c][2 * e + 1])};
                   Tri t = tri_of(d);
-                  const float sc = oz_pow2c(eb[i >> 1] - em) * fn;
-                  t = {t.h * sc, t.m * sc, t.l * sc};
+                  const F2 sc = both(oz_pow2c(eb[i] - em) * fn);
+                  t = {mul2(t.h, sc), mul2(t.m, sc), mul2(t.l, sc)};
                   if (!first) {
-                    Tri o{H[q][i] * fo, M3[q][i] * fo, L[q][i] * fo};
+                    const F2 fo2 = both(fo);
+                    Tri o{mul2(H[q][i], fo2), mul2(M3[q][i], fo2), mul2(L[q][i], fo2)};
                     tri_add(o, t);
                     t = o;
                   }
@@ -695,13 +726,15 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
 #pragma unroll
             for (int e = 0; e < 8; ++e)
               if (e < nv[q]) {
+                const F2 h = H[q][e], l = L[q][e];
                 double re, im;
                 if constexpr (NS == 6) {
-                  re = scalbn((double)H[q][2 * e] + ((double)M3[q][2 * e] + (double)L[q][2 * e]), ex[q]);
-                  im = scalbn((double)H[q][2 * e + 1] + ((double)M3[q][2 * e + 1] + (double)L[q][2 * e + 1]), ex[q]);
+                  const F2 m = M3[q][e];
+                  re = scalbn((double)h.x + ((double)m.x + (double)l.x), ex[q]);
+                  im = scalbn((double)h.y + ((double)m.y + (double)l.y), ex[q]);
                 } else {
-                  re = (double)H[q][2 * e] + (double)L[q][2 * e];
-                  im = (double)H[q][2 * e + 1] + (double)L[q][2 * e + 1];
+                  re = (double)h.x + (double)l.x;
+                  im = (double)h.y + (double)l.y;
                 }
                 o[(int64_t)(n0 + e) * d.sn] = make_double2(re, im);
               }
@@ -716,9 +749,10 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
             valid[q] = gi[q] < Gm && (STAGE == 0 ? rg < M : rw[q].dst >= 0);
             float mo[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-              mo[e] = NS == 3 ? fmaxf(fabsf(H[q][2 * e] + L[q][2 * e]), fabsf(H[q][2 * e + 1] + L[q][2 * e + 1]))
-                              : fmaxf(fabsf(H[q][2 * e]), fabsf(H[q][2 * e + 1]));
+            for (int e = 0; e < 8; ++e) {
+              const F2 v = NS == 3 ? add2(H[q][e], L[q][e]) : H[q][e];
+              mo[e] = fmaxf(fabsf(v.x), fabsf(v.y));
+            }
             mx[q] = fmaxf(fmaxf(fmaxf(mo[0], mo[1]), fmaxf(mo[2], mo[3])),
                           fmaxf(fmaxf(mo[4], mo[5]), fmaxf(mo[6], mo[7])));
             ee[q] = mx[q] > 0.f || mx[q] != mx[q] ? oz_exponent(mx[q]) + ex[q] : OZ_ENONE;
@@ -787,7 +821,7 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
               scale = __int_as_float(e2 - 8);
             }
             // NS = 6: 2^(8 - e2 + ex); e2 - ex is at least the exponent of an FP32 value
-            const float f = NS == 3 ? oz_pow2(15 - e2) : oz_pow2c(8 - e2 + ex[q]), m1 = oz_m1(nksb);
+            const F2 f = both(NS == 3 ? oz_pow2(15 - e2) : oz_pow2c(8 - e2 + ex[q])), m1 = both(oz_m1(nksb));
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               if (e == 4 && nv[q] <= 4) {  // the second half is padding
@@ -795,16 +829,13 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
                 for (int p = 0; p < NS; ++p) w[p][4] = w[p][5] = w[p][6] = w[p][7] = 0u;
                 break;
               }
-              float sr[NS], si[NS];
-              if constexpr (NS == 3) {
-                oz_slice(H[q][2 * e], L[q][2 * e], H[q][2 * e] + L[q][2 * e], f, m1, sr);
-                oz_slice(H[q][2 * e + 1], L[q][2 * e + 1], H[q][2 * e + 1] + L[q][2 * e + 1], f, m1, si);
-              } else {
-                tri_digits({H[q][2 * e], M3[q][2 * e], L[q][2 * e]}, f, sr);
-                tri_digits({H[q][2 * e + 1], M3[q][2 * e + 1], L[q][2 * e + 1]}, f, si);
-              }
+              F2 sl[NS];
+              if constexpr (NS == 3)
+                oz_slice(H[q][e], L[q][e], add2(H[q][e], L[q][e]), f, m1, sl);
+              else
+                tri_digits({H[q][e], M3[q][e], L[q][e]}, f, sl);
 #pragma unroll
-              for (int p = 0; p < NS; ++p) w[p][e] = h2(sr[p], si[p]);
+              for (int p = 0; p < NS; ++p) w[p][e] = h2(sl[p]);
             }
             char *o = blob + ks * (int)SA + rr * 32;
             const bool sw = (rr >> 2) & 1;
@@ -926,23 +957,26 @@ __global__ void __launch_bounds__(128) oz_build_kernel(const OzBuild *__restrict
     }
     if (q < nks) {
       uint32_t w[NS][8];
-      float sr[8][NS], si[8][NS];
+      F2 sl[8][NS];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         if constexpr (NS == 3) {
-          const float hr = (float)v[e].x, hi = (float)v[e].y;
-          oz_slice(hr, (float)(v[e].x - (double)hr), hr, f, m1, sr[e]);
-          oz_slice(hi, (float)(v[e].y - (double)hi), hi, f, m1, si[e]);
+          const F2 h{(float)v[e].x, (float)v[e].y};
+          const F2 l{(float)(v[e].x - (double)h.x), (float)(v[e].y - (double)h.y)};
+          oz_slice(h, l, h, both(f), both(m1), sl[e]);
         } else {
-          double_digits(v[e].x, e2, sr[e]);
-          double_digits(v[e].y, e2, si[e]);
+          float sr[6], si[6];
+          double_digits(v[e].x, e2, sr);
+          double_digits(v[e].y, e2, si);
+#pragma unroll
+          for (int p = 0; p < NS; ++p) sl[e][p] = {sr[p], si[p]};
         }
       }
       if (!t.isb) {
 #pragma unroll
         for (int p = 0; p < NS; ++p) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) w[p][e] = h2(sr[e][p], si[e][p]);
+          for (int e = 0; e < 8; ++e) w[p][e] = h2(sl[e][p]);
           st_octet(blob + (q * NS + p) * pstride + lr * 32, w[p], (lr >> 2) & 1);
         }
       } else {  // rows (n, 0) = [Br -Bi], (n, 1) = [Bi Br]
@@ -950,10 +984,10 @@ __global__ void __launch_bounds__(128) oz_build_kernel(const OzBuild *__restrict
         for (int p = 0; p < NS; ++p) {
           char *o = blob + (q * NS + p) * pstride + lr * 64;
 #pragma unroll
-          for (int e = 0; e < 8; ++e) w[p][e] = h2(sr[e][p], -si[e][p]);
+          for (int e = 0; e < 8; ++e) w[p][e] = h2({sl[e][p].x, -sl[e][p].y});
           st_octet(o, w[p], (lr >> 1) & 1);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) w[p][e] = h2(si[e][p], sr[e][p]);
+          for (int e = 0; e < 8; ++e) w[p][e] = h2({sl[e][p].y, sl[e][p].x});
           st_octet(o + 32, w[p], (lr >> 1) & 1);
         }
       }
