@@ -271,14 +271,14 @@ template <int NS, int STAGE> struct Job {
   }
 };
 
-constexpr int OZ_RING = 16;             // largest operand ring
-constexpr int OZ_SC = 32;               // scale rings: deeper than the operand rings plus the accumulator sets
+constexpr int OZ_RING = 8;              // largest operand ring of a set
+constexpr int OZ_SC = 16;               // scale rings of a set: deeper than its operand ring plus its row tiles
 constexpr int OZ_SMEM = 200 * 1024;
 // Drain warps (then one warp copies and one issues the MMAs): three slices take two octets per
 // thread in 8 warps (hex 8 k: 61 ms against 69 with one octet in 16 warps), six slices one octet
 // in 16 warps (s+p+d: 24 ms against 33: unrolled over two octets the code misses the instruction cache).
 template <int NS> constexpr int oz_drain = 4 * OzCfg<NS>::OCT / OzCfg<NS>::HO;
-template <int NS> constexpr int oz_threads = 32 * (oz_drain<NS> + 2);
+template <int NS> constexpr int oz_threads = 32 * (oz_drain<NS> + 2 * OzCfg<NS>::SETS);
 
 // One lane of a converged warp.  The copy and MMA loops are warp-uniform and
 // elect a lane only around the instruction itself: their descriptors then stay in
@@ -308,10 +308,14 @@ struct Ring {
 // work at all, a K step (8 complex) is 8 MMAs, and two TMEM accumulator sets let
 // one round multiply while the other drains.  Operands stream through rings of
 // segments of SEG K steps; stages 1 and 2 hold the column operand of a task over
-// its row tiles.  The copy and MMA warps' own loops count: with one K step per
-// segment and a table entry read per step they alone took 7.0 of the 10.4 ms of the
-// hexagonal 8 k Sigma stage (three slices).  With segments of 4 it takes 7.0 (of 2: 7.7); stages
-// 1 and 2 keep 2, which leaves room for the next task's columns (s+p+d: 1.33 ms against 1.52).
+// its row tiles.  The issue of an MMA blocks its warp while the tensor pipe is
+// busy, so whatever that warp does in between (barriers, commits, the round
+// table) adds to the time: measured, 200 idle cycles per 4 K steps cost 240.  Each
+// accumulator set therefore has a copy and an MMA warp and rings of its own, and
+// one set's loop overhead is hidden behind the other's MMAs (two issuing warps:
+// 1200 idle cycles cost 100).  Stage 3 of the hexagonal 8 k crystal (three
+// slices), Sigma: one K step per segment and one MMA warp 10.4 ms, segments of four
+// 6.5, an MMA warp per set 6.2.
 // A column tile of one octet (two) fills a quarter (half) of an accumulator set, so
 // stages 2 and 3 put G = OCT / noct row tiles into one.
 //
@@ -330,26 +334,27 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
   static_assert(SETS * SETC <= 512, "the accumulator sets must fit TMEM");
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint32_t tslot;
-  __shared__ __align__(8) uint64_t full[OZ_RING], emptyA[OZ_RING], emptyB[OZ_RING], fullB[2], done[SETS], tfree[SETS], last;
-  __shared__ __align__(16) float sA[OZ_SC][OZ_M], sB[OZ_SC][8 * OCT];
+  __shared__ __align__(8) uint64_t full[SETS][OZ_RING], emptyA[SETS][OZ_RING], emptyB[SETS][OZ_RING], fullB[2],
+      done[SETS], tfree[SETS], last;
+  __shared__ __align__(16) float sA[SETS][OZ_SC][OZ_M], sB[SETS][OZ_SC][8 * OCT];
   __shared__ float gmax[2][OCT][OZ_M];
   __shared__ int abort_flag;
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   if (warp == 0) tc::tmem_alloc(&tslot, 512);
   if (tid == 0) {
-    for (int j = 0; j < OZ_RING; ++j) {
-      tc::mbar_init(&full[j], 1);
-      tc::mbar_init(&emptyA[j], 1);
-      tc::mbar_init(&emptyB[j], 1);
-    }
-    tc::mbar_init(&fullB[0], 1);
-    tc::mbar_init(&fullB[1], 1);
     for (int j = 0; j < SETS; ++j) {
+      for (int k = 0; k < OZ_RING; ++k) {
+        tc::mbar_init(&full[j][k], 1);
+        tc::mbar_init(&emptyA[j][k], 1);
+        tc::mbar_init(&emptyB[j][k], STAGE == 2 ? 1 : SETS);  // stages 1 and 2 use emptyB[0]
+      }
       tc::mbar_init(&done[j], 1);
       tc::mbar_init(&tfree[j], DW);
     }
-    tc::mbar_init(&last, 1);
+    tc::mbar_init(&fullB[0], 1);
+    tc::mbar_init(&fullB[1], 1);
+    tc::mbar_init(&last, SETS);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -381,20 +386,22 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
     }
     return __all_sync(0xffffffffu, hit);
   };
-  // rings: nA segments of A, then nB segments of B (stage 3) or tasksB tasks' B of nB K steps
-  const uint32_t smA = tc::smem_u32(smem), smB = smA + (uint32_t)g.nA * SEG * SA;
+  // rings: nA segments of A per set, then nB segments of B per set (stage 3) or tasksB tasks' B of nB K steps
+  const uint32_t smA0 = tc::smem_u32(smem), smB0 = smA0 + (uint32_t)(SETS * g.nA) * SEG * SA;
 
-  if (warp == DW) {
+  if (warp >= DW && warp < DW + SETS) {
     // ------------------------------ copies ------------------------------
+    const int set = warp - DW;
+    const uint32_t smA = smA0 + set * (g.nA * SEG * SA), smB = smB0 + (STAGE == 2 ? set * (g.nB * SEG * SB) : 0);
     Ring ra(g.nA), rb(STAGE == 2 ? g.nB : g.tasksB);
-    int ia = 0, ib = 0, na = 0, nb = 0;  // segments (of A, of B or tasks), rounds copied
+    int ia = 0, ib = 0, na = 0, nb = 0, n = 0;  // segments (of A, of B or tasks), scales, fills of the sets
     bool ok = true;
     for (int ti = blockIdx.x; ti < g.ntasks && ok; ti += gridDim.x) {
       Job<NS, STAGE> job;
       job.init(g, g.tasks[ti]);
       const uint32_t bb = (uint32_t)(job.noct * NS * 512), sb = (uint32_t)(32 * job.noct);
-      if constexpr (STAGE != 2) {  // the task's column operand, all rounds
-        if (ib >= g.tasksB && !bwait(&emptyB[rb.slot], rb.phase ^ 1)) { ok = false; break; }
+      if (STAGE != 2 && set == 0) {  // the task's column operand, all rounds
+        if (ib >= g.tasksB && !bwait(&emptyB[0][rb.slot], rb.phase ^ 1)) { ok = false; break; }
         if (elect_one()) {
           uint64_t *f = &fullB[rb.slot];
           expect_tx(f, job.kos * bb + job.R * sb);
@@ -402,7 +409,7 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
             const int nks = min(OCT, job.kos - r * OCT);
             const char *bp = job.bptr(r, OzRnd{});
             bulk_load(smB + rb.slot * (g.nB * SB) + r * OCT * bb, bp, nks * bb, f);
-            bulk_load(tc::smem_u32(sB[(nb + r) & (OZ_SC - 1)]), bp + nks * bb, sb, f);
+            bulk_load(tc::smem_u32(sB[0][(nb + r) & (OZ_SC - 1)]), bp + nks * bb, sb, f);
           }
         }
         __syncwarp();
@@ -412,25 +419,27 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
       }
       for (int m0 = 0; m0 < job.outer && ok; m0 += job.G) {
         const int Gm = min(job.G, job.outer - m0);
-        OzRnd nx = job.round(0);
-        for (int r = 0; r < job.R && ok; ++r) {
+        int r = (n ^ set) & (SETS - 1);  // this set's rounds
+        n += job.R;
+        OzRnd nx = job.round(r);
+        for (; r < job.R && ok; r += SETS) {
           const OzRnd q = nx;
-          nx = job.round(r + 1);
+          nx = job.round(r + SETS);
           for (int gi = 0; gi < Gm && ok; ++gi) {
             const bool withb = STAGE == 2 && gi == 0;
             const char *ap = job.aptr(m0 + gi, r, q), *bp = job.bptr(r, q);
             for (int ks = 0; ks < q.nks; ks += SEG) {
-              const int n = min(SEG, q.nks - ks);
-              if (ia >= g.nA && !bwait(&emptyA[ra.slot], ra.phase ^ 1)) { ok = false; break; }
-              if (withb && ib >= g.nB && !bwait(&emptyB[rb.slot], rb.phase ^ 1)) { ok = false; break; }
+              const int nk = min(SEG, q.nks - ks);
+              if (ia >= g.nA && !bwait(&emptyA[set][ra.slot], ra.phase ^ 1)) { ok = false; break; }
+              if (withb && ib >= g.nB && !bwait(&emptyB[set][rb.slot], rb.phase ^ 1)) { ok = false; break; }
               if (elect_one()) {
-                uint64_t *f = &full[ra.slot];
-                expect_tx(f, n * SA + (ks == 0 ? 512u : 0u) + (withb ? n * bb + (ks == 0 ? sb : 0u) : 0u));
-                bulk_load(smA + ra.slot * (SEG * SA), ap + ks * SA, n * SA, f);
-                if (withb) bulk_load(smB + rb.slot * (SEG * SB), bp + ks * bb, n * bb, f);
+                uint64_t *f = &full[set][ra.slot];
+                expect_tx(f, nk * SA + (ks == 0 ? 512u : 0u) + (withb ? nk * bb + (ks == 0 ? sb : 0u) : 0u));
+                bulk_load(smA + ra.slot * (SEG * SA), ap + ks * SA, nk * SA, f);
+                if (withb) bulk_load(smB + rb.slot * (SEG * SB), bp + ks * bb, nk * bb, f);
                 if (ks == 0) {
-                  bulk_load(tc::smem_u32(sA[na & (OZ_SC - 1)]), ap + q.nks * SA, 512, f);
-                  if (withb) bulk_load(tc::smem_u32(sB[nb & (OZ_SC - 1)]), bp + q.nks * bb, sb, f);
+                  bulk_load(tc::smem_u32(sA[set][na & (OZ_SC - 1)]), ap + q.nks * SA, 512, f);
+                  if (withb) bulk_load(tc::smem_u32(sB[set][nb & (OZ_SC - 1)]), bp + q.nks * bb, sb, f);
                 }
               }
               __syncwarp();
@@ -451,20 +460,23 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
     Ring rw(g.nA);
     const int first = max(0, ia - g.nA);
     for (int q = 0; q < ia; ++q) {
-      if (q >= first) tc::mbar_wait(&full[rw.slot], rw.phase, 4000000);
+      if (q >= first) tc::mbar_wait(&full[set][rw.slot], rw.phase, 4000000);
       rw.next();
     }
-    if constexpr (STAGE != 2) {
+    if (STAGE != 2 && set == 0) {
       Ring rv(g.tasksB);
       for (int q = 0; q < ib; ++q) {
         if (q >= ib - g.tasksB) tc::mbar_wait(&fullB[rv.slot], rv.phase, 4000000);
         rv.next();
       }
     }
-  } else if (warp == DW + 1) {
+  } else if (warp >= DW + SETS) {
     // ------------------------------ MMAs ------------------------------
+    const int set = warp - DW - SETS;
+    const uint32_t smA = smA0 + set * (g.nA * SEG * SA), smB = smB0 + (STAGE == 2 ? set * (g.nB * SEG * SB) : 0);
+    const uint32_t ts = tm + set * SETC;
     Ring ra(g.nA), rb(STAGE == 2 ? g.nB : g.tasksB);
-    int n = 0;  // accumulator sets filled
+    int n = 0, fills = 0;  // fills of the sets, of this set
     bool ok = true;
     for (int ti = blockIdx.x; ti < g.ntasks && ok; ti += gridDim.x) {
       Job<NS, STAGE> job;
@@ -476,17 +488,19 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
       const uint32_t bt = smB + rb.slot * (g.nB * SB);
       for (int m0 = 0; m0 < job.outer && ok; m0 += job.G) {
         const int Gm = min(job.G, job.outer - m0);
-        OzRnd nx = job.round(0);
-        for (int r = 0; r < job.R && ok; ++r, ++n) {
-          const int set = n % SETS, nks = __shfl_sync(0xffffffffu, nx.nks, 0);
-          nx = job.round(r + 1);
-          if (n >= SETS && !bwait(&tfree[set], (n / SETS - 1) & 1)) { ok = false; break; }
+        int r = (n ^ set) & (SETS - 1);
+        n += job.R;
+        OzRnd nx = job.round(r);
+        for (; r < job.R && ok; r += SETS, ++fills) {
+          const int nks = __shfl_sync(0xffffffffu, nx.nks, 0);
+          nx = job.round(r + SETS);
+          if (fills >= 1 && !bwait(&tfree[set], (fills - 1) & 1)) { ok = false; break; }
           const Ring rr = rb;
           for (int gi = 0; gi < Gm && ok; ++gi) {
             if (STAGE == 2) rb = rr;
-            const uint32_t d0 = tm + (uint32_t)(set * SETC + gi * 16 * noct);
+            const uint32_t d0 = ts + (uint32_t)(gi * 16 * noct);
             for (int ks = 0; ks < nks; ks += SEG) {
-              if (!bwait(&full[ra.slot], ra.phase)) { ok = false; break; }
+              if (!bwait(&full[set][ra.slot], ra.phase)) { ok = false; break; }
               tc::fence_after_sync();
               const uint32_t a0 = smA + ra.slot * (SEG * SA);
               const uint32_t b0 = STAGE == 2 ? smB + rb.slot * (SEG * SB) : bt + (r * OCT + ks) * NS * bstep;
@@ -509,8 +523,8 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
                                    fresh ? more : 1u);  // kind::f16, types from the descriptor
                     }
                 }
-                tc::commit(&emptyA[ra.slot]);
-                if (STAGE == 2 && gi == Gm - 1) tc::commit(&emptyB[rb.slot]);
+                tc::commit(&emptyA[set][ra.slot]);
+                if (STAGE == 2 && gi == Gm - 1) tc::commit(&emptyB[set][rb.slot]);
               }
               __syncwarp();
               ra.next();
@@ -524,7 +538,7 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
       }
       if (STAGE != 2) {
         if (!ok) break;
-        if (elect_one()) tc::commit(&emptyB[rb.slot]);
+        if (elect_one()) tc::commit(&emptyB[0][rb.slot]);
         __syncwarp();
         rb.next();
       }
@@ -537,7 +551,7 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
     // The rows' destinations are read while the set still multiplies.
     const int lq = warp & 3, os0 = HO * (warp >> 2), row = 32 * lq + lane;
     const uint32_t tbase = tm + ((uint32_t)(32 * lq) << 16) + 16u * os0;
-    int n = 0, i0 = 0, j0 = 0, tile = 0;  // sets, row tiles and column images consumed
+    int n = 0, tile = 0, i0[SETS] = {}, j0[SETS] = {};  // fills, tiles; row tiles and column images by set
     bool dead = false;
     OzTask tk1{};
     if (blockIdx.x < (unsigned)g.ntasks) tk1 = g.tasks[blockIdx.x];
@@ -623,8 +637,10 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
 #pragma unroll
           for (int e = 0; e < 8; ++e) H[q][e] = L[q][e] = M3[NS == 6 ? q : 0][e] = both(0.f);
         }
-        for (int r = 0; r < job.R; ++r, ++n, i0 += Gm) {
-          const int set = n % SETS;
+        for (int r = 0; r < job.R; ++r, ++n) {
+          const int set = n % SETS, ia = set ? i0[SETS - 1] : i0[0], jb = STAGE != 2 ? j0[0] + r : set ? j0[SETS - 1] : j0[0];
+          (set ? i0[SETS - 1] : i0[0]) += Gm;
+          if (STAGE == 2) ++(set ? j0[SETS - 1] : j0[0]);
           if (!dead) dead = !bwait(&done[set], (n / SETS) & 1);
           if (dead) continue;
           tc::fence_after_sync();
@@ -632,9 +648,9 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
 #pragma unroll
           for (int q = 0; q < HO; ++q) {
             if (gi[q] >= Gm) continue;
-            const float *sbp = sB[(j0 + r) & (OZ_SC - 1)] + 8 * oct[q];
+            const float *sbp = sB[STAGE == 2 ? set : 0][jb & (OZ_SC - 1)] + 8 * oct[q];
             const uint32_t base = tbase + (uint32_t)(set * SETC) + 16u * q;
-            const float sa = sA[(i0 + gi[q]) & (OZ_SC - 1)][row];
+            const float sa = sA[set][(ia + gi[q]) & (OZ_SC - 1)][row];
             if constexpr (NS == 3) {
 #pragma unroll
               for (int hf = 0; hf < 2; ++hf) {
@@ -715,7 +731,6 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
           if (lane == 0) tc::mbar_arrive(&tfree[set]);
         }
         if constexpr (STAGE == 2) {  // FP64 partial of this K slice
-          j0 += job.R;
           const OzS3 d = static_cast<const OzS3 *>(g.desc)[tk.d];
 #pragma unroll
           for (int q = 0; q < HO; ++q) {
@@ -857,7 +872,7 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
           for (int q = 0; q < HO; ++q) rw[q] = rw1[q];
         }
       }
-      if (STAGE != 2) j0 += job.R;
+      if (STAGE != 2) j0[0] += job.R;
     }
   }
   __syncthreads();
@@ -1016,12 +1031,14 @@ void oz_rings(int ns, int stage, int max_kos, OzArgs *a) {
   const int seg = ns == 3 ? (stage == 2 ? OzCfg<3>::SEG3 : OzCfg<3>::SEG)
                           : (stage == 2 ? OzCfg<6>::SEG3 : OzCfg<6>::SEG);
   const int slotA = seg * ns * 4096, stepB = ns * 512 * OZ_OCT;
+  const int sets = ns == 3 ? OzCfg<3>::SETS : OzCfg<6>::SETS;
   if (stage == 2) {
-    a->nA = a->nB = std::min(OZ_RING, OZ_SMEM / (slotA + seg * stepB));
+    a->nA = a->nB = std::min(OZ_RING, OZ_SMEM / (sets * (slotA + seg * stepB)));
   } else {
     a->nB = max_kos;
-    a->tasksB = (OZ_SMEM - 2 * a->nB * stepB) / slotA >= 3 ? 2 : 1;
-    a->nA = std::min(OZ_RING, (OZ_SMEM - a->tasksB * a->nB * stepB) / slotA);
+    auto ring = [&](int tasks) { return std::min(OZ_RING, (OZ_SMEM - tasks * a->nB * stepB) / (sets * slotA)); };
+    a->tasksB = ring(2) >= 3 ? 2 : 1;
+    a->nA = ring(a->tasksB);
   }
   GWGB_REQUIRE(a->nA >= 2, GWGB_E_UNSUPPORTED, "sliced GEMM rings too small");
 }

@@ -29,11 +29,12 @@ constexpr int OZ_M = 128;   // rows per tile (TMEM lanes)
 constexpr int64_t OZ_CHUNK_BYTES = 8ll << 30;
 
 // Geometry of one slicing: NS planes; OCT octets (of 8 complex) per round and per column tile; NACC
-// accumulators of slice products up to class CMAX, SETS sets of them in TMEM; HO octets per drain thread;
+// accumulators of slice products up to class CMAX, SETS sets of them in TMEM, each with a copy and an MMA warp
+// and operand rings of its own; HO octets per drain thread;
 // SEG K steps per operand copy (SEG3: in stage 3).
 template <int NS> struct OzCfg;
 template <> struct OzCfg<3> {  // 33-bit operands: the split-precision path
-  static constexpr int OCT = 4, NACC = 4, CMAX = 3, SETS = 2, HO = 2, SEG = 2, SEG3 = 4;
+  static constexpr int OCT = 4, NACC = 4, CMAX = 3, SETS = 2, HO = 2, SEG = 2, SEG3 = 2;
 };
 template <> struct OzCfg<6> {  // 57-bit operands: the FP64 contractions
   static constexpr int OCT = 4, NACC = 7, CMAX = 6, SETS = 1, HO = 1, SEG = 1, SEG3 = 1;
@@ -120,7 +121,7 @@ struct OzArgs {
   const char *A, *B;
   char *X;                   // stages 1, 2: output images
   double2 *part;             // stage 3
-  int nA, nB;                // operand rings (segments of K steps); stages 1, 2: nB K steps of B per task,
+  int nA, nB;                // operand rings of a set (segments of K steps); stages 1, 2: nB K steps of B per task,
   int tasksB;                // for one or two tasks
   int *err;
 };
