@@ -568,13 +568,13 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
         oct[q] = os0 + q - gi[q] * job.noct;
       }
       // stage 1: the row and its destination
-      int rg = 0, M = 0, nL = 1, tau = 0, Lr = 0, dtau = 0, dL = 0, gs = 1, goff = 0, nLg = 1, glog = 0, nt2 = 1;
+      int rg = 0, M = 0, nL = 1, tau = 0, Lr = 0, dtau = 0, dL = 0, gs = 1, glog = 0, nt2 = 1, nLp = 0, nx = 0;
+      int slot0 = 0, ksq[HO], xq[HO];  // first slot; K step and x of the octets
       int64_t t2bytes = 0;
       char *xbase = g.X;
       // stage 2
       const OzRow *rows = nullptr;
       OzRow rw[HO];
-      int zos = 1;
       if constexpr (STAGE == 0) {
         const OzS1 d = static_cast<const OzS1 *>(g.desc)[tk.d];
         const OzCol1 col = static_cast<const OzCol1 *>(g.aux1)[tk.i];
@@ -582,9 +582,9 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
         M = d.M;
         nL = d.nL;
         gs = col.gs;
-        nLg = d1.nLg;
-        glog = d1.glog;
-        goff = d1.gbase + col.x0 * nLg;
+        slot0 = d1.slot0;
+        nLp = d1.nLp;
+        nx = d1.nx;
         nt2 = d1.nt2;
         t2bytes = d1.t2bytes;
         xbase += d1.base + col.yoff;
@@ -594,19 +594,23 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
         dtau = OZ_M / nL;
         dL = OZ_M - dtau * nL;
 #pragma unroll
-        for (int q = 0; q < HO; ++q) nv[q] = col.ny - 8 * (oct[q] % gs);
+        for (int q = 0; q < HO; ++q) {
+          const int grp = oct[q] / gs;
+          ksq[q] = oct[q] - grp * gs;
+          xq[q] = col.x0 + grp;
+          nv[q] = col.ny - 8 * ksq[q];
+                  }
       } else if constexpr (STAGE == 1) {
         const OzS2 d = static_cast<const OzS2 *>(g.desc)[tk.d];
         gs = job.noct;
         glog = d.glog;
-        zos = d.zos;
         tau = tk.i & 0xffff;
         xbase += (tk.i >> 16) * oz_abytes(NS, OCT);
         rows = static_cast<const OzRow *>(g.aux1) + d.rows + tk.m0 * OZ_M + row;
 #pragma unroll
         for (int q = 0; q < HO; ++q) {
           nv[q] = d.nz - 8 * ((tk.i >> 16) * OCT + oct[q]);
-          rw[q] = {-1, 0, 0};
+          rw[q].pk = OZ_NOROW;
           if (gi[q] < min(job.G, job.outer)) rw[q] = rows[gi[q] * OZ_M];
         }
       } else {
@@ -618,13 +622,11 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
       }
       for (int m0 = 0; m0 < job.outer; m0 += job.G, ++tile) {
         const int Gm = min(job.G, job.outer - m0);
-        OzDst2 d2[HO];
         OzRow rw1[HO];
         if constexpr (STAGE == 1) {
 #pragma unroll
           for (int q = 0; q < HO; ++q) {
-            if (rw[q].dst >= 0) d2[q] = static_cast<const OzDst2 *>(g.aux2)[rw[q].dst];
-            rw1[q] = {-1, 0, 0};
+            rw1[q].pk = OZ_NOROW;
             if (m0 + job.G + gi[q] < job.outer) rw1[q] = rows[(m0 + job.G + gi[q]) * OZ_M];
           }
         }
@@ -761,7 +763,7 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
           int ee[HO];
 #pragma unroll
           for (int q = 0; q < HO; ++q) {
-            valid[q] = gi[q] < Gm && (STAGE == 0 ? rg < M : rw[q].dst >= 0);
+            valid[q] = gi[q] < Gm && (STAGE == 0 ? rg < M : rw[q].pk != OZ_NOROW);
             float mo[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
@@ -815,16 +817,16 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
             char *blob = xbase;
             int nksb = gs, rr, ks;
             if constexpr (STAGE == 0) {
-              const int grp = oct[q] / gs;
-              const int slot = ((goff + grp * nLg + (Lr >> glog)) << glog) + (Lr & ((1 << glog) - 1));
+              const int Lq = Lr & ~3, slot = slot0 + Lq * nx + xq[q] * min(4, nLp - Lq) + (Lr & 3);
               blob += ((int64_t)tau * nt2 + (slot >> 7)) * t2bytes;
               rr = slot & 127;
-              ks = oct[q] - grp * gs;
+              ks = ksq[q];
             } else {
-              const int fr = tau * d2[q].nx + rw[q].x, Lg = rw[q].L >> glog;
-              if (glog) nksb = min(1 << glog, d2[q].nL - (Lg << glog)) * zos;
-              ks = (rw[q].L & ((1 << glog) - 1)) * zos + oct[q];
-              blob += d2[q].base + (fr >> 7) * d2[q].fbytes + d2[q].kbase + (int64_t)Lg * d2[q].lgbytes;
+              const uint32_t pk = rw[q].pk;
+              const int fr = tau * (int)((pk >> 8) & 255) + (int)(pk & 255);
+              if (glog) nksb = (int)(pk >> 24);
+              ks = (int)((pk >> 16) & 255) + oct[q];
+              blob += rw[q].base + (int64_t)(fr >> 7) * rw[q].f16 * 16;
               rr = fr & 127;
             }
             uint32_t w[NS][8];

@@ -62,12 +62,16 @@ struct OzCol1 {
   int8_t ngrp, gs;
   int32_t ny;      // valid y of this round
 };
-// Where the stage-1 output of a contribution goes: stage-2 row slots
-//   group gi = gbase + x * nLg + (L >> glog), slot = (gi << glog) + (L & (2^glog - 1)),
-// tile slot / 128 of base + (tau * nt2 + tile) * t2bytes.
+// Where the stage-1 output of a contribution goes: row slots of stage 2.  Blocks of four L, in each the x, in each x the
+// L of the block: with Lq = L & ~3 and n = min(4, nLp - Lq),
+//   slot = slot0 + Lq * nx + x * n + (L & 3)
+// (slot0 a multiple of 4, nLp = nL padded to 2^glog), tile slot / 128 of base + (tau * nt2 + tile) * t2bytes.  A warp
+// of the stage-1 drain (consecutive L) then writes whole 128-byte lines of four rows, and one of the stage-2 drain
+// holds 8 x of 4 L, which are 8 neighbouring rows of 4 images; with the L of an x next to one another its 32 rows
+// were 32 lines (stage 2 of Sigma, hexagonal 8 k: three slices 15.4 ms, with blocks of four 13.1; six slices, 4 k: 7.4, 5.95).
 struct OzDst1 {
   int64_t base, t2bytes;
-  int32_t nt2, gbase, nLg, glog;
+  int32_t nt2, slot0, nLp, nx;
 };
 // Stage 2: one pack (contributions that share the B2 operand and glog).
 struct OzS2 {
@@ -77,13 +81,14 @@ struct OzS2 {
   int32_t rows;            // first entry of the row map
   int32_t nz;              // valid z
 };
-struct OzRow { int32_t dst; int16_t x, L; };  // stage-2 row slot; dst < 0: empty
-// Where the stage-2 output of a contribution goes: final row tau * nx + x in
-// row tile f at base + f * fbytes; the round of L group Lg at kbase + Lg * lgbytes.
-struct OzDst2 {
-  int64_t base, fbytes;
-  int32_t kbase, lgbytes, nx, nL;
+// A row slot of stage 2: row tau * nx + x of the stage-3 image at base + (row / 128) * f16 * 16, octets of K from ks
+// on; nks: octets of the image (glog > 0).
+struct OzRow {
+  int64_t base;
+  int32_t f16;
+  uint32_t pk;  // x | nx << 8 | ks << 16 | nks << 24; OZ_NOROW: empty
 };
+constexpr uint32_t OZ_NOROW = 0xffffffffu;
 // Stage 3: one unit (a K slice of an output block).
 struct OzS3 {
   int64_t a, fbytes;       // X2 images: a + f * fbytes + round offset
@@ -117,7 +122,7 @@ struct OzArgs {
   const void *desc;
   const OzTask *tasks;
   int ntasks;
-  const void *aux1, *aux2;   // stage 1: OzCol1, OzDst1; stage 2: OzRow, OzDst2; stage 3: OzRnd
+  const void *aux1, *aux2;   // stage 1: OzCol1, OzDst1; stage 2: OzRow; stage 3: OzRnd
   const char *A, *B;
   char *X;                   // stages 1, 2: output images
   double2 *part;             // stage 3

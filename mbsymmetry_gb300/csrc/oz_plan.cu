@@ -58,7 +58,6 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
   std::vector<OzDst1> dst1;
   std::vector<OzS2> s2;
   std::vector<OzRow> rows;
-  std::vector<OzDst2> dst2;
   std::vector<OzS3> s3;
   std::vector<OzRnd> rnd;
   std::vector<RedTask> red;
@@ -243,12 +242,11 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
     }
     int64_t voff = vbase;
     const size_t bv0 = builds.size();
-    struct Pack { std::vector<int> cs; std::vector<int> dst; int groups = 0; int64_t base = 0; };
+    struct Pack { std::vector<int> cs; int64_t slots = 0; };
     std::map<std::tuple<int64_t, int, int>, Pack> packs;  // (B2 block, conj, glog)
-    struct Use { int c, pack_g, d1, d2; };
+    struct Use { int c, d1; int64_t slot, x2, fb, kbase, lgb; };
     std::vector<Use> uses;
-    const size_t s3_0 = s3.size(), t3a = 0;
-    (void)t3a;
+    const size_t s3_0 = s3.size();
     int64_t x2 = 0;
     std::vector<OzTask> t3;
     OzLaunch l1, l2, l3;
@@ -320,13 +318,10 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
         const OzContrib &x = cs[c];
         const int g = 1 << glog[c], zos = cdiv(x.nz, 8), R = cdiv(zos, OCT), nLg = cdiv(x.nL, g);
         const int64_t lgb = R > 1 ? (int64_t)NS * zos * 4096 + 512 * R : oz_abytes(NS, g * zos);
-        const int d2 = (int)dst2.size();
-        dst2.push_back({x2, fb, (int32_t)kbase[c - un.c0], (int32_t)lgb, x.nx, x.nL});
-        GWGB_REQUIRE(kbase[c - un.c0] < INT32_MAX, GWGB_E_UNSUPPORTED, "sliced unit too large");
         Pack &p = packs[std::make_tuple(x.b2, (int)x.b2conj, glog[c])];
-        uses.push_back({c, p.groups, 0, d2});
+        uses.push_back({c, 0, p.slots, x2, fb, kbase[c - un.c0], lgb});
         p.cs.push_back((int)uses.size() - 1);
-        p.groups += x.nx * nLg;
+        p.slots += ((int64_t)x.nx * nLg * g + 3) / 4 * 4;
         const double rowsx = (double)ntau * x.nx * x.nL;
         l1.flops += 8.0 * rowsx * x.ny * x.K1;
         l2.flops += 8.0 * rowsx * x.ny * x.nz;
@@ -346,7 +341,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
     std::vector<OzTask> t2;
     int m_kos2 = 1;
     int64_t npk_tiles = 0;
-    for (auto &kv : packs) npk_tiles += (int64_t)ntau * cdiv((int64_t)kv.second.groups << std::get<2>(kv.first), OZ_M);
+    for (auto &kv : packs) npk_tiles += (int64_t)ntau * cdiv(kv.second.slots, OZ_M);
     // row tiles per task: enough tasks for about eight waves, at most 16 tiles
     const int per2 = (int)std::max<int64_t>(1, std::min<int64_t>(16, npk_tiles / (8 * (int64_t)std::max(1, nsm))));
     for (auto &kv : packs) {
@@ -354,26 +349,29 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
       const int gl = std::get<2>(kv.first);
       const OzContrib &x0 = cs[uses[p.cs[0]].c];
       const int kos = cdiv(x0.ny, 8), R = cdiv(kos, OCT), zos = cdiv(x0.nz, 8), nzt = cdiv(zos, OCT);
-      const int nt2 = cdiv((int64_t)p.groups << gl, OZ_M);
+      const int nt2 = cdiv(p.slots, OZ_M);
       const int64_t t2b = (int64_t)NS * kos * 4096 + 512 * R;
       const B2 &b2 = b2_of[std::make_pair(x0.b2, (int)x0.b2conj)];
       const int id = (int)s2.size();
       s2.push_back({x1, t2b, b2.b, b2.bt, b2.bz, nt2, kos, zos, gl, (int32_t)rows.size(), x0.nz});
       const size_t r0 = rows.size();
-      rows.resize(r0 + (size_t)nt2 * OZ_M, OzRow{-1, 0, 0});
+      rows.resize(r0 + (size_t)nt2 * OZ_M, OzRow{0, 0, OZ_NOROW});
       for (int ui : p.cs) {
         Use &us = uses[ui];
         const OzContrib &x = cs[us.c];
         GWGB_REQUIRE(x.ny == x0.ny && x.nz == x0.nz && x.b2z == x0.b2z && x.b2y == x0.b2y && x.b2t == x0.b2t,
                      GWGB_E_INVALID, "sliced pack of unequal blocks");
-        const int nLg = cdiv(x.nL, 1 << gl);
+        const int g = 1 << gl, nLp = cdiv(x.nL, g) * g;
         us.d1 = (int)dst1.size();
-        dst1.push_back({x1, t2b, nt2, us.pack_g, nLg, gl});
+        dst1.push_back({x1, t2b, nt2, (int32_t)us.slot, nLp, x.nx});
         for (int xx = 0; xx < x.nx; ++xx)
           for (int L = 0; L < x.nL; ++L) {
-            const int64_t slot = ((int64_t)(us.pack_g + xx * nLg + (L >> gl)) << gl) + (L & ((1 << gl) - 1));
+            const int Lq = L & ~3, Lg = L >> gl;
+            const int64_t slot = us.slot + Lq * x.nx + xx * std::min(4, nLp - Lq) + (L & 3);
             check_range(slot, 1, (int64_t)nt2 * OZ_M, "sliced stage-2 row");
-            rows[r0 + slot] = {us.d2, (int16_t)xx, (int16_t)L};
+            rows[r0 + slot] = {us.x2 + us.kbase + Lg * us.lgb, (int32_t)(us.fb / 16),
+                               (uint32_t)xx | (uint32_t)x.nx << 8 | (uint32_t)((L & (g - 1)) * zos) << 16 |
+                                   (uint32_t)(gl ? std::min(g, x.nL - Lg * g) * zos : 0) << 24};
           }
       }
       x1 += (int64_t)ntau * nt2 * t2b;
@@ -485,7 +483,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
   };
   auto each = [&](auto &&f) {
     f(builds, builds_); f(tasks, tasks_); f(s1, s1_); f(col1, col1_); f(dst1, dst1_); f(s2, s2_); f(rows, rows_);
-    f(dst2, dst2_); f(s3, s3_); f(rnd, rnd_); f(red, red_);
+    f(s3, s3_); f(rnd, rnd_); f(red, red_);
   };
   each(place);
   host_.resize(total);
@@ -497,7 +495,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
 void OzPlan::upload(cudaStream_t st) {
   lists_.alloc(host_.size());
   auto at = [&](auto &l) { l.p = reinterpret_cast<decltype(l.p)>(lists_.p + reinterpret_cast<size_t>(l.p)); };
-  at(builds_); at(tasks_); at(s1_); at(col1_); at(dst1_); at(s2_); at(rows_); at(dst2_); at(s3_); at(rnd_); at(red_);
+  at(builds_); at(tasks_); at(s1_); at(col1_); at(dst1_); at(s2_); at(rows_); at(s3_); at(rnd_); at(red_);
   if (!host_.empty()) GWGB_CUDA(cudaMemcpyAsync(lists_.p, host_.data(), host_.size(), cudaMemcpyHostToDevice, st));
   GWGB_CUDA(cudaStreamSynchronize(st));
   host_ = std::vector<char>();
@@ -533,7 +531,6 @@ void OzPlan::run_one(const OzLaunch &l, OzShared &sh, const double2 *V, const do
   } else if (l.d0 == 1) {
     a.desc = s2_.p;
     a.aux1 = rows_.p;
-    a.aux2 = dst2_.p;
     a.A = sh.X1.p;
     a.B = sh.B2.p;
     a.X = sh.X2.p;

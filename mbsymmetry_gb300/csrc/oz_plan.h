@@ -124,7 +124,6 @@ class OzPlan {
   List<OzDst1> dst1_;
   List<OzS2> s2_;
   List<OzRow> rows_;
-  List<OzDst2> dst2_;
   List<OzS3> s3_;
   List<OzRnd> rnd_;
   List<RedTask> red_;
