@@ -26,7 +26,7 @@ namespace gwgb {
 
 constexpr int OZ_M = 128;   // rows per tile (TMEM lanes)
 // X1 + X2 of one chunk, when that is at most an eighth of the free memory.
-constexpr int64_t OZ_CHUNK_BYTES = 8ll << 30;
+constexpr int64_t OZ_CHUNK_BYTES = 16ll << 30;
 
 // Geometry of one slicing: NS planes; OCT octets (of 8 complex) per round and per column tile; NACC
 // accumulators of slice products up to class CMAX, SETS sets of them in TMEM, each with a copy and an MMA warp

@@ -249,6 +249,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
     const size_t s3_0 = s3.size();
     int64_t x2 = 0;
     std::vector<OzTask> t3;
+    std::vector<std::pair<int64_t, int64_t>> s3_cost;  // of the chunk's units: drains, K steps
     OzLaunch l1, l2, l3;
     l1.stage = stage0; l2.stage = stage0 + 1; l3.stage = stage0 + 2;
     // stage 3: X2 and V3 layout of every unit
@@ -311,6 +312,9 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
       s3.push_back({x2, fb, hit->second.first, bz, part, (int32_t)rnd.size(), (int32_t)rr.size(), ntau * ow.nx, ow.N,
                     ow.nx, ow.N * ow.nx, ow.sn, ow.sx, OCT, 0});
       rnd.insert(rnd.end(), rr.begin(), rr.end());
+      int64_t steps = 0;
+      for (const OzRnd &q : rr) steps += q.nks;
+      s3_cost.push_back({3 * (int64_t)rr.size(), steps});
       for (int ct = 0; ct < nct; ++ct)
         for (int f = 0, G = OCT / std::min(OCT, nos - ct * OCT); f < nf; f += G)
           t3.push_back({id, f | ct << 16, 0, std::min(G, nf - f)});
@@ -426,17 +430,29 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
         for (int m = 0; m < k.n; m += per1) t.push_back({k.d, k.i, m, std::min(per1, k.n - m)});
       t1.swap(t);
     }
-    std::stable_sort(t3.begin(), t3.end(), [&](const OzTask &a, const OzTask &b) { return s3[a.d].nkr > s3[b.d].nkr; });
     GWGB_REQUIRE(ntau < 65536, GWGB_E_UNSUPPORTED, "too many tau points");
     vimg_ = std::max(vimg_, voff);
     add_build(persist ? static_ : launches_, bv0, builds.size(), 0, IMG_V, stage0);
     if (persist) vbase = voff;
+    // Longest tasks first: CTA c takes tasks c, c + grid, ..., so the loads differ by one task at most.  Cost in K
+    // steps of MMAs: a drain of the accumulators takes about eight in stages 1 and 2, three in stage 3.
+    auto cost = [&](const OzTask &k, int stage) -> int64_t {
+      if (stage == 0) return (int64_t)k.n * (8 * cdiv(s1[k.d].kos, OCT) + s1[k.d].kos);
+      if (stage == 1) {
+        const int G = OCT / std::min(OCT, s2[k.d].zos - (k.i >> 16) * OCT);
+        return (int64_t)cdiv(k.n, G) * 8 * cdiv(s2[k.d].kos, OCT) + (int64_t)k.n * s2[k.d].kos;
+      }
+      return s3_cost[k.d - s3_0].first + k.n * s3_cost[k.d - s3_0].second;
+    };
     auto add_gemm = [&](OzLaunch l, const std::vector<OzTask> &t, int stage, int kos) {
       l.kind = 0;
       l.t0 = (int64_t)tasks.size();
       l.n = (int64_t)t.size();
       if (t.empty()) return;
-      tasks.insert(tasks.end(), t.begin(), t.end());
+      std::vector<std::pair<int64_t, int>> order(t.size());
+      for (size_t i = 0; i < t.size(); ++i) order[i] = {-cost(t[i], stage), (int)i};
+      std::sort(order.begin(), order.end());
+      for (const auto &o : order) tasks.push_back(t[o.second]);
       oz_rings(NS, stage, kos, &l.args);
       l.d0 = stage;
       launches_.push_back(l);
