@@ -102,20 +102,26 @@ struct Tri {
   F2 h, m, l;
 };
 
-// The value of the class sums D0 .. D6 (weights 2^(-9c)); D0 to D3 are exact integers.
+// The value of the class sums D0 .. D6 (weights 2^(-9c)).  Carries instead of two-sums (26 steps against 44): D0 to D3
+// are exact integers, at most 64 sums of c + 1 products of digits, of which at most one is 256 in each factor, so D3 and
+// a carry of 2^15.4 stay below 2^24 and each step is exact (but for the last bits of D4 to D6, which the tensor core
+// rounds to 24 bits).
 __device__ __forceinline__ Tri tri_of(const F2 (&d)[7]) {
-  const F2 W1 = both(0x1p-9f), W2 = both(0x1p-18f), W3 = both(0x1p-27f), W4 = both(0x1p-36f);
-  F2 h, e1, s, e2, e3;
-  two_sum(d[0], mul2(d[1], W1), h, e1);
-  two_sum(mul2(d[2], W2), mul2(d[3], W3), s, e2);
-  two_sum(e1, s, e1, e3);
-  const F2 l = fma2(fma2(fma2(d[6], W1, d[5]), W1, d[4]), W4, add2(e2, e3));
-  // h is zero only when the value is (all of it can lie in the low classes)
-  two_sum(h, e1, h, e1);
-  two_sum(e1, l, e1, e2);
+  const F2 W = both(0x1p-9f), MG = both(1.5f * 8388608.f), NM = both(-1.5f * 8388608.f), NB = both(-512.f);
+  auto carry = [&](F2 x) { return add2(fma2(x, W, MG), NM); };  // x / 512 to an integer
+  const F2 d4 = fma2(fma2(d[6], W, d[5]), W, d[4]), c4 = carry(d4);
+  const F2 d3 = add2(d[3], c4), c3 = carry(d3);
+  const F2 d2 = add2(d[2], c3), c2 = carry(d2);
+  const F2 d1 = add2(d[1], c2), c1 = carry(d1);
+  // a an integer, m a multiple of 2^-18 below 0.51, l below 2^-18 0.51: each zero or larger than the next
+  const F2 a = add2(d[0], c1);
+  const F2 m = fma2(fma2(c1, NB, d1), both(0x1p-9f), mul2(fma2(c2, NB, d2), both(0x1p-18f)));
+  const F2 l = fma2(fma2(c3, NB, d3), both(0x1p-27f), mul2(fma2(c4, NB, d4), both(0x1p-36f)));
+  const F2 m1 = add2(m, l);
   Tri t;
-  two_sum(h, e1, t.h, t.m);
-  t.l = e2;
+  t.h = add2(a, m1);
+  t.m = sub2(m1, sub2(t.h, a));
+  t.l = sub2(l, sub2(m1, m));
   return t;
 }
 
