@@ -284,7 +284,7 @@ constexpr int OZ_SMEM = 200 * 1024;
 // thread in 8 warps (hex 8 k: 61 ms against 69 with one octet in 16 warps), six slices one octet
 // in 16 warps (s+p+d: 24 ms against 33: unrolled over two octets the code misses the instruction cache).
 template <int NS> constexpr int oz_drain = 4 * OzCfg<NS>::OCT / OzCfg<NS>::HO;
-template <int NS> constexpr int oz_threads = 32 * (oz_drain<NS> + 2 * OzCfg<NS>::SETS);
+template <int NS> constexpr int oz_threads = NS == 6 ? 640 : 32 * (oz_drain<NS> + 2 * OzCfg<NS>::SETS);
 
 // One lane of a converged warp.  The copy and MMA loops are warp-uniform and
 // elect a lane only around the instruction itself: their descriptors then stay in
@@ -395,163 +395,9 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
   // rings: nA segments of A per set, then nB segments of B per set (stage 3) or tasksB tasks' B of nB K steps
   const uint32_t smA0 = tc::smem_u32(smem), smB0 = smA0 + (uint32_t)(SETS * g.nA) * SEG * SA;
 
-  if (warp >= DW && warp < DW + SETS) {
-    // ------------------------------ copies ------------------------------
-    const int set = warp - DW;
-    const uint32_t smA = smA0 + set * (g.nA * SEG * SA), smB = smB0 + (STAGE == 2 ? set * (g.nB * SEG * SB) : 0);
-    Ring ra(g.nA), rb(STAGE == 2 ? g.nB : g.tasksB);
-    int ia = 0, ib = 0, na = 0, nb = 0, n = 0;  // segments (of A, of B or tasks), scales, fills of the sets
-    bool ok = true;
-    for (int ti = blockIdx.x; ti < g.ntasks && ok; ti += gridDim.x) {
-      Job<NS, STAGE> job;
-      job.init(g, g.tasks[ti]);
-      const uint32_t bb = (uint32_t)(job.noct * NS * 512), sb = (uint32_t)(32 * job.noct);
-      if (STAGE != 2 && set == 0) {  // the task's column operand, all rounds
-        if (ib >= g.tasksB && !bwait(&emptyB[0][rb.slot], rb.phase ^ 1)) { ok = false; break; }
-        if (elect_one()) {
-          uint64_t *f = &fullB[rb.slot];
-          expect_tx(f, job.kos * bb + job.R * sb);
-          for (int r = 0; r < job.R; ++r) {
-            const int nks = min(OCT, job.kos - r * OCT);
-            const char *bp = job.bptr(r, OzRnd{});
-            bulk_load(smB + rb.slot * (g.nB * SB) + r * OCT * bb, bp, nks * bb, f);
-            bulk_load(tc::smem_u32(sB[0][(nb + r) & (OZ_SC - 1)]), bp + nks * bb, sb, f);
-          }
-        }
-        __syncwarp();
-        nb += job.R;
-        rb.next();
-        ++ib;
-      }
-      for (int m0 = 0; m0 < job.outer && ok; m0 += job.G) {
-        const int Gm = min(job.G, job.outer - m0);
-        int r = (n ^ set) & (SETS - 1);  // this set's rounds
-        n += job.R;
-        OzRnd nx = job.round(r);
-        for (; r < job.R && ok; r += SETS) {
-          const OzRnd q = nx;
-          nx = job.round(r + SETS);
-          for (int gi = 0; gi < Gm && ok; ++gi) {
-            const bool withb = STAGE == 2 && gi == 0;
-            const char *ap = job.aptr(m0 + gi, r, q), *bp = job.bptr(r, q);
-            for (int ks = 0; ks < q.nks; ks += SEG) {
-              const int nk = min(SEG, q.nks - ks);
-              if (ia >= g.nA && !bwait(&emptyA[set][ra.slot], ra.phase ^ 1)) { ok = false; break; }
-              if (withb && ib >= g.nB && !bwait(&emptyB[set][rb.slot], rb.phase ^ 1)) { ok = false; break; }
-              if (elect_one()) {
-                uint64_t *f = &full[set][ra.slot];
-                expect_tx(f, nk * SA + (ks == 0 ? 512u : 0u) + (withb ? nk * bb + (ks == 0 ? sb : 0u) : 0u));
-                bulk_load(smA + ra.slot * (SEG * SA), ap + ks * SA, nk * SA, f);
-                if (withb) bulk_load(smB + rb.slot * (SEG * SB), bp + ks * bb, nk * bb, f);
-                if (ks == 0) {
-                  bulk_load(tc::smem_u32(sA[set][na & (OZ_SC - 1)]), ap + q.nks * SA, 512, f);
-                  if (withb) bulk_load(tc::smem_u32(sB[set][nb & (OZ_SC - 1)]), bp + q.nks * bb, sb, f);
-                }
-              }
-              __syncwarp();
-              if (withb) {
-                rb.next();
-                ++ib;
-              }
-              ra.next();
-              ++ia;
-            }
-            ++na;
-            if (withb) ++nb;
-          }
-        }
-      }
-    }
-    // every copy issued has landed before the CTA may end
-    Ring rw(g.nA);
-    const int first = max(0, ia - g.nA);
-    for (int q = 0; q < ia; ++q) {
-      if (q >= first) tc::mbar_wait(&full[set][rw.slot], rw.phase, 4000000);
-      rw.next();
-    }
-    if (STAGE != 2 && set == 0) {
-      Ring rv(g.tasksB);
-      for (int q = 0; q < ib; ++q) {
-        if (q >= ib - g.tasksB) tc::mbar_wait(&fullB[rv.slot], rv.phase, 4000000);
-        rv.next();
-      }
-    }
-  } else if (warp >= DW + SETS) {
-    // ------------------------------ MMAs ------------------------------
-    const int set = warp - DW - SETS;
-    const uint32_t smA = smA0 + set * (g.nA * SEG * SA), smB = smB0 + (STAGE == 2 ? set * (g.nB * SEG * SB) : 0);
-    const uint32_t ts = tm + set * SETC;
-    Ring ra(g.nA), rb(STAGE == 2 ? g.nB : g.tasksB);
-    int n = 0, fills = 0;  // fills of the sets, of this set
-    bool ok = true;
-    for (int ti = blockIdx.x; ti < g.ntasks && ok; ti += gridDim.x) {
-      Job<NS, STAGE> job;
-      job.init(g, g.tasks[ti]);
-      const int noct = __shfl_sync(0xffffffffu, job.noct, 0);
-      const uint32_t id = idesc_f16(16 * noct);
-      const uint32_t bstep = 512u * noct;  // one plane of one K step
-      if (STAGE != 2 && !bwait(&fullB[rb.slot], rb.phase)) { ok = false; break; }
-      const uint32_t bt = smB + rb.slot * (g.nB * SB);
-      for (int m0 = 0; m0 < job.outer && ok; m0 += job.G) {
-        const int Gm = min(job.G, job.outer - m0);
-        int r = (n ^ set) & (SETS - 1);
-        n += job.R;
-        OzRnd nx = job.round(r);
-        for (; r < job.R && ok; r += SETS, ++fills) {
-          const int nks = __shfl_sync(0xffffffffu, nx.nks, 0);
-          nx = job.round(r + SETS);
-          if (fills >= 1 && !bwait(&tfree[set], (fills - 1) & 1)) { ok = false; break; }
-          const Ring rr = rb;
-          for (int gi = 0; gi < Gm && ok; ++gi) {
-            if (STAGE == 2) rb = rr;
-            const uint32_t d0 = ts + (uint32_t)(gi * 16 * noct);
-            for (int ks = 0; ks < nks; ks += SEG) {
-              if (!bwait(&full[set][ra.slot], ra.phase)) { ok = false; break; }
-              tc::fence_after_sync();
-              const uint32_t a0 = smA + ra.slot * (SEG * SA);
-              const uint32_t b0 = STAGE == 2 ? smB + rb.slot * (SEG * SB) : bt + (r * OCT + ks) * NS * bstep;
-              if (elect_one()) {
-#pragma unroll
-                for (int k = 0; k < SEG; ++k) {
-                  if (ks + k >= nks) break;
-                  const uint32_t more = ks + k > 0 ? 1u : 0u;
-#pragma unroll
-                  for (int c = 0; c <= OzCfg<NS>::CMAX; ++c)
-#pragma unroll
-                    for (int p = 0; p < NS; ++p) {
-                      const int q = c - p;
-                      if (q < 0 || q >= NS) continue;
-                      // NS = 3: (0,0) | (0,1) | (1,0) | the rest; NS = 6: one per class
-                      const int acc = NS == 6 ? c : c == 0 ? 0 : c == 1 ? 1 + p : 3;
-                      const bool fresh = NS == 6 ? p == max(0, c - NS + 1) : c < 2 || (c == 2 && p == 0);
-                      tc::mma_bf16(d0 + acc * NR, sw32_desc(a0 + k * SA + p * 4096u),
-                                   sw32_desc(b0 + (k * NS + q) * bstep), id,
-                                   fresh ? more : 1u);  // kind::f16, types from the descriptor
-                    }
-                }
-                tc::commit(&emptyA[set][ra.slot]);
-                if (STAGE == 2 && gi == Gm - 1) tc::commit(&emptyB[set][rb.slot]);
-              }
-              __syncwarp();
-              ra.next();
-              if (STAGE == 2) rb.next();
-            }
-          }
-          if (!ok) break;
-          if (elect_one()) tc::commit(&done[set]);
-          __syncwarp();
-        }
-      }
-      if (STAGE != 2) {
-        if (!ok) break;
-        if (elect_one()) tc::commit(&emptyB[0][rb.slot]);
-        __syncwarp();
-        rb.next();
-      }
-    }
-    if (elect_one()) tc::commit(&last);  // arrives when every MMA issued above has completed
-    __syncwarp();
-  } else {
+  // six slices: 16 x 32 x 112 + 4 x 32 x 32 registers are the launch's 640 x 96
+  if (warp < DW) {
+    if constexpr (NS == 6) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
     // ------------------------------ drain ------------------------------
     // warp w: TMEM lanes (rows) 32 (w & 3) .. + 31, octets HO (w >> 2) .. + HO - 1 of the set.
     // The rows' destinations are read while the set still multiplies.
@@ -881,6 +727,165 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
         }
       }
       if (STAGE != 2) j0[0] += job.R;
+    }
+  } else {
+    if constexpr (NS == 6) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+    if (warp < DW + SETS) {
+      // ------------------------------ copies ------------------------------
+      const int set = warp - DW;
+      const uint32_t smA = smA0 + set * (g.nA * SEG * SA), smB = smB0 + (STAGE == 2 ? set * (g.nB * SEG * SB) : 0);
+      Ring ra(g.nA), rb(STAGE == 2 ? g.nB : g.tasksB);
+      int ia = 0, ib = 0, na = 0, nb = 0, n = 0;  // segments (of A, of B or tasks), scales, fills of the sets
+      bool ok = true;
+      for (int ti = blockIdx.x; ti < g.ntasks && ok; ti += gridDim.x) {
+        Job<NS, STAGE> job;
+        job.init(g, g.tasks[ti]);
+        const uint32_t bb = (uint32_t)(job.noct * NS * 512), sb = (uint32_t)(32 * job.noct);
+        if (STAGE != 2 && set == 0) {  // the task's column operand, all rounds
+          if (ib >= g.tasksB && !bwait(&emptyB[0][rb.slot], rb.phase ^ 1)) { ok = false; break; }
+          if (elect_one()) {
+            uint64_t *f = &fullB[rb.slot];
+            expect_tx(f, job.kos * bb + job.R * sb);
+            for (int r = 0; r < job.R; ++r) {
+              const int nks = min(OCT, job.kos - r * OCT);
+              const char *bp = job.bptr(r, OzRnd{});
+              bulk_load(smB + rb.slot * (g.nB * SB) + r * OCT * bb, bp, nks * bb, f);
+              bulk_load(tc::smem_u32(sB[0][(nb + r) & (OZ_SC - 1)]), bp + nks * bb, sb, f);
+            }
+          }
+          __syncwarp();
+          nb += job.R;
+          rb.next();
+          ++ib;
+        }
+        for (int m0 = 0; m0 < job.outer && ok; m0 += job.G) {
+          const int Gm = min(job.G, job.outer - m0);
+          int r = (n ^ set) & (SETS - 1);  // this set's rounds
+          n += job.R;
+          OzRnd nx = job.round(r);
+          for (; r < job.R && ok; r += SETS) {
+            const OzRnd q = nx;
+            nx = job.round(r + SETS);
+            for (int gi = 0; gi < Gm && ok; ++gi) {
+              const bool withb = STAGE == 2 && gi == 0;
+              const char *ap = job.aptr(m0 + gi, r, q), *bp = job.bptr(r, q);
+              for (int ks = 0; ks < q.nks; ks += SEG) {
+                const int nk = min(SEG, q.nks - ks);
+                if (ia >= g.nA && !bwait(&emptyA[set][ra.slot], ra.phase ^ 1)) { ok = false; break; }
+                if (withb && ib >= g.nB && !bwait(&emptyB[set][rb.slot], rb.phase ^ 1)) { ok = false; break; }
+                if (elect_one()) {
+                  uint64_t *f = &full[set][ra.slot];
+                  expect_tx(f, nk * SA + (ks == 0 ? 512u : 0u) + (withb ? nk * bb + (ks == 0 ? sb : 0u) : 0u));
+                  bulk_load(smA + ra.slot * (SEG * SA), ap + ks * SA, nk * SA, f);
+                  if (withb) bulk_load(smB + rb.slot * (SEG * SB), bp + ks * bb, nk * bb, f);
+                  if (ks == 0) {
+                    bulk_load(tc::smem_u32(sA[set][na & (OZ_SC - 1)]), ap + q.nks * SA, 512, f);
+                    if (withb) bulk_load(tc::smem_u32(sB[set][nb & (OZ_SC - 1)]), bp + q.nks * bb, sb, f);
+                  }
+                }
+                __syncwarp();
+                if (withb) {
+                  rb.next();
+                  ++ib;
+                }
+                ra.next();
+                ++ia;
+              }
+              ++na;
+              if (withb) ++nb;
+            }
+          }
+        }
+      }
+      // every copy issued has landed before the CTA may end
+      Ring rw(g.nA);
+      const int first = max(0, ia - g.nA);
+      for (int q = 0; q < ia; ++q) {
+        if (q >= first) tc::mbar_wait(&full[set][rw.slot], rw.phase, 4000000);
+        rw.next();
+      }
+      if (STAGE != 2 && set == 0) {
+        Ring rv(g.tasksB);
+        for (int q = 0; q < ib; ++q) {
+          if (q >= ib - g.tasksB) tc::mbar_wait(&fullB[rv.slot], rv.phase, 4000000);
+          rv.next();
+        }
+      }
+    } else if (warp < DW + 2 * SETS) {
+      // ------------------------------ MMAs ------------------------------
+      const int set = warp - DW - SETS;
+      const uint32_t smA = smA0 + set * (g.nA * SEG * SA), smB = smB0 + (STAGE == 2 ? set * (g.nB * SEG * SB) : 0);
+      const uint32_t ts = tm + set * SETC;
+      Ring ra(g.nA), rb(STAGE == 2 ? g.nB : g.tasksB);
+      int n = 0, fills = 0;  // fills of the sets, of this set
+      bool ok = true;
+      for (int ti = blockIdx.x; ti < g.ntasks && ok; ti += gridDim.x) {
+        Job<NS, STAGE> job;
+        job.init(g, g.tasks[ti]);
+        const int noct = __shfl_sync(0xffffffffu, job.noct, 0);
+        const uint32_t id = idesc_f16(16 * noct);
+        const uint32_t bstep = 512u * noct;  // one plane of one K step
+        if (STAGE != 2 && !bwait(&fullB[rb.slot], rb.phase)) { ok = false; break; }
+        const uint32_t bt = smB + rb.slot * (g.nB * SB);
+        for (int m0 = 0; m0 < job.outer && ok; m0 += job.G) {
+          const int Gm = min(job.G, job.outer - m0);
+          int r = (n ^ set) & (SETS - 1);
+          n += job.R;
+          OzRnd nx = job.round(r);
+          for (; r < job.R && ok; r += SETS, ++fills) {
+            const int nks = __shfl_sync(0xffffffffu, nx.nks, 0);
+            nx = job.round(r + SETS);
+            if (fills >= 1 && !bwait(&tfree[set], (fills - 1) & 1)) { ok = false; break; }
+            const Ring rr = rb;
+            for (int gi = 0; gi < Gm && ok; ++gi) {
+              if (STAGE == 2) rb = rr;
+              const uint32_t d0 = ts + (uint32_t)(gi * 16 * noct);
+              for (int ks = 0; ks < nks; ks += SEG) {
+                if (!bwait(&full[set][ra.slot], ra.phase)) { ok = false; break; }
+                tc::fence_after_sync();
+                const uint32_t a0 = smA + ra.slot * (SEG * SA);
+                const uint32_t b0 = STAGE == 2 ? smB + rb.slot * (SEG * SB) : bt + (r * OCT + ks) * NS * bstep;
+                if (elect_one()) {
+#pragma unroll
+                  for (int k = 0; k < SEG; ++k) {
+                    if (ks + k >= nks) break;
+                    const uint32_t more = ks + k > 0 ? 1u : 0u;
+#pragma unroll
+                    for (int c = 0; c <= OzCfg<NS>::CMAX; ++c)
+#pragma unroll
+                      for (int p = 0; p < NS; ++p) {
+                        const int q = c - p;
+                        if (q < 0 || q >= NS) continue;
+                        // NS = 3: (0,0) | (0,1) | (1,0) | the rest; NS = 6: one per class
+                        const int acc = NS == 6 ? c : c == 0 ? 0 : c == 1 ? 1 + p : 3;
+                        const bool fresh = NS == 6 ? p == max(0, c - NS + 1) : c < 2 || (c == 2 && p == 0);
+                        tc::mma_bf16(d0 + acc * NR, sw32_desc(a0 + k * SA + p * 4096u),
+                                     sw32_desc(b0 + (k * NS + q) * bstep), id,
+                                     fresh ? more : 1u);  // kind::f16, types from the descriptor
+                      }
+                  }
+                  tc::commit(&emptyA[set][ra.slot]);
+                  if (STAGE == 2 && gi == Gm - 1) tc::commit(&emptyB[set][rb.slot]);
+                }
+                __syncwarp();
+                ra.next();
+                if (STAGE == 2) rb.next();
+              }
+            }
+            if (!ok) break;
+            if (elect_one()) tc::commit(&done[set]);
+            __syncwarp();
+          }
+        }
+        if (STAGE != 2) {
+          if (!ok) break;
+          if (elect_one()) tc::commit(&emptyB[0][rb.slot]);
+          __syncwarp();
+          rb.next();
+        }
+      }
+      if (elect_one()) tc::commit(&last);  // arrives when every MMA issued above has completed
+      __syncwarp();
     }
   }
   __syncthreads();
