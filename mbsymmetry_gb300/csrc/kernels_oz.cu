@@ -102,14 +102,14 @@ struct Tri {
   F2 h, m, l;
 };
 
-// The value of the class sums D0 .. D6 (weights 2^(-9c)).  Carries instead of two-sums (26 steps against 44): D0 to D3
+// The value of the class sums D0 .. D3 and d4 = D4 + 2^-9 D5 + 2^-18 D6 (weights 2^(-9c)).  Carries instead of two-sums (26 steps against 44): D0 to D3
 // are exact integers, at most 64 sums of c + 1 products of digits, of which at most one is 256 in each factor, so D3 and
 // a carry of 2^15.4 stay below 2^24 and each step is exact (but for the last bits of D4 to D6, which the tensor core
 // rounds to 24 bits).
-__device__ __forceinline__ Tri tri_of(const F2 (&d)[7]) {
+__device__ __forceinline__ Tri tri_of(const F2 (&d)[4], F2 d4) {
   const F2 W = both(0x1p-9f), MG = both(1.5f * 8388608.f), NM = both(-1.5f * 8388608.f), NB = both(-512.f);
   auto carry = [&](F2 x) { return add2(fma2(x, W, MG), NM); };  // x / 512 to an integer
-  const F2 d4 = fma2(fma2(d[6], W, d[5]), W, d[4]), c4 = carry(d4);
+  const F2 c4 = carry(d4);
   const F2 d3 = add2(d[3], c4), c3 = carry(d3);
   const F2 d2 = add2(d[2], c3), c2 = carry(d2);
   const F2 d1 = add2(d[1], c2), c1 = carry(d1);
@@ -308,6 +308,25 @@ struct Ring {
   }
 };
 
+// The MMAs of one K step, classes C0 to C1 of slice products (one lane).  NS = 3: accumulators (0,0) | (0,1) |
+// (1,0) | the rest; NS = 6: one per class.
+template <int NS, int C0, int C1>
+__device__ __forceinline__ void oz_mmas(uint32_t d0, uint32_t a0, uint32_t b0, uint32_t bstep, uint32_t id,
+                                        uint32_t more) {
+  constexpr int NR = 16 * OzCfg<NS>::OCT;
+#pragma unroll
+  for (int c = C0; c <= C1; ++c)
+#pragma unroll
+    for (int p = 0; p < NS; ++p) {
+      const int q = c - p;
+      if (q < 0 || q >= NS) continue;
+      const int acc = NS == 6 ? c : c == 0 ? 0 : c == 1 ? 1 + p : 3;
+      const bool fresh = NS == 6 ? p == max(0, c - NS + 1) : c < 2 || (c == 2 && p == 0);
+      tc::mma_bf16(d0 + acc * NR, sw32_desc(a0 + p * 4096u), sw32_desc(b0 + q * bstep), id,
+                   fresh ? more : 1u);  // kind::f16, types from the descriptor
+    }
+}
+
 // Persistent warp-specialised GEMM over operand images.  Bound: the drain's
 // CUDA-core work (about 40 FP32 instructions per complex output of stages 1
 // and 2) and the L2 / HBM traffic of the images; the operands need no CUDA-core
@@ -322,6 +341,11 @@ struct Ring {
 // 1200 idle cycles cost 100).  Stage 3 of the hexagonal 8 k crystal (three
 // slices), Sigma: one K step per segment and one MMA warp 10.4 ms, segments of four
 // 6.5, an MMA warp per set 6.2.
+// Six slices have room for one set in TMEM.  There a round's MMAs go in two groups, the
+// classes 4 to 6 (16 of the 26 products of a K step) and 0 to 3, with barriers of their
+// own: the drain reads the high classes while the low ones multiply and the low ones
+// while the next round's high ones do.  In one group the multiplies and the TMEM reads
+// of a set took turns: stage 3 of Sigma, hexagonal 4 k, 5.33 ms, in two 4.45.
 // A column tile of one octet (two) fills a quarter (half) of an accumulator set, so
 // stages 2 and 3 put G = OCT / noct row tiles into one.
 //
@@ -341,7 +365,7 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint32_t tslot;
   __shared__ __align__(8) uint64_t full[SETS][OZ_RING], emptyA[SETS][OZ_RING], emptyB[SETS][OZ_RING], fullB[2],
-      done[SETS], tfree[SETS], last;
+      done[SETS], tfree[SETS], doneH, tfreeH, last;
   __shared__ __align__(16) float sA[SETS][OZ_SC][OZ_M], sB[SETS][OZ_SC][8 * OCT];
   __shared__ float gmax[2][OCT][OZ_M];
   __shared__ int abort_flag;
@@ -360,6 +384,8 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
     }
     tc::mbar_init(&fullB[0], 1);
     tc::mbar_init(&fullB[1], 1);
+    tc::mbar_init(&doneH, 1);
+    tc::mbar_init(&tfreeH, DW);
     tc::mbar_init(&last, SETS);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -495,6 +521,31 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
           const int set = n % SETS, ia = set ? i0[SETS - 1] : i0[0], jb = STAGE != 2 ? j0[0] + r : set ? j0[SETS - 1] : j0[0];
           (set ? i0[SETS - 1] : i0[0]) += Gm;
           if (STAGE == 2) ++(set ? j0[SETS - 1] : j0[0]);
+          F2 d4[NS == 6 ? 8 : 1];  // six slices: classes 4 to 6 of this octet (HO is 1)
+          if constexpr (NS == 6) {
+            if (!dead) dead = !bwait(&doneH, n & 1);
+            if (dead) continue;
+            tc::fence_after_sync();
+            if (gi[0] < Gm) {
+              const F2 W = both(0x1p-9f);
+#pragma unroll
+              for (int hf = 0; hf < 4; ++hf) {
+                if (2 * hf >= nv[0]) continue;
+                uint32_t x[3][4];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) tmem_ld4(tbase + (4 + c) * NR + 4 * hf, x[c]);
+                tmem_wait_ld();
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                  auto at = [&](int c) { return F2{__uint_as_float(x[c][2 * e]), __uint_as_float(x[c][2 * e + 1])}; };
+                  d4[2 * hf + e] = fma2(fma2(at(2), W, at(1)), W, at(0));
+                }
+              }
+            }
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&tfreeH);
+          }
           if (!dead) dead = !bwait(&done[set], (n / SETS) & 1);
           if (dead) continue;
           tc::fence_after_sync();
@@ -554,17 +605,17 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
 #pragma unroll
               for (int hf = 0; hf < 4; ++hf) {
                 if (2 * hf >= nv[q]) continue;
-                uint32_t x[7][4];
+                uint32_t x[4][4];
 #pragma unroll
-                for (int c = 0; c < 7; ++c) tmem_ld4(base + c * NR + 4 * hf, x[c]);
+                for (int c = 0; c < 4; ++c) tmem_ld4(base + c * NR + 4 * hf, x[c]);
                 tmem_wait_ld();
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                   const int i = 2 * hf + e;
-                  F2 d[7];
+                  F2 d[4];
 #pragma unroll
-                  for (int c = 0; c < 7; ++c) d[c] = {__uint_as_float(x[c][2 * e]), __uint_as_float(x[c][2 * e + 1])};
-                  Tri t = tri_of(d);
+                  for (int c = 0; c < 4; ++c) d[c] = {__uint_as_float(x[c][2 * e]), __uint_as_float(x[c][2 * e + 1])};
+                  Tri t = tri_of(d, d4[i]);
                   const F2 sc = both(oz_pow2c(eb[i] - em) * fn);
                   t = {mul2(t.h, sc), mul2(t.m, sc), mul2(t.l, sc)};
                   if (!first) {
@@ -835,41 +886,62 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
           for (; r < job.R && ok; r += SETS, ++fills) {
             const int nks = __shfl_sync(0xffffffffu, nx.nks, 0);
             nx = job.round(r + SETS);
-            if (fills >= 1 && !bwait(&tfree[set], (fills - 1) & 1)) { ok = false; break; }
             const Ring rr = rb;
-            for (int gi = 0; gi < Gm && ok; ++gi) {
-              if (STAGE == 2) rb = rr;
-              const uint32_t d0 = ts + (uint32_t)(gi * 16 * noct);
-              for (int ks = 0; ks < nks; ks += SEG) {
-                if (!bwait(&full[set][ra.slot], ra.phase)) { ok = false; break; }
-                tc::fence_after_sync();
-                const uint32_t a0 = smA + ra.slot * (SEG * SA);
-                const uint32_t b0 = STAGE == 2 ? smB + rb.slot * (SEG * SB) : bt + (r * OCT + ks) * NS * bstep;
-                if (elect_one()) {
-#pragma unroll
-                  for (int k = 0; k < SEG; ++k) {
-                    if (ks + k >= nks) break;
-                    const uint32_t more = ks + k > 0 ? 1u : 0u;
-#pragma unroll
-                    for (int c = 0; c <= OzCfg<NS>::CMAX; ++c)
-#pragma unroll
-                      for (int p = 0; p < NS; ++p) {
-                        const int q = c - p;
-                        if (q < 0 || q >= NS) continue;
-                        // NS = 3: (0,0) | (0,1) | (1,0) | the rest; NS = 6: one per class
-                        const int acc = NS == 6 ? c : c == 0 ? 0 : c == 1 ? 1 + p : 3;
-                        const bool fresh = NS == 6 ? p == max(0, c - NS + 1) : c < 2 || (c == 2 && p == 0);
-                        tc::mma_bf16(d0 + acc * NR, sw32_desc(a0 + k * SA + p * 4096u),
-                                     sw32_desc(b0 + (k * NS + q) * bstep), id,
-                                     fresh ? more : 1u);  // kind::f16, types from the descriptor
-                      }
-                  }
-                  tc::commit(&emptyA[set][ra.slot]);
-                  if (STAGE == 2 && gi == Gm - 1) tc::commit(&emptyB[set][rb.slot]);
+            if constexpr (NS == 6) {  // per row tile the high classes, then the low ones; its K steps stay in the ring
+              if (fills >= 1 && !bwait(&tfreeH, (fills - 1) & 1)) { ok = false; break; }
+              for (int gi = 0; gi < Gm && ok; ++gi) {
+                if (STAGE == 2) rb = rr;
+                const uint32_t d0 = ts + (uint32_t)(gi * 16 * noct);
+                const Ring a1 = ra, b1 = rb;
+                auto bat = [&](int ks) { return STAGE == 2 ? smB + rb.slot * SB : bt + (r * OCT + ks) * NS * bstep; };
+                for (int ks = 0; ks < nks; ++ks) {
+                  if (!bwait(&full[set][ra.slot], ra.phase)) { ok = false; break; }
+                  tc::fence_after_sync();
+                  if (elect_one()) oz_mmas<NS, 4, OzCfg<NS>::CMAX>(d0, smA + ra.slot * SA, bat(ks), bstep, id, ks > 0);
+                  __syncwarp();
+                  ra.next();
+                  if (STAGE == 2) rb.next();
                 }
+                if (!ok) break;
+                if (gi == Gm - 1 && elect_one()) tc::commit(&doneH);
                 __syncwarp();
-                ra.next();
-                if (STAGE == 2) rb.next();
+                if (gi == 0 && fills >= 1 && !bwait(&tfree[set], (fills - 1) & 1)) { ok = false; break; }
+                ra = a1;
+                rb = b1;
+                for (int ks = 0; ks < nks; ++ks) {
+                  if (elect_one()) {
+                    oz_mmas<NS, 0, 3>(d0, smA + ra.slot * SA, bat(ks), bstep, id, ks > 0);
+                    tc::commit(&emptyA[set][ra.slot]);
+                    if (STAGE == 2 && gi == Gm - 1) tc::commit(&emptyB[set][rb.slot]);
+                  }
+                  __syncwarp();
+                  ra.next();
+                  if (STAGE == 2) rb.next();
+                }
+              }
+            } else {
+              if (fills >= 1 && !bwait(&tfree[set], (fills - 1) & 1)) { ok = false; break; }
+              for (int gi = 0; gi < Gm && ok; ++gi) {
+                if (STAGE == 2) rb = rr;
+                const uint32_t d0 = ts + (uint32_t)(gi * 16 * noct);
+                for (int ks = 0; ks < nks; ks += SEG) {
+                  if (!bwait(&full[set][ra.slot], ra.phase)) { ok = false; break; }
+                  tc::fence_after_sync();
+                  const uint32_t a0 = smA + ra.slot * (SEG * SA);
+                  const uint32_t b0 = STAGE == 2 ? smB + rb.slot * (SEG * SB) : bt + (r * OCT + ks) * NS * bstep;
+                  if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < SEG; ++k) {
+                      if (ks + k >= nks) break;
+                      oz_mmas<NS, 0, OzCfg<NS>::CMAX>(d0, a0 + k * SA, b0 + k * NS * bstep, bstep, id, ks + k > 0 ? 1u : 0u);
+                    }
+                    tc::commit(&emptyA[set][ra.slot]);
+                    if (STAGE == 2 && gi == Gm - 1) tc::commit(&emptyB[set][rb.slot]);
+                  }
+                  __syncwarp();
+                  ra.next();
+                  if (STAGE == 2) rb.next();
+                }
               }
             }
             if (!ok) break;
@@ -1050,10 +1122,10 @@ void oz_rings(int ns, int stage, int max_kos, OzArgs *a) {
   } else {
     a->nB = max_kos;
     auto ring = [&](int tasks) { return std::min(OZ_RING, (OZ_SMEM - tasks * a->nB * stepB) / (sets * slotA)); };
-    a->tasksB = ring(2) >= 3 ? 2 : 1;
+    a->tasksB = ring(2) >= (ns == 6 ? OZ_OCT : 3) ? 2 : 1;  // six slices hold a round of A
     a->nA = ring(a->tasksB);
   }
-  GWGB_REQUIRE(a->nA >= 2, GWGB_E_UNSUPPORTED, "sliced GEMM rings too small");
+  GWGB_REQUIRE(a->nA >= (ns == 6 ? OZ_OCT : 2), GWGB_E_UNSUPPORTED, "sliced GEMM rings too small");
 }
 
 template <int NS>
