@@ -137,24 +137,32 @@ __device__ __forceinline__ void tri_add(Tri &a, const Tri &b) {
   two_sum(h, m, a.h, a.m);
 }
 
-// The six digits of h + m + l (f = 2^(8-E)).
-__device__ __forceinline__ void tri_digits(const Tri &x, F2 f, F2 (&s)[6]) {
-  const F2 MG = both(1.5f * 8388608.f), NM = both(-1.5f * 8388608.f);  // 1.5 2^23: rounds to integers
-  const F2 B = both(512.f);
-  s[0] = add2(fma2(x.h, f, MG), NM);
-  F2 t, te;
-  two_sum(sub2(mul2(x.h, f), s[0]), mul2(x.m, f), t, te);  // products and difference are exact
-  te = fma2(x.l, f, te);
-  s[1] = add2(fma2(t, B, MG), NM);
-  t = sub2(mul2(t, B), s[1]);
-  s[2] = add2(fma2(t, B, MG), NM);
-  t = sub2(mul2(t, B), s[2]);
-  two_sum(t, mul2(te, both(262144.f)), t, te);
-  s[3] = add2(fma2(t, B, MG), NM);
-  t = sub2(mul2(t, B), s[3]);
-  s[4] = add2(fma2(t, B, MG), NM);
-  t = sub2(mul2(t, B), s[4]);
-  s[5] = fma2(te, both(134217728.f), mul2(t, B));  // te 2^27
+// a + b for a zero or |a| > |b|: s the rounded sum, b what it leaves.
+__device__ __forceinline__ F2 fast_two_sum(F2 a, F2 &b) {
+  const F2 s = add2(a, b);
+  b = sub2(b, sub2(s, a));
+  return s;
+}
+
+// The six digits of h + m + l (nf = -2^(8-E)).  Of the negative: rounding by 1.5 2^23 - (1.5 2^23 + t) gives the digit of
+// the positive number and, added, the remainder, three steps a digit.  Remainders are multiples of an ulp of the
+// number they are left of and so zero or larger than the part that follows.
+__device__ __forceinline__ void tri_digits(const Tri &x, F2 nf, F2 (&s)[6]) {
+  const F2 MG = both(1.5f * 8388608.f), B = both(512.f);
+  auto digit = [&](F2 a, F2 f, F2 &d) {  // a f = -d + what is returned
+    d = sub2(MG, fma2(a, f, MG));
+    return fma2(a, f, d);
+  };
+  F2 t = digit(x.h, nf, s[0]), te = mul2(x.m, nf);
+  t = fast_two_sum(t, te);
+  te = fma2(x.l, nf, te);
+  t = digit(t, B, s[1]);
+  t = digit(t, B, s[2]);
+  te = mul2(te, both(262144.f));
+  t = fast_two_sum(t, te);
+  t = digit(t, B, s[3]);
+  t = digit(t, B, s[4]);
+  s[5] = fma2(te, both(-134217728.f), mul2(t, both(-512.f)));  // te 2^27
 }
 
 // 2^e for any e, 0 below the FP32 range.
@@ -421,9 +429,11 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
   // rings: nA segments of A per set, then nB segments of B per set (stage 3) or tasksB tasks' B of nB K steps
   const uint32_t smA0 = tc::smem_u32(smem), smB0 = smA0 + (uint32_t)(SETS * g.nA) * SEG * SA;
 
-  // six slices: 16 x 32 x 112 + 4 x 32 x 32 registers are the launch's 640 x 96
+  // six slices: registers of the drain and other warps, 512 x 112 + 128 x 32 and 512 x 104 + 128 x 56 of the launch's
+  // 640 x 96 (which of the two spills less; 150 bytes spilled in stage 2 took Sigma's, hexagonal 4 k, from 4.5 to 7.0 ms)
+  constexpr int DREG = STAGE == 1 ? 104 : 112, OREG = STAGE == 1 ? 56 : 32;
   if (warp < DW) {
-    if constexpr (NS == 6) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+    if constexpr (NS == 6) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(DREG));
     // ------------------------------ drain ------------------------------
     // warp w: TMEM lanes (rows) 32 (w & 3) .. + 31, octets HO (w >> 2) .. + HO - 1 of the set.
     // The rows' destinations are read while the set still multiplies.
@@ -488,8 +498,6 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
 #pragma unroll
         for (int q = 0; q < HO; ++q) {
           nv[q] = d.nz - 8 * ((tk.i >> 16) * OCT + oct[q]);
-          rw[q].pk = OZ_NOROW;
-          if (gi[q] < min(job.G, job.outer)) rw[q] = rows[gi[q] * OZ_M];
         }
       } else {
 #pragma unroll
@@ -500,12 +508,11 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
       }
       for (int m0 = 0; m0 < job.outer; m0 += job.G, ++tile) {
         const int Gm = min(job.G, job.outer - m0);
-        OzRow rw1[HO];
-        if constexpr (STAGE == 1) {
+        if constexpr (STAGE == 1) {  // used after the wait for the accumulators
 #pragma unroll
           for (int q = 0; q < HO; ++q) {
-            rw1[q].pk = OZ_NOROW;
-            if (m0 + job.G + gi[q] < job.outer) rw1[q] = rows[(m0 + job.G + gi[q]) * OZ_M];
+            rw[q].pk = OZ_NOROW;
+            if (gi[q] < Gm) rw[q] = rows[(m0 + gi[q]) * OZ_M];
           }
         }
         // this thread's octets: value H + L (NS = 3), (H + M + L) 2^ex (NS = 6)
@@ -740,8 +747,8 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
             } else {
               scale = __int_as_float(e2 - 8);
             }
-            // NS = 6: 2^(8 - e2 + ex); e2 - ex is at least the exponent of an FP32 value
-            const F2 f = both(NS == 3 ? oz_pow2(15 - e2) : oz_pow2c(8 - e2 + ex[q])), m1 = both(oz_m1(nksb));
+            // NS = 6: -2^(8 - e2 + ex); e2 - ex is at least the exponent of an FP32 value
+            const F2 f = both(NS == 3 ? oz_pow2(15 - e2) : -oz_pow2c(8 - e2 + ex[q])), m1 = both(oz_m1(nksb));
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               if (e == 4 && nv[q] <= 4) {  // the second half is padding
@@ -772,15 +779,12 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
             Lr -= nL;
             ++tau;
           }
-        } else if constexpr (STAGE == 1) {
-#pragma unroll
-          for (int q = 0; q < HO; ++q) rw[q] = rw1[q];
         }
       }
       if (STAGE != 2) j0[0] += job.R;
     }
   } else {
-    if constexpr (NS == 6) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+    if constexpr (NS == 6) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(OREG));
     if (warp < DW + SETS) {
       // ------------------------------ copies ------------------------------
       const int set = warp - DW;
