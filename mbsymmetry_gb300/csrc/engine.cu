@@ -388,8 +388,8 @@ class Engine {
     }
     build_oz();
     if (OzSet *o = oz_set(); o && alloc_oz(*o) && !o->ready) {
-      o->plan[0].build_static(V_.p, st_);
-      o->plan[1].build_static(Vt_.p, st_);
+      if (!o->off[0]) o->plan[0].build_static(V_.p, st_);
+      if (!o->off[1]) o->plan[1].build_static(Vt_.p, st_);
       o->ready = true;
       built = true;
     }
@@ -420,7 +420,7 @@ class Engine {
   }
   struct OzSet {
     OzPlan plan[2];
-    bool built = false, alloc = false, ready = false, off = false;
+    bool built = false, alloc = false, ready = false, off[2] = {false, false};
   };
   OzSet oz_[2];
   OzShared oz_buf_;
@@ -428,7 +428,11 @@ class Engine {
   bool alloc_oz(OzSet &set);
   OzSet *oz_set() {  // the set that runs the contractions, if one does
     OzSet *o = prec_ == GWGB_PREC_OZAKI ? &oz_[0] : prec_ == GWGB_PREC_FP64 ? &oz_[1] : nullptr;
-    return o && o->built && !o->off ? o : nullptr;
+    return o && o->built && !(o->off[0] && o->off[1]) ? o : nullptr;
+  }
+  OzSet *oz_set(int which) {  // that runs one contraction (0: P0, 1: Sigma)
+    OzSet *o = oz_set();
+    return o && !o->off[which] ? o : nullptr;
   }
   // per-launch profile (gwgb_set_launch_timing): records [0, n_p0) P0, then Sigma
   bool lt_on_ = false, lt_ran_p0_ = false, lt_ran_sig_ = false;
@@ -1471,8 +1475,8 @@ bool Engine::alloc_oz(OzSet &set) {
     if (m > (int64_t)buf.n) buf.alloc((size_t)m);
   };
   try {
-    set.plan[0].alloc_images();
-    set.plan[1].alloc_images();
+    for (int k = 0; k < 2; ++k)
+      if (!set.off[k]) set.plan[k].alloc_images();
     grow(oz_buf_.A1, p.bytes_A1(), s.bytes_A1());
     grow(oz_buf_.B2, p.bytes_B2(), s.bytes_B2());
     grow(oz_buf_.X1, p.bytes_X1(), s.bytes_X1());
@@ -1481,7 +1485,7 @@ bool Engine::alloc_oz(OzSet &set) {
   } catch (const Error &e) {
     if (&set != &oz_[1] || e.code != GWGB_E_NOMEM) throw;
     cudaGetLastError();
-    set.off = true;
+    set.off[0] = set.off[1] = true;
     set.plan[0].free();
     set.plan[1].free();
     oz_buf_.free();
@@ -1514,7 +1518,7 @@ void Engine::build_oz() {
   const bool f64 = prec_ == GWGB_PREC_FP64;
   OzSet &set = oz_[f64 ? 1 : 0];
   if (set.built) {
-    if (lt_set_ != &set && !set.off) lt_build();
+    if (lt_set_ != &set && oz_set()) lt_build();
     return;
   }
   const int NS = f64 ? 6 : 3;
@@ -1576,6 +1580,24 @@ void Engine::build_oz() {
   set.plan[1].build(NS, cs, own, nts, 3, budget, persist / 2, nsm_, (int64_t)Vt_.n, (int64_t)Gall_.n, (int64_t)Pall_.n,
                     (int64_t)nts * ns * l.flat_ao);
   p0_built.get();
+  if (f64) {
+    // Six slices against the FMA kernels, one contraction at a time: the MMAs (padded to octets of columns and 128 rows)
+    // run at 190 TFLOP/s and more including their drains, the launches around them take about 0.05 ms; the FMA
+    // kernels run at 1.2 TFLOP/s.  s+p (AO blocks 1-4): P0 0.45 ms against 0.40, Sigma 0.44 against 0.70; s+p+d
+    // (1-8): 17 against 94; hexagonal 4 k (AO 7-30): 18.5 against 222; blocks of a single orbital stay on the FMA
+    // kernels.  (GWGB_FP64_SLICES=1 / 0 in the environment forces one or the other)
+    const char *force = std::getenv("GWGB_FP64_SLICES");
+    for (int k = 0; k < 2; ++k) {
+      double ops = 0;
+      for (const OzLaunch &x : set.plan[k].launches()) ops += x.ops;
+      set.off[k] = force ? force[0] == '0' : ops / 1.9e14 + 5e-5 > (k ? sig_flops_ : p0_flops_) / 1.2e12;
+      if (set.off[k]) set.plan[k].free();
+    }
+    if (set.off[0] && set.off[1]) {
+      set.built = true;
+      return;
+    }
+  }
   {  // the buffers (shared with the other set, if it is built) must fit the free memory
     const OzPlan &p = set.plan[0], &s = set.plan[1];
     auto grow = [](int64_t a, int64_t b, size_t have) {
@@ -1595,20 +1617,10 @@ void Engine::build_oz() {
       msg += std::string(" ") + x.first + " " + std::to_string(x.second >> 20) + " MB";
     }
     GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    // Six slices against the FMA kernels: the MMAs (padded to octets of columns and 128 rows) run at 160 to
-    // 400 TFLOP/s including their drains, the launches around them take about 0.1 ms; the FMA kernels run at
-    // 1.2 TFLOP/s.  s+p (AO blocks 1-4): 1.03 ms against 1.04; s+p+d (1-8): 21 against 94; hexagonal 4 k
-    // (AO 7-30): 28 against 222; blocks of a single orbital stay on the FMA kernels.
-    double ops = 0;
-    for (const OzPlan *q : {&p, &s})
-      for (const OzLaunch &x : q->launches()) ops += x.ops;
-    // (GWGB_FP64_SLICES=1 / 0 in the environment forces one or the other)
-    const char *force = std::getenv("GWGB_FP64_SLICES");
-    const bool slow = f64 && force ? force[0] == '0' : f64 && ops / 1.8e14 + 1e-4 > (p0_flops_ + sig_flops_) / 1.2e12;
-    const bool fits = !slow && tot + (256ll << 20) + (V_.p ? 0 : 16 * l.flat_V) <= (int64_t)free_b;
+    const bool fits = tot + (256ll << 20) + (V_.p ? 0 : 16 * l.flat_V) <= (int64_t)free_b;
     set.built = true;
     if (f64 && !fits) {  // the FMA kernels, which need no images
-      set.off = true;
+      set.off[0] = set.off[1] = true;
       set.plan[0].free();
       set.plan[1].free();
       return;
@@ -1617,8 +1629,8 @@ void Engine::build_oz() {
     GWGB_REQUIRE(fits, GWGB_E_UNSUPPORTED,
                  "sliced-precision buffers need " + std::to_string(tot >> 20) + " MB (" + msg + " ), " +
                      std::to_string(free_b >> 20) + " MB free");
-    set.plan[0].upload(st_);
-    set.plan[1].upload(st_);
+    for (int k = 0; k < 2; ++k)
+      if (!set.off[k]) set.plan[k].upload(st_);
   }
   set.ready = false;
   lt_build();
@@ -1725,7 +1737,7 @@ void Engine::k_rotate_G() {
 
 void Engine::k_p0(int mirror) {
   const double pref = -1.0 / l_.nk * (ns_ == 1 ? 2.0 : 1.0);  // cugw_qkpt_block.cu:210, cugw_solver_block.cpp:303
-  if (OzSet *o = oz_set()) {
+  if (OzSet *o = oz_set(0)) {
     GWGB_REQUIRE(o->ready, GWGB_E_STATE, "sliced operands not prepared");
     GWGB_CUDA(cudaMemsetAsync(Pall_.p, 0, Pall_.n * sizeof(double2), st_));  // blocks without contributions
     oz_run(0, pref);
@@ -1757,7 +1769,7 @@ void Engine::k_pq(bool mirror_first) {
 
 
 void Engine::k_sigma() {
-  if (OzSet *o = oz_set()) {
+  if (OzSet *o = oz_set(1)) {
     GWGB_REQUIRE(o->ready, GWGB_E_STATE, "sliced operands not prepared");
     GWGB_CUDA(cudaMemsetAsync(Sig_.p, 0, Sig_.n * sizeof(double2), st_));  // blocks without contributions
     oz_run(1, -1.0 / l_.nk);
@@ -1849,11 +1861,9 @@ void Engine::finish_stats(bool with_dyson, bool with_gw, bool with_pq, bool with
                           : (p0_tiles_.n ? 1 : 0) + (p0_red_.n ? 1 : 0);
     const int64_t sg = tc ? sgt
                           : (sig_tiles_.n ? 1 : 0) + (sig_red_.n ? 1 : 0);
-    if (OzSet *o = oz_set()) {
-      const int64_t a = (int64_t)o->plan[0].launches().size(), b = (int64_t)o->plan[1].launches().size();
-      launches += (rotG_.n ? 1 : 0) + a + 1 + 3 + b;  // 1: the tau mirror of P0
-    } else
-    launches += (rotG_.n ? 1 : 0) + p0 + 3 + sg;
+    OzSet *o0 = oz_set(0), *o1 = oz_set(1);  // (+ 1: the tau mirror of P0)
+    launches += (rotG_.n ? 1 : 0) + (o0 ? (int64_t)o0->plan[0].launches().size() + 1 : p0) + 3 +
+                (o1 ? (int64_t)o1->plan[1].launches().size() : sg);
   }
   if (with_dyson) launches += 3 + (has_tct_ ? 1 : 0);
   s.kernel_launches = launches;

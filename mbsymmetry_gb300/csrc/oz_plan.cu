@@ -669,6 +669,7 @@ void OzPlan::free() {
   host_ = std::vector<char>();
   launches_.clear();
   static_.clear();
+  vimg_ = a1_ = b2_ = x1_ = x2_ = part_ = 0;
 }
 
 }  // namespace gwgb
