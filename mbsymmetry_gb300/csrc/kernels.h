@@ -8,15 +8,14 @@ namespace gwgb {
 // Largest irrep block (AO or aux) the FP64 kernels accept.
 constexpr int MAX_BLOCK = 64;
 
-// Block inverses: one warp per block; as many warps per CTA as fit in ~48 KB
-// of shared memory (2 n^2 complex + 3 n ints per warp), 1 to 8.
-__host__ __device__ constexpr int inv_bytes_per_warp(int nmax) { return 2 * nmax * nmax * 16 + 3 * nmax * 4; }
-__host__ __device__ constexpr int inv_warps_per_block(int nmax) {
-  return (48 * 1024) / inv_bytes_per_warp(nmax) < 1 ? 1
-         : ((48 * 1024) / inv_bytes_per_warp(nmax) > 8 ? 8 : (48 * 1024) / inv_bytes_per_warp(nmax));
+// Block inverses: shared memory of one matrix (A, in mode 0 P, three rows, 2 n ints); up to n = 16 one warp per
+// block and as many warps per CTA as fit in ~48 KB, 1 to 8.
+__host__ __device__ constexpr int inv_bytes(int nmax, int mode) {
+  return ((mode == 0 ? 2 : 1) * nmax * nmax + 3 * nmax) * 16 + 2 * nmax * 4;
 }
-__host__ __device__ constexpr int inv_smem_bytes(int nmax) {
-  return inv_warps_per_block(nmax) * inv_bytes_per_warp(nmax);
+__host__ __device__ constexpr int inv_warps_per_block(int nmax, int mode) {
+  return (48 * 1024) / inv_bytes(nmax, mode) < 1 ? 1
+         : ((48 * 1024) / inv_bytes(nmax, mode) > 8 ? 8 : (48 * 1024) / inv_bytes(nmax, mode));
 }
 __host__ __device__ constexpr int rotate_smem_bytes(int nmax) { return 3 * nmax * nmax * 16; }
 

@@ -373,281 +373,244 @@ __global__ void __launch_bounds__(256) transform_kernel(const TSlab *__restrict_
 }
 
 // ---------------------------------------------------------------------------
-// Batched block inverses by Gauss-Jordan elimination with full pivoting (the
-// pivoting strategy of Eigen::FullPivLU, sc_type_block.cpp:55), one warp per
-// matrix.  An exactly singular block sets *bad and leaves its output
-// untouched.
+// Batched block inverses.  An exactly singular block sets *bad and leaves its
+// output untouched.
 //   mode 0 (W~ solve, cugw_solver_block.cpp:412-424):
 //     A = I - (P + P^H)/2 ; A^-1 ; R = (A^-1 + A^-H)/2 ; P <- R P
 //   mode 1 (Dyson, sc_type_block.cpp:48-57):
 //     A = (i w_n + mu) S - F - Sigma(i w_n) ; G = A^-1   (in place)
+// Bound: the FP64 pipe (2 FMA per cycle and SM; a DFMA of one warp takes 64 cycles
+// of its scheduler), so what counts is the number of FP64 instructions:
+//  - the A of mode 0 is Hermitian and, at bosonic frequencies, positive definite: symmetric sweeps over its
+//    lower triangle, no pivot search (2 n^3 FMA against 6 n^3 and the search).  A pivot that is not clearly
+//    positive sends the block to the general elimination;
+//  - the general one is Gauss-Jordan with full pivoting (the strategy of Eigen::FullPivLU,
+//    sc_type_block.cpp:55), 4 FMA per element and step; the pivot is the largest
+//    component by its upper 32 bits, found in integers while the elimination writes the elements.
+// One warp per matrix up to n = 16, one CTA above (NT threads either way), elements spread over the threads.
+// The W~ solve of the 27 k s+p+d+4 crystal (aux 2-40): 3.36 ms with the elimination for all, 1.40; hexagonal 8 k:
+// 3.15, 1.14; Dyson, hexagonal 8 k (AO 2-30): 0.61, 0.18; s+p (n up to 12): W~ and Dyson 0.17, 0.07.
 // ---------------------------------------------------------------------------
-// nm = largest block of the launch; every warp of the CTA owns 2*nm^2 complex
-// and 3*nm ints of shared memory.
-__global__ void inverse_kernel(const InvTask *__restrict__ tasks, int ntasks, double2 *__restrict__ W,
-                               const double2 *__restrict__ S, const double2 *__restrict__ F,
-                               const int64_t *__restrict__ wsample, double beta, double mu, int mode,
-                               int *__restrict__ bad, int nm, const double *__restrict__ mu_ptr,
-                               double2 *__restrict__ Wout, const int *__restrict__ skip) {
-  if (skip && *skip) return;  // the mu search has converged (uniform over the grid)
-  const int WPB = blockDim.x >> 5;
-  extern __shared__ double2 smem_inv[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double2 *A = smem_inv + (size_t)warp * 2 * nm * nm;
-  double2 *B = A + nm * nm;
-  int *ipiv = reinterpret_cast<int *>(smem_inv + (size_t)WPB * 2 * nm * nm) + warp * 3 * nm;
-  int *indxr = ipiv + nm;
-  int *indxc = indxr + nm;
-  const int ti = blockIdx.x * WPB + warp;
-  if (ti >= ntasks) return;
-  const InvTask tk = tasks[ti];
-  const int n = tk.n;
-  double2 *g = W + tk.a;
-  if (mode == 0) {
-    for (int e = lane; e < n * n; e += 32) B[e] = g[e];
+constexpr int INV_CTA_THREADS = 128;
+
+template <int NT> __device__ __forceinline__ void inv_sync() {
+  if constexpr (NT == 32)
     __syncwarp();
-    for (int e = lane; e < n * n; e += 32) {
+  else
+    __syncthreads();
+}
+
+// Size of a component pair for the pivot choice: upper word of the larger one; 0 for NaN and for
+// what underflows when squared.
+__device__ __forceinline__ unsigned inv_key(double2 v) {
+  const unsigned k = max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu);
+  return k > 0x7ff00000u || k < (unsigned)(1023 - 537) << 20 ? 0u : k;
+}
+
+// Inverse of the n x n matrix A of NT threads, in place, columns permuted: column m of A is column perm[m] of the
+// inverse.  rowk, old, fcol: n complex each; used, perm: n ints; red: NT / 32 pairs.  False if singular.
+template <int NT>
+__device__ __forceinline__ bool gauss_jordan(double2 *A, int n, double2 *rowk, double2 *old, double2 *fcol, int *used,
+                                             int *perm, unsigned (*red)[2], int tid) {
+  const int lane = tid & 31, warp = tid >> 5, nn = n * n;
+  for (int j = tid; j < n; j += NT) {
+    used[j] = 0;
+    perm[j] = j;
+  }
+  unsigned best = 0u;
+  int bidx = 0x7fffffff;
+  for (int e = tid; e < nn; e += NT) {
+    const unsigned k = inv_key(A[e]);
+    if (k > best) { best = k; bidx = e; }
+  }
+  for (int it = 0; it < n; ++it) {
+    {  // largest key, first in row-major order
+      const unsigned wb = __reduce_max_sync(0xffffffffu, best);
+      const unsigned wi = __reduce_min_sync(0xffffffffu, best == wb ? (unsigned)bidx : 0x7fffffffu);
+      best = wb;
+      bidx = (int)wi;
+    }
+    if constexpr (NT > 32) {
+      if (lane == 0) {
+        red[warp][0] = best;
+        red[warp][1] = (unsigned)bidx;
+      }
+    }
+    inv_sync<NT>();
+    if constexpr (NT > 32) {
+      best = red[0][0];
+      bidx = (int)red[0][1];
+#pragma unroll
+      for (int w = 1; w < NT / 32; ++w)
+        if (red[w][0] > best || (red[w][0] == best && (int)red[w][1] < bidx)) {
+          best = red[w][0];
+          bidx = (int)red[w][1];
+        }
+    }
+    if (best == 0u) return false;  // uniform
+    const int irow = bidx / n, icol = bidx - irow * n;
+    // scaled pivot row, the row it trades places with, the pivot's column after that
+    for (int l = tid; l < n; l += NT) {
+      const double2 pv = A[irow * n + icol];
+      const double den = 1.0 / (pv.x * pv.x + pv.y * pv.y);
+      const double2 pinv = make_double2(pv.x * den, -pv.y * den);
+      rowk[l] = l == icol ? pinv : cmul(A[irow * n + l], pinv);
+      old[l] = A[icol * n + l];
+      fcol[l] = A[(l == irow ? icol : l) * n + icol];
+    }
+    if (tid == 0) {
+      used[icol] = 1;
+      const int t = perm[irow];
+      perm[irow] = perm[icol];
+      perm[icol] = t;
+    }
+    inv_sync<NT>();
+    best = 0u;
+    bidx = 0x7fffffff;
+    for (int e = tid; e < nn; e += NT) {
+      const int i = e / n, j = e - i * n;
+      const double2 r = rowk[j];
+      double2 a = r;
+      if (i != icol) {
+        const double2 f = fcol[i];
+        a = j == icol ? make_double2(0.0, 0.0) : i == irow ? old[j] : A[e];
+        a.x = fma(-r.x, f.x, fma(r.y, f.y, a.x));
+        a.y = fma(-r.x, f.y, fma(-r.y, f.x, a.y));
+        if (!used[i] && !used[j]) {
+          const unsigned k = inv_key(a);
+          if (k > best) { best = k; bidx = e; }
+        }
+      }
+      A[e] = a;
+    }
+  }
+  inv_sync<NT>();
+  return true;
+}
+
+// -A^-1 of a positive definite A (lower triangle, in place) by symmetric sweeps.  c, w: n complex each.  False (A
+// overwritten) where a pivot is not clearly positive: below 2^-40 of its diagonal element 1 - Re P.
+template <int NT>
+__device__ __forceinline__ bool sweep_inverse(double2 *A, const double2 *P, int n, double2 *c, double2 *w, int tid) {
+  const int half = (n + 1) / 2, ne = half * (n + 1);
+  for (int k = 0; k < n; ++k) {
+    const double p = A[k * n + k].x;
+    const double p0 = 1.0 - P[k * n + k].x;
+    if (!(p > 0x1p-40 * p0) || !(p0 > 0.0) || isinf(p)) return false;  // uniform
+    for (int i = tid; i < n; i += NT) {  // column k, and its conjugate over the pivot
+      const double d = 1.0 / p;
+      const double2 v = i >= k ? A[i * n + k] : cconj(A[k * n + i]);
+      c[i] = v;
+      w[i] = i == k ? make_double2(-d, 0.0) : make_double2(v.x * d, -v.y * d);
+    }
+    inv_sync<NT>();
+    // rows q and n - 1 - q of the triangle together have n + 1 elements
+    for (int e = tid; e < ne; e += NT) {
+      const int q = e / (n + 1), r = e - q * (n + 1), lng = n - q;
+      const int i = r < lng ? n - 1 - q : q, j = r < lng ? r : r - lng;
+      if (r >= lng && n - 1 - q == q) continue;
+      double2 a;
+      if (i == k) {
+        a = w[j];
+      } else if (j == k) {
+        a = cconj(w[i]);
+      } else {
+        const double2 x = c[i], y = w[j];
+        a = A[i * n + j];
+        a.x = fma(-x.x, y.x, fma(x.y, y.y, a.x));
+        a.y = fma(-x.x, y.y, fma(-x.y, y.x, a.y));
+      }
+      A[i * n + j] = a;
+    }
+    inv_sync<NT>();
+  }
+  return true;
+}
+
+// nm = largest block of the launch.  Shared, per matrix: A [nm^2] | P [nm^2] (mode 0) | three rows [nm] (complex) |
+// 2 nm ints.
+template <int NT>
+__global__ void __launch_bounds__(NT == 32 ? 256 : NT) inverse_kernel(
+    const InvTask *__restrict__ tasks, int ntasks, double2 *__restrict__ W, const double2 *__restrict__ S,
+    const double2 *__restrict__ F, const int64_t *__restrict__ wsample, double beta, double mu, int mode,
+    int *__restrict__ bad, int nm, const double *__restrict__ mu_ptr, double2 *__restrict__ Wout,
+    const int *__restrict__ skip) {
+  if (skip && *skip) return;  // the mu search has converged (uniform over the grid)
+  extern __shared__ double2 smem_inv[];
+  __shared__ unsigned red[NT / 32][2];
+  const int per = NT == 32 ? blockDim.x / 32 : 1, mat = NT == 32 ? threadIdx.x >> 5 : 0, tid = threadIdx.x % NT;
+  const int ti = blockIdx.x * per + mat;
+  if (ti >= ntasks) return;
+  const int na = (mode == 0 ? 2 : 1) * nm * nm + 3 * nm;
+  double2 *A = smem_inv + (size_t)mat * na;
+  double2 *B = A + (mode == 0 ? nm * nm : 0);
+  double2 *rowk = A + na - 3 * nm, *old = rowk + nm, *fcol = old + nm;
+  int *used = reinterpret_cast<int *>(smem_inv + (size_t)per * na) + mat * 2 * nm, *perm = used + nm;
+  const InvTask tk = tasks[ti];
+  const int n = tk.n, nn = n * n;
+  double2 *g = W + tk.a;
+  auto hermitian = [&]() {  // A = I - (P + P^H)/2
+    for (int e = tid; e < nn; e += NT) {
       const int i = e / n, j = e - i * n;
       const double2 pij = B[e], pji = B[j * n + i];
       A[e] = make_double2((i == j ? 1.0 : 0.0) - 0.5 * (pij.x + pji.x), -0.5 * (pij.y - pji.y));
     }
-  } else {
+    inv_sync<NT>();
+  };
+  if (mode == 1) {
     if (mu_ptr) mu = *mu_ptr;
     const double wn = (2.0 * (double)wsample[tk.w] + 1.0) * 3.14159265358979323846 / beta;
-    for (int e = lane; e < n * n; e += 32) {
+    for (int e = tid; e < nn; e += NT) {
       const double2 sv = S[tk.s + e], fv = F[tk.f + e], sg = g[e];
       // (mu + i wn) * S - F - Sigma
       A[e] = make_double2(mu * sv.x - wn * sv.y - fv.x - sg.x, mu * sv.y + wn * sv.x - fv.y - sg.y);
     }
-  }
-  for (int j = lane; j < n; j += 32) ipiv[j] = 0;
-  __syncwarp();
-  int singular = 0;
-  for (int it = 0; it < n; ++it) {
-    // pivot: largest |A[j][k]| over unused rows j and columns k, first in row-major order on ties
-    double best = -1.0;
-    int bidx = 0x7fffffff;
-    for (int e = lane; e < n * n; e += 32) {
-      const int j = e / n, k = e - j * n;
-      if (ipiv[j] == 1 || ipiv[k] != 0) continue;
-      const double2 v = A[e];
-      const double av = v.x * v.x + v.y * v.y;
-      if (av > best || (av == best && e < bidx)) { best = av; bidx = e; }
+    inv_sync<NT>();
+    if (!gauss_jordan<NT>(A, n, rowk, old, fcol, used, perm, red, tid)) {
+      if (tid == 0) atomicExch(bad, 1);
+      return;
     }
-    for (int off = 16; off > 0; off >>= 1) {
-      const double ob = __shfl_down_sync(0xffffffffu, best, off);
-      const int oi = __shfl_down_sync(0xffffffffu, bidx, off);
-      if (ob > best || (ob == best && oi < bidx)) { best = ob; bidx = oi; }
-    }
-    best = __shfl_sync(0xffffffffu, best, 0);
-    bidx = __shfl_sync(0xffffffffu, bidx, 0);
-    if (!(best > 0.0)) { singular = 1; break; }
-    const int irow = bidx / n, icol = bidx - irow * n;
-    __syncwarp();
-    if (lane == 0) { ipiv[icol] += 1; indxr[it] = irow; indxc[it] = icol; }
-    if (irow != icol)
-      for (int l = lane; l < n; l += 32) {
-        const double2 t = A[irow * n + l];
-        A[irow * n + l] = A[icol * n + l];
-        A[icol * n + l] = t;
-      }
-    __syncwarp();
-    const double2 pv = A[icol * n + icol];
-    const double den = pv.x * pv.x + pv.y * pv.y;
-    const double2 pinv = make_double2(pv.x / den, -pv.y / den);
-    __syncwarp();
-    for (int l = lane; l < n; l += 32) {
-      const double2 v = (l == icol) ? make_double2(1.0, 0.0) : A[icol * n + l];
-      A[icol * n + l] = cmul(v, pinv);
-    }
-    __syncwarp();
-    for (int ll = lane; ll < n; ll += 32) {
-      if (ll == icol) continue;
-      const double2 f = A[ll * n + icol];
-      A[ll * n + icol] = make_double2(0.0, 0.0);
-      for (int l = 0; l < n; ++l) {
-        const double2 r = A[icol * n + l];
-        A[ll * n + l] = make_double2(A[ll * n + l].x - (r.x * f.x - r.y * f.y),
-                                     A[ll * n + l].y - (r.x * f.y + r.y * f.x));
-      }
-    }
-    __syncwarp();
-  }
-  if (singular) {
-    if (lane == 0) atomicExch(bad, 1);
-    return;
-  }
-  // undo the column permutation in reverse order
-  for (int l = n - 1; l >= 0; --l) {
-    const int r = indxr[l], c = indxc[l];
-    if (r != c)
-      for (int k = lane; k < n; k += 32) {
-        const double2 t = A[k * n + r];
-        A[k * n + r] = A[k * n + c];
-        A[k * n + c] = t;
-      }
-    __syncwarp();
-  }
-  if (mode == 1) {
     double2 *o = Wout ? Wout + tk.a : g;
-    for (int e = lane; e < n * n; e += 32) o[e] = A[e];
+    for (int e = tid; e < nn; e += NT) {
+      const int i = e / n, j = e - i * n;
+      o[i * n + perm[j]] = A[e];
+    }
     return;
   }
-  // R = (A^-1 + A^-H)/2, each unordered pair by one lane
-  for (int e = lane; e < n * n; e += 32) {
-    const int i = e / n, j = e - i * n;
-    if (j < i) continue;
-    const double2 aij = A[e], aji = A[j * n + i];
-    const double2 r = make_double2(0.5 * (aij.x + aji.x), 0.5 * (aij.y - aji.y));
-    A[e] = r;
-    A[j * n + i] = cconj(r);
-  }
-  __syncwarp();
-  for (int e = lane; e < n * n; e += 32) {
-    const int i = e / n, j = e - i * n;
-    double2 a = make_double2(0.0, 0.0);
-    for (int l = 0; l < n; ++l) a = cfma(A[i * n + l], B[l * n + j], a);
-    g[e] = a;
-  }
-}
-
-// Same Gauss-Jordan inverse with one CTA per block (blocks larger than 16):
-// the pivot search, the row scaling and the elimination run over all n^2
-// elements with the same per-element arithmetic and the same pivot order as
-// inverse_kernel.  Shared: A [n^2] | B [n^2] | fcol [n] (complex) | 3n ints.
-constexpr int INV_CTA_THREADS = 128;
-__host__ __device__ constexpr int inv_cta_smem_bytes(int n) { return (2 * n * n + n) * 16 + 3 * n * 4 + 64; }
-
-__global__ void __launch_bounds__(INV_CTA_THREADS) inverse_cta_kernel(
-    const InvTask *__restrict__ tasks, double2 *__restrict__ W, const double2 *__restrict__ S,
-    const double2 *__restrict__ F, const int64_t *__restrict__ wsample, double beta, double mu, int mode,
-    int *__restrict__ bad, int nm, const double *__restrict__ mu_ptr, double2 *__restrict__ Wout,
-    const int *__restrict__ skip) {
-  if (skip && *skip) return;
-  constexpr int NT = INV_CTA_THREADS, NW = NT / 32;
-  extern __shared__ double2 smem_inv[];
-  __shared__ double red_best[NW];
-  __shared__ int red_idx[NW];
-  __shared__ int piv[3];  // irow, icol, singular
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const InvTask tk = tasks[blockIdx.x];
-  const int n = tk.n;
-  double2 *A = smem_inv;
-  double2 *B = A + nm * nm;
-  double2 *fcol = B + nm * nm;
-  int *ipiv = reinterpret_cast<int *>(fcol + nm);
-  int *indxr = ipiv + nm;
-  int *indxc = indxr + nm;
-  double2 *g = W + tk.a;
-  if (mode == 0) {
-    for (int e = tid; e < n * n; e += NT) B[e] = g[e];
-    __syncthreads();
-    for (int e = tid; e < n * n; e += NT) {
+  for (int e = tid; e < nn; e += NT) B[e] = g[e];
+  inv_sync<NT>();
+  hermitian();
+  if (sweep_inverse<NT>(A, B, n, rowk, old, tid)) {
+    // R = -A, both triangles
+    for (int e = tid; e < nn; e += NT) {
       const int i = e / n, j = e - i * n;
-      const double2 pij = B[e], pji = B[j * n + i];
-      A[e] = make_double2((i == j ? 1.0 : 0.0) - 0.5 * (pij.x + pji.x), -0.5 * (pij.y - pji.y));
+      if (j > i) continue;
+      const double2 v = A[e];
+      A[e] = make_double2(-v.x, i == j ? 0.0 : -v.y);
+      if (j < i) A[j * n + i] = make_double2(-v.x, v.y);
     }
   } else {
-    if (mu_ptr) mu = *mu_ptr;
-    const double wn = (2.0 * (double)wsample[tk.w] + 1.0) * 3.14159265358979323846 / beta;
-    for (int e = tid; e < n * n; e += NT) {
-      const double2 sv = S[tk.s + e], fv = F[tk.f + e], sg = g[e];
-      A[e] = make_double2(mu * sv.x - wn * sv.y - fv.x - sg.x, mu * sv.y + wn * sv.x - fv.y - sg.y);
+    inv_sync<NT>();
+    hermitian();
+    if (!gauss_jordan<NT>(A, n, rowk, old, fcol, used, perm, red, tid)) {
+      if (tid == 0) atomicExch(bad, 1);
+      return;
     }
+    for (int e = tid; e < nn; e += NT) {  // columns in order, by way of B
+      const int i = e / n, j = e - i * n;
+      B[i * n + perm[j]] = A[e];
+    }
+    inv_sync<NT>();
+    for (int e = tid; e < nn; e += NT) {  // R = (A^-1 + A^-H)/2
+      const int i = e / n, j = e - i * n;
+      const double2 aij = B[e], aji = B[j * n + i];
+      A[e] = make_double2(0.5 * (aij.x + aji.x), 0.5 * (aij.y - aji.y));
+    }
+    inv_sync<NT>();
+    for (int e = tid; e < nn; e += NT) B[e] = g[e];
   }
-  for (int j = tid; j < n; j += NT) ipiv[j] = 0;
-  __syncthreads();
-  for (int it = 0; it < n; ++it) {
-    double best = -1.0;
-    int bidx = 0x7fffffff;
-    for (int e = tid; e < n * n; e += NT) {
-      const int j = e / n, k = e - j * n;
-      if (ipiv[j] == 1 || ipiv[k] != 0) continue;
-      const double2 v = A[e];
-      const double av = v.x * v.x + v.y * v.y;
-      if (av > best || (av == best && e < bidx)) { best = av; bidx = e; }
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-      const double ob = __shfl_down_sync(0xffffffffu, best, off);
-      const int oi = __shfl_down_sync(0xffffffffu, bidx, off);
-      if (ob > best || (ob == best && oi < bidx)) { best = ob; bidx = oi; }
-    }
-    if (lane == 0) { red_best[warp] = best; red_idx[warp] = bidx; }
-    __syncthreads();
-    if (tid == 0) {
-      double b = red_best[0];
-      int bi = red_idx[0];
-      for (int w = 1; w < NW; ++w)
-        if (red_best[w] > b || (red_best[w] == b && red_idx[w] < bi)) { b = red_best[w]; bi = red_idx[w]; }
-      if (!(b > 0.0)) {
-        piv[2] = 1;
-      } else {
-        const int irow = bi / n, icol = bi - irow * n;
-        piv[0] = irow; piv[1] = icol; piv[2] = 0;
-        ipiv[icol] += 1; indxr[it] = irow; indxc[it] = icol;
-      }
-    }
-    __syncthreads();
-    if (piv[2]) break;
-    const int irow = piv[0], icol = piv[1];
-    if (irow != icol) {
-      for (int l = tid; l < n; l += NT) {
-        const double2 t = A[irow * n + l];
-        A[irow * n + l] = A[icol * n + l];
-        A[icol * n + l] = t;
-      }
-      __syncthreads();
-    }
-    const double2 pv = A[icol * n + icol];
-    const double den = pv.x * pv.x + pv.y * pv.y;
-    const double2 pinv = make_double2(pv.x / den, -pv.y / den);
-    __syncthreads();
-    for (int l = tid; l < n; l += NT) {
-      const double2 v = (l == icol) ? make_double2(1.0, 0.0) : A[icol * n + l];
-      A[icol * n + l] = cmul(v, pinv);
-    }
-    for (int ll = tid; ll < n; ll += NT) fcol[ll] = A[ll * n + icol];
-    __syncthreads();
-    for (int e = tid; e < n * n; e += NT) {
-      const int ll = e / n, l = e - ll * n;
-      if (ll == icol) continue;
-      const double2 f = fcol[ll];
-      const double2 r = A[icol * n + l];
-      const double2 a = (l == icol) ? make_double2(0.0, 0.0) : A[e];
-      A[e] = make_double2(a.x - (r.x * f.x - r.y * f.y), a.y - (r.x * f.y + r.y * f.x));
-    }
-    __syncthreads();
-  }
-  if (piv[2]) {
-    if (tid == 0) atomicExch(bad, 1);
-    return;
-  }
-  for (int l = n - 1; l >= 0; --l) {
-    const int r = indxr[l], c = indxc[l];
-    if (r != c) {
-      for (int k = tid; k < n; k += NT) {
-        const double2 t = A[k * n + r];
-        A[k * n + r] = A[k * n + c];
-        A[k * n + c] = t;
-      }
-      __syncthreads();
-    }
-  }
-  if (mode == 1) {
-    double2 *o = Wout ? Wout + tk.a : g;
-    for (int e = tid; e < n * n; e += NT) o[e] = A[e];
-    return;
-  }
-  for (int e = tid; e < n * n; e += NT) {
-    const int i = e / n, j = e - i * n;
-    if (j < i) continue;
-    const double2 aij = A[e], aji = A[j * n + i];
-    const double2 r = make_double2(0.5 * (aij.x + aji.x), 0.5 * (aij.y - aji.y));
-    A[e] = r;
-    A[j * n + i] = cconj(r);
-  }
-  __syncthreads();
-  for (int e = tid; e < n * n; e += NT) {
+  inv_sync<NT>();
+  for (int e = tid; e < nn; e += NT) {
     const int i = e / n, j = e - i * n;
     double2 a = make_double2(0.0, 0.0);
     for (int l = 0; l < n; ++l) a = cfma(A[i * n + l], B[l * n + j], a);
@@ -814,11 +777,11 @@ void launch_inverse(const InvTask *tasks, int ntasks, int nmax, double2 *W, cons
                     cudaStream_t st, const double *mu_ptr, double2 *Wout, const int *skip) {
   if (ntasks == 0) return;
   if (nmax > 16) {  // one CTA per block
-    inverse_cta_kernel<<<ntasks, INV_CTA_THREADS, inv_cta_smem_bytes(nmax), st>>>(
-        tasks, W, S, F, wsample, beta, mu, mode, bad, nmax, mu_ptr, Wout, skip);
+    inverse_kernel<INV_CTA_THREADS><<<ntasks, INV_CTA_THREADS, inv_bytes(nmax, mode), st>>>(
+        tasks, ntasks, W, S, F, wsample, beta, mu, mode, bad, nmax, mu_ptr, Wout, skip);
   } else {          // one warp per block
-    const int w = inv_warps_per_block(nmax);
-    inverse_kernel<<<(ntasks + w - 1) / w, 32 * w, inv_smem_bytes(nmax), st>>>(
+    const int w = inv_warps_per_block(nmax, mode);
+    inverse_kernel<32><<<(ntasks + w - 1) / w, 32 * w, w * inv_bytes(nmax, mode), st>>>(
         tasks, ntasks, W, S, F, wsample, beta, mu, mode, bad, nmax, mu_ptr, Wout, skip);
   }
   GWGB_CUDA(cudaGetLastError());
@@ -841,9 +804,8 @@ void set_fp64_kernel_attributes(int smem_bytes) {
 }
 
 void set_inverse_kernel_attributes() {
-  GWGB_CUDA(cudaFuncSetAttribute(inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, inv_smem_bytes(MAX_BLOCK)));
-  GWGB_CUDA(cudaFuncSetAttribute(inverse_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 inv_cta_smem_bytes(MAX_BLOCK)));
+  GWGB_CUDA(cudaFuncSetAttribute(inverse_kernel<INV_CTA_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 inv_bytes(MAX_BLOCK, 0)));
 }
 
 }  // namespace gwgb
