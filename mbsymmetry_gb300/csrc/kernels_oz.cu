@@ -97,7 +97,7 @@ __device__ __forceinline__ void oz_slice(F2 h, F2 l, F2 v, F2 f, F2 m1, F2 (&s)[
   s[2] = sub2(t, s[1]);
 }
 
-// Unevaluated sums of three FP32 numbers, h the rounded value.
+// Unevaluated sums of three FP32 numbers; normalised: h the rounded value, m that of the rest.
 struct Tri {
   F2 h, m, l;
 };
@@ -105,8 +105,8 @@ struct Tri {
 // The value of the class sums D0 .. D3 and d4 = D4 + 2^-9 D5 + 2^-18 D6 (weights 2^(-9c)).  Carries instead of two-sums (26 steps against 44): D0 to D3
 // are exact integers, at most 64 sums of c + 1 products of digits, of which at most one is 256 in each factor, so D3 and
 // a carry of 2^15.4 stay below 2^24 and each step is exact (but for the last bits of D4 to D6, which the tensor core
-// rounds to 24 bits).
-__device__ __forceinline__ Tri tri_of(const F2 (&d)[4], F2 d4) {
+// rounds to 24 bits).  NORM: normalised.
+template <bool NORM> __device__ __forceinline__ Tri tri_of(const F2 (&d)[4], F2 d4) {
   const F2 W = both(0x1p-9f), MG = both(1.5f * 8388608.f), NM = both(-1.5f * 8388608.f), NB = both(-512.f);
   auto carry = [&](F2 x) { return add2(fma2(x, W, MG), NM); };  // x / 512 to an integer
   const F2 c4 = carry(d4);
@@ -117,6 +117,7 @@ __device__ __forceinline__ Tri tri_of(const F2 (&d)[4], F2 d4) {
   const F2 a = add2(d[0], c1);
   const F2 m = fma2(fma2(c1, NB, d1), both(0x1p-9f), mul2(fma2(c2, NB, d2), both(0x1p-18f)));
   const F2 l = fma2(fma2(c3, NB, d3), both(0x1p-27f), mul2(fma2(c4, NB, d4), both(0x1p-36f)));
+  if constexpr (!NORM) return {a, m, l};
   const F2 m1 = add2(m, l);
   Tri t;
   t.h = add2(a, m1);
@@ -125,16 +126,20 @@ __device__ __forceinline__ Tri tri_of(const F2 (&d)[4], F2 d4) {
   return t;
 }
 
-// a += b, and a normalised (h the rounded value).
+// a += b without normalising: sums and their errors stay in order of size, which leaves R rounds within 2^-70 R^2 of
+// the largest (21 steps a round; normalised every time it was 36, and the FP32 pipe bounds the drains).
 __device__ __forceinline__ void tri_add(Tri &a, const Tri &b) {
-  F2 h, e1, m, e2, e3;
-  two_sum(a.h, b.h, h, e1);
+  F2 e1, m, e2, e3;
+  two_sum(a.h, b.h, a.h, e1);
   two_sum(a.m, b.m, m, e2);
-  two_sum(m, e1, m, e3);
-  const F2 l = add2(add2(a.l, b.l), add2(e2, e3));
+  two_sum(m, e1, a.m, e3);
+  a.l = add2(add2(a.l, b.l), add2(e2, e3));
+}
+
+__device__ __forceinline__ void tri_norm(F2 &h, F2 &m, F2 &l) {
   two_sum(h, m, h, m);
-  two_sum(m, l, m, a.l);
-  two_sum(h, m, a.h, a.m);
+  two_sum(m, l, m, l);
+  two_sum(h, m, h, m);
 }
 
 // a + b for a zero or |a| > |b|: s the rounded sum, b what it leaves.
@@ -622,7 +627,7 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
                   F2 d[4];
 #pragma unroll
                   for (int c = 0; c < 4; ++c) d[c] = {__uint_as_float(x[c][2 * e]), __uint_as_float(x[c][2 * e + 1])};
-                  Tri t = tri_of(d, d4[i]);
+                  Tri t = tri_of<STAGE != 2 && !MULTI>(d, d4[i]);
                   const F2 sc = both(oz_pow2c(eb[i] - em) * fn);
                   t = {mul2(t.h, sc), mul2(t.m, sc), mul2(t.l, sc)};
                   if (!first) {
@@ -641,6 +646,10 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
           tc::fence_before_sync();
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(&tfree[set]);
+        }
+        if constexpr (NS == 6 && STAGE != 2 && MULTI) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) tri_norm(H[0][e], M3[0][e], L[0][e]);
         }
         if constexpr (STAGE == 2) {  // FP64 partial of this K slice
           const OzS3 d = static_cast<const OzS3 *>(g.desc)[tk.d];
