@@ -336,6 +336,7 @@ class Engine {
   bool vt_ready_ = false;
   DBuf<TSlab> slab_p_fwd_, slab_p_bwd_, slab_s_fwd_, slab_g_bwd_;
   DBuf<InvTask> inv_w_, inv_d_;
+  std::vector<InvClass> inv_w_cls_, inv_d_cls_;
   int p0_maxo_ = 8, sig_maxo_ = 8, rot_smem_ = 0;
   int fp64_smem_ = 0, nsm_ = 0;  // FP64 contraction CTA shared memory; SM count
   // tcgen05 Sigma path: W-GEMM tiles, conj(V) operand tasks, per-contribution W references
@@ -1431,6 +1432,8 @@ void Engine::build_work_lists() {
       check_range(t.s, (int64_t)t.n * t.n, (int64_t)ns_ * fa, "S/F block");
     }
   }
+  inv_w_cls_ = inv_classes(iw);
+  inv_d_cls_ = inv_classes(id);
   inv_w_.upload(iw, st_);
   inv_d_.upload(id, st_);
   {  // algorithmic work of the transforms (16 (n_in + n_out) B per column + T once per launch) and
@@ -1761,7 +1764,7 @@ void Engine::k_pq(bool mirror_first) {
   record(8);
   transform(XF_P0, slab_p_fwd_, max_cols_p_, TntBF_.p, nw_b_, ncheb_, 1, Pall_.p, Pw_.p);
   record(9);
-  launch_inverse(inv_w_.p, (int)inv_w_.n, l_.max_aux, Pw_.p, nullptr, nullptr, nullptr, beta_, 0.0, 0, bad_.p, st_);
+  launch_inverse(inv_w_.p, inv_w_cls_, Pw_.p, nullptr, nullptr, nullptr, beta_, 0.0, 0, bad_.p, st_);
   record(10);
   transform(XF_P, slab_p_bwd_, max_cols_p_, TtnFB_.p, nts_, nw_b_, 0, Pw_.p, Pall_.p);
   record(11);
@@ -1792,7 +1795,7 @@ void Engine::k_sigma() {
 
 void Engine::k_dyson() {
   transform(XF_SIGMA, slab_s_fwd_, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p);
-  launch_inverse(inv_d_.p, (int)inv_d_.n, l_.max_ao, Ww_.p, S_.p, F_.p, ws_.p, beta_, 0.0, 1, bad_.p + 1, st_);
+  launch_inverse(inv_d_.p, inv_d_cls_, Ww_.p, S_.p, F_.p, ws_.p, beta_, 0.0, 1, bad_.p + 1, st_);
   transform(XF_G, slab_g_bwd_, max_cols_g_, Ttn_.p, nts_, nw_, 0, Ww_.p, Gall_.p);
   if (has_tct_) {
     GWGB_CUDA(cudaMemsetAsync(leak_.p, 0, 2 * sizeof(unsigned long long), st_));
@@ -1850,6 +1853,7 @@ void Engine::finish_stats(bool with_dyson, bool with_gw, bool with_pq, bool with
     s.solve_flops += solve_flops_dy_;
   }
   int64_t launches = 0;
+  auto xf = [&](int i) { return xf_[i].ready ? 2 : 1; };  // a transform in six slices builds its images first
   if (with_gw) {
     const bool tc = tc_split();
     int64_t sgt = 0, p0t = 0;
@@ -1862,10 +1866,11 @@ void Engine::finish_stats(bool with_dyson, bool with_gw, bool with_pq, bool with
     const int64_t sg = tc ? sgt
                           : (sig_tiles_.n ? 1 : 0) + (sig_red_.n ? 1 : 0);
     OzSet *o0 = oz_set(0), *o1 = oz_set(1);  // (+ 1: the tau mirror of P0)
-    launches += (rotG_.n ? 1 : 0) + (o0 ? (int64_t)o0->plan[0].launches().size() + 1 : p0) + 3 +
+    launches += (rotG_.n ? 1 : 0) + (o0 ? (int64_t)o0->plan[0].launches().size() + 1 : p0) + xf(XF_P0) +
+                (int64_t)inv_w_cls_.size() + xf(XF_P) +
                 (o1 ? (int64_t)o1->plan[1].launches().size() : sg);
   }
-  if (with_dyson) launches += 3 + (has_tct_ ? 1 : 0);
+  if (with_dyson) launches += xf(XF_SIGMA) + (int64_t)inv_d_cls_.size() + xf(XF_G) + (has_tct_ ? 1 : 0);
   s.kernel_launches = launches;
   stats_ = s;
 }
@@ -1956,7 +1961,7 @@ void Engine::dyson(double mu) {
   record(5);
   transform(XF_SIGMA, slab_s_fwd_, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p);
   record(12);
-  launch_inverse(inv_d_.p, (int)inv_d_.n, l_.max_ao, Ww_.p, S_.p, F_.p, ws_.p, beta_, mu, 1, bad_.p + 1, st_);
+  launch_inverse(inv_d_.p, inv_d_cls_, Ww_.p, S_.p, F_.p, ws_.p, beta_, mu, 1, bad_.p + 1, st_);
   record(13);
   transform(XF_G, slab_g_bwd_, max_cols_g_, Ttn_.p, nts_, nw_, 0, Ww_.p, Gall_.p);
   record(14);
@@ -1995,7 +2000,7 @@ void Engine::iteration(double mu) {
     record(5);
     transform(XF_SIGMA, slab_s_fwd_, max_cols_g_, Tnt_.p, nw_, ncheb_, 1, Sig_.p, Ww_.p);
     record(12);
-    launch_inverse(inv_d_.p, (int)inv_d_.n, l_.max_ao, Ww_.p, S_.p, F_.p, ws_.p, beta_, mu, 1, bad_.p + 1, st_);
+    launch_inverse(inv_d_.p, inv_d_cls_, Ww_.p, S_.p, F_.p, ws_.p, beta_, mu, 1, bad_.p + 1, st_);
     record(13);
     transform(XF_G, slab_g_bwd_, max_cols_g_, Ttn_.p, nts_, nw_, 0, Ww_.p, Gall_.p);
     record(14);
@@ -2071,7 +2076,7 @@ void Engine::k_mu_search(const gwgb_mu_search &ms) {
   const int *done = reinterpret_cast<const int *>(reinterpret_cast<const char *>(mus_.p) + offsetof(MuState, done));
   launch_mu_begin(mus_.p, mu_dev_.p, ms.step, st_);
   for (int e = 0; e < ms.max_evals; ++e) {
-    launch_inverse(inv_d_.p, (int)inv_d_.n, l_.max_ao, Ww_.p, S_.p, F_.p, ws_.p, beta_, 0.0, 1, bad_.p + 1, st_,
+    launch_inverse(inv_d_.p, inv_d_cls_, Ww_.p, S_.p, F_.p, ws_.p, beta_, 0.0, 1, bad_.p + 1, st_,
                    mu_dev_.p, Wg_.p, done);
     // G(beta) only: the last row of Ttn
     launch_transform(slab_g_bwd_.p, (int)slab_g_bwd_.n, max_cols_g_, Ttn_.p + (int64_t)(nts_ - 1) * nw_, 1, nw_, 0,
@@ -2082,7 +2087,7 @@ void Engine::k_mu_search(const gwgb_mu_search &ms) {
 }
 
 void Engine::k_dyson_dev() {
-  launch_inverse(inv_d_.p, (int)inv_d_.n, l_.max_ao, Ww_.p, S_.p, F_.p, ws_.p, beta_, 0.0, 1, bad_.p + 1, st_,
+  launch_inverse(inv_d_.p, inv_d_cls_, Ww_.p, S_.p, F_.p, ws_.p, beta_, 0.0, 1, bad_.p + 1, st_,
                  mu_dev_.p);
   transform(XF_G, slab_g_bwd_, max_cols_g_, Ttn_.p, nts_, nw_, 0, Ww_.p, Gall_.p);
   if (has_tct_) {

@@ -1,6 +1,8 @@
 // Launchers of the GW engine kernels (host side).
 #pragma once
 
+#include <vector>
+
 #include "common.h"
 
 namespace gwgb {
@@ -8,6 +10,11 @@ namespace gwgb {
 // Largest irrep block (AO or aux) the FP64 kernels accept.
 constexpr int MAX_BLOCK = 64;
 
+// Tasks [first, first + count) of a launch of the block inverses, none larger than nmax.
+struct InvClass { int first, count, nmax; };
+// Sorts the tasks by size, largest first, and splits them where the kernel changes: the shared memory of a CTA is that of
+// the largest block of its launch, so small blocks would run one per SM beside one of 64.
+std::vector<InvClass> inv_classes(std::vector<InvTask> &tasks);
 // Block inverses: shared memory of one matrix (A, in mode 0 P, three rows, 2 n ints); up to n = 16 one warp per
 // block and as many warps per CTA as fit in ~48 KB, 1 to 8.
 __host__ __device__ constexpr int inv_bytes(int nmax, int mode) {
@@ -52,7 +59,8 @@ void launch_transform(const TSlab *slabs, int nslabs, int max_cols, const double
 // Batched block inverses.  mode 0: W~ (R = sym((1 - sym(P))^-1), R P); mode 1:
 // Dyson ((mu + i w_n) S - F - Sigma)^-1.  Optional: mu read from *mu_ptr,
 // output to Wout instead of in place, nothing done while *skip != 0.
-void launch_inverse(const InvTask *tasks, int ntasks, int nmax, double2 *W, const double2 *S,
+// One launch per class of block sizes (inv_classes: tasks sorted, largest first).
+void launch_inverse(const InvTask *tasks, const std::vector<InvClass> &classes, double2 *W, const double2 *S,
                     const double2 *F, const int64_t *wsample, double beta, double mu, int mode, int *bad,
                     cudaStream_t st, const double *mu_ptr = nullptr, double2 *Wout = nullptr,
                     const int *skip = nullptr);

@@ -10,6 +10,8 @@
 #include "common.h"
 #include "kernels.h"
 
+#include <algorithm>
+
 namespace gwgb {
 
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
@@ -387,12 +389,11 @@ __global__ void __launch_bounds__(256) transform_kernel(const TSlab *__restrict_
 //  - the general one is Gauss-Jordan with full pivoting (the strategy of Eigen::FullPivLU,
 //    sc_type_block.cpp:55), 4 FMA per element and step; the pivot is the largest
 //    component by its upper 32 bits, found in integers while the elimination writes the elements.
-// One warp per matrix up to n = 16, one CTA above (NT threads either way), elements spread over the threads.
-// The W~ solve of the 27 k s+p+d+4 crystal (aux 2-40): 3.36 ms with the elimination for all, 1.40; hexagonal 8 k:
-// 3.15, 1.14; Dyson, hexagonal 8 k (AO 2-30): 0.61, 0.18; s+p (n up to 12): W~ and Dyson 0.17, 0.07.
+// One warp per matrix up to n = 16, a CTA of 128 threads up to 32, of 256 above (NT), elements spread over the threads.
+// Measured, before and now: W~ s+p+d+4 (aux 9-46) 3.36 and 1.32 ms, hexagonal 8 k (aux 2-30) 3.15 and 1.02; Dyson there
+// (AO 2-30) 0.61 and 0.20; s+p (n up to 12), both solves, 0.17 and 0.07.  Tried and slower: the product R P from one
+// triangle (R commutes with the Hermitian part of P), the rest in FP32.
 // ---------------------------------------------------------------------------
-constexpr int INV_CTA_THREADS = 128;
-
 template <int NT> __device__ __forceinline__ void inv_sync() {
   if constexpr (NT == 32)
     __syncwarp();
@@ -772,19 +773,34 @@ void launch_transform(const TSlab *slabs, int nslabs, int max_cols, const double
   GWGB_CUDA(cudaGetLastError());
 }
 
-void launch_inverse(const InvTask *tasks, int ntasks, int nmax, double2 *W, const double2 *S,
+std::vector<InvClass> inv_classes(std::vector<InvTask> &tasks) {
+  std::stable_sort(tasks.begin(), tasks.end(), [](const InvTask &x, const InvTask &y) { return x.n > y.n; });
+  std::vector<InvClass> c;
+  auto kind = [](int n) { return n > 32 ? 2 : n > 16 ? 1 : 0; };
+  for (size_t i = 0; i < tasks.size(); ++i) {
+    if (i == 0 || kind(tasks[i].n) != kind(tasks[i - 1].n)) c.push_back({(int)i, 0, tasks[i].n});
+    ++c.back().count;
+  }
+  return c;
+}
+
+void launch_inverse(const InvTask *tasks, const std::vector<InvClass> &classes, double2 *W, const double2 *S,
                     const double2 *F, const int64_t *wsample, double beta, double mu, int mode, int *bad,
                     cudaStream_t st, const double *mu_ptr, double2 *Wout, const int *skip) {
-  if (ntasks == 0) return;
-  if (nmax > 16) {  // one CTA per block
-    inverse_kernel<INV_CTA_THREADS><<<ntasks, INV_CTA_THREADS, inv_bytes(nmax, mode), st>>>(
-        tasks, ntasks, W, S, F, wsample, beta, mu, mode, bad, nmax, mu_ptr, Wout, skip);
-  } else {          // one warp per block
-    const int w = inv_warps_per_block(nmax, mode);
-    inverse_kernel<32><<<(ntasks + w - 1) / w, 32 * w, w * inv_bytes(nmax, mode), st>>>(
-        tasks, ntasks, W, S, F, wsample, beta, mu, mode, bad, nmax, mu_ptr, Wout, skip);
+  for (const InvClass &c : classes) {
+    const int bytes = inv_bytes(c.nmax, mode);
+    auto run = [&](auto kernel, int per, int threads) {
+      kernel<<<(c.count + per - 1) / per, per * threads, per * bytes, st>>>(
+          tasks + c.first, c.count, W, S, F, wsample, beta, mu, mode, bad, c.nmax, mu_ptr, Wout, skip);
+    };
+    if (c.nmax > 32)
+      run(inverse_kernel<256>, 1, 256);
+    else if (c.nmax > 16)
+      run(inverse_kernel<128>, 1, 128);
+    else  // one warp per block
+      run(inverse_kernel<32>, inv_warps_per_block(c.nmax, mode), 32);
+    GWGB_CUDA(cudaGetLastError());
   }
-  GWGB_CUDA(cudaGetLastError());
 }
 
 void launch_leakage(const TSlab *slabs, int nslabs, const double2 *G, const double *tf, const double *tl,
@@ -804,8 +820,8 @@ void set_fp64_kernel_attributes(int smem_bytes) {
 }
 
 void set_inverse_kernel_attributes() {
-  GWGB_CUDA(cudaFuncSetAttribute(inverse_kernel<INV_CTA_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 inv_bytes(MAX_BLOCK, 0)));
+  GWGB_CUDA(cudaFuncSetAttribute(inverse_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, inv_bytes(MAX_BLOCK, 0)));
+  GWGB_CUDA(cudaFuncSetAttribute(inverse_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, inv_bytes(32, 0)));
 }
 
 }  // namespace gwgb

@@ -141,7 +141,7 @@ extern "C" int gwgb_wsolve_noalloc(int32_t device, const double *P0_t, double *P
     const int ncheb = nts - 2;
     launch_transform(slabs, 1, (int)qslice, reinterpret_cast<const double2 *>(Tnt_BF), nw_b, ncheb, 1,
                      reinterpret_cast<const double2 *>(P0_t), Pw, st);
-    launch_inverse(tasks, nw_b * nblocks, nmax, Pw, nullptr, nullptr, nullptr, 1.0, 0.0, 0, status, st);
+    launch_inverse(tasks, {{0, nw_b * nblocks, nmax}}, Pw, nullptr, nullptr, nullptr, 1.0, 0.0, 0, status, st);
     launch_transform(slabs + 1, 1, (int)qslice, reinterpret_cast<const double2 *>(Ttn_FB), nts, nw_b, 0, Pw,
                      reinterpret_cast<double2 *>(P_t), st);
     int host_status = 0;
