@@ -217,7 +217,8 @@ PREC_LABEL = {
     "ozaki": ("fp16 x3 slices per operand row (Ozaki scheme, 33 bits) on tcgen05 kind::f16, 8 products, "
               "exact leading sums in FP32, float-float accumulation; FP64 W~ solve, Dyson, "
               "transforms, mu search, energies"),
-    "fp64": "complex128 contractions on CUDA cores (the drop-in)",
+    "fp64": ("complex128 contractions (the drop-in): fp16 x6 slices per operand row (57 bits) on tcgen05 kind::f16, "
+             "26 products, exact leading sums in FP32; blocks too small for that in FP64 FMAs"),
     "tf32x3": ("tf32x3 (tcgen05 kind::tf32, 2 planes, 3 products, FP32 accumulate within an aux block or "
                "aux-row chunk, FP64 across): FP32-class error, no 1e-7 claim"),
     "bf16x3": ("bf16x3 (tcgen05 kind::f16, 3 BF16 planes, 6 products, FP32 accumulate within an aux block or "
@@ -430,12 +431,13 @@ def run_gpu(args):
     a64 = s64[f"{dom64}_flops"] / (st64[f"{dom64}_ms"] * 1e-3) / 1e12
     fp64 = {"precision": PREC_LABEL["fp64"], "s_per_iteration": ms64 / 1e3, "stages_ms": st64,
             "contraction_tflops": {k: s64[f"{k}_flops"] / (st64[f"{k}_ms"] * 1e-3) / 1e12 for k in ("p0", "sigma")},
-            "roofline": {"bound": "fp64 (CUDA-core FMA)", "kernel": f"{dom64}_fp64_kernel", "achieved": a64,
-                         "peak": fp64_peak, "unit": "TFLOP/s", "frac": a64 / fp64_peak if fp64_peak > 0 else None,
-                         "traffic": {"sigma": 0.0703e9, "p0": 0.0563e9}[dom64],
-                         "traffic_unit": "bytes per launch (ncu)",
-                         "note": "FP64 FMA on CUDA cores: the FP64 tensor path (DMMA) measures slower on this "
-                                 "GPU (peaks.fp64_dmma_tflops)"},
+            "roofline": {"bound": "tensor (six FP16 slices, 26 products)", "kernel": "oz_gemm_kernel",
+                         "contraction": dom64, "achieved": a64, "peak": peaks["tcgen05_bf16_tflops"] / 26,
+                         "unit": "TFLOP/s", "frac": a64 / (peaks["tcgen05_bf16_tflops"] / 26),
+                         "times_fp64_fma_peak": a64 / fp64_peak if fp64_peak > 0 else None,
+                         "note": "algorithmic FP64 FLOPs of the whole contraction / its stage time, against the measured "
+                                 "kind::f16 rate over the 26 slice products; the FP64 FMA rate (peaks.fp64_fma_tflops) "
+                                 "bounds the kernels used for small blocks"},
             "transforms": {"ms": st64["transform_ms"], "bytes_alg": s64["transform_bytes"],
                            "achieved_gbs": s64["transform_bytes"] / (st64["transform_ms"] * 1e-3) / 1e9,
                            "flops_alg": s64["transform_flops"],
@@ -510,7 +512,7 @@ def run_gpu(args):
     line = {
         "metric": METRIC, "value": reps.seconds_per_iteration(ms), "unit": "s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": False,
-        "scaling": "weak", "vs_baseline": None, "dtype": "bf16x4 slices (c128 in/out, fp64 solves)",
+        "scaling": "weak", "vs_baseline": None, "dtype": "fp16x3 slices (c128 in/out, fp64 solves)",
         "data": "synthetic (seeded)",
         "config": {"workload": WORKLOAD},
         "precision": "ozaki: " + PREC_LABEL["ozaki"], "l2": "flushed (256 MiB write) before each step",
