@@ -5,7 +5,7 @@ nao=26, naux=120, nts=100, beta=100, ns=1, V stored for all 729 k pairs),
 synthetic seeded data (see mbsymmetry_gb300/crystal.py).  One step = one GW
 iteration P0 -> P~ (W~ solve) -> Sigma -> Dyson with all tau <-> i omega
 transforms, replayed as one CUDA graph, with the P0 and Sigma contractions on
-the sliced split-precision path (BF16 fixed-point slices on tcgen05, Sigma
+the sliced split-precision path (FP16 fixed-point slices on tcgen05, Sigma
 within 1e-7 Ha of FP64: the error is measured and reported in the line); the
 FP64 drop-in, the FP32-class split paths, mixed-vs-FP64 blocks for C3, C4 and
 C2's sizes built from Gaussian orbitals, and the self-consistent loop are

@@ -1473,26 +1473,20 @@ bool Engine::alloc_oz(OzSet &set) {
   if (set.alloc) return true;
   const OzPlan &p = set.plan[0], &s = set.plan[1];
   drop_graphs();  // they may hold the addresses of smaller buffers
-  auto grow = [](auto &buf, int64_t a, int64_t b) {
-    const int64_t m = std::max(a, b);
-    if (m > (int64_t)buf.n) buf.alloc((size_t)m);
-  };
   try {
     for (int k = 0; k < 2; ++k)
       if (!set.off[k]) set.plan[k].alloc_images();
-    grow(oz_buf_.A1, p.bytes_A1(), s.bytes_A1());
-    grow(oz_buf_.B2, p.bytes_B2(), s.bytes_B2());
-    grow(oz_buf_.X1, p.bytes_X1(), s.bytes_X1());
-    grow(oz_buf_.X2, p.bytes_X2(), s.bytes_X2());
-    grow(oz_buf_.part, p.part_elems(), s.part_elems());
+    auto m = [](int64_t a, int64_t b) { return std::max(a, b); };
+    oz_buf_.grow(m(p.bytes_A1(), s.bytes_A1()), m(p.bytes_B2(), s.bytes_B2()), m(p.bytes_X1(), s.bytes_X1()),
+                 m(p.bytes_X2(), s.bytes_X2()), m(p.part_elems(), s.part_elems()));
   } catch (const Error &e) {
+    oz_buf_.free();
+    for (OzSet &o : oz_) o.alloc = o.ready = false;  // the other set's buffers, too, are allocated again on its next use
     if (&set != &oz_[1] || e.code != GWGB_E_NOMEM) throw;
     cudaGetLastError();
     set.off[0] = set.off[1] = true;
     set.plan[0].free();
     set.plan[1].free();
-    oz_buf_.free();
-    oz_[0].alloc = oz_[0].ready = false;  // its buffers, too, are allocated again on its next use
     return false;
   }
   set.alloc = true;
@@ -1534,7 +1528,8 @@ void Engine::build_oz() {
   GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
   const int64_t avail = (int64_t)free_b - (V_.p ? 0 : 16 * l.flat_V);
   const int64_t persist = std::max<int64_t>(0, avail / 4);
-  // intermediates of one chunk: large chunks mean fewer, fuller launches (hex 8 k: 1 GB 66 ms, 8 GB 56 ms)
+  // intermediates of one chunk: large chunks mean fewer, fuller launches (hexagonal 8 k, the stages of both
+  // contractions in three slices: 1 GB 47.5 ms, 8 GB 37.2, 16 GB 36.6)
   const int64_t budget = tc_chunk_env_ ? tc_chunk_bytes_ : std::min<int64_t>(OZ_CHUNK_BYTES, std::max<int64_t>(64ll << 20, avail / 8));
   // P0[Q][P] = sum V[Q][p][m] G1(beta - tau)[t][p] conj(V[P][t][n]) G2(tau)[m][n]
   for (const P0Group &g : p0_groups_) {
@@ -1587,7 +1582,7 @@ void Engine::build_oz() {
     // Six slices against the FMA kernels, one contraction at a time: the MMAs (padded to octets of columns and 128 rows)
     // run at 190 TFLOP/s and more including their drains, the launches around them take about 0.05 ms; the FMA
     // kernels run at 1.2 TFLOP/s.  s+p (AO blocks 1-4): P0 0.45 ms against 0.40, Sigma 0.44 against 0.70; s+p+d
-    // (1-8): 17 against 94; hexagonal 4 k (AO 7-30): 18.5 against 222; blocks of a single orbital stay on the FMA
+    // (1-8), both: 14 against 94; hexagonal 4 k (AO 7-30): 18 against 222; blocks of a single orbital stay on the FMA
     // kernels.  (GWGB_FP64_SLICES=1 / 0 in the environment forces one or the other)
     const char *force = std::getenv("GWGB_FP64_SLICES");
     for (int k = 0; k < 2; ++k) {

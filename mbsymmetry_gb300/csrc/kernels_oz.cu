@@ -293,9 +293,10 @@ template <int NS, int STAGE> struct Job {
 constexpr int OZ_RING = 8;              // largest operand ring of a set
 constexpr int OZ_SC = 16;               // scale rings of a set: deeper than its operand ring plus its row tiles
 constexpr int OZ_SMEM = 200 * 1024;
-// Drain warps (then one warp copies and one issues the MMAs): three slices take two octets per
-// thread in 8 warps (hex 8 k: 61 ms against 69 with one octet in 16 warps), six slices one octet
-// in 16 warps (s+p+d: 24 ms against 33: unrolled over two octets the code misses the instruction cache).
+// Drain warps (then per accumulator set one that copies and one that issues the MMAs): three slices take two
+// octets per thread in 8 warps (stage 1 of Sigma, hexagonal 8 k, 7.5 ms against 8.8 with one octet in 16 warps),
+// six slices one octet in 16 warps (s+p+d: 24 ms an iteration against 33 when that was measured: unrolled over two
+// octets the code misses the instruction cache).
 template <int NS> constexpr int oz_drain = 4 * OzCfg<NS>::OCT / OzCfg<NS>::HO;
 template <int NS> constexpr int oz_threads = NS == 6 ? 640 : 32 * (oz_drain<NS> + 2 * OzCfg<NS>::SETS);
 
@@ -340,10 +341,11 @@ __device__ __forceinline__ void oz_mmas(uint32_t d0, uint32_t a0, uint32_t b0, u
     }
 }
 
-// Persistent warp-specialised GEMM over operand images.  Bound: the drain's
-// CUDA-core work (about 40 FP32 instructions per complex output of stages 1
-// and 2) and the L2 / HBM traffic of the images; the operands need no CUDA-core
-// work at all, a K step (8 complex) is 8 MMAs, and two TMEM accumulator sets let
+// Persistent warp-specialised GEMM over operand images.  Bound, three slices: HBM in
+// stages 2 and 3 (hexagonal 8 k, Sigma: 6.0 and 5.6 TB/s of 6.8), the drains in stage 1
+// (2800 cycles per accumulator set, its MMAs 880); six slices: the drains' FP32 work, in
+// stage 3 about as long as the MMAs.  The operands need no CUDA-core work at all, a K step
+// (8 complex) is 8 or 26 MMAs, and the two accumulator sets of three slices let
 // one round multiply while the other drains.  Operands stream through rings of
 // segments of SEG K steps; stages 1 and 2 hold the column operand of a task over
 // its row tiles.  The issue of an MMA blocks its warp while the tensor pipe is

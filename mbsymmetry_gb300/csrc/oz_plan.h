@@ -1,6 +1,7 @@
 // Work lists and buffers of one sliced contraction (P0 or Sigma).
 #pragma once
 
+#include <algorithm>
 #include <vector>
 
 #include "dbuf.h"
@@ -45,11 +46,37 @@ struct OzLaunch {
 };
 
 // Buffers that the plans of one handle share (they run one after the other).
-struct OzShared {
-  DBuf<char> A1, B2, X1, X2;
-  DBuf<double2> part;
+struct OzShared {  // one allocation (a first pass waits for it)
+  template <typename T> struct Part {
+    T *p = nullptr;
+    size_t n = 0;
+  };
+  Part<char> A1, B2, X1, X2;
+  Part<double2> part;
+  DBuf<char> pool;
+  // At least these sizes (the contents are lost when that means a new allocation).
+  void grow(int64_t a1, int64_t b2, int64_t x1, int64_t x2, int64_t np) {
+    auto fits = [](const auto &x, int64_t n) { return n <= (int64_t)x.n; };
+    if (fits(A1, a1) && fits(B2, b2) && fits(X1, x1) && fits(X2, x2) && fits(part, np)) return;
+    size_t at = 0;
+    auto place = [&](auto &x, int64_t n, auto *q) {
+      x.n = std::max(x.n, (size_t)n);
+      x.p = reinterpret_cast<decltype(q)>(at);
+      at = (at + x.n * sizeof(*q) + 1023) / 1024 * 1024;
+    };
+    auto all = [&](auto &&f) { f(A1); f(B2); f(X1); f(X2); };
+    pool.free();
+    place(A1, a1, (char *)nullptr); place(B2, b2, (char *)nullptr);
+    place(X1, x1, (char *)nullptr); place(X2, x2, (char *)nullptr);
+    place(part, np, (double2 *)nullptr);
+    pool.alloc(at);
+    all([&](auto &x) { x.p = pool.p + reinterpret_cast<size_t>(x.p); });
+    part.p = reinterpret_cast<double2 *>(pool.p + reinterpret_cast<size_t>(part.p));
+  }
   void free() {
-    A1.free(); B2.free(); X1.free(); X2.free(); part.free();
+    pool.free();
+    A1 = B2 = X1 = X2 = {};
+    part = {};
   }
 };
 
