@@ -25,8 +25,8 @@
 // accumulator per class; classes 0 to 3 are exact in FP32 (at most 4 products of
 // 2^16 over 64 real terms), classes 4 to 6 have weight 2^-36 and less, class 7 is
 // dropped (2^-61).  The drain sums the classes without error into three FP32
-// numbers.  Measured against 64-bit references the error is below the FP64
-// FMA kernels'.  Their rate is the FP64 pipe's (2 FMA per cycle and SM); one
+// numbers.  Against extended precision the error of P0 and Sigma is 0.7 to
+// 1.8e-16, the FMA kernels' 1.7 to 5.2e-16.  Their rate is the FP64 pipe's (2 FMA per cycle and SM); one
 // complex output of K = 32 takes 64 cycles there and about 3 here.  Complex products use
 // the real embedding A = [Ar Ai] (K interleaved), B rows (n, 0) = [Br -Bi],
 // (n, 1) = [Bi Br], so D[r][(n,0)] = Re, D[r][(n,1)] = Im of sum_k A[r][k] B[n][k].
