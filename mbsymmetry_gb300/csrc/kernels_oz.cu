@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
   __shared__ __align__(8) uint64_t full[SETS][OZ_RING], emptyA[SETS][OZ_RING], emptyB[SETS][OZ_RING], fullB[2],
       done[SETS], tfree[SETS], doneH, tfreeH, last;
   __shared__ __align__(16) float sA[SETS][OZ_SC][OZ_M], sB[SETS][OZ_SC][8 * OCT];
-  __shared__ float gmax[2][OCT][OZ_M];
+  __shared__ float gmax[2][OCT / HO][OZ_M];
   __shared__ int abort_flag;
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -699,25 +699,28 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
               ee[q] = OZ_ENONE;
             }
           }
-          if (gs > HO) {  // octets that share the exponent are in other warps of this lane quarter
-#pragma unroll
-            for (int q = 0; q < HO; ++q) gmax[tile & 1][os0 + q][row] = NS == 6 ? __int_as_float(ee[q]) : mx[q];
-            asm volatile("bar.sync %0, %1;" ::"r"(1 + lq), "n"(32 * OCT / HO) : "memory");
-#pragma unroll
-            for (int q = 0; q < HO; ++q) {
-              const int g0 = os0 + q - oct[q] % gs;
-              for (int k = 0; k < gs; ++k) {
-                const float o = gmax[tile & 1][min(g0 + k, OCT - 1)][row];
-                if constexpr (NS == 6) {
-                  ee[q] = max(ee[q], __float_as_int(o));
-                } else {
-                  mx[q] = fmaxf(mx[q], o);
-                }
+          // Octets that share an exponent: gs = 2 the pairs (0, 1) and (2, 3), gs > 2 all of them (octets past the
+          // third are then invalid and do not count).  Beyond a thread's own they are in the other warps of its
+          // lane quarter.
+          if constexpr (HO == 2) {
+            if (gs >= 2) {
+              mx[0] = fmaxf(mx[0], mx[1]);
+              if (gs > 2) {
+                gmax[tile & 1][os0 / HO][row] = mx[0];
+                asm volatile("bar.sync %0, %1;" ::"r"(1 + lq), "n"(32 * OCT / HO) : "memory");
+                mx[0] = fmaxf(mx[0], gmax[tile & 1][1 - os0 / HO][row]);
               }
+              mx[1] = mx[0];
             }
-          } else if (HO == 2 && gs == 2) {
-            mx[0] = mx[HO - 1] = fmaxf(mx[0], mx[HO - 1]);
-            ee[0] = ee[HO - 1] = max(ee[0], ee[HO - 1]);
+          } else if (gs > 1) {
+            gmax[tile & 1][os0][row] = __int_as_float(ee[0]);
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + lq), "n"(32 * OCT / HO) : "memory");
+            if (gs == 2) {
+              ee[0] = max(ee[0], __float_as_int(gmax[tile & 1][os0 ^ 1][row]));
+            } else {
+#pragma unroll
+              for (int k = 0; k < OCT; ++k) ee[0] = max(ee[0], __float_as_int(gmax[tile & 1][k][row]));
+            }
           }
           if constexpr (STAGE == 1) {  // rows L of one K round share the exponent of their (tau, x)
             for (int dlt = 1; dlt < (1 << glog); dlt <<= 1) {
