@@ -342,8 +342,8 @@ __device__ __forceinline__ void oz_mmas(uint32_t d0, uint32_t a0, uint32_t b0, u
 }
 
 // Persistent warp-specialised GEMM over operand images.  Bound, three slices: HBM in
-// stages 2 and 3 (hexagonal 8 k, Sigma: 6.0 and 5.6 TB/s of 6.8), the drains in stage 1
-// (2800 cycles per accumulator set, its MMAs 880); six slices: the drains' FP32 work, in
+// stages 2 and 3 (hexagonal 8 k, Sigma: 6.1 and 5.6 TB/s of 6.8), the drains in stage 1
+// (2500 cycles per accumulator set, its MMAs 880); six slices: the drains' FP32 work, in
 // stage 3 about as long as the MMAs.  The operands need no CUDA-core work at all, a K step
 // (8 complex) is 8 or 26 MMAs, and the two accumulator sets of three slices let
 // one round multiply while the other drains.  Operands stream through rings of
