@@ -47,7 +47,8 @@ WORKLOADS = {
 WORKLOAD = WORKLOADS[CONFIG]
 METRIC = "s/GW iteration + tensor TFLOP/s: mixed vs FP64 GPU at Sigma err<=1e-7 Ha; CPU ref"
 # dram__bytes_read.sum + dram__bytes_write.sum summed over one iteration's launches of
-# each sliced-path GEMM kernel on C2, from one ncu capture of `bench.py --profile`.
+# each sliced-path GEMM kernel on C2 (none recorded for the present kernels; by stage on
+# hexagonal crystals: profiles/sliced_gemm_stages.md).
 OZ_TRAFFIC = {}
 L2_BYTES = 129 * 1024 * 1024
 
