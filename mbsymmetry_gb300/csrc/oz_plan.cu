@@ -625,10 +625,13 @@ void OzTransform::build(const std::vector<TSlab> &slabs, int nout, int nin, int 
   s3_.upload(s3, st);
   rnd_.upload(rnd, st);
   T_.alloc((size_t)tb);
+  scale_.alloc(2 * (size_t)nin);
   GWGB_CUDA(cudaStreamSynchronize(st));
 }
 
+// In place: a captured graph holds the addresses of T_ and scale_.
 void OzTransform::set_matrix(const double *T_host, const double2 *T, cudaStream_t st) {
+  ready = false;
   std::vector<double> scale(2 * (size_t)nin_, 1.0);
   for (int i = 0; i < nin_; ++i) {
     double m = 0.0;
@@ -642,7 +645,7 @@ void OzTransform::set_matrix(const double *T_host, const double2 *T, cudaStream_
     scale[i] = std::ldexp(1.0, e);
     scale[nin_ + i] = std::ldexp(1.0, -e);
   }
-  scale_.upload(scale, st);
+  GWGB_CUDA(cudaMemcpyAsync(scale_.p, scale.data(), scale.size() * sizeof(double), cudaMemcpyHostToDevice, st));
   launch_oz_build(6, builds_.p + nbuild_, nT_, T, T_.p, st, scale_.p);
   GWGB_CUDA(cudaStreamSynchronize(st));
   ready = true;

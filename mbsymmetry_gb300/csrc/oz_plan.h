@@ -91,7 +91,7 @@ class OzTransform {
   int64_t bytes_A() const { return a_; }
   bool built() const { return gemm_.n > 0; }
   bool ready = false;           // the matrix has been set
-  // T: host and device copies, [nout][nin]
+  // T: host and device copies, [nout][nin]; may be set again, the buffers stay where they are
   void set_matrix(const double *T_host, const double2 *T, cudaStream_t st);
   // A: bytes_A() bytes of scratch
   void run(const double2 *X, double2 *Y, char *A, int nsm, int *err, cudaStream_t st) const;
