@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
   __shared__ __align__(8) uint64_t full[SETS][OZ_RING], emptyA[SETS][OZ_RING], emptyB[SETS][OZ_RING], fullB[2],
       done[SETS], tfree[SETS], doneH, tfreeH, last;
   __shared__ __align__(16) float sA[SETS][OZ_SC][OZ_M], sB[SETS][OZ_SC][8 * OCT];
-  __shared__ float gmax[2][OCT / HO][OZ_M];
+  __shared__ float gmax[2][OCT / HO][OZ_M];  // exchange n of a warp in gmax[n & 1]
   __shared__ int abort_flag;
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
     // The rows' destinations are read while the set still multiplies.
     const int lq = warp & 3, os0 = HO * (warp >> 2), row = 32 * lq + lane;
     const uint32_t tbase = tm + ((uint32_t)(32 * lq) << 16) + 16u * os0;
-    int n = 0, tile = 0, i0[SETS] = {}, j0[SETS] = {};  // fills, tiles; row tiles and column images by set
+    int n = 0, xch = 0, i0[SETS] = {}, j0[SETS] = {};  // fills, exchanges; row tiles and column images by set
     bool dead = false;
     OzTask tk1{};
     if (blockIdx.x < (unsigned)g.ntasks) tk1 = g.tasks[blockIdx.x];
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
           nv[q] = d.N - 8 * ((tk.i >> 16) * d.oct + oct[q]);
         }
       }
-      for (int m0 = 0; m0 < job.outer; m0 += job.G, ++tile) {
+      for (int m0 = 0; m0 < job.outer; m0 += job.G) {
         const int Gm = min(job.G, job.outer - m0);
         if constexpr (STAGE == 1) {  // used after the wait for the accumulators
 #pragma unroll
@@ -701,26 +701,31 @@ __global__ void __launch_bounds__(oz_threads<NS>, 1) oz_gemm_kernel(const OzArgs
           }
           // Octets that share an exponent: gs = 2 the pairs (0, 1) and (2, 3), gs > 2 all of them (octets past the
           // third are then invalid and do not count).  Beyond a thread's own they are in the other warps of its
-          // lane quarter.
+          // lane quarter: gmax, one barrier per exchange.  The buffers alternate by exchange (gs is the same in these
+          // warps), not by tile: a warp writes buffer n & 1 again in exchange n + 2, after the barrier of n + 1, which
+          // every warp reaches only when it has read exchange n.  By tile, one without an exchange in between left
+          // nothing to order the two (the warps of a quarter may be two fills of the accumulators apart).
           if constexpr (HO == 2) {
             if (gs >= 2) {
               mx[0] = fmaxf(mx[0], mx[1]);
               if (gs > 2) {
-                gmax[tile & 1][os0 / HO][row] = mx[0];
+                gmax[xch & 1][os0 / HO][row] = mx[0];
                 asm volatile("bar.sync %0, %1;" ::"r"(1 + lq), "n"(32 * OCT / HO) : "memory");
-                mx[0] = fmaxf(mx[0], gmax[tile & 1][1 - os0 / HO][row]);
+                mx[0] = fmaxf(mx[0], gmax[xch & 1][1 - os0 / HO][row]);
+                ++xch;
               }
               mx[1] = mx[0];
             }
           } else if (gs > 1) {
-            gmax[tile & 1][os0][row] = __int_as_float(ee[0]);
+            gmax[xch & 1][os0][row] = __int_as_float(ee[0]);
             asm volatile("bar.sync %0, %1;" ::"r"(1 + lq), "n"(32 * OCT / HO) : "memory");
             if (gs == 2) {
-              ee[0] = max(ee[0], __float_as_int(gmax[tile & 1][os0 ^ 1][row]));
+              ee[0] = max(ee[0], __float_as_int(gmax[xch & 1][os0 ^ 1][row]));
             } else {
 #pragma unroll
-              for (int k = 0; k < OCT; ++k) ee[0] = max(ee[0], __float_as_int(gmax[tile & 1][k][row]));
+              for (int k = 0; k < OCT; ++k) ee[0] = max(ee[0], __float_as_int(gmax[xch & 1][k][row]));
             }
+            ++xch;
           }
           if constexpr (STAGE == 1) {  // rows L of one K round share the exponent of their (tau, x)
             for (int dlt = 1; dlt < (1 << glog); dlt <<= 1) {
