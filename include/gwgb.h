@@ -359,6 +359,11 @@ int gwgb_test_raise_status(gwgb_handle h, int32_t which);
  * the wait did not run out. */
 int gwgb_test_wait_timeout(int32_t device, int32_t polls);
 
+/* Test hook: of the calling thread's device allocations, counted from now on,
+ * number `first` (from 1) and the following ones fail with GWGB_E_NOMEM,
+ * `count` in all; count 0 switches it off.  No GPU call is made. */
+int gwgb_test_fail_alloc(int32_t first, int32_t count);
+
 /* ---- W~ solve without device allocation -------------------------------
  * No counterpart in the reference.  For callers that cannot allocate device
  * memory while they run (a host code whose own pool owns all of HBM, a plugin

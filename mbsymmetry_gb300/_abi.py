@@ -133,6 +133,7 @@ SIGNATURES = {
                                POINTER(GwgbScRecord)]),
     "gwgb_test_raise_status": (c_int32, [c_void_p, c_int32]),
     "gwgb_test_wait_timeout": (c_int32, [c_int32, c_int32]),
+    "gwgb_test_fail_alloc": (c_int32, [c_int32, c_int32]),
     "gwgb_wsolve_noalloc": (c_int32, [c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32,
                                       c_void_p, c_int32, c_void_p]),
 }

@@ -11,6 +11,11 @@ namespace gwgb {
 
 // Device bytes held by the buffers of every live handle in this process.
 extern std::atomic<int64_t> g_device_bytes;
+// Test hook (gwgb_test_fail_alloc): this thread's device allocations first, first + 1, ... fail, `count` of them.
+struct FailAlloc {
+  int32_t first = 0, count = 0;
+};
+extern thread_local FailAlloc g_fail_alloc;
 
 template <typename T>
 struct DBuf {
@@ -18,7 +23,17 @@ struct DBuf {
   size_t n = 0;
   void alloc(size_t count) {
     free();
-    if (count) GWGB_CUDA(cudaMalloc(&p, count * sizeof(T)));
+    if (!count) return;
+    if (FailAlloc &f = g_fail_alloc; f.count > 0 && --f.first <= 0) {
+      --f.count;
+      throw Error(GWGB_E_NOMEM, "device allocation failed (test hook)");
+    }
+    const cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+    if (e != cudaSuccess) {
+      p = nullptr;
+      cudaGetLastError();  // or the next kernel launch would report it
+    }
+    GWGB_CUDA(e);
     n = count;
     g_device_bytes += (int64_t)(n * sizeof(T));
   }

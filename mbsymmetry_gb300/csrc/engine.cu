@@ -189,6 +189,7 @@ static Lay derive_layout(const gwgb_layout &L) {
 }
 
 std::atomic<int64_t> g_device_bytes{0};
+thread_local FailAlloc g_fail_alloc;
 
 // An output block of a contraction and the contributions it sums.
 struct Owner {
@@ -426,6 +427,7 @@ class Engine {
   OzSet oz_[2];
   OzShared oz_buf_;
   void build_oz();
+  void plan_oz(OzSet &set);
   bool alloc_oz(OzSet &set);
   OzSet *oz_set() {  // the set that runs the contractions, if one does
     OzSet *o = prec_ == GWGB_PREC_OZAKI ? &oz_[0] : prec_ == GWGB_PREC_FP64 ? &oz_[1] : nullptr;
@@ -451,9 +453,11 @@ class Engine {
     lt_set_ = oz_set();
     lt_info_.clear();
     lt_free();
+    lt_n_p0_ = 0;
     lt_ran_p0_ = lt_ran_sig_ = false;
+    if (!lt_set_) return;
     for (int l = 0; l < 2; ++l) {
-      for (const OzLaunch &x : oz_set()->plan[l].launches()) {
+      for (const OzLaunch &x : lt_set_->plan[l].launches()) {
         gwgb_launch_stat g{};
         g.stage = x.stage;
         g.kernel = x.kind;
@@ -1481,12 +1485,16 @@ bool Engine::alloc_oz(OzSet &set) {
                  m(p.bytes_X2(), s.bytes_X2()), m(p.part_elems(), s.part_elems()));
   } catch (const Error &e) {
     oz_buf_.free();
-    for (OzSet &o : oz_) o.alloc = o.ready = false;  // the other set's buffers, too, are allocated again on its next use
+    for (OzSet &o : oz_) {  // the other set's buffers, too, are allocated again on its next use
+      o.alloc = o.ready = false;
+      o.plan[0].free_images();
+      o.plan[1].free_images();
+    }
     if (&set != &oz_[1] || e.code != GWGB_E_NOMEM) throw;
-    cudaGetLastError();
     set.off[0] = set.off[1] = true;
     set.plan[0].free();
     set.plan[1].free();
+    lt_build();
     return false;
   }
   set.alloc = true;
@@ -1510,14 +1518,36 @@ void Engine::build_xf(int which, const std::vector<TSlab> &slabs, int nout, int 
   xf_img_.alloc((size_t)xf_[which].bytes_A());
 }
 
+// The lists of the active precision's set, once.  FP64 needs none where they or their buffers do not fit:
+// it has the FMA kernels.
 void Engine::build_oz() {
   if (prec_ != GWGB_PREC_OZAKI && prec_ != GWGB_PREC_FP64) return;
   const bool f64 = prec_ == GWGB_PREC_FP64;
   OzSet &set = oz_[f64 ? 1 : 0];
-  if (set.built) {
-    if (lt_set_ != &set && oz_set()) lt_build();
-    return;
+  if (!set.built) {
+    auto none = [&] {
+      set.plan[0].free();
+      set.plan[1].free();
+      set.off[0] = set.off[1] = f64;
+    };
+    try {
+      plan_oz(set);
+    } catch (const Error &e) {
+      none();
+      if (!f64 || (e.code != GWGB_E_NOMEM && e.code != GWGB_E_UNSUPPORTED)) throw;
+    } catch (const std::bad_alloc &) {
+      none();
+      if (!f64) throw;
+    }
+    set.built = true;
+    set.ready = false;
   }
+  if (lt_set_ != oz_set()) lt_build();
+}
+
+// Plans of both contractions, their lists on the device; throws where they do not fit.
+void Engine::plan_oz(OzSet &set) {
+  const bool f64 = &set == &oz_[1];
   const int NS = f64 ? 6 : 3;
   const Lay &l = l_;
   const int ns = ns_, nts = nts_;
@@ -1591,10 +1621,7 @@ void Engine::build_oz() {
       set.off[k] = force ? force[0] == '0' : ops / 1.9e14 + 5e-5 > (k ? sig_flops_ : p0_flops_) / 1.2e12;
       if (set.off[k]) set.plan[k].free();
     }
-    if (set.off[0] && set.off[1]) {
-      set.built = true;
-      return;
-    }
+    if (set.off[0] && set.off[1]) return;
   }
   {  // the buffers (shared with the other set, if it is built) must fit the free memory
     const OzPlan &p = set.plan[0], &s = set.plan[1];
@@ -1616,22 +1643,12 @@ void Engine::build_oz() {
     }
     GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const bool fits = tot + (256ll << 20) + (V_.p ? 0 : 16 * l.flat_V) <= (int64_t)free_b;
-    set.built = true;
-    if (f64 && !fits) {  // the FMA kernels, which need no images
-      set.off[0] = set.off[1] = true;
-      set.plan[0].free();
-      set.plan[1].free();
-      return;
-    }
-    set.built = fits;
     GWGB_REQUIRE(fits, GWGB_E_UNSUPPORTED,
                  "sliced-precision buffers need " + std::to_string(tot >> 20) + " MB (" + msg + " ), " +
                      std::to_string(free_b >> 20) + " MB free");
     for (int k = 0; k < 2; ++k)
       if (!set.off[k]) set.plan[k].upload(st_);
   }
-  set.ready = false;
-  lt_build();
 }
 
 // ---------------------------------------------------------------------------
@@ -2361,6 +2378,13 @@ int gwgb_test_wait_timeout(int32_t device, int32_t polls) {
     return GWGB_E_TIMEOUT;
   }
   return GWGB_OK;
+}
+
+int gwgb_test_fail_alloc(int32_t first, int32_t count) {
+  return guarded([&] {
+    GWGB_REQUIRE(first >= 1 && count >= 0, GWGB_E_INVALID, "first must be positive and count not negative");
+    gwgb::g_fail_alloc = {first, count};
+  });
 }
 
 GWGB_FORWARD(gwgb_set_hcore, (gwgb_handle h, const double *H), e.set_hcore(H))

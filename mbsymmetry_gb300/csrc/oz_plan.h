@@ -125,6 +125,7 @@ class OzPlan {
   int64_t bytes_X2() const { return x2_; }
   int64_t part_elems() const { return part_; }
   void alloc_images() { V_.alloc((size_t)vimg_); }
+  void free_images() { V_.free(); }
   // the operand images that do not change between iterations (after a V / rotation upload)
   void build_static(const double2 *V, cudaStream_t st);
   void run_one(const OzLaunch &l, OzShared &sh, const double2 *V, const double2 *G, const double2 *B2, double2 *out,

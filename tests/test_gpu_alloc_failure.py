@@ -1,0 +1,97 @@
+"""Device allocations that fail (injected on the host): lists, operand images and
+work buffers of the sliced contractions.  FP64, which has kernels that need none
+of them, still answers; the split precision reports the failure or answers, and the
+same handle answers once memory is there again."""
+import numpy as np
+import pytest
+
+from _helpers import crystal
+from mbsymmetry_gb300 import _abi
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def fail_alloc():
+    lib = _abi.load()
+    yield lambda first, count: _abi.check(lib.gwgb_test_fail_alloc(first, count))
+    lib.gwgb_test_fail_alloc(1, 0)
+
+
+def _solver(precision):
+    from mbsymmetry_gb300.solver import GWSolver
+    cr, tr = crystal("C1")
+    return cr, tr, GWSolver(cr.layout, cr.ns, tr, precision=precision)
+
+
+def _inputs(cr, s):
+    s.set_shared_Coulomb(cr.V)
+    s.set_fock(cr.F, cr.S)
+
+
+def _solve(cr, s):
+    s.set_Selfenergy(np.zeros(s.g_size, np.complex128))
+    s.dyson(cr.mu)
+    s.solve()
+    return s.P0_q_t_QP(), s.Selfenergy()
+
+
+def _reference(precision):
+    cr, _, s = _solver(precision)
+    _inputs(cr, s)
+    out = _solve(cr, s)
+    s.close()
+    return out
+
+
+@pytest.mark.parametrize("first,count", [(n, 1) for n in range(1, 7)] + [(1, 1000), (3, 1000), (5, 1000)])
+def test_fp64_answers_without_the_buffers(first, count, fail_alloc, monkeypatch):
+    monkeypatch.setenv("GWGB_FP64_SLICES", "1")
+    ref = _reference("fp64")
+    cr, _, s = _solver("fp64")
+    fail_alloc(first, count)
+    _inputs(cr, s)
+    got = _solve(cr, s)
+    again = _solve(cr, s)
+    fail_alloc(1, 0)
+    s.close()
+    for a, b, c in zip(ref, got, again):
+        assert np.abs(a - b).max() < 1e-12 * np.abs(a).max()
+        assert np.array_equal(b, c)
+
+
+@pytest.mark.parametrize("first,count", [(n, 1) for n in range(1, 4)] + [(1, 1000), (3, 1000)])
+def test_split_precision_recovers(first, count, fail_alloc):
+    ref = _reference("ozaki")
+    cr, _, s = _solver("ozaki")
+    _inputs(cr, s)
+    fail_alloc(first, count)
+    try:
+        got = _solve(cr, s)
+    except _abi.GwgbError as e:
+        assert e.code in (_abi.GWGB_E_NOMEM, _abi.GWGB_E_UNSUPPORTED)
+        got = None
+    assert got is None or count == 1
+    fail_alloc(1, 0)
+    for out in (got, _solve(cr, s)):
+        assert out is None or all(np.array_equal(a, b) for a, b in zip(ref, out))
+    s.close()
+
+
+def test_split_precision_lists_fail(fail_alloc):
+    """Switching the precision fails with the lists; switching it again works."""
+    ref = _reference("ozaki")
+    cr, _, s = _solver("fp64")
+    _inputs(cr, s)
+    fail_alloc(2, 1000)
+    try:
+        s.single_prec_run(True)
+        with pytest.raises(_abi.GwgbError) as e:
+            _solve(cr, s)
+        assert e.value.code in (_abi.GWGB_E_NOMEM, _abi.GWGB_E_UNSUPPORTED)
+    except _abi.GwgbError as e:
+        assert e.code in (_abi.GWGB_E_NOMEM, _abi.GWGB_E_UNSUPPORTED)
+    fail_alloc(1, 0)
+    s.single_prec_run(True)
+    assert all(np.array_equal(a, b) for a, b in zip(ref, _solve(cr, s)))
+    s.close()
