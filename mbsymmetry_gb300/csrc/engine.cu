@@ -389,7 +389,14 @@ class Engine {
       built = true;
     }
     build_oz();
-    if (OzSet *o = oz_set(); o && alloc_oz(*o) && !o->ready) {
+    for (OzSet *o; (o = oz_set()) && !alloc_oz(*o);) {  // less memory than cudaMemGetInfo said: the next level
+      o->plan[0].free();
+      o->plan[1].free();
+      o->built = false;
+      ++o->level;
+      build_oz();
+    }
+    if (OzSet *o = oz_set(); o && !o->ready) {
       if (!o->off[0]) o->plan[0].build_static(V_.p, st_);
       if (!o->off[1]) o->plan[1].build_static(Vt_.p, st_);
       o->ready = true;
@@ -423,6 +430,7 @@ class Engine {
   struct OzSet {
     OzPlan plan[2];
     bool built = false, alloc = false, ready = false, off[2] = {false, false};
+    int level = 0;  // of memory: 0 what is fastest, each further one a quarter of the chunks
   };
   OzSet oz_[2];
   OzShared oz_buf_;
@@ -1472,7 +1480,7 @@ void Engine::build_work_lists() {
 // sliced (Ozaki) path: the two contractions as chains of block GEMMs (oz_plan.h)
 // ---------------------------------------------------------------------------
 // The images and work buffers of the active set, on its first use (a handle that only solves
-// Dyson or W~ never needs them).  False: no memory (FP64 falls back to the FMA kernels).
+// Dyson or W~ never needs them).  False: no memory.
 bool Engine::alloc_oz(OzSet &set) {
   if (set.alloc) return true;
   const OzPlan &p = set.plan[0], &s = set.plan[1];
@@ -1490,11 +1498,7 @@ bool Engine::alloc_oz(OzSet &set) {
       o.plan[0].free_images();
       o.plan[1].free_images();
     }
-    if (&set != &oz_[1] || e.code != GWGB_E_NOMEM) throw;
-    set.off[0] = set.off[1] = true;
-    set.plan[0].free();
-    set.plan[1].free();
-    lt_build();
+    if (e.code != GWGB_E_NOMEM) throw;
     return false;
   }
   set.alloc = true;
@@ -1518,31 +1522,35 @@ void Engine::build_xf(int which, const std::vector<TSlab> &slabs, int nout, int 
   xf_img_.alloc((size_t)xf_[which].bytes_A());
 }
 
-// The lists of the active precision's set, once.  FP64 needs none where they or their buffers do not fit:
-// it has the FMA kernels.
+// The lists of the active precision's set, once, at the first memory level whose buffers fit.  FP64 needs none where
+// no level fits: it has the FMA kernels.
 void Engine::build_oz() {
   if (prec_ != GWGB_PREC_OZAKI && prec_ != GWGB_PREC_FP64) return;
   const bool f64 = prec_ == GWGB_PREC_FP64;
   OzSet &set = oz_[f64 ? 1 : 0];
-  if (!set.built) {
-    auto none = [&] {
+  constexpr int LEVELS = 8;
+  const bool fresh = !set.built;
+  while (!set.built) {
+    auto next = [&](bool memory) {  // true: try again with less
       set.plan[0].free();
       set.plan[1].free();
-      set.off[0] = set.off[1] = f64;
+      if (memory && ++set.level < LEVELS) return true;
+      set.level = 0;
+      if (f64 && memory) set.off[0] = set.off[1] = set.built = true;
+      return f64 && memory;
     };
     try {
+      GWGB_REQUIRE(set.level < LEVELS, GWGB_E_NOMEM, "no device memory for the sliced-precision buffers");
       plan_oz(set);
+      set.built = true;
     } catch (const Error &e) {
-      none();
-      if (!f64 || (e.code != GWGB_E_NOMEM && e.code != GWGB_E_UNSUPPORTED)) throw;
+      if (!next(e.code == GWGB_E_NOMEM || e.code == GWGB_E_UNSUPPORTED)) throw;
     } catch (const std::bad_alloc &) {
-      none();
-      if (!f64) throw;
+      if (!next(true)) throw;
     }
-    set.built = true;
     set.ready = false;
   }
-  if (lt_set_ != oz_set()) lt_build();
+  if (fresh || lt_set_ != oz_set()) lt_build();
 }
 
 // Plans of both contractions, their lists on the device; throws where they do not fit.
@@ -1553,14 +1561,17 @@ void Engine::plan_oz(OzSet &set) {
   const int ns = ns_, nts = nts_;
   std::vector<OzContrib> cs;
   std::vector<OzOwner> own;
-  // memory free for the images of V that do not change between iterations (V itself may not be allocated yet)
+  // Memory free now (V itself may not be allocated yet).  At most a quarter of it holds the images of V that do not
+  // change between iterations, an eighth the intermediates of one chunk: large chunks mean fewer, fuller launches
+  // (hexagonal 8 k, the stages of both contractions in three slices: 1 GB 47.5 ms, 8 GB 37.2, 16 GB 36.6).  Where
+  // that does not fit: no images of V kept, the chunks and the images of G and P~ (by ranges of tau) a quarter, ...
   size_t free_b = 0, total_b = 0;
   GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
   const int64_t avail = (int64_t)free_b - (V_.p ? 0 : 16 * l.flat_V);
-  const int64_t persist = std::max<int64_t>(0, avail / 4);
-  // intermediates of one chunk: large chunks mean fewer, fuller launches (hexagonal 8 k, the stages of both
-  // contractions in three slices: 1 GB 47.5 ms, 8 GB 37.2, 16 GB 36.6)
-  const int64_t budget = tc_chunk_env_ ? tc_chunk_bytes_ : std::min<int64_t>(OZ_CHUNK_BYTES, std::max<int64_t>(64ll << 20, avail / 8));
+  const int64_t persist = set.level ? 0 : std::max<int64_t>(0, avail / 4);
+  const int64_t chunk = tc_chunk_env_ ? tc_chunk_bytes_ : std::min<int64_t>(OZ_CHUNK_BYTES, std::max<int64_t>(64ll << 20, avail / 8));
+  const int64_t budget = set.level ? std::max<int64_t>(1ll << 20, chunk >> (2 * set.level)) : chunk;
+  const int64_t taus = set.level ? budget : INT64_MAX;
   // P0[Q][P] = sum V[Q][p][m] G1(beta - tau)[t][p] conj(V[P][t][n]) G2(tau)[m][n]
   for (const P0Group &g : p0_groups_) {
     const int c0 = (int)cs.size();
@@ -1581,9 +1592,11 @@ void Engine::plan_oz(OzSet &set) {
     own.push_back({g.pout, g.pstride, g.qb, g.qb, g.qb, 1, c0, (int32_t)cs.size()});
   }
   // the lists of the two contractions are built side by side
-  auto p0_built = std::async(std::launch::async, [&set, cs, own, NS, nts, budget, persist, this] {
-    set.plan[0].build(NS, cs, own, nts / 2, 0, budget, persist / 2, nsm_, l_.flat_V, (int64_t)Gall_.n, (int64_t)Gall_.n,
-                      (int64_t)Pall_.n);
+  const bool first = set.level == 0;  // which contractions run in slices is decided there
+  auto p0_built = std::async(std::launch::async, [&set, cs, own, NS, nts, budget, persist, taus, first, this] {
+    if (first || !set.off[0])
+      set.plan[0].build(NS, cs, own, nts / 2, 0, budget, persist / 2, taus, nsm_, l_.flat_V, (int64_t)Gall_.n,
+                        (int64_t)Gall_.n, (int64_t)Pall_.n);
   });
   // Sigma[i][j] = sum Vt[Q][i][m] G2(tau)[m][n] P~(tau)[Q][P] conj(Vt[P][j][n])
   cs.clear();
@@ -1605,10 +1618,11 @@ void Engine::plan_oz(OzSet &set) {
     }
     own.push_back({ow.out, ow.ostride, ow.n, ow.n, 1, ow.n, c0, (int32_t)cs.size()});
   }
-  set.plan[1].build(NS, cs, own, nts, 3, budget, persist / 2, nsm_, (int64_t)Vt_.n, (int64_t)Gall_.n, (int64_t)Pall_.n,
-                    (int64_t)nts * ns * l.flat_ao);
+  if (first || !set.off[1])
+    set.plan[1].build(NS, cs, own, nts, 3, budget, persist / 2, taus, nsm_, (int64_t)Vt_.n, (int64_t)Gall_.n,
+                      (int64_t)Pall_.n, (int64_t)nts * ns * l.flat_ao);
   p0_built.get();
-  if (f64) {
+  if (f64 && first) {
     // Six slices against the FMA kernels, one contraction at a time: the MMAs (padded to octets of columns and 128 rows)
     // run at 190 TFLOP/s and more including their drains, the launches around them take about 0.05 ms; the FMA
     // kernels run at 1.2 TFLOP/s.  s+p (AO blocks 1-4): P0 0.45 ms against 0.40, Sigma 0.44 against 0.70; s+p+d
@@ -1623,7 +1637,7 @@ void Engine::plan_oz(OzSet &set) {
     }
     if (set.off[0] && set.off[1]) return;
   }
-  {  // the buffers (shared with the other set, if it is built) must fit the free memory
+  {  // the lists and the buffers (shared with the other set, if it is built) must fit the free memory
     const OzPlan &p = set.plan[0], &s = set.plan[1];
     auto grow = [](int64_t a, int64_t b, size_t have) {
       const int64_t m = std::max(a, b);
@@ -1632,7 +1646,8 @@ void Engine::plan_oz(OzSet &set) {
     const int64_t a1 = grow(p.bytes_A1(), s.bytes_A1(), oz_buf_.A1.n), b2 = grow(p.bytes_B2(), s.bytes_B2(), oz_buf_.B2.n),
                   x1 = grow(p.bytes_X1(), s.bytes_X1(), oz_buf_.X1.n), x2 = grow(p.bytes_X2(), s.bytes_X2(), oz_buf_.X2.n),
                   part = grow(p.part_elems(), s.part_elems(), oz_buf_.part.n);
-    const std::pair<const char *, int64_t> need[] = {{"V images", p.bytes_V() + s.bytes_V()}, {"G images", a1},
+    const std::pair<const char *, int64_t> need[] = {{"lists", p.bytes_lists() + s.bytes_lists()},
+                                                     {"V images", p.bytes_V() + s.bytes_V()}, {"G images", a1},
                                                      {"stage-2 operands", b2}, {"X1", x1}, {"X2", x2},
                                                      {"partials", 16 * part}};
     int64_t tot = 0;
@@ -1641,11 +1656,9 @@ void Engine::plan_oz(OzSet &set) {
       tot += x.second;
       msg += std::string(" ") + x.first + " " + std::to_string(x.second >> 20) + " MB";
     }
-    GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const bool fits = tot + (256ll << 20) + (V_.p ? 0 : 16 * l.flat_V) <= (int64_t)free_b;
-    GWGB_REQUIRE(fits, GWGB_E_UNSUPPORTED,
+    GWGB_REQUIRE(tot + std::min<int64_t>(256ll << 20, avail / 8) <= avail, GWGB_E_UNSUPPORTED,
                  "sliced-precision buffers need " + std::to_string(tot >> 20) + " MB (" + msg + " ), " +
-                     std::to_string(free_b >> 20) + " MB free");
+                     std::to_string(avail >> 20) + " MB free");
     for (int k = 0; k < 2; ++k)
       if (!set.off[k]) set.plan[k].upload(st_);
   }

@@ -6,7 +6,9 @@
 // stage 3, with an FP64 partial of its own; the partials are summed in order
 // at the end).  Units depend on the block alone, so no result bit depends on
 // the chunking.  Chunk: consecutive units whose intermediates X1 and X2 fit
-// the budget; each chunk is one launch per stage.
+// the budget; each chunk is one launch per stage.  Where the images of G and of
+// the stage-2 operand at every tau exceed their limit, the chunks are those of one
+// tau range after the other.
 #include "oz_plan.h"
 
 #include <algorithm>
@@ -42,7 +44,8 @@ int choose_glog(int zos, int nL, int oct) {
 }  // namespace
 
 void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<OzOwner> &own, int ntau, int stage0,
-                   int64_t budget, int64_t persist_bytes, int nsm, int64_t nV, int64_t nG, int64_t nB2, int64_t nout) {
+                   int64_t budget, int64_t persist_bytes, int64_t tau_bytes, int nsm, int64_t nV, int64_t nG, int64_t nB2,
+                   int64_t nout) {
   ns_ = ns;
   const int OCT = OZ_OCT, NS = ns;
   const int FK = 8 * OCT;  // complex K of a full round
@@ -82,44 +85,30 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
                 "sliced stage-2 operand");
   }
 
-  // --- images of G rows (tau, L) and of the stage-2 operand, for the whole contraction
-  std::map<int64_t, int> s1_of;
+  // --- distinct operands of stage 1 and of stage 2 (their first contribution), and the tau ranges
   struct B2 { int64_t b, bt, bz; };
-  std::map<std::pair<int64_t, int>, B2> b2_of;
-  const size_t ga0 = builds.size();
-  for (const OzContrib &c : cs) {
-    if (s1_of.count(c.ga)) continue;
-    const int kos = cdiv(c.K1, 8), R = cdiv(kos, OCT), M = ntau * c.nL;
-    s1_of[c.ga] = (int)s1.size();
-    s1.push_back({a1_, M, c.nL, kos, 0});
-    for (int mt = 0; mt * OZ_M < M; ++mt)
-      for (int r = 0; r < R; ++r) {
-        const int nks = std::min(OCT, kos - r * OCT);
-        builds.push_back({c.ga + (int64_t)r * FK * c.gk, a1_, c.gt, 0, c.gL, c.gk, c.nL, 1 << 20, c.nL,
-                          c.K1 - r * FK, ntau, 1, mt * OZ_M, OZ_M, (int16_t)nks, 0, 0, 0, -1, 0});
-        a1_ += oz_abytes(NS, nks);
-      }
+  std::map<int64_t, int> s1_of;                       // G block -> OzS1 of the tau range
+  std::map<std::pair<int64_t, int>, B2> b2_of;        // (block, conj) -> images of the tau range
+  std::vector<int> s1_first, b2_first;
+  for (size_t c = 0; c < cs.size(); ++c) {
+    if (s1_of.emplace(cs[c].ga, 0).second) s1_first.push_back((int)c);
+    if (b2_of.emplace(std::make_pair(cs[c].b2, (int)cs[c].b2conj), B2{}).second) b2_first.push_back((int)c);
   }
-  const size_t gb0 = builds.size();
-  for (const OzContrib &c : cs) {
-    const auto key = std::make_pair(c.b2, (int)c.b2conj);
-    if (b2_of.count(key)) continue;
-    const int kos = cdiv(c.ny, 8), R = cdiv(kos, OCT), zos = cdiv(c.nz, 8);
-    const int64_t per = (int64_t)NS * kos * 512 + 32 * R;
-    b2_of[key] = {b2_, zos * per, OCT * per};
-    for (int t = 0; t < ntau; ++t)
-      for (int z0 = 0; z0 < zos; z0 += OCT) {
-        const int noct = std::min(OCT, zos - z0);
-        for (int r = 0; r < R; ++r) {
-          const int nks = std::min(OCT, kos - r * OCT);
-          builds.push_back({c.b2 + t * c.b2t + (int64_t)z0 * 8 * c.b2z + (int64_t)r * FK * c.b2y, b2_, 0, 0, c.b2z,
-                            c.b2y, 1 << 20, 1 << 20, c.nz - 8 * z0, c.ny - r * FK, 1, 1, 0, (int16_t)(8 * noct),
-                            (int16_t)nks, 1, c.b2conj, 0, -1, 0});
-          b2_ += noct * oz_bbytes1(NS, nks);
-        }
-      }
-  }
-  const size_t gv0 = builds.size();
+  auto b2_bytes = [&](const OzContrib &c) {  // of one tau and octet of columns
+    const int kos = cdiv(c.ny, 8);
+    return (int64_t)NS * kos * 512 + 32 * cdiv(kos, OCT);
+  };
+  auto image_bytes = [&](int nt) {
+    int64_t n = 0;
+    for (int i : s1_first) {
+      const int kos = cdiv(cs[i].K1, 8);
+      n += cdiv((int64_t)nt * cs[i].nL, OZ_M) * ((int64_t)NS * kos * 4096 + 512 * cdiv(kos, OCT));
+    }
+    for (int i : b2_first) n += (int64_t)nt * cdiv(cs[i].nz, 8) * b2_bytes(cs[i]);
+    return n;
+  };
+  int ntr = ntau;  // tau of a range
+  while (ntr > 1 && image_bytes(ntr) > tau_bytes) ntr = (ntr + 1) / 2;
   auto add_build = [&](std::vector<OzLaunch> &v, size_t lo, size_t hi, int src, int dst, int stage) {
     if (lo == hi) return;
     OzLaunch l;
@@ -135,8 +124,46 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
     }
     v.push_back(l);
   };
-  add_build(launches_, ga0, gb0, 1, IMG_A1, stage0);
-  add_build(launches_, gb0, gv0, 2, IMG_B2, stage0 + 1);
+  // images of G rows (tau, L) and of the stage-2 operand, tau in [t0, t0 + nt)
+  auto add_images = [&](int t0, int nt) {
+    const size_t ga0 = builds.size();
+    int64_t a1 = 0, b2 = 0;
+    for (int i : s1_first) {
+      const OzContrib &c = cs[i];
+      const int kos = cdiv(c.K1, 8), R = cdiv(kos, OCT), M = nt * c.nL;
+      s1_of[c.ga] = (int)s1.size();
+      s1.push_back({a1, M, c.nL, kos, 0});
+      for (int mt = 0; mt * OZ_M < M; ++mt)
+        for (int r = 0; r < R; ++r) {
+          const int nks = std::min(OCT, kos - r * OCT);
+          builds.push_back({c.ga + t0 * c.gt + (int64_t)r * FK * c.gk, a1, c.gt, 0, c.gL, c.gk, c.nL, 1 << 20, c.nL,
+                            c.K1 - r * FK, nt, 1, mt * OZ_M, OZ_M, (int16_t)nks, 0, 0, 0, -1, 0});
+          a1 += oz_abytes(NS, nks);
+        }
+    }
+    const size_t gb0 = builds.size();
+    for (int i : b2_first) {
+      const OzContrib &c = cs[i];
+      const int kos = cdiv(c.ny, 8), R = cdiv(kos, OCT), zos = cdiv(c.nz, 8);
+      const int64_t per = b2_bytes(c);
+      b2_of[std::make_pair(c.b2, (int)c.b2conj)] = {b2, zos * per, OCT * per};
+      for (int t = t0; t < t0 + nt; ++t)
+        for (int z0 = 0; z0 < zos; z0 += OCT) {
+          const int noct = std::min(OCT, zos - z0);
+          for (int r = 0; r < R; ++r) {
+            const int nks = std::min(OCT, kos - r * OCT);
+            builds.push_back({c.b2 + t * c.b2t + (int64_t)z0 * 8 * c.b2z + (int64_t)r * FK * c.b2y, b2, 0, 0, c.b2z,
+                              c.b2y, 1 << 20, 1 << 20, c.nz - 8 * z0, c.ny - r * FK, 1, 1, 0, (int16_t)(8 * noct),
+                              (int16_t)nks, 1, c.b2conj, 0, -1, 0});
+            b2 += noct * oz_bbytes1(NS, nks);
+          }
+        }
+    }
+    a1_ = std::max(a1_, a1);
+    b2_ = std::max(b2_, b2);
+    add_build(launches_, ga0, gb0, 1, IMG_A1, stage0);
+    add_build(launches_, gb0, builds.size(), 2, IMG_B2, stage0 + 1);
+  };
 
   // --- units
   struct Unit { int own, c0, c1, idx, nunits; int64_t bytes; };
@@ -148,7 +175,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
     const int yos = cdiv(x.ny, 8), zos = cdiv(x.nz, 8), nLg = cdiv(x.nL, 1 << glog[c]);
     const int64_t r1 = (int64_t)x.nx * (nLg << glog[c]) * (NS * 32 * yos + 4 * cdiv(yos, OCT));
     const int64_t r2 = (int64_t)x.nx * (NS * 32 * (int64_t)x.nL * zos + 4 * rounds_of(c));
-    return ntau * (r1 + r2);
+    return ntr * (r1 + r2);
   };
   for (size_t o = 0; o < own.size(); ++o) {
     const OzOwner &ow = own[o];
@@ -202,7 +229,8 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
   struct V1 { size_t col0; std::vector<OzCol1> cols; };
   std::map<int, V1> v1_of;                                     // vid -> column tiles (dst filled per use)
   std::map<std::tuple<int, int, int>, std::pair<int64_t, std::vector<OzRnd>>> v3_of;  // (first vid, last vid, n) -> images
-  const int64_t PART_MAX = (int64_t)1 << 26;                   // FP64 partials held before a reduction (1 GB)
+  // FP64 partials held before a reduction: the chunk's budget, at most 1 GB
+  const int64_t PART_MAX = std::min<int64_t>((int64_t)1 << 26, budget / 16);
   int64_t part = 0, vbase = 0;
   size_t red0 = 0;
   auto flush_red = [&]() {
@@ -224,17 +252,21 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
     red0 = red.size();
     part = 0;
   };
-  for (size_t u0 = 0; u0 < units.size();) {
+  GWGB_REQUIRE(ntau < 65536, GWGB_E_UNSUPPORTED, "too many tau points");
+  size_t u0 = 0;  // the next chunk's first unit, in the tau range from t0 on
+  for (int t0 = 0; t0 < ntau && !units.empty();) {
+    const int nt = std::min(ntr, ntau - t0);
+    if (u0 == 0) add_images(t0, nt);
     size_t u1 = u0;
     int64_t tot = 0;
     while (u1 < units.size() && (u1 == u0 || tot + units[u1].bytes <= budget)) {
       if (u1 > u0 && units[u1].idx == 0 && part >= PART_MAX) break;
       tot += units[u1].bytes;
       const OzOwner &ow = own[units[u1].own];
-      part += (int64_t)ntau * ow.N * ow.nx;
+      part += (int64_t)nt * ow.N * ow.nx;
       ++u1;
     }
-    for (size_t u = u0; u < u1; ++u) part -= (int64_t)ntau * own[units[u].own].N * own[units[u].own].nx;
+    for (size_t u = u0; u < u1; ++u) part -= (int64_t)nt * own[units[u].own].N * own[units[u].own].nx;
     if (!persist) {
       v1_of.clear();
       v3_of.clear();
@@ -256,7 +288,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
     for (size_t u = u0; u < u1; ++u) {
       const Unit &un = units[u];
       const OzOwner &ow = own[un.own];
-      const int nf = cdiv((int64_t)ntau * ow.nx, OZ_M), nos = cdiv(ow.N, 8), nct = cdiv(nos, OCT);
+      const int nf = cdiv((int64_t)nt * ow.nx, OZ_M), nos = cdiv(ow.N, 8), nct = cdiv(nos, OCT);
       const auto vkey = std::make_tuple(cs[un.c0].vid, cs[un.c1 - 1].vid, un.c1 - un.c0);
       auto hit = v3_of.find(vkey);
       const bool fresh = hit == v3_of.end();
@@ -309,7 +341,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
         voff += (int64_t)nos * vb;
       }
       const int id = (int)s3.size();
-      s3.push_back({x2, fb, hit->second.first, bz, part, (int32_t)rnd.size(), (int32_t)rr.size(), ntau * ow.nx, ow.N,
+      s3.push_back({x2, fb, hit->second.first, bz, part, (int32_t)rnd.size(), (int32_t)rr.size(), nt * ow.nx, ow.N,
                     ow.nx, ow.N * ow.nx, ow.sn, ow.sx, OCT, 0});
       rnd.insert(rnd.end(), rr.begin(), rr.end());
       int64_t steps = 0;
@@ -326,7 +358,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
         uses.push_back({c, 0, p.slots, x2, fb, kbase[c - un.c0], lgb});
         p.cs.push_back((int)uses.size() - 1);
         p.slots += ((int64_t)x.nx * nLg * g + 3) / 4 * 4;
-        const double rowsx = (double)ntau * x.nx * x.nL;
+        const double rowsx = (double)nt * x.nx * x.nL;
         l1.flops += 8.0 * rowsx * x.ny * x.K1;
         l2.flops += 8.0 * rowsx * x.ny * x.nz;
         l3.flops += 8.0 * rowsx * x.nz * x.N;
@@ -334,8 +366,8 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
       for (const OzRnd &q : rr) l3.ops += nprod * 2.0 * OZ_M * 16.0 * nos * 16.0 * q.nks * nf;
       // partials
       if (un.idx == 0)
-        red.push_back({part, ow.out, ow.ostride, ow.N * ow.nx, 0, ntau, un.nunits, 0});
-      part += (int64_t)ntau * ow.N * ow.nx;
+        red.push_back({part, ow.out, ow.ostride, ow.N * ow.nx, t0, nt, un.nunits, 0});
+      part += (int64_t)nt * ow.N * ow.nx;
       part_ = std::max(part_, part);
       x2 += (int64_t)nf * fb;
     }
@@ -347,7 +379,7 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
     int64_t npk_tiles = 0;
     int64_t nrow = (int64_t)rows.size();
     for (auto &kv : packs) {
-      npk_tiles += (int64_t)ntau * cdiv(kv.second.slots, OZ_M);
+      npk_tiles += (int64_t)nt * cdiv(kv.second.slots, OZ_M);
       nrow += (int64_t)cdiv(kv.second.slots, OZ_M) * OZ_M;
     }
     if (nrow > (int64_t)rows.capacity()) rows.reserve(std::max<int64_t>(nrow, 2 * (int64_t)rows.capacity()));
@@ -383,12 +415,12 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
           for (int xx = 0; xx < x.nx; ++xx, ++row.pk) to[(int64_t)xx * step] = row;
         }
       }
-      x1 += (int64_t)ntau * nt2 * t2b;
+      x1 += (int64_t)nt * nt2 * t2b;
       m_kos2 = std::max(m_kos2, kos);
-      for (int t = 0; t < ntau; ++t)
+      for (int t = 0; t < nt; ++t)
         for (int zt = 0; zt < nzt; ++zt)
           for (int m = 0; m < nt2; m += per2) t2.push_back({id, t | zt << 16, m, std::min(per2, nt2 - m)});
-      l2.ops += nprod * 2.0 * OZ_M * 16.0 * zos * 16.0 * kos * nt2 * ntau;
+      l2.ops += nprod * 2.0 * OZ_M * 16.0 * zos * 16.0 * kos * nt2 * nt;
     }
     x1_ = std::max(x1_, x1);
     // stage 1: column tiles of every use
@@ -435,7 +467,6 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
         for (int m = 0; m < k.n; m += per1) t.push_back({k.d, k.i, m, std::min(per1, k.n - m)});
       t1.swap(t);
     }
-    GWGB_REQUIRE(ntau < 65536, GWGB_E_UNSUPPORTED, "too many tau points");
     vimg_ = std::max(vimg_, voff);
     add_build(persist ? static_ : launches_, bv0, builds.size(), 0, IMG_V, stage0);
     if (persist) vbase = voff;
@@ -485,10 +516,14 @@ void OzPlan::build(int ns, const std::vector<OzContrib> &cs, const std::vector<O
     const bool owner_end = u1 == units.size() || units[u1].idx == 0;
     if (u1 == units.size() || (owner_end && part >= PART_MAX)) flush_red();
     u0 = u1;
+    if (u0 == units.size()) {
+      u0 = 0;
+      t0 += ntr;
+    }
   }
   for (const RedTask &r : red) {
     check_range(r.part, (int64_t)r.nslice * r.nt * r.elems, std::max<int64_t>(1, part_), "sliced partials");
-    check_range(r.out, (int64_t)(r.nt - 1) * r.ostride + r.elems, nout, "sliced output block");
+    check_range(r.out, (int64_t)(r.t0 + r.nt - 1) * r.ostride + r.elems, nout, "sliced output block");
   }
   for (const OzBuild &b : builds)
     check_range(b.dst, b.isb ? (int64_t)(b.rows / 8) * oz_bbytes1(NS, b.nks) : oz_abytes(NS, b.nks),

@@ -113,11 +113,14 @@ class OzPlan {
  public:
   enum { IMG_V, IMG_A1, IMG_B2 };
   // stage0: gwgb_launch_stat.stage of stage 1; budget: bytes of X1 + X2 per chunk; persist_bytes: the
-  // V images are kept (built once per upload) when they take at most this, else built per chunk.
+  // V images are kept (built once per upload) when they take at most this, else built per chunk; tau_bytes: the images
+  // of G and of the stage-2 operand, for a range of tau if those of all take more.
   // Host side only (no CUDA calls); upload() then moves the lists to the device.
   void build(int ns, const std::vector<OzContrib> &cs, const std::vector<OzOwner> &own, int ntau, int stage0,
-             int64_t budget, int64_t persist_bytes, int nsm, int64_t nV, int64_t nG, int64_t nB2, int64_t nout);
+             int64_t budget, int64_t persist_bytes, int64_t tau_bytes, int nsm, int64_t nV, int64_t nG, int64_t nB2,
+             int64_t nout);
   void upload(cudaStream_t st);
+  int64_t bytes_lists() const { return (int64_t)host_.size(); }  // until upload()
   int64_t bytes_V() const { return vimg_; }
   int64_t bytes_A1() const { return a1_; }
   int64_t bytes_B2() const { return b2_; }

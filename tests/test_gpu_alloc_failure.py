@@ -95,3 +95,37 @@ def test_split_precision_lists_fail(fail_alloc):
     s.single_prec_run(True)
     assert all(np.array_equal(a, b) for a, b in zip(ref, _solve(cr, s)))
     s.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "ozaki"])
+@pytest.mark.parametrize("ns", [1, 2])
+def test_less_memory_means_smaller_chunks(precision, ns, fail_alloc, monkeypatch):
+    """An allocation that fails makes the engine plan again with smaller chunks, the
+    images of G and P~ by ranges of tau and none of V kept: more launches, the same bits."""
+    from mbsymmetry_gb300.solver import GWSolver
+    monkeypatch.setenv("GWGB_FP64_SLICES", "1")
+    cr, tr = crystal("C1", ns=ns)
+    out = []
+    for chunk, fails in ((None, 0), (None, 1), ("1", 1), (None, 5)):
+        if chunk:
+            monkeypatch.setenv("GWGB_TC_CHUNK_MB", chunk)
+        else:
+            monkeypatch.delenv("GWGB_TC_CHUNK_MB", raising=False)
+        s = GWSolver(cr.layout, ns, tr, precision=precision)
+        _inputs(cr, s)
+        s.set_Selfenergy(np.zeros(s.g_size, np.complex128))
+        s.dyson(cr.mu)
+        G0 = s.G_tau()
+        fail_alloc(1, fails)
+        s.solve()
+        fail_alloc(1, 0)
+        n = s.stats()["kernel_launches"]
+        first = (s.P0_q_t_QP(), s.Selfenergy())
+        s.set_G(G0)
+        s.iteration(cr.mu)  # the same plan in a captured graph
+        assert np.array_equal(first[1], s.Selfenergy())
+        out.append((n, *first))
+        s.close()
+    assert out[2][0] > 5 * out[0][0]  # one tau range after the other
+    for n, P, S in out[1:]:
+        assert np.array_equal(P, out[0][1]) and np.array_equal(S, out[0][2])
