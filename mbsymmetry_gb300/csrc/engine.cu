@@ -513,7 +513,7 @@ class Engine {
   std::vector<P0Contrib> pc_host_;
   std::vector<SigContrib> sc_host_;
   std::vector<Owner> sig_own_host_;
-  bool tc_chunk_env_ = false;  // GWGB_TC_CHUNK_MB given: it caps the sliced path's chunks too
+  bool tc_chunk_env_ = false;  // GWGB_TC_CHUNK_MB given: it caps the sliced path's chunks and kept V images too
   // Run a contraction's plan (0: P0 into Pall_, 1: Sigma into Sig_).
   void oz_run(int which, double scale) {
     OzSet &o = *oz_set();
@@ -1568,7 +1568,8 @@ void Engine::plan_oz(OzSet &set) {
   size_t free_b = 0, total_b = 0;
   GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
   const int64_t avail = (int64_t)free_b - (V_.p ? 0 : 16 * l.flat_V);
-  const int64_t persist = set.level ? 0 : std::max<int64_t>(0, avail / 4);
+  int64_t persist = set.level ? 0 : std::max<int64_t>(0, avail / 4);
+  if (tc_chunk_env_) persist = std::min(persist, tc_chunk_bytes_);
   const int64_t chunk = tc_chunk_env_ ? tc_chunk_bytes_ : std::min<int64_t>(OZ_CHUNK_BYTES, std::max<int64_t>(64ll << 20, avail / 8));
   const int64_t budget = set.level ? std::max<int64_t>(1ll << 20, chunk >> (2 * set.level)) : chunk;
   const int64_t taus = set.level ? budget : INT64_MAX;
