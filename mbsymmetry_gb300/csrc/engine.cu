@@ -653,9 +653,7 @@ Engine::Engine(const gwgb_params &p, const gwgb_layout &L) {
     tc_chunk_bytes_ = (int64_t)mb << 20;
     tc_chunk_env_ = true;
   }
-  build_work_lists();
-  if (p.precision != GWGB_PREC_FP64) set_precision(p.precision);
-  // buffers
+  // buffers, V first: what is sized by the free memory comes after them
   const int64_t fa = l_.flat_ao, fq = l_.flat_aux;
   V_.alloc(l_.flat_V);
   Sig_.alloc((size_t)nts_ * ns_ * fa);
@@ -675,6 +673,8 @@ Engine::Engine(const gwgb_params &p, const gwgb_layout &L) {
   mus_.alloc(1);
   counter_.alloc(1);
   recs_.alloc(16);
+  build_work_lists();
+  if (p.precision != GWGB_PREC_FP64) set_precision(p.precision);
   for (auto &e : sc_ev_) GWGB_CUDA(cudaEventCreate(&e));
   GWGB_CUDA(cudaMemsetAsync(Gall_.p, 0, Gall_.n * sizeof(double2), st_));
   GWGB_CUDA(cudaMemsetAsync(Pall_.p, 0, Pall_.n * sizeof(double2), st_));
@@ -1511,15 +1511,21 @@ void Engine::build_xf(int which, const std::vector<TSlab> &slabs, int nout, int 
   double flops = 0;
   for (const TSlab &x : slabs) flops += 8.0 * x.ncols * nout * nin;
   if (flops < 4e7) return;
-  xf_[which].build(slabs, nout, nin, row0, nX, nY, nsm_, st_);
-  if (!xf_[which].built() || xf_[which].bytes_A() <= (int64_t)xf_img_.n) return;
-  size_t free_b = 0, total_b = 0;
-  GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  if (xf_[which].bytes_A() > (int64_t)(free_b / 16)) {
-    xf_[which].free();
-    return;
+  OzTransform &x = xf_[which];
+  try {
+    x.build(slabs, nout, nin, row0, nX, nY, nsm_, st_);
+    if (!x.built() || x.bytes_A() <= (int64_t)xf_img_.n) return;
+    size_t free_b = 0, total_b = 0;
+    GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    GWGB_REQUIRE(x.bytes_A() <= (int64_t)(free_b / 16), GWGB_E_NOMEM, "transform images");
+    DBuf<char> img;
+    img.alloc((size_t)x.bytes_A());
+    xf_img_.free();
+    xf_img_ = img;
+  } catch (const Error &e) {  // the FP64 kernel, which needs none of this
+    x.free();
+    if (e.code != GWGB_E_NOMEM && e.code != GWGB_E_UNSUPPORTED) throw;
   }
-  xf_img_.alloc((size_t)xf_[which].bytes_A());
 }
 
 // The lists of the active precision's set, once, at the first memory level whose buffers fit.  FP64 needs none where
@@ -1561,13 +1567,13 @@ void Engine::plan_oz(OzSet &set) {
   const int ns = ns_, nts = nts_;
   std::vector<OzContrib> cs;
   std::vector<OzOwner> own;
-  // Memory free now (V itself may not be allocated yet).  At most a quarter of it holds the images of V that do not
+  // Memory free now.  At most a quarter of it holds the images of V that do not
   // change between iterations, an eighth the intermediates of one chunk: large chunks mean fewer, fuller launches
   // (hexagonal 8 k, the stages of both contractions in three slices: 1 GB 47.5 ms, 8 GB 37.2, 16 GB 36.6).  Where
   // that does not fit: no images of V kept, the chunks and the images of G and P~ (by ranges of tau) a quarter, ...
   size_t free_b = 0, total_b = 0;
   GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  const int64_t avail = (int64_t)free_b - (V_.p ? 0 : 16 * l.flat_V);
+  const int64_t avail = (int64_t)free_b;
   int64_t persist = set.level ? 0 : std::max<int64_t>(0, avail / 4);
   if (tc_chunk_env_) persist = std::min(persist, tc_chunk_bytes_);
   const int64_t chunk = tc_chunk_env_ ? tc_chunk_bytes_ : std::min<int64_t>(OZ_CHUNK_BYTES, std::max<int64_t>(64ll << 20, avail / 8));

@@ -129,3 +129,58 @@ def test_less_memory_means_smaller_chunks(precision, ns, fail_alloc, monkeypatch
     assert out[2][0] > 5 * out[0][0]  # one tau range after the other
     for n, P, S in out[1:]:
         assert np.array_equal(P, out[0][1]) and np.array_equal(S, out[0][2])
+
+
+def test_transforms_run_without_their_images(fail_alloc):
+    """Every single allocation of a handle's creation in turn: either the creation
+    fails with GWGB_E_NOMEM, or a transform goes on with the FP64 kernel and the W~
+    solve and Dyson agree with the undisturbed handle's (60 to 150 terms a transform,
+    a solve in between: 1e-12 of the largest element)."""
+    from mbsymmetry_gb300.crystal import CrystalSpec, load_ir, make_crystal
+    from mbsymmetry_gb300.solver import GWSolver
+    from mbsymmetry_gb300.transformer import build_transforms
+    cr = make_crystal(CrystalSpec("xf", "fcc", (1, 1, 1), 48, 50, 150, 50.0, ao_block=(14, 18), aux_block=(16, 17),
+                                  seed=7))
+    tr = build_transforms(load_ir(150), 50.0)
+    assert 8.0 * (tr.nts - 2) * tr.nw * cr.layout.flat_ao_size > 4e7 < 8.0 * (tr.nts - 2) * tr.nw_b * cr.layout.flat_aux_size
+    rng = np.random.default_rng(4)
+    P0 = np.zeros(tr.nts * cr.layout.flat_aux_size, np.complex128).reshape(tr.nts, -1)
+    o = 0
+    for n in cr.layout.aux_sizes[0]:
+        x = rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))
+        P0[:, o:o + n * n] = -0.02 * (x @ x.conj().T).ravel() * np.exp(-np.abs(np.arange(tr.nts) - 74.5) / 9)[:, None]
+        o += n * n
+
+    def run(s):
+        s.set_shared_Coulomb(cr.V)
+        s.set_fock(cr.F, cr.S)
+        s.set_Selfenergy(np.zeros(s.g_size, np.complex128))
+        s.dyson(cr.mu)
+        s.set_P0(P0.ravel())
+        s.compute_Pq_from_P0q()
+        return s.G_tau(), s.P0_q_t_QP()
+
+    first = GWSolver(cr.layout, 1, tr)
+    ref, fell_back = run(first), 0
+    b0 = first.stats()["device_bytes"]
+    second = GWSolver(cr.layout, 1, tr)
+    size = second.stats()["device_bytes"] - b0 if run(second) else 0
+    second.close()
+    for n in range(1, 121):
+        run(first)
+        b0 = first.stats()["device_bytes"]
+        fail_alloc(n, 1)
+        try:
+            s = GWSolver(cr.layout, 1, tr)
+        except _abi.GwgbError as e:
+            assert e.code == _abi.GWGB_E_NOMEM
+            continue
+        finally:
+            fail_alloc(1, 0)
+        got = run(s)
+        fell_back += s.stats()["device_bytes"] - b0 < size
+        s.close()
+        for a, b in zip(ref, got):
+            assert np.abs(a - b).max() < 1e-12 * np.abs(a).max()
+    first.close()
+    assert fell_back >= 4
