@@ -6,6 +6,9 @@
 // Sigma(tau), the frequency-domain work buffers and the work lists of the
 // kernels.  An iteration is a fixed sequence of kernel launches over static
 // work lists, so it is captured once as a CUDA graph and replayed.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -1678,8 +1681,22 @@ static void h2d(void *d, const void *h, size_t bytes, cudaStream_t st) {
   GWGB_REQUIRE(h != nullptr || bytes == 0, GWGB_E_INVALID, "NULL host pointer");
   GWGB_CUDA(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st));
 }
+// Pages of a host array that the process has not touched yet would be faulted in by the GPU's writes: 9 MB took 0.5
+// to 6 ms (as the heap happened to be), 0.08 into resident pages; populated at once by the operating system 0.35.
+static void populate_pages(void *h, size_t bytes) {
+  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  char *p = (char *)((uintptr_t)h / page * page), *end = (char *)h + bytes;
+  unsigned char in[1024];
+  for (size_t n; p < end; p += n * page) {
+    n = std::min(sizeof(in), ((size_t)(end - p) + page - 1) / page);
+    if (n < 16 || mincore(p, n * page, in) != 0) return;  // small, or not ordinary memory
+    if (std::any_of(in, in + n, [](unsigned char r) { return !(r & 1); }))
+      madvise(p, n * page, 23 /* MADV_POPULATE_WRITE; fails on older kernels: then as before */);
+  }
+}
 static void d2h(void *h, const void *d, size_t bytes, cudaStream_t st) {
   GWGB_REQUIRE(h != nullptr || bytes == 0, GWGB_E_INVALID, "NULL host pointer");
+  populate_pages(h, bytes);
   GWGB_CUDA(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, st));
 }
 
@@ -1690,7 +1707,10 @@ void Engine::upload_V(const double *V, int64_t n) {
   GWGB_CUDA(cudaStreamSynchronize(st_));
   have_V_ = true;
   vt_ready_ = vcat_ready_ = oz_[0].ready = oz_[1].ready = false;  // rebuilt before the next solve
-  build_oz();  // the lists, with the other set-up of a handle that will contract
+  // The lists of a small crystal, 2 ms (s+p), which would double its first contraction.  Larger ones wait for that: a
+  // handle that only solves Dyson or W~ never needs them (hexagonal 8 k 28 ms, s+p+d+4 8 k 13), and with them the first
+  // contraction still takes a fraction of the FMA kernels' time (s+p+d+4 8 k 44 ms against 260).
+  if (prec_ == GWGB_PREC_FP64 && p0_flops_ + sig_flops_ < 6e9) build_oz();
 }
 
 void Engine::set_reps(const double *orep, int64_t no, const double *auxrep, int64_t na) {
