@@ -42,12 +42,27 @@ extern "C" {
 #define GWGB_E_UNSUPPORTED   7  /* shape beyond the limits of the built kernels */
 
 /* ---- contraction precision -------------------------------------------- */
-#define GWGB_PREC_FP64       0  /* complex128 everywhere: the drop-in path */
+#define GWGB_PREC_FP64       0  /* complex128 in and out, the drop-in path (arithmetic: GWGB_FLAG_FP64_FMA below) */
 #define GWGB_PREC_TF32X3     1  /* P0/Sigma on tcgen05 kind::tf32, 3-pass split, FP32 accumulate */
 #define GWGB_PREC_BF16X3     2  /* P0/Sigma on tcgen05 kind::f16 (BF16), 3-way split, 6 products, FP32 accumulate */
 #define GWGB_PREC_OZAKI      3  /* P0/Sigma on tcgen05 kind::f16 (FP16): three slices per operand row (Ozaki scheme),
                                    8 products, exact leading sums in FP32, float-float accumulation; Sigma error
                                    below 1e-9 of the FP64 path */
+
+/* gwgb_params.flags.  Large enough FP64 contractions, and in every precision large
+ * enough tau <-> omega transforms, run on tcgen05 with six FP16 slices per operand:
+ * a number is held to 2^-57 of the largest one of its row (an operand's row over at
+ * most 32 complex summation indices; rows of an intermediate may share theirs),
+ * against 2^-53 of itself in an FP64 FMA.  Relative to the products of row scales the
+ * results are at least as accurate as FP64 (on crystals of the configurations' sizes
+ * every quantile of the element-wise error is smaller, too), but sums of products
+ * that are all far below the product of their rows' largest elements are not: those
+ * of strongly graded data lose about log2 of that ratio minus 4 bits.  Contractions
+ * too small to gain, and all of them where no plan fits the device memory, run in
+ * FP64 FMAs.  With this flag all contractions of GWGB_PREC_FP64 and all transforms
+ * do, at about the FP64 rate of the GPU.  (GWGB_FP64_SLICES=0 / 1 in the environment
+ * forces FMAs or slices for the contractions of handles without the flag.) */
+#define GWGB_FLAG_FP64_FMA   1
 
 typedef struct gwgb_handle_s *gwgb_handle;
 
@@ -62,7 +77,7 @@ typedef struct gwgb_params {
   int32_t precision; /* GWGB_PREC_* */
   int32_t device;    /* CUDA device ordinal */
   int32_t nt_batch;  /* accepted for params_t compatibility; the kernels choose their own tau tiles */
-  int32_t flags;     /* reserved, 0 */
+  int32_t flags;     /* GWGB_FLAG_*, else 0 */
   /* Tile-shape settings of the tcgen05 Sigma path, 0 = the built-in choice;
    * mbsymmetry_gb300/autotune.py picks them by timing a workload. */
   int32_t uvt_smem_kb; /* shared memory per U/Sigma CTA (60..227 KB; sets tau per tile and aux rows per chunk) */

@@ -138,6 +138,8 @@ SIGNATURES = {
                                       c_void_p, c_int32, c_void_p]),
 }
 
+FLAG_FP64_FMA = 1
+
 NOALLOC_SCRATCH_BYTES = 8 << 20
 NOALLOC_MAX_BLOCKS = 64
 

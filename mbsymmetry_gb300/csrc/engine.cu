@@ -303,6 +303,7 @@ class Engine {
  private:
   // parameters
   int ns_, nts_, nw_, nw_b_, ncheb_, prec_, dev_;
+  bool fma64_ = false;  // GWGB_FLAG_FP64_FMA
   double beta_;
   Lay l_;
   cudaStream_t st_ = nullptr;
@@ -626,6 +627,7 @@ Engine::Engine(const gwgb_params &p, const gwgb_layout &L) {
   if (p.sw_npk_max) tune_npk_ = p.sw_npk_max;
   if (p.uv_waves) tune_waves_ = p.uv_waves;
   beta_ = p.beta; prec_ = GWGB_PREC_FP64; dev_ = p.device;
+  fma64_ = (p.flags & GWGB_FLAG_FP64_FMA) != 0;
   l_ = derive_layout(L);
   GWGB_CUDA(cudaSetDevice(dev_));
   GWGB_CUDA(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
@@ -1513,7 +1515,7 @@ void Engine::build_xf(int which, const std::vector<TSlab> &slabs, int nout, int 
   // 12000 columns at 120 points: 1.28 ms there, 0.20 here
   double flops = 0;
   for (const TSlab &x : slabs) flops += 8.0 * x.ncols * nout * nin;
-  if (flops < 4e7) return;
+  if (flops < 4e7 || fma64_) return;
   OzTransform &x = xf_[which];
   try {
     x.build(slabs, nout, nin, row0, nX, nY, nsm_, st_);
@@ -1539,6 +1541,7 @@ void Engine::build_oz() {
   OzSet &set = oz_[f64 ? 1 : 0];
   constexpr int LEVELS = 8;
   const bool fresh = !set.built;
+  if (f64 && fma64_) set.off[0] = set.off[1] = set.built = true;
   while (!set.built) {
     auto next = [&](bool memory) {  // true: try again with less
       set.plan[0].free();

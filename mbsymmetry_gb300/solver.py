@@ -31,11 +31,15 @@ def _ptr(a: np.ndarray):
 
 class GWSolver:
     def __init__(self, layout: BlockLayout, ns: int, transforms: IRTransforms,
-                 precision: str = "fp64", device: int = 0, tune: dict = None):
+                 precision: str = "fp64", device: int = 0, tune: dict = None, fp64_fma: bool = False):
         """tune: optional gwgb_params settings chosen by autotune.autotune()
         (its "best" entry): the tile settings of the FP32-class tcgen05 Sigma
         path (uvt_smem_kb, sw_npk_max, uv_waves); oz_simt_cols is accepted
-        without effect."""
+        without effect.
+
+        fp64_fma: contractions of "fp64" and all transforms in FP64 FMAs, every
+        number with its own 53 bits, instead of slices of 57 bits per row where
+        those are faster (GWGB_FLAG_FP64_FMA in gwgb.h)."""
         self.lib = _abi.load()
         self.layout = layout
         self.ns = ns
@@ -43,7 +47,8 @@ class GWSolver:
         self.nts = transforms.nts
         p = _abi.GwgbParams(ns=ns, nts=transforms.nts, nw=transforms.nw, nw_b=transforms.nw_b,
                             beta=transforms.beta, precision=_abi.PREC_NAMES[precision], device=device,
-                            nt_batch=0, flags=0, **{k: int(v) for k, v in (tune or {}).items()})
+                            nt_batch=0, flags=_abi.FLAG_FP64_FMA if fp64_fma else 0,
+                            **{k: int(v) for k, v in (tune or {}).items()})
         self._lay_c, self._keep = layout.to_c()
         h = ctypes.c_void_p()
         _abi.check(self.lib.gwgb_create(ctypes.byref(p), ctypes.byref(self._lay_c), ctypes.byref(h)))
