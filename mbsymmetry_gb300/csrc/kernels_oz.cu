@@ -9,8 +9,8 @@
 // ISC 2020 for FP16 tensor cores):
 //   x 2^(15-E) = s0 + s1 + s2,  s0 a multiple of 2^6 (|s0| <= 2^15),
 //   s1 a multiple of 2^(5-b) (|s1| <= 2^5), s2 the rest rounded to FP16,
-// b = 9 bits for rounds of 3 or 4 octets of K, 10 for 2, 11 for 1.  The
-// remainder is below 2^(E-32) and 2^(E-33) rms (s2 floats).  The products
+// b = 9 bits for rounds of 3 or 4 octets of K, 10 for 2, 11 for 1.  What is
+// left out is below 1.13 x 2^(E-32) and 2^(E-33) rms (s2 floats).  The products
 // (i, j) with i + j <= 3 (8 MMAs per K step) go to four TMEM accumulators:
 //   (0, 0): multiples of 2^12, at most 2^30 each: a round of 64 real terms stays
 //           within 24 bits, so FP32 accumulation is exact;
@@ -20,13 +20,16 @@
 //
 // The FP64 contractions are the same chains with six slices: x 2^(8-E) = sum_p
 // d_p 2^(-9p), |d_p| <= 2^8, d_0 .. d_4 integers and d_5 the rest rounded to FP16,
-// so a row is held to 2^(E-57) of its scale (FP64 itself holds an element to
-// 2^-53).  The products of class i + j <= 6 (26 MMAs per K step) go to one
+// so a row is held to about 2^(E-57) (FP64 itself holds each element to 2^-53 of
+// itself: elements more than 2^4 below their row's largest have fewer bits here).
+// The products of class i + j <= 6 (26 MMAs per K step) go to one
 // accumulator per class; classes 0 to 3 are exact in FP32 (at most 4 products of
 // 2^16 over 64 real terms), classes 4 to 6 have weight 2^-36 and less, class 7 is
 // dropped (2^-61).  The drain sums the classes without error into three FP32
-// numbers.  Against extended precision the error of P0 and Sigma is 0.7 to
-// 1.8e-16, the FMA kernels' 1.7 to 5.2e-16.  Their rate is the FP64 pipe's (2 FMA per cycle and SM); one
+// numbers.  Against extended precision the error of P0 and Sigma (2-norm) is 0.6 to
+// 1.8e-16, the FMA kernels' 1.0 to 5.2e-16; element by element (s+p+d, hexagonal and
+// Gaussian-orbital crystals) the median is 0.5 to 1.9e-16 against 0.7 to 14e-16, the
+// largest 0.2 to 9e-15 against 0.6 to 210e-15.  Their rate is the FP64 pipe's (2 FMA per cycle and SM); one
 // complex output of K = 32 takes 64 cycles there and about 3 here.  Complex products use
 // the real embedding A = [Ar Ai] (K interleaved), B rows (n, 0) = [Br -Bi],
 // (n, 1) = [Bi Br], so D[r][(n,0)] = Re, D[r][(n,1)] = Im of sum_k A[r][k] B[n][k].
@@ -102,10 +105,15 @@ struct Tri {
   F2 h, m, l;
 };
 
-// The value of the class sums D0 .. D3 and d4 = D4 + 2^-9 D5 + 2^-18 D6 (weights 2^(-9c)).  Carries instead of two-sums (26 steps against 44): D0 to D3
-// are exact integers, at most 64 sums of c + 1 products of digits, of which at most one is 256 in each factor, so D3 and
-// a carry of 2^15.4 stay below 2^24 and each step is exact (but for the last bits of D4 to D6, which the tensor core
-// rounds to 24 bits).  NORM: normalised.
+// The value of the class sums D0 .. D3 and d4 = D4 + 2^-9 D5 + 2^-18 D6 (weights 2^(-9c)).  Carries instead of
+// two-sums (26 steps against 44).  D0 to D3 are exact integers, sums of 64 (c + 1) products of digits; D2 and below leave
+// room for a carry.  D3 with its carry stays within 2^24: a digit of 256 turns the sign of the next one (the remainder
+// is at most half a unit), so a term whose four products of class 3 all have 256 in both factors and one sign has
+// three of the other sign in class 4; a factor below 256 takes at least 1/256 of a product off class 3, twice what a
+// whole product of class 4 carries.  In the worst mixture, three such products and one of 255 x 256, class 3 lacks 2/512 of a
+// product and class 4 adds 1/512.  So each step is exact, but for the last bits of D4 to D6, which the tensor core
+// rounds to 24 bits.  (The fourth digit of a drain's image may reach 260; class 3 could pass 2^24 only in rounds all of
+// whose elements have the magnitude 2^E 512/513 to eight digits, and would lose its last bit there.)  NORM: normalised.
 template <bool NORM> __device__ __forceinline__ Tri tri_of(const F2 (&d)[4], F2 d4) {
   const F2 W = both(0x1p-9f), MG = both(1.5f * 8388608.f), NM = both(-1.5f * 8388608.f), NB = both(-512.f);
   auto carry = [&](F2 x) { return add2(fma2(x, W, MG), NM); };  // x / 512 to an integer
@@ -126,8 +134,9 @@ template <bool NORM> __device__ __forceinline__ Tri tri_of(const F2 (&d)[4], F2 
   return t;
 }
 
-// a += b without normalising: sums and their errors stay in order of size, which leaves R rounds within 2^-70 R^2 of
-// the largest (21 steps a round; normalised every time it was 36, and the FP32 pipe bounds the drains).
+// a += b without normalising: sums and their errors stay in order of size, which leaves up to 4096 rounds within 2^-57
+// of the largest partial sum (measured with a model of these steps; an FP64 addition rounds to 2^-53).  21 steps a
+// round; normalised every time it was 36, and the FP32 pipe bounds the drains.
 __device__ __forceinline__ void tri_add(Tri &a, const Tri &b) {
   F2 e1, m, e2, e3;
   two_sum(a.h, b.h, a.h, e1);
@@ -355,7 +364,7 @@ __device__ __forceinline__ void oz_mmas(uint32_t d0, uint32_t a0, uint32_t b0, u
 // one set's loop overhead is hidden behind the other's MMAs (two issuing warps:
 // 1200 idle cycles cost 100).  Stage 3 of the hexagonal 8 k crystal (three
 // slices), Sigma: one K step per segment and one MMA warp 10.4 ms, segments of four
-// 6.5, an MMA warp per set 6.2.
+// 6.5; an MMA warp per set, with segments of two in rings of its own, 6.2.
 // Six slices have room for one set in TMEM.  There a round's MMAs go in two groups, the
 // classes 4 to 6 (16 of the 26 products of a K step) and 0 to 3, with barriers of their
 // own: the drain reads the high classes while the low ones multiply and the low ones
