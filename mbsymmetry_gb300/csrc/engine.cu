@@ -1606,7 +1606,7 @@ void Engine::plan_oz(OzSet &set) {
   }
   // the lists of the two contractions are built side by side
   const bool first = set.level == 0;  // which contractions run in slices is decided there
-  auto p0_built = std::async(std::launch::async, [&set, cs, own, NS, nts, budget, persist, taus, first, this] {
+  auto p0_built = std::async(std::launch::async | std::launch::deferred, [&set, cs, own, NS, nts, budget, persist, taus, first, this] {
     if (first || !set.off[0])
       set.plan[0].build(NS, cs, own, nts / 2, 0, budget, persist / 2, taus, nsm_, l_.flat_V, (int64_t)Gall_.n,
                         (int64_t)Gall_.n, (int64_t)Pall_.n);

@@ -34,6 +34,11 @@ __device__ __forceinline__ double2 cfma_conja(double2 a, double2 b, double2 c) {
   c.y = fma(-a.y, b.x, c.y);
   return c;
 }
+// c - a * b, the product first: three instructions a component.  Two, fma(-a.x, b.x, fma(a.y, b.y, c.x)), round twice at
+// the size of c; in the eliminations below that makes the error of the inverses 12 to 26% larger.
+__device__ __forceinline__ double2 csub(double2 c, double2 a, double2 b) {
+  return make_double2(c.x - fma(a.x, b.x, -(a.y * b.y)), c.y - fma(a.x, b.y, a.y * b.x));
+}
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 __device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
 
@@ -384,15 +389,16 @@ __global__ void __launch_bounds__(256) transform_kernel(const TSlab *__restrict_
 // Bound: the FP64 pipe (2 FMA per cycle and SM; a DFMA of one warp takes 64 cycles
 // of its scheduler), so what counts is the number of FP64 instructions:
 //  - the A of mode 0 is Hermitian and, at bosonic frequencies, positive definite: symmetric sweeps over its
-//    lower triangle, no pivot search (2 n^3 FMA against 6 n^3 and the search).  A pivot that is not clearly
+//    lower triangle, no pivot search (3 n^3 instructions against 6 n^3 and the search).  A pivot that is not clearly
 //    positive sends the block to the general elimination;
 //  - the general one is Gauss-Jordan with full pivoting (the strategy of Eigen::FullPivLU,
-//    sc_type_block.cpp:55), 4 FMA per element and step; the pivot is the largest
+//    sc_type_block.cpp:55), 6 instructions per element and step; the pivot is the largest
 //    component by its upper 32 bits, found in integers while the elimination writes the elements.
 // One warp per matrix up to n = 16, a CTA of 128 threads up to 32, of 256 above (NT), elements spread over the threads.
-// Measured, before and now: W~ s+p+d+4 (aux 9-46) 3.36 and 1.32 ms, hexagonal 8 k (aux 2-30) 3.15 and 1.02; Dyson there
-// (AO 2-30) 0.61 and 0.20; s+p (n up to 12), both solves, 0.17 and 0.07.  Tried and slower: the product R P from one
-// triangle (R commutes with the Hermitian part of P), the rest in FP32.
+// Measured, with one general elimination per warp or CTA of 128 and now: W~ s+p+d+4 (aux 9-46) 3.36 and 1.53 ms,
+// hexagonal 8 k (aux 2-30) 3.15 and 0.95; Dyson there (AO 2-30) 0.61 and 0.26; s+p (n up to 12), both solves, 0.17 and 0.075.
+// With 4 instead of 6 instructions per element (csub) 1.33, 0.83, 0.20 and 0.071, at an error 12 to 26% larger.  Tried
+// and slower: the product R P from one triangle (R commutes with the Hermitian part of P), the rest in FP32.
 // ---------------------------------------------------------------------------
 template <int NT> __device__ __forceinline__ void inv_sync() {
   if constexpr (NT == 32)
@@ -481,9 +487,7 @@ __device__ __forceinline__ bool gauss_jordan(double2 *A, int n, double2 *rowk, d
       double2 a = r;
       if (i != icol) {
         const double2 f = fcol[i];
-        a = j == icol ? make_double2(0.0, 0.0) : i == irow ? old[j] : A[e];
-        a.x = fma(-r.x, f.x, fma(r.y, f.y, a.x));
-        a.y = fma(-r.x, f.y, fma(-r.y, f.x, a.y));
+        a = csub(j == icol ? make_double2(0.0, 0.0) : i == irow ? old[j] : A[e], r, f);
         if (!used[i] && !used[j]) {
           const unsigned k = inv_key(a);
           if (k > best) { best = k; bidx = e; }
@@ -523,10 +527,7 @@ __device__ __forceinline__ bool sweep_inverse(double2 *A, const double2 *P, int 
       } else if (j == k) {
         a = cconj(w[i]);
       } else {
-        const double2 x = c[i], y = w[j];
-        a = A[i * n + j];
-        a.x = fma(-x.x, y.x, fma(x.y, y.y, a.x));
-        a.y = fma(-x.x, y.y, fma(-x.y, y.x, a.y));
+        a = csub(A[i * n + j], c[i], w[j]);
       }
       A[i * n + j] = a;
     }
