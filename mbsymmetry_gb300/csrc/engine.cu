@@ -427,7 +427,7 @@ class Engine {
   void transform(int which, const DBuf<TSlab> &slabs, int max_cols, const double2 *T, int nout, int nin, int row0,
                  const double2 *X, double2 *Y) {
     if (xf_[which].ready)
-      xf_[which].run(X, Y, xf_img_.p, nsm_, bad_.p + 2, st_);
+      xf_[which].run(slabs.p, (int)slabs.n, T, X, Y, xf_img_.p, nsm_, bad_.p + 2, st_);
     else
       launch_transform(slabs.p, (int)slabs.n, max_cols, T, nout, nin, row0, X, Y, st_);
   }
@@ -1518,7 +1518,7 @@ void Engine::build_xf(int which, const std::vector<TSlab> &slabs, int nout, int 
   if (flops < 4e7 || fma64_) return;
   OzTransform &x = xf_[which];
   try {
-    x.build(slabs, nout, nin, row0, nX, nY, nsm_, st_);
+    x.build(slabs, nout, nin, row0, which != XF_P0 && which != XF_SIGMA, nX, nY, nsm_, st_);
     if (!x.built() || x.bytes_A() <= (int64_t)xf_img_.n) return;
     size_t free_b = 0, total_b = 0;
     GWGB_CUDA(cudaMemGetInfo(&free_b, &total_b));
@@ -1747,9 +1747,8 @@ void Engine::set_transforms(const double *Tnt, const double *Ttn, const double *
     h2d(tct_l_.p, tl, ncheb_ * sizeof(double), st_);
   }
   const double2 *T[XF_E] = {TntBF_.p, TtnFB_.p, Tnt_.p, Ttn_.p};
-  const double *Th[XF_E] = {TntBF, TtnFB, Tnt, Ttn};
   for (int i = 0; i < XF_E; ++i)
-    if (xf_[i].built()) xf_[i].set_matrix(Th[i], T[i], st_);
+    if (xf_[i].built()) xf_[i].set_matrix(T[i], st_);
   GWGB_CUDA(cudaStreamSynchronize(st_));
   have_T_ = true;
 }
@@ -1908,7 +1907,7 @@ void Engine::finish_stats(bool with_dyson, bool with_gw, bool with_pq, bool with
     s.solve_flops += solve_flops_dy_;
   }
   int64_t launches = 0;
-  auto xf = [&](int i) { return xf_[i].ready ? 2 : 1; };  // a transform in six slices builds its images first
+  auto xf = [&](int i) { return xf_[i].ready ? xf_[i].launches() : 1; };
   if (with_gw) {
     const bool tc = tc_split();
     int64_t sgt = 0, p0t = 0;
@@ -2101,7 +2100,7 @@ void Engine::set_energy_matrix(const double *M, int n) {
   for (size_t i = 0; i < m.size(); ++i) m[i] = make_double2(M[i], 0.0);
   if (!Me_.p) Me_.alloc(m.size());
   h2d(Me_.p, m.data(), m.size() * sizeof(double2), st_);
-  if (xf_[XF_E].built()) xf_[XF_E].set_matrix(&m[0].x, Me_.p, st_);
+  if (xf_[XF_E].built()) xf_[XF_E].set_matrix(Me_.p, st_);
   GWGB_CUDA(cudaStreamSynchronize(st_));
   if (!have_M_) drop_graphs();
   have_M_ = true;

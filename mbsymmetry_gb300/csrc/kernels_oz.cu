@@ -1128,6 +1128,35 @@ __global__ void __launch_bounds__(128) oz_build_kernel(const OzBuild *__restrict
   }
 }
 
+// One CTA per row (launch_oz_row_scale).  Bound: reading X once, 10 us where the transform takes 100.
+__global__ void __launch_bounds__(1024) oz_row_scale_kernel(const TSlab *__restrict__ slabs, int nslabs,
+                                                            const double2 *__restrict__ X, int row0, int nin,
+                                                            double *__restrict__ scale) {
+  __shared__ int part[32];
+  const int i = blockIdx.x;
+  int m = 0;  // upper word of the largest component
+  for (int s = 0; s < nslabs; ++s) {
+    const TSlab sl = slabs[s];
+    const double2 *x = X + sl.x + (int64_t)(row0 + i) * sl.ldx;
+#pragma unroll 4
+    for (int c = threadIdx.x; c < sl.ncols; c += 1024) {
+      const double2 v = x[c];
+      m = max(m, max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff));
+    }
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    m = __reduce_max_sync(0xffffffffu, part[threadIdx.x]);
+    if (threadIdx.x == 0) {
+      const int be = m >> 20, e = be == 0 || be == 0x7ff ? 0 : min(max(be - 1022, -500), 500);
+      scale[i] = __hiloint2double((1023 - e) << 20, 0);
+      scale[nin + i] = __hiloint2double((1023 + e) << 20, 0);
+    }
+  }
+}
+
 }  // namespace
 
 template <int NS>
@@ -1175,6 +1204,12 @@ void launch_oz_gemm(int ns, int stage, bool multi, const OzArgs &a, int nsm, cud
     launch<3>(stage, multi, a, grid, st);
   else
     launch<6>(stage, multi, a, grid, st);
+  GWGB_CUDA(cudaGetLastError());
+}
+
+void launch_oz_row_scale(const TSlab *slabs, int nslabs, const double2 *X, int row0, int nin, double *scale,
+                         cudaStream_t st) {
+  oz_row_scale_kernel<<<nin, 1024, 0, st>>>(slabs, nslabs, X, row0, nin, scale);
   GWGB_CUDA(cudaGetLastError());
 }
 

@@ -603,12 +603,13 @@ void OzPlan::run_one(const OzLaunch &l, OzShared &sh, const double2 *V, const do
   launch_oz_gemm(ns_, (int)l.d0, l.multi, a, nsm, st);
 }
 
-void OzTransform::build(const std::vector<TSlab> &slabs, int nout, int nin, int row0, int64_t nX, int64_t nY, int nsm,
-                        cudaStream_t st) {
+void OzTransform::build(const std::vector<TSlab> &slabs, int nout, int nin, int row0, bool scaled, int64_t nX, int64_t nY,
+                        int nsm, cudaStream_t st) {
   const int NS = 6, OCT = OZ_OCT, FK = 8 * OCT;
   const int kos = cdiv(nin, 8), R = cdiv(kos, OCT), nos = cdiv(nout, 8);
-  nout_ = nout;
   nin_ = nin;
+  row0_ = row0;
+  scaled_ = scaled;
   const int64_t fb = (int64_t)NS * kos * 4096 + 512 * R, vb = (int64_t)NS * kos * 512 + 32 * R;
   std::vector<OzBuild> builds;
   std::vector<OzTask> tasks;
@@ -632,7 +633,7 @@ void OzTransform::build(const std::vector<TSlab> &slabs, int nout, int nin, int 
       for (int r = 0; r < R; ++r) {
         const int nks = std::min(OCT, kos - r * OCT);
         builds.push_back({x.x + (int64_t)(row0 + r * FK) * x.ldx, a_, 0, 0, 1, x.ldx, 1 << 30, 1 << 20, x.ncols,
-                          nin - r * FK, 1, 1, f * OZ_M, OZ_M, (int16_t)nks, 0, 0, 0, r * FK, 0});
+                          nin - r * FK, 1, 1, f * OZ_M, OZ_M, (int16_t)nks, 0, 0, 0, scaled ? r * FK : -1, 0});
         a_ += oz_abytes(NS, nks);
       }
       GWGB_REQUIRE(f < 65536, GWGB_E_UNSUPPORTED, "transform slab too large");
@@ -646,7 +647,7 @@ void OzTransform::build(const std::vector<TSlab> &slabs, int nout, int nin, int 
     for (int r = 0; r < R; ++r) {
       const int nks = std::min(OCT, kos - r * OCT);
       builds.push_back({(int64_t)ct * oct * 8 * nin + r * FK, tb, 0, 0, nin, 1, 1 << 20, 1 << 20, nout - ct * oct * 8,
-                        nin - r * FK, 1, 1, 0, (int16_t)(8 * noct), (int16_t)nks, 1, 0, 0, nin + r * FK, 0});
+                        nin - r * FK, 1, 1, 0, (int16_t)(8 * noct), (int16_t)nks, 1, 0, 0, scaled ? nin + r * FK : -1, 0});
       tb += noct * oz_bbytes1(NS, nks);
     }
   }
@@ -660,33 +661,24 @@ void OzTransform::build(const std::vector<TSlab> &slabs, int nout, int nin, int 
   s3_.upload(s3, st);
   rnd_.upload(rnd, st);
   T_.alloc((size_t)tb);
-  scale_.alloc(2 * (size_t)nin);
+  if (scaled) scale_.alloc(2 * (size_t)nin);
   GWGB_CUDA(cudaStreamSynchronize(st));
 }
 
-// In place: a captured graph holds the addresses of T_ and scale_.
-void OzTransform::set_matrix(const double *T_host, const double2 *T, cudaStream_t st) {
+// In place: a captured graph holds the address of T_ (and, scaled, of T).
+void OzTransform::set_matrix(const double2 *T, cudaStream_t st) {
   ready = false;
-  std::vector<double> scale(2 * (size_t)nin_, 1.0);
-  for (int i = 0; i < nin_; ++i) {
-    double m = 0.0;
-    for (int r = 0; r < nout_; ++r) {
-      const double *t = T_host + 2 * ((size_t)r * nin_ + i);
-      m = std::max(m, std::max(std::fabs(t[0]), std::fabs(t[1])));
-    }
-    if (!(m > 0x1p-500 && m < 0x1p500)) continue;
-    int e;
-    std::frexp(m, &e);
-    scale[i] = std::ldexp(1.0, e);
-    scale[nin_ + i] = std::ldexp(1.0, -e);
-  }
-  GWGB_CUDA(cudaMemcpyAsync(scale_.p, scale.data(), scale.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-  launch_oz_build(6, builds_.p + nbuild_, nT_, T, T_.p, st, scale_.p);
+  if (!scaled_) launch_oz_build(6, builds_.p + nbuild_, nT_, T, T_.p, st);
   GWGB_CUDA(cudaStreamSynchronize(st));
   ready = true;
 }
 
-void OzTransform::run(const double2 *X, double2 *Y, char *A, int nsm, int *err, cudaStream_t st) const {
+void OzTransform::run(const TSlab *slabs, int nslabs, const double2 *T, const double2 *X, double2 *Y, char *A, int nsm,
+                      int *err, cudaStream_t st) const {
+  if (scaled_) {
+    launch_oz_row_scale(slabs, nslabs, X, row0_, nin_, scale_.p, st);
+    launch_oz_build(6, builds_.p + nbuild_, nT_, T, T_.p, st, scale_.p);
+  }
   launch_oz_build(6, builds_.p, nbuild_, X, A, st, scale_.p);
   OzArgs a = gemm_.args;
   a.desc = s3_.p;

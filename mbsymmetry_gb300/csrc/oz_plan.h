@@ -81,32 +81,39 @@ struct OzShared {  // one allocation (a first pass waits for it)
 };
 
 // A tau <-> omega transform Y[slab][r][c] = sum_i T[r][i] X[slab][row0 + i][c] as a stage-3
-// GEMM in six slices: rows c, K = i, columns r.  The tau grids are dense at their ends, where the
-// weights in T are small and X is large: X[i] is scaled by the power of two of the largest
-// |T[r][i]| and T by its inverse, so that the slices of a row are relative to its largest term.
+// GEMM in six slices: rows c, K = i, columns r.  Scaled: X[i] by the power of two below its largest
+// element over all columns and T[.][i] by the inverse, in every run, so that the slices of a row of T follow its terms.
+// The transforms to tau need that: their terms fall off with frequency in X and, towards the middle of the tau axis, in T,
+// where the result is a small rest of them.  Errors against extended precision, relative to the FP64 kernel's, over the
+// committed grids, G and P~ of s+p+d crystals, geometric mean and worst: 2-norm 0.1 and 0.2, largest of a row r relative to that
+// row 0.08 and 0.3; scaled by the columns of T alone 0.39 and 0.64, but rows 12 and 900.  The transforms from tau
+// are as good without (0.05 and 0.2, rows 0.05 and 0.15).
 class OzTransform {
  public:
-  void build(const std::vector<TSlab> &slabs, int nout, int nin, int row0, int64_t nX, int64_t nY, int nsm,
+  void build(const std::vector<TSlab> &slabs, int nout, int nin, int row0, bool scaled, int64_t nX, int64_t nY, int nsm,
              cudaStream_t st);
   int64_t bytes_A() const { return a_; }
   bool built() const { return gemm_.n > 0; }
   bool ready = false;           // the matrix has been set
-  // T: host and device copies, [nout][nin]; may be set again, the buffers stay where they are
-  void set_matrix(const double *T_host, const double2 *T, cudaStream_t st);
-  // A: bytes_A() bytes of scratch
-  void run(const double2 *X, double2 *Y, char *A, int nsm, int *err, cudaStream_t st) const;
+  int launches() const { return scaled_ ? 4 : 2; }
+  // T: [nout][nin] on the device; may be set again, the buffers stay where they are
+  void set_matrix(const double2 *T, cudaStream_t st);
+  // slabs: those of build(), on the device; A: bytes_A() bytes of scratch
+  void run(const TSlab *slabs, int nslabs, const double2 *T, const double2 *X, double2 *Y, char *A, int nsm, int *err,
+           cudaStream_t st) const;
   void free();
 
  private:
   int64_t a_ = 0, nbuild_ = 0, nT_ = 0;
-  int nout_ = 0, nin_ = 0;
+  int nin_ = 0, row0_ = 0;
+  bool scaled_ = false;
   OzLaunch gemm_;
   DBuf<OzBuild> builds_;        // images of X, then those of T
   DBuf<OzTask> tasks_;
   DBuf<OzS3> s3_;
   DBuf<OzRnd> rnd_;
   DBuf<char> T_;
-  DBuf<double> scale_;          // [nin] of X, [nin] of T
+  DBuf<double> scale_;          // [nin] of X, [nin] of T, of the last run
 };
 
 class OzPlan {

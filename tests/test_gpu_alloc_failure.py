@@ -144,12 +144,12 @@ def test_transforms_run_without_their_images(fail_alloc):
     tr = build_transforms(load_ir(150), 50.0)
     assert 8.0 * (tr.nts - 2) * tr.nw * cr.layout.flat_ao_size > 4e7 < 8.0 * (tr.nts - 2) * tr.nw_b * cr.layout.flat_aux_size
     rng = np.random.default_rng(4)
-    P0 = np.zeros(tr.nts * cr.layout.flat_aux_size, np.complex128).reshape(tr.nts, -1)
-    o = 0
-    for n in cr.layout.aux_sizes[0]:
+    tau = np.asarray(tr.tau_fermi)
+    P0 = np.zeros((tr.nts, cr.layout.flat_aux_size), np.complex128)
+    for n, o in zip(cr.layout.aux_sizes[0], cr.layout.aux_offsets[0]):  # negative definite, one bosonic pole a block
         x = rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))
-        P0[:, o:o + n * n] = -0.02 * (x @ x.conj().T).ravel() * np.exp(-np.abs(np.arange(tr.nts) - 74.5) / 9)[:, None]
-        o += n * n
+        w = rng.uniform(0.5, 2.0)
+        P0[:, o:o + n * n] = (-0.02 * (np.exp(-tau * w) + np.exp(-(tr.beta - tau) * w)))[:, None] * (x @ x.conj().T).ravel()
 
     def run(s):
         s.set_shared_Coulomb(cr.V)
