@@ -392,8 +392,9 @@ __global__ void __launch_bounds__(256) transform_kernel(const TSlab *__restrict_
 //    lower triangle, no pivot search (3 n^3 instructions against 6 n^3 and the search).  A pivot that is not clearly
 //    positive sends the block to the general elimination;
 //  - the general one is Gauss-Jordan with full pivoting (the strategy of Eigen::FullPivLU,
-//    sc_type_block.cpp:55), 6 instructions per element and step; the pivot is the largest
-//    component by its upper 32 bits, found in integers while the elimination writes the elements.
+//    sc_type_block.cpp:55), 6 instructions per element and step; the pivot is the element of
+//    largest modulus to 20 bits, found in integers and FP32 while the elimination writes the elements (the largest
+//    component instead made Dyson's error up to 12% larger).
 // One warp per matrix up to n = 16, a CTA of 128 threads up to 32, of 256 above (NT), elements spread over the threads.
 // Measured, with one general elimination per warp or CTA of 128 and now: W~ s+p+d+4 (aux 9-46) 3.36 and 1.53 ms,
 // hexagonal 8 k (aux 2-30) 3.15 and 0.95; Dyson there (AO 2-30) 0.61 and 0.26; s+p (n up to 12), both solves, 0.17 and 0.075.
@@ -407,11 +408,16 @@ template <int NT> __device__ __forceinline__ void inv_sync() {
     __syncthreads();
 }
 
-// Size of a component pair for the pivot choice: upper word of the larger one; 0 for NaN and for
-// what underflows when squared.
+// Size of an element for the pivot choice: |v|^2 to 20 bits as an ordered integer, from the upper words in FP32 (the
+// FP64 pipe bounds the elimination).  0 for NaN and for what underflows when squared.
 __device__ __forceinline__ unsigned inv_key(double2 v) {
-  const unsigned k = max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu);
-  return k > 0x7ff00000u || k < (unsigned)(1023 - 537) << 20 ? 0u : k;
+  const unsigned x = (unsigned)__double2hiint(v.x) & 0x7fffffffu, y = (unsigned)__double2hiint(v.y) & 0x7fffffffu;
+  const unsigned k = max(x, y), s = min(x, y), e = k >> 20, d = e - (s >> 20);
+  if (k >= 0x7ff00000u) return k == 0x7ff00000u ? 0xffffffffu : 0u;
+  if (k < (unsigned)(1023 - 537) << 20) return 0u;
+  const float fk = __uint_as_float(0x3f800000u | (k & 0xfffffu) << 3);                             // [1, 2)
+  const float fs = d < 16u ? __uint_as_float((127u - d) << 23 | (s & 0xfffffu) << 3) : 0.f;  // on the scale of fk
+  return (e << 21) + ((__float_as_uint(fmaf(fk, fk, fs * fs)) - 0x3f800000u) >> 3);          // fk^2 + fs^2 < 8
 }
 
 // Inverse of the n x n matrix A of NT threads, in place, columns permuted: column m of A is column perm[m] of the
