@@ -216,10 +216,11 @@ def _peaks(dev):
 STAGE_KEYS = ("rotate_G_ms", "p0_ms", "pq_ms", "sigma_ms", "dyson_ms", "transform_ms", "solve_ms")
 PREC_LABEL = {
     "ozaki": ("fp16 x3 slices per operand row (Ozaki scheme, 33 bits) on tcgen05 kind::f16, 8 products, "
-              "exact leading sums in FP32, float-float accumulation; FP64 W~ solve, Dyson, "
-              "transforms, mu search, energies"),
+              "exact leading sums in FP32, float-float accumulation; transforms in fp16 x6 slices (57 bits), "
+              "FP64 W~ solve, Dyson inverses, mu search, energies"),
     "fp64": ("complex128 contractions (the drop-in): fp16 x6 slices per operand row (57 bits) on tcgen05 kind::f16, "
-             "26 products, exact leading sums in FP32; blocks too small for that in FP64 FMAs"),
+             "26 products, exact leading sums in FP32, transforms likewise; blocks too small for that, W~ solve and "
+             "Dyson inverses in FP64 FMAs"),
     "tf32x3": ("tf32x3 (tcgen05 kind::tf32, 2 planes, 3 products, FP32 accumulate within an aux block or "
                "aux-row chunk, FP64 across): FP32-class error, no 1e-7 claim"),
     "bf16x3": ("bf16x3 (tcgen05 kind::f16, 3 BF16 planes, 6 products, FP32 accumulate within an aux block or "

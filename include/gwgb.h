@@ -51,7 +51,7 @@ extern "C" {
 
 /* gwgb_params.flags.  Large enough FP64 contractions, and in every precision large
  * enough tau <-> omega transforms, run on tcgen05 with six FP16 slices per operand:
- * a number is held to 2^-57 of the largest one of its row (an operand's row over at
+ * a number is held to about 2^-57 of the largest one of its row (an operand's row over at
  * most 32 complex summation indices; rows of an intermediate may share theirs),
  * against 2^-53 of itself in an FP64 FMA.  Relative to the products of row scales the
  * results are at least as accurate as FP64 (on crystals of the configurations' sizes
@@ -254,7 +254,8 @@ int gwgb_get_stats(gwgb_handle h, gwgb_stats *out);
 /* Block until all work of the handle is done. */
 int gwgb_synchronize(gwgb_handle h);
 
-/* ---- per-launch profile of the sliced path (GWGB_PREC_OZAKI) ----
+/* ---- per-launch profile of the contractions in slices (GWGB_PREC_OZAKI, and
+ * GWGB_PREC_FP64 where it runs them in slices; no entries otherwise) ----
  * With timing on, every GEMM and reduction launch of the P0 and Sigma stages
  * is bracketed by CUDA events (recorded into the iteration's graph); after a
  * solve or iteration gwgb_get_launch_stats returns one entry per launch, in
@@ -268,7 +269,7 @@ typedef struct gwgb_launch_stat {
   double ms;        /* CUDA-event time of the launch */
   double flops;     /* algorithmic: 8 M N K per complex block GEMM (0 for reductions) */
   double mma_flops; /* kernel 0: FP16 MMA FLOPs issued (128-row tiles, N and K padded to the MMA shape,
-                       8 slice products, real embedding) */
+                       8 slice products with three slices, 26 with six, real embedding) */
   double bytes;     /* kernels 2, 3: bytes read + written */
 } gwgb_launch_stat;
 
