@@ -1134,14 +1134,18 @@ __global__ void __launch_bounds__(1024) oz_row_scale_kernel(const TSlab *__restr
                                                             double *__restrict__ scale) {
   __shared__ int part[32];
   const int i = blockIdx.x;
-  int m = 0;  // upper word of the largest component
+  int m = 0;  // upper word of the largest finite component, at least 1 if there is one but zero
+  auto word = [](double v) {
+    const int h = __double2hiint(v) & 0x7fffffff;
+    return h >= 0x7ff00000 ? 0 : h ? h : __double2loint(v) ? 1 : 0;
+  };
   for (int s = 0; s < nslabs; ++s) {
     const TSlab sl = slabs[s];
     const double2 *x = X + sl.x + (int64_t)(row0 + i) * sl.ldx;
 #pragma unroll 4
     for (int c = threadIdx.x; c < sl.ncols; c += 1024) {
       const double2 v = x[c];
-      m = max(m, max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff));
+      m = max(m, max(word(v.x), word(v.y)));
     }
   }
   m = __reduce_max_sync(0xffffffffu, m);
@@ -1150,9 +1154,9 @@ __global__ void __launch_bounds__(1024) oz_row_scale_kernel(const TSlab *__restr
   if (threadIdx.x < 32) {
     m = __reduce_max_sync(0xffffffffu, part[threadIdx.x]);
     if (threadIdx.x == 0) {
-      const int be = m >> 20, e = be == 0 || be == 0x7ff ? 0 : min(max(be - 1022, -500), 500);
-      scale[i] = __hiloint2double((1023 - e) << 20, 0);
-      scale[nin + i] = __hiloint2double((1023 + e) << 20, 0);
+      const int e = min(max((m >> 20) - 1022, -500), 500);
+      scale[i] = m ? __hiloint2double((1023 - e) << 20, 0) : 1.0;
+      scale[nin + i] = m ? __hiloint2double((1023 + e) << 20, 0) : 0.0;
     }
   }
 }

@@ -136,8 +136,8 @@ void set_oz_kernel_attributes();
 void oz_rings(int ns, int stage, int max_kos, OzArgs *a);
 // multi (stages 1 and 2): the tasks have more than one round of K.
 void launch_oz_gemm(int ns, int stage, bool multi, const OzArgs &a, int nsm, cudaStream_t st);
-// scale[i] = 2^-e and scale[nin + i] = 2^e with 2^(e-1) <= the largest component of row row0 + i over all slabs < 2^e (1
-// where it is zero or not finite).
+// scale[i] = 2^-e and scale[nin + i] = 2^e with 2^(e-1) <= the largest finite component of row row0 + i over all slabs <
+// 2^e, |e| at most 500; 1 and 0 for a row without one, so that its matrix elements do not set the scale of theirs.
 void launch_oz_row_scale(const TSlab *slabs, int nslabs, const double2 *X, int row0, int nin, double *scale,
                          cudaStream_t st);
 void launch_oz_build(int ns, const OzBuild *tasks, int64_t ntasks, const double2 *src, char *dst, cudaStream_t st,

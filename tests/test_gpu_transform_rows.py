@@ -93,3 +93,31 @@ def test_dyson_rows():
         return s.G_tau()
 
     _compare(run, tr.Ttn.astype(CL) @ g)
+
+
+def test_zero_rows_do_not_set_the_scale():
+    """Frequencies at which W~ vanishes, beside others at 10^-25: both handles agree to
+    rounding (120 terms, row by row)."""
+    from mbsymmetry_gb300 import _abi
+    from mbsymmetry_gb300.solver import GWSolver
+    cr, tr = _crystal()
+    L, nts, rng = cr.layout, tr.nts, np.random.default_rng(3)
+    T = np.array(tr.Tnt_BF)
+    T[3::4] = 0.0
+    P0 = np.zeros((nts, L.flat_aux_size), np.complex128)
+    for n, o in zip(L.aux_sizes[0], L.aux_offsets[0]):
+        x = rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))
+        P0[:, o:o + n * n] = -1e-25 * np.cosh(np.linspace(-3, 3, nts))[:, None] * (x @ x.conj().T).reshape(1, n * n)
+    out = []
+    for fma in (False, True):
+        s = GWSolver(L, 1, tr, fp64_fma=fma)
+        _abi.check(s.lib.gwgb_set_transforms(s.h, *(a.ctypes.data for a in (tr.Tnt, tr.Ttn, T, tr.Ttn_FB,
+                                                                            tr.wsample_fermi)), None, None))
+        s.set_shared_Coulomb(cr.V)
+        s.set_P0(P0.ravel())
+        s.compute_Pq_from_P0q()
+        out.append(s.P0_q_t_QP().reshape(nts, -1))
+        s.close()
+    scale = np.abs(tr.Ttn_FB) @ np.abs(T @ P0[1:-1]).max(1)
+    assert np.abs(out[1]).max() > 0
+    assert (np.abs(out[0] - out[1]).max(1) < 120 * 2.0 ** -52 * scale).all()
