@@ -1139,14 +1139,23 @@ __global__ void __launch_bounds__(1024) oz_row_scale_kernel(const TSlab *__restr
     const int h = __double2hiint(v) & 0x7fffffff;
     return h >= 0x7ff00000 ? 0 : h ? h : __double2loint(v) ? 1 : 0;
   };
+  // chunks of 128 columns dealt to the warps over all slabs: small slabs are read side by side (54 of 89 columns: 8 us less
+  // of a Dyson pass's 0.245 ms of transforms than one after the other)
+  const int lane = threadIdx.x & 31;
+  int first = threadIdx.x >> 5;  // this warp's first chunk of the slab, modulo 32
   for (int s = 0; s < nslabs; ++s) {
     const TSlab sl = slabs[s];
     const double2 *x = X + sl.x + (int64_t)(row0 + i) * sl.ldx;
-#pragma unroll 4
-    for (int c = threadIdx.x; c < sl.ncols; c += 1024) {
-      const double2 v = x[c];
-      m = max(m, max(word(v.x), word(v.y)));
+    const int chunks = (sl.ncols + 127) >> 7;
+    for (int k = first & 31; k < chunks; k += 32) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int c = k * 128 + j * 32 + lane;
+        const double2 v = c < sl.ncols ? x[c] : make_double2(0.0, 0.0);
+        m = max(m, max(word(v.x), word(v.y)));
+      }
     }
+    first -= chunks;
   }
   m = __reduce_max_sync(0xffffffffu, m);
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
